@@ -46,6 +46,15 @@ int m_slot(int M) { return M == 1 ? 0 : M == 2 ? 1 : M == 4 ? 2 : 3; }
 
 uint64_t align256(uint64_t x) { return (x + 255) & ~255ull; }
 
+// Subtiles of M words that hold patterns in the last tile a circuit lays
+// out (at least one, so that item counts divide), and its sweep items.
+uint32_t last_subtiles(const BatchCirc& c, int M) {
+  return std::max<uint32_t>(1, (tile_words(c.W, c.tiles - 1) + M - 1) / M);
+}
+unsigned long long sweep_items(const BatchCirc& c, int M) {
+  return ((unsigned long long)(c.tiles - 1) * (kTileWords / M) + last_subtiles(c, M)) * c.n_sweeps;
+}
+
 // Runs f(i) for i in [0, n) on up to hardware_concurrency threads; the
 // first exception a worker raised is rethrown on the calling thread.
 template <class F>
@@ -275,8 +284,9 @@ void BatchExec::layout(const std::vector<BatchJob>& jobs, const std::vector<Clas
       res_off[i] = fo;
       fo += j.F;
       fault_patterns += j.F * j.pats->P;
-      dense_gate_words += p.dense_sweep_gates * kTileWords * tiles;
-      sweep_alg_bytes += p.dense_sweep_bytes * kTileWords * tiles;
+      const uint64_t swept = (uint64_t)(tiles - 1) * kTileWords + (uint64_t)last_subtiles(c, j.M) * j.M;
+      dense_gate_words += p.dense_sweep_gates * swept;
+      sweep_alg_bytes += p.dense_sweep_bytes * swept;
       good_gate_words += (uint64_t)(p.N - p.n_pi) * kTileWords * tiles;
     }
     char* rb = d_res.as<char>();
@@ -330,7 +340,7 @@ void BatchExec::layout(const std::vector<BatchJob>& jobs, const std::vector<Clas
       if (jobs[i].cls != (int)ci || circs[i].n_sweeps == 0) continue;
       if (jobs[i].M != sh.M) throw ArgError{"batch job's words per item differ from its class"};
       const unsigned long long ci_items =
-          (unsigned long long)circs[i].tiles * circs[i].n_sweeps * (kTileWords / sh.M);
+          sweep_items(circs[i], sh.M);
       if (ci_items >= 0xFFFFFFFFull)
         throw LimitError{"a batch circuit has 2^32 or more sweep items; run it on its own"};
       k.circ_ids.push_back((uint32_t)i);
@@ -523,7 +533,9 @@ uint64_t BatchExec::enqueue_sweeps(cudaStream_t s, int only) {
         d.N = c.N;
         d.n_sweeps = c.n_sweeps;
         d.max_gate_level = c.max_gate_level;
-        d.n_items = c.tiles * c.n_sweeps * (kTileWords / (uint32_t)k.shape.M);
+        d.n_items = (uint32_t)sweep_items(c, k.shape.M);
+        d.tiles = c.tiles;
+        d.last_sub = last_subtiles(c, k.shape.M);
         chunk_items += d.n_items;
       }
       params.queue = d_ctl.as<unsigned long long>() + 1 + k.queue_base + j0;
@@ -753,8 +765,6 @@ struct fsimb_batch {
     for (size_t i = 0; i < n; ++i) {
       std::vector<uint32_t> w;
       level_widths(i, w);
-      uint32_t widest = 1;
-      for (uint32_t x : w) widest = std::max(widest, x);
       int M = 0, occ = 1, t = 0;
       default_sweep_shape(
           members[i]->plan, [&](int m) -> const Schedule& { return schedule_at(i, m); },
@@ -764,7 +774,7 @@ struct fsimb_batch {
             CK(sweep_batch_occupancy(m, th, smem, &got));
             return got;
           },
-          std::move(w), widest, smem_optin, smem_per_sm, M, occ, t);
+          std::move(w), (uint32_t)std::min<uint64_t>(members[i]->pats.W, kTileWords), smem_optin, smem_per_sm, M, occ, t);
       if (sweep_vals_bytes(schedule_at(i, M).max_live, M) > smem_share(occ))
         throw LimitError{"batch member " + std::to_string(i) +
                          " has more live values than shared memory holds at 1 word per item"};

@@ -80,12 +80,16 @@ namespace fsimb {
 
 void default_sweep_shape(const Plan& plan, const std::function<const Schedule&(int)>& sched_at,
                          const std::function<int(int, int, size_t)>& occupancy,
-                         std::vector<uint32_t> widths, uint32_t widest, size_t smem_optin,
+                         std::vector<uint32_t> widths, uint32_t words, size_t smem_optin,
                          size_t smem_per_sm, int& M, int& occ, int& threads) {
-  (void)widest;
+  // Words beyond the pattern block are work for nothing: no more words per
+  // item than the block has, rounded up to a power of two.
+  int most = 1;
+  while (most < 8 && (uint32_t)most < words) most *= 2;
   const size_t share1 = sweep_smem_share(smem_optin, smem_per_sm, 1);
   const size_t share2 = sweep_smem_share(smem_optin, smem_per_sm, 2);
   for (int m : {8, 4}) {
+    if (m > most) continue;
     // plan.max_live (no bank constraints) bounds every schedule's slots from below
     if (plan.max_live > kMaxSlots || sweep_vals_bytes(plan.max_live, m) + 64 * 32 > share2) continue;
     const Schedule& sc = sched_at(m);
@@ -101,7 +105,7 @@ void default_sweep_shape(const Plan& plan, const std::function<const Schedule&(i
     threads = t;
     return;
   }
-  M = 8;
+  M = most;
   while (M > 1 && sweep_vals_bytes(plan.max_live, M) > share1) M /= 2;
   while (M > 1 && (sched_at(M).max_live > kMaxSlots || sweep_vals_bytes(sched_at(M).max_live, M) > share1))
     M /= 2;
@@ -111,8 +115,7 @@ void default_sweep_shape(const Plan& plan, const std::function<const Schedule&(i
 
 }  // namespace fsimb
 
-void fsimb_handle::default_shape(std::vector<uint32_t> widths, uint32_t widest, int& M, int& occ,
-                                 int& threads) {
+void fsimb_handle::default_shape(std::vector<uint32_t> widths, int& M, int& occ, int& threads) {
   default_sweep_shape(
       plan, [&](int m) -> const Schedule& { return cached_schedule(m); },
       [&](int m, int t, size_t smem) {
@@ -121,10 +124,11 @@ void fsimb_handle::default_shape(std::vector<uint32_t> widths, uint32_t widest, 
         CK(sweep_occupancy(m, t, smem, &got));
         return got;
       },
-      std::move(widths), widest, smem_optin, smem_per_sm, M, occ, threads);
+      std::move(widths), (uint32_t)std::min<uint64_t>(pats.W, kTileWords), smem_optin, smem_per_sm, M, occ,
+      threads);
 }
 
-void fsimb_handle::tune_shape(cudaStream_t s, const std::vector<uint32_t>& widths, uint32_t widest) {
+void fsimb_handle::tune_shape(cudaStream_t s, const std::vector<uint32_t>& widths) {
   const uint32_t N = plan.N;
   const uint32_t n_sweeps = (uint32_t)plan.sweeps.size();
   for (auto& e : tune_ev)
@@ -159,7 +163,7 @@ void fsimb_handle::tune_shape(cudaStream_t s, const std::vector<uint32_t>& width
   // faster by more than 2% on the sample (the sample favours no shape, but
   // its time carries a few percent of noise).
   int dM = 0, docc = 1, dT = 0;
-  default_shape(widths, widest, dM, docc, dT);
+  default_shape(widths, dM, docc, dT);
   float default_ms = -1;
   struct Cand {
     int M, occ, T;
@@ -209,6 +213,7 @@ void fsimb_handle::tune_shape(cudaStream_t s, const std::vector<uint32_t>& width
     sa.list = d_tune_list.as<uint32_t>();
     sa.wait_ns = kWaitLimitNs;
     sa.n_list = (uint32_t)list.size();
+    sa.n_words = tile_words(pats.W, 0);
     sa.max_gate_level = plan.max_gate_level;
     sa.N = N;
     sa.good = d_good.as<uint64_t>();
@@ -217,7 +222,7 @@ void fsimb_handle::tune_shape(cudaStream_t s, const std::vector<uint32_t>& width
     sa.vals_bytes = vals;
     sa.rec_buf = rec_buf;
     sa.err = d_err.as<int>();
-    const int nb = (int)std::min<uint64_t>((uint64_t)n_sms * got, (uint64_t)sa.n_list * (kTileWords / M));
+    const int nb = (int)std::min<uint64_t>((uint64_t)n_sms * got, (uint64_t)sa.n_list * ((sa.n_words + M - 1) / M));
     // an untimed run of the first candidate warms the GPU up; then the
     // fastest of two timed runs counts
     float ms = 1e30f;
@@ -297,12 +302,9 @@ void fsimb_handle::run(const fsimb_opts* opts) {
   if (W_pad > (1ull << 31) || tiles * (uint64_t)N * kTileWords > (1ull << 40))
     throw LimitError{"pattern block too large"};
 
-  uint32_t widest = 1;
   std::vector<uint32_t> widths;
-  for (uint32_t l = 1; l <= plan.max_gate_level && l < plan.n_levels; ++l) {
+  for (uint32_t l = 1; l <= plan.max_gate_level && l < plan.n_levels; ++l)
     widths.push_back(plan.level_off[l + 1] - plan.level_off[l]);
-    widest = std::max(widest, widths.back());
-  }
   cudaEvent_t e0 = ev(0), e1 = ev(1), e2 = ev(2), e3 = ev(3);
   CK(cudaEventRecord(e0, s));
   if (!plan_uploaded) {
@@ -365,7 +367,7 @@ void fsimb_handle::run(const fsimb_opts* opts) {
       } else if (o.tune && tiles) {
         if (tuned_gen != plan_gen) {
           const auto t0 = std::chrono::steady_clock::now();
-          tune_shape(s, widths, widest);
+          tune_shape(s, widths);
           tune_ms_now =
               std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
         }
@@ -373,7 +375,7 @@ void fsimb_handle::run(const fsimb_opts* opts) {
         occ = tuned_occ;
         threads = tuned_T;
       } else {
-        default_shape(widths, widest, M, occ, threads);
+        default_shape(widths, M, occ, threads);
       }
       const size_t budget = sweep_smem_share(smem_optin, smem_per_sm, occ);
       const bool fixed_M = M != 0;
@@ -407,7 +409,7 @@ void fsimb_handle::run(const fsimb_opts* opts) {
   }
   int blocks = 0, occ_got = 0;
   if (wide) {
-    M = o.words_per_item == 1 ? 1 : 2;
+    M = o.words_per_item == 1 || (!o.words_per_item && W == 1) ? 1 : 2;
     threads = 256;
     if (!eflag_uploaded) {
       std::vector<uint8_t> fl(N, 0);
@@ -480,7 +482,8 @@ void fsimb_handle::run(const fsimb_opts* opts) {
     cudaEvent_t a0 = ev(4 + 3 * t), a1 = ev(5 + 3 * t), a2 = ev(6 + 3 * t);
     CK(cudaEventRecord(a0, s));
     if (n_sw) {
-      const uint32_t subtiles = kTileWords / M;
+      const uint32_t n_words = tile_words(W, t);
+      const uint32_t subtiles = (n_words + M - 1) / M;
       const int nb = (int)std::min<uint64_t>((uint64_t)blocks, (uint64_t)n_sw * subtiles);
       if (wide) {
         SweepWideArgs wa{};
@@ -493,6 +496,7 @@ void fsimb_handle::run(const fsimb_opts* opts) {
         wa.inj = d_inj.as<InjRec>();
         wa.list = sw_list;
         wa.n_list = n_sw;
+        wa.n_words = n_words;
         wa.max_gate_level = plan.max_gate_level;
         wa.N = N;
         wa.good = good_t;
@@ -513,6 +517,7 @@ void fsimb_handle::run(const fsimb_opts* opts) {
         sa.inj = d_inj.as<InjRec>();
         sa.list = sw_list;
         sa.n_list = n_sw;
+        sa.n_words = n_words;
         sa.max_gate_level = plan.max_gate_level;
         sa.N = N;
         sa.good = good_t;
@@ -528,8 +533,8 @@ void fsimb_handle::run(const fsimb_opts* opts) {
       ++launches;
       items += (uint64_t)n_sw * subtiles;
       if (!sw_list) {
-        dense += plan.dense_sweep_gates * kTileWords;
-        alg_bytes += plan.dense_sweep_bytes * kTileWords;
+        dense += plan.dense_sweep_gates * subtiles * M;
+        alg_bytes += plan.dense_sweep_bytes * subtiles * M;
       } else {
         host_sw.resize(n_sw);
         CK(cudaMemcpyAsync(host_sw.data(), sw_list, n_sw * 4, cudaMemcpyDeviceToHost, s));
@@ -537,8 +542,8 @@ void fsimb_handle::run(const fsimb_opts* opts) {
         for (uint32_t si : host_sw) {
           uint32_t L0 = nl.level[plan.sweeps[si].elem] + 1;
           if (L0 <= plan.max_gate_level) {
-            dense += (uint64_t)(plan.eval_prefix[gates_end] - plan.eval_prefix[plan.level_off[L0]]) * kTileWords;
-            alg_bytes += (plan.nfp_prefix[gates_end] - plan.nfp_prefix[plan.level_off[L0]]) * kTileWords;
+            dense += (uint64_t)(plan.eval_prefix[gates_end] - plan.eval_prefix[plan.level_off[L0]]) * subtiles * M;
+            alg_bytes += (plan.nfp_prefix[gates_end] - plan.nfp_prefix[plan.level_off[L0]]) * subtiles * M;
           }
         }
       }
@@ -707,7 +712,6 @@ void fsimb_handle::run(const fsimb_opts* opts) {
   stats.block_threads = (uint32_t)threads;
   stats.blocks = (uint32_t)blocks;
   stats.smem_bytes = (uint32_t)smem;
-  (void)widest;
   stats.device_bytes = device_bytes();
 }
 

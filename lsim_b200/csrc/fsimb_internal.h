@@ -117,6 +117,11 @@ inline size_t sweep_smem_share(size_t smem_optin, size_t smem_per_sm, int occ) {
   return per > static_smem + reserved ? std::min(budget, per - static_smem - reserved) : 0;
 }
 
+// Pattern words of tile t of a block of W words.
+inline uint32_t tile_words(uint64_t W, uint64_t t) {
+  return (uint32_t)std::min<uint64_t>(kTileWords, W > t * kTileWords ? W - t * kTileWords : 0);
+}
+
 // Bytes of a sweep CTA's value slots: max_live slots of M words, 16-byte rounded.
 inline uint32_t sweep_vals_bytes(uint32_t max_live, int M) {
   return (uint32_t)(((size_t)max_live * M * 8 + 15) / 16 * 16);
@@ -153,11 +158,12 @@ struct PinnedBuf {
 // item when the value slots leave room for at least 64 staged records (the
 // CTA size then lowered until two fit), else the largest words per item
 // whose slots fit one CTA per SM, with the width heuristic's CTA size.
-// sched_at(M) returns the schedule at M; occupancy(M, threads, smem) the
-// sweep kernel's CTAs per SM.
+// At most `words` words per item (rounded up to a power of two): the pattern
+// words a tile of the block has.  sched_at(M) returns the schedule at M;
+// occupancy(M, threads, smem) the sweep kernel's CTAs per SM.
 void default_sweep_shape(const Plan& plan, const std::function<const Schedule&(int)>& sched_at,
                          const std::function<int(int, int, size_t)>& occupancy,
-                         std::vector<uint32_t> widths, uint32_t widest, size_t smem_optin,
+                         std::vector<uint32_t> widths, uint32_t words, size_t smem_optin,
                          size_t smem_per_sm, int& M, int& occ, int& threads);
 
 // A fresh value for fsimb_handle::gen: every change of a handle's circuit,
@@ -329,11 +335,11 @@ struct fsimb_handle {
   // Makes `sched` the schedule at M (re-uploaded before the next sweep).
   void use_schedule(int M);
   // default_sweep_shape for this circuit and the plain sweep kernel.
-  void default_shape(std::vector<uint32_t> widths, uint32_t widest, int& M, int& occ, int& threads);
+  void default_shape(std::vector<uint32_t> widths, int& M, int& occ, int& threads);
   // Times candidate shapes on a strided sample of tile 0's sweeps and keeps
   // the fastest in tuned_M / tuned_T / tuned_occ.  Needs the plan and the
   // patterns on the device.
-  void tune_shape(cudaStream_t s, const std::vector<uint32_t>& widths, uint32_t widest);
+  void tune_shape(cudaStream_t s, const std::vector<uint32_t>& widths);
 };
 
 // Wraps a C ABI body: exceptions become status codes and (h)->err.

@@ -600,7 +600,9 @@ __global__ void __maxnreg__(M >= 8 ? 120 : (M >= 4 ? 72 : (M >= 2 ? 56 : 64))) k
                     (a.wait_test && blockIdx.x == 0) ? 1u : 0u);
   const SweepView v{a.blob, a.lvl, a.level, a.li_off, a.li, a.fi_off, a.fi_idx, a.type, a.good,
                     a.max_gate_level};
-  constexpr uint32_t subtiles = kTileWords / M;
+  // Subtiles that hold pattern words: the last tile of a block is rarely full
+  // (16 words of 32 for 1,000 patterns), and the tracing masks the others.
+  const uint32_t subtiles = (a.n_words + M - 1) / M;
   const uint32_t n_items = a.n_list * subtiles;
   for (;;) {
     if (threadIdx.x == 0) s_item = atomicAdd(a.queue, 1);
@@ -646,10 +648,12 @@ __global__ void __maxnreg__(M >= 8 ? 96 : (M >= 4 ? 72 : (M >= 2 ? 56 : 64)))
       const uint32_t item = s_item;
       __syncthreads();  // s_item is rewritten only after every thread read it
       if (item == 0xFFFFFFFFu) break;
-      const uint32_t tile = item / per_tile;
+      // The last tile has items only for the subtiles that hold pattern words.
+      const uint32_t tile = min(item / per_tile, c.tiles - 1);
       const uint32_t rem = item - tile * per_tile;
-      const uint32_t si = rem / subtiles;
-      const uint32_t w0 = (rem % subtiles) * M;
+      const uint32_t sub = tile == c.tiles - 1 ? c.last_sub : subtiles;
+      const uint32_t si = rem / sub;
+      const uint32_t w0 = (rem % sub) * M;
       const SweepView v{c.blob, c.lvl, c.level, c.li_off, c.li, c.fi_off, c.fi_idx, c.type,
                         c.good + (uint64_t)tile * c.N * 32, c.max_gate_level};
       if (!sweep_item<M>(k, v, c.inj[si], w0, c.out + ((uint64_t)tile * c.n_sweeps + si) * 32)) {
@@ -674,7 +678,9 @@ __global__ void __launch_bounds__(256) k_sweep_wide(SweepWideArgs a) {
   uint64_t* gv = a.gvals + (size_t)blockIdx.x * a.N * M;
   const uint32_t tid = threadIdx.x, nth = blockDim.x;
   const uint32_t m = tid % M, step = nth / M;
-  constexpr uint32_t subtiles = kTileWords / M;
+  // Subtiles that hold pattern words: the last tile of a block is rarely full
+  // (16 words of 32 for 1,000 patterns), and the tracing masks the others.
+  const uint32_t subtiles = (a.n_words + M - 1) / M;
   const uint32_t n_items = a.n_list * subtiles;
   for (;;) {
     if (tid == 0) s_item = atomicAdd(a.queue, 1);

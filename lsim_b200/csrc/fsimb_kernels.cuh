@@ -33,6 +33,7 @@ struct SweepArgs {
   const InjRec* inj;
   const uint32_t* list;    // sweep indices to run (nullptr: 0..n_list-1)
   uint32_t n_list;
+  uint32_t n_words;        // pattern words of this tile (1..32): the others are not swept
   uint32_t max_gate_level;
   uint32_t N;
   const uint64_t* good;    // this tile: [N][32]
@@ -56,6 +57,7 @@ struct SweepWideArgs {
   const InjRec* inj;
   const uint32_t* list;      // sweep indices to run (nullptr: 0..n_list-1)
   uint32_t n_list;
+  uint32_t n_words;          // pattern words of this tile (1..32)
   uint32_t max_gate_level;
   uint32_t N;
   const uint64_t* good;      // this tile: [N][32]
@@ -165,10 +167,12 @@ struct SweepCirc {
   const uint64_t* good;  // [tiles][N][32]
   uint64_t* out;         // [tiles][n_sweeps][32]
   uint32_t N, n_sweeps, max_gate_level;
-  uint32_t n_items;      // tiles * n_sweeps * (32 / M): (tile, sweep, subtile), tile-major
+  uint32_t n_items;      // (tile, sweep, subtile), tile-major: n_sweeps * (32 / M) per tile,
+                         // n_sweeps * last_sub for the last one
+  uint32_t tiles, last_sub;
 };
 
-constexpr int kSweepCircsPerLaunch = 300;
+constexpr int kSweepCircsPerLaunch = 280;
 
 struct BatchSweepParams {
   SweepCirc c[kSweepCircsPerLaunch];

@@ -265,12 +265,9 @@ struct fsimb_server {
     build_circuit_plan(nl, c->cp);
     // the default shape, for the batch kernel
     std::vector<uint32_t> widths;
-    uint32_t widest = 1;
     const Plan& B = c->cp.base;
-    for (uint32_t l = 1; l <= B.max_gate_level && l < B.n_levels; ++l) {
+    for (uint32_t l = 1; l <= B.max_gate_level && l < B.n_levels; ++l)
       widths.push_back(B.level_off[l + 1] - B.level_off[l]);
-      widest = std::max(widest, widths.back());
-    }
     Schedule sc[4];
     bool has[4] = {false, false, false, false};
     auto sched_at = [&](int m) -> const Schedule& {
@@ -295,7 +292,7 @@ struct fsimb_server {
             CK(sweep_batch_occupancy(m, th, smem, &got));
             return got;
           },
-          widths, widest, smem_optin, smem_per_sm, M, occ, T);
+          widths, kTileWords, smem_optin, smem_per_sm, M, occ, T);
     }
     const Schedule& chosen = sched_at(M);
     if (chosen.max_live > kMaxSlots ||
@@ -427,8 +424,7 @@ struct fsimb_server {
         if (j.good_resident)
           j.dev.good = c.d_good.as<uint64_t>() + (r->row0 / kTileWords) * (uint64_t)c.nl.N * kTileWords;
         r->bytes = batch_job_bytes(j, false);
-        r->work = (double)r->plan.dense_sweep_gates * kTileWords *
-                  (double)std::max<uint64_t>(1, (r->pats.W + kTileWords - 1) / kTileWords);
+        r->work = (double)r->plan.dense_sweep_gates * (double)std::max<uint64_t>(1, r->pats.W);
         WaveBytes need = overhead();
         add(need, r->bytes);
         if (!slots.empty() && !fits(need, slots[0]->cap))

@@ -59,8 +59,8 @@ typedef struct {
   uint32_t words_per_item;   /* sweep words per work item: 0 auto, or 1,2,4,8
                                 (1 or 2 for the wide-circuit sweep) */
   uint32_t block_threads;    /* sweep CTA size: 0 auto, or a multiple of 32 up to 1024 */
-  uint32_t ctas_per_sm;      /* sweep CTAs sharing an SM: 0 auto, or 1..8; sizes the
-                                record buffer so that many fit */
+  uint32_t ctas_per_sm;      /* sweep CTAs sharing an SM: 0 auto, or 1..8; the live
+                                values must leave room for that many */
   uint32_t tune;             /* 1, with the three above 0: on the first run of a circuit and
                                 fault list, time candidate sweep shapes on a strided sample
                                 of the first tile's sweeps and keep the fastest */
@@ -71,7 +71,7 @@ typedef struct {
                                 in global memory; 1 shared memory (FSIMB_ERR_LIMIT when
                                 they do not fit); 2 global memory */
   uint32_t wait_test;        /* test hook, normally 0.  1: one sweep CTA waits on a barrier
-                                that no copy completes; the wait gives up after 20 ms and
+                                that nothing completes; the wait gives up after 20 ms and
                                 the run fails with FSIMB_ERR_CUDA, results discarded, the
                                 handle still usable.  Shared-memory sweep only. */
   uint32_t pad;
@@ -262,7 +262,8 @@ typedef struct {
   uint32_t words_per_item;   /* 0 auto, or 1, 2, 4, 8 (members whose live values
                                 do not fit take the next smaller value) */
   uint32_t block_threads;    /* 0 auto, or a multiple of 32 up to 1024 */
-  uint32_t ctas_per_sm;      /* 0 auto (1), or 1..4: sizes the sweep CTA's record buffer */
+  uint32_t ctas_per_sm;      /* 0 auto (1), or 1..4: the live values must leave room for
+                                that many sweep CTAs on an SM */
   uint32_t tune;             /* 1, with the three above 0: time candidate shapes on a
                                 sample of the batch (the first tile of a spread of its
                                 circuits) the first time a membership runs; the winner

@@ -107,10 +107,9 @@ uint64_t batch_job_static_bytes(const BatchJob& j) {
     t(nl.type.size());
     t(nl.fi_off.size() * 4);
     t(nl.fi_idx.size() * 4);
-    t(nl.level.size() * 4);
-    t(sc.lvl.size() * sizeof(LevelDesc));
-    t(sc.blob.size() * 8);
-    t(sc.li_off.size() * 4);
+    t(p.net.lev_up.size() * 4);
+    t(sc.lvl.size() * 16);
+    t(sc.blob.size() * 4);
     t(sc.li.size() * 4);
   }
   t(p.sweeps.size() * sizeof(InjRec));
@@ -198,17 +197,15 @@ uint64_t BatchExec::upload_static(const std::vector<BatchJob>& jobs, cudaStream_
       c.level = j.dev.level;
       c.lvl = j.dev.lvl;
       c.blob = j.dev.blob;
-      c.li_off = j.dev.li_off;
       c.li = j.dev.li;
     } else {
       const Schedule& sc = *j.sched;
       c.type = (const uint8_t*)put(nl.type.data(), nl.type.size());
       c.fi_off = (const uint32_t*)put(nl.fi_off.data(), nl.fi_off.size() * 4);
       c.fi_idx = (const uint32_t*)put(nl.fi_idx.data(), nl.fi_idx.size() * 4);
-      c.level = (const uint32_t*)put(nl.level.data(), nl.level.size() * 4);
-      c.lvl = (const uint4*)put(sc.lvl.data(), sc.lvl.size() * sizeof(LevelDesc));
-      c.blob = (const uint4*)put(sc.blob.data(), sc.blob.size() * 8);
-      c.li_off = (const uint32_t*)put(sc.li_off.data(), sc.li_off.size() * 4);
+      c.level = (const uint32_t*)put(p.net.lev_up.data(), p.net.lev_up.size() * 4);
+      c.lvl = (const uint4*)put(sc.lvl.data(), sc.lvl.size() * 16);
+      c.blob = (const uint4*)put(sc.blob.data(), sc.blob.size() * 4);
       c.li = (const uint32_t*)put(sc.li.data(), sc.li.size() * 4);
     }
     c.inj = (const InjRec*)put(p.sweeps.data(), p.sweeps.size() * sizeof(InjRec));
@@ -277,6 +274,10 @@ void BatchExec::layout(const std::vector<BatchJob>& jobs, const std::vector<Clas
       c.max_gate_level = p.max_gate_level;
       c.n_levels = p.n_levels;
       c.n_slots = (uint32_t)(p.members.size() + p.roots.size());
+      c.stream_recs = j.sched->stream_recs;
+      c.fix0 = j.sched->fix0;
+      c.inj_slot = j.sched->max_live - 1;
+      c.split = j.sched->split;
       c.good = j.good_resident ? j.dev.good : (uint64_t*)take((uint64_t)tiles * p.N * kTileWords * 8);
       c.out = (uint64_t*)take((uint64_t)tiles * std::max<uint32_t>(c.n_sweeps, 1) * kTileWords * 8);
       c.sens = first_tile_only ? nullptr
@@ -338,7 +339,8 @@ void BatchExec::layout(const std::vector<BatchJob>& jobs, const std::vector<Clas
     unsigned long long items = 0;
     for (size_t i = 0; i < n; ++i) {
       if (jobs[i].cls != (int)ci || circs[i].n_sweeps == 0) continue;
-      if (jobs[i].M != sh.M) throw ArgError{"batch job's words per item differ from its class"};
+      if (jobs[i].M != sh.M || (int)jobs[i].sched->T != sh.threads)
+        throw ArgError{"a batch job's words per item or CTA size differ from its class"};
       const unsigned long long ci_items =
           sweep_items(circs[i], sh.M);
       if (ci_items >= 0xFFFFFFFFull)
@@ -347,12 +349,13 @@ void BatchExec::layout(const std::vector<BatchJob>& jobs, const std::vector<Clas
       items += ci_items;
       k.work += (double)jobs[i].plan->dense_sweep_gates * circs[i].tiles;
       max_live = std::max(max_live, jobs[i].sched->max_live);
-      widest = std::max(widest, jobs[i].sched->max_block16);
+      const std::vector<uint32_t>& ro = jobs[i].sched->rec_off;
+      for (size_t l = 0; l + 1 < ro.size(); ++l) widest = std::max(widest, ro[l + 1] - ro[l]);
     }
     if (k.circ_ids.empty()) continue;
     k.n_items = items;
-    k.max_live = max_live;
     k.widest = widest;
+    k.max_live = max_live;
     k.queue_base = n_counters;
     n_counters += (uint32_t)k.circ_ids.size();
     size_class(k, sh);
@@ -389,7 +392,7 @@ void BatchExec::layout(const std::vector<BatchJob>& jobs, const std::vector<Clas
     CK(cudaMemcpyAsync(d_desc.p, h_desc.p, at, cudaMemcpyHostToDevice, s));
     desc_bytes = at;
   }
-  // Control words: one work counter per class and the error flag.
+  // Control words: one work counter per swept circuit.
   ctl_bytes = align256(((uint64_t)n_counters + 1) * 8);
   d_ctl.ensure(wb_need.ctl);
   h_res.ensure(wb_need.res);
@@ -400,32 +403,20 @@ void BatchExec::layout(const std::vector<BatchJob>& jobs, const std::vector<Clas
 
 void BatchExec::size_class(SweepClass& k, const ClassShape& sh) {
   k.shape = sh;
-  const size_t share = sweep_smem_share(smem_optin, smem_per_sm, sh.occ);
-  k.vals_bytes = sweep_vals_bytes(k.max_live, sh.M);
-  if (k.vals_bytes > share)
+  const size_t share = sweep_smem_share(smem_optin, smem_per_sm, 1);
+  const uint32_t vals = sweep_vals_bytes(k.max_live, sh.M);
+  if (vals > share)
     throw LimitError{"a batch circuit needs " + std::to_string(k.max_live) + " live values at " +
-                     std::to_string(sh.M) + " word(s) per item; " + std::to_string(sh.occ) +
-                     " CTA(s) per SM leave room for " + std::to_string(share / (8 * sh.M))};
-  k.rec_buf = (uint32_t)std::min<size_t>(k.widest, (share - k.vals_bytes) / 32);
-  k.smem = std::max<size_t>(16, k.vals_bytes + (size_t)k.rec_buf * 32);
-  k.threads = std::min<int>(sh.threads, (int)sweep_max_threads(sh.M));
+                     std::to_string(sh.M) + " word(s) per item; shared memory holds " +
+                     std::to_string(share / (8 * sh.M))};
+  k.smem = std::max<size_t>(16, vals);
   size_t& attr = smem_attr[m_slot(sh.M)];
   attr = std::max(attr, k.smem);
   CK(sweep_batch_set_smem(sh.M, attr));
-  int occ = 0;
-  CK(sweep_batch_occupancy(sh.M, k.threads, k.smem, &occ));
-  if (occ < 1) throw LimitError{"batch sweep kernel does not fit on an SM with this shape"};
-  k.blocks = (int)std::min<unsigned long long>((unsigned long long)n_sms * occ, k.n_items);
-}
-
-void BatchExec::relaunch_shapes(const std::vector<ClassShape>& shapes) {
-  // Same circuits and classes (same words per item); new CTA size / CTAs per SM.
-  for (SweepClass& k : classes) {
-    const ClassShape& sh = shapes[k.id];
-    if (sh.M != k.shape.M) throw ArgError{"a class's words per item cannot change without a new layout"};
-    size_class(k, sh);
-  }
-  invalidate_graph();
+  k.occ = 0;
+  CK(sweep_batch_occupancy(sh.M, sh.threads, k.smem, &k.occ));
+  if (k.occ < 1) throw LimitError{"batch sweep kernel does not fit on an SM with this shape"};
+  k.blocks = (int)std::min<unsigned long long>((unsigned long long)n_sms * k.occ, k.n_items);
 }
 
 void BatchExec::apply_attributes() {
@@ -522,7 +513,10 @@ uint64_t BatchExec::enqueue_sweeps(cudaStream_t s, int only) {
         d.blob = c.blob;
         d.level = c.level;
         d.lvl = c.lvl;
-        d.li_off = c.li_off;
+        d.stream_recs = c.stream_recs;
+        d.fix0 = c.fix0;
+        d.inj_slot = c.inj_slot;
+        d.split = c.split;
         d.li = c.li;
         d.fi_off = c.fi_off;
         d.fi_idx = c.fi_idx;
@@ -538,13 +532,9 @@ uint64_t BatchExec::enqueue_sweeps(cudaStream_t s, int only) {
         d.last_sub = last_subtiles(c, k.shape.M);
         chunk_items += d.n_items;
       }
-      params.queue = d_ctl.as<unsigned long long>() + 1 + k.queue_base + j0;
-      params.err = d_ctl.as<int>();
-      params.wait_ns = kWaitLimitNs;
-      params.vals_bytes = k.vals_bytes;
-      params.rec_buf = k.rec_buf;
+      params.queue = d_ctl.as<unsigned long long>() + k.queue_base + j0;
       const int blocks = (int)std::min<unsigned long long>((unsigned long long)k.blocks, chunk_items);
-      CK(launch_sweep_batch(k.shape.M, k.threads, std::max(blocks, 1), k.smem, params, s));
+      CK(launch_sweep_batch(k.shape.M, k.shape.threads, std::max(blocks, 1), k.smem, params, s));
       ++launches;
     }
   }
@@ -576,7 +566,7 @@ uint64_t BatchExec::run_graph(cudaStream_t capture_stream, cudaStream_t s) {
   return graph_launches;
 }
 
-void BatchExec::fetch(cudaStream_t s, int* kerr) {
+void BatchExec::fetch(cudaStream_t s) {
   const uint64_t Fp = std::max<uint64_t>(F_total, 1);
   char* hb = h_res.as<char>();
   if (F_total) {
@@ -584,9 +574,7 @@ void BatchExec::fetch(cudaStream_t s, int* kerr) {
     CK(cudaMemcpyAsync(hb + Fp * 8, d_first, F_total * 8, cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(hb + Fp * 16, d_lastflag, F_total, cudaMemcpyDeviceToHost, s));
   }
-  CK(cudaMemcpyAsync(hb + Fp * 17, d_ctl.p, sizeof(int), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
-  std::memcpy(kerr, hb + Fp * 17, sizeof(int));
 }
 
 void BatchExec::results(size_t i, const BatchJob& j, fsimb_fault_result* out) const {
@@ -628,7 +616,7 @@ struct MemberCache {
 bool same_shapes(const std::vector<ClassShape>& a, const std::vector<ClassShape>& b) {
   if (a.size() != b.size()) return false;
   for (size_t i = 0; i < a.size(); ++i)
-    if (a[i].M != b[i].M || a[i].threads != b[i].threads || a[i].occ != b[i].occ) return false;
+    if (a[i].M != b[i].M || a[i].threads != b[i].threads) return false;
   return true;
 }
 
@@ -638,7 +626,6 @@ bool same_shapes(const std::vector<ClassShape>& a, const std::vector<ClassShape>
 struct BatchAssign {
   std::vector<int> M, cls;
   std::vector<ClassShape> shapes;
-  std::vector<uint32_t> max_live;  // per class: the largest member schedule's slots
 };
 
 struct fsimb_batch {
@@ -713,12 +700,17 @@ struct fsimb_batch {
         h->plan_valid = true;
         h->plan_uploaded = false;
         h->sched_M = 0;
-        h->sched_uploaded = false;
       }
     });
   }
 
   size_t smem_share(int occ) const { return sweep_smem_share(smem_optin, smem_per_sm, occ); }
+
+  // The documented limit: every gate's live value at one word per item.
+  bool gates_fit(size_t i, size_t share) const {
+    const Plan& p = members[i]->plan;
+    return p.max_live <= kMaxSlots && sweep_vals_bytes(p.max_live, 1) <= share;
+  }
 
   // Schedules for every member at words per item M or the largest smaller
   // value whose slots fit `share`; returns that value per member.
@@ -726,6 +718,7 @@ struct fsimb_batch {
     std::vector<int> got(members.size(), 0);
     parallel_for(members.size(), [&](size_t i) {
       for (int m = M; m >= 1; m /= 2) {
+        if (!gates_fit(i, share)) return;
         const Schedule& sc = schedule_at(i, m);
         if (sc.max_live <= kMaxSlots && sweep_vals_bytes(sc.max_live, m) <= share) {
           got[i] = m;
@@ -740,65 +733,42 @@ struct fsimb_batch {
     return got;
   }
 
-  void level_widths(size_t i, std::vector<uint32_t>& widths) const {
-    const Plan& p = members[i]->plan;
-    for (uint32_t l = 1; l <= p.max_gate_level && l < p.n_levels; ++l)
-      widths.push_back(p.level_off[l + 1] - p.level_off[l]);
-  }
-
   // Automatic classes: each member at the default shape the plain path would
-  // give it alone (default_sweep_shape, with the batch kernel's occupancy),
-  // and members of the same shape share a class.  A class's shared memory is
-  // capped at the share of its CTAs per SM, so no member runs at a lower
-  // occupancy than alone.
+  // give it alone (default_sweep_shape), and members of the same shape share
+  // a class.
   BatchAssign auto_assign() {
     BatchAssign a;
     const size_t n = members.size();
     a.M.resize(n);
     std::vector<ClassShape> shape(n);
     std::vector<long long> key(n);
-    const size_t share2 = smem_share(2);
-    parallel_for(n, [&](size_t i) {  // the schedules the default shape looks at first
-      for (int m : {8, 4})
-        if (sweep_vals_bytes(members[i]->plan.max_live, m) <= share2) schedule_at(i, m);
-    });
-    for (size_t i = 0; i < n; ++i) {
-      std::vector<uint32_t> w;
-      level_widths(i, w);
-      int M = 0, occ = 1, t = 0;
-      default_sweep_shape(
-          members[i]->plan, [&](int m) -> const Schedule& { return schedule_at(i, m); },
-          [&](int m, int th, size_t smem) {
-            CK(sweep_batch_set_smem(m, smem));
-            int got = 0;
-            CK(sweep_batch_occupancy(m, th, smem, &got));
-            return got;
-          },
-          std::move(w), (uint32_t)std::min<uint64_t>(members[i]->pats.W, kTileWords), smem_optin, smem_per_sm, M, occ, t);
-      if (sweep_vals_bytes(schedule_at(i, M).max_live, M) > smem_share(occ))
+    parallel_for(n, [&](size_t i) {
+      if (!gates_fit(i, smem_share(1)))
         throw LimitError{"batch member " + std::to_string(i) +
                          " has more live values than shared memory holds at 1 word per item"};
+      int M = 0, t = 0;
+      default_sweep_shape(
+          members[i]->plan, [&](int m) -> const Schedule& { return schedule_at(i, m); },
+          (uint32_t)std::min<uint64_t>(members[i]->pats.W, kTileWords), smem_optin, smem_per_sm, M, t);
       a.M[i] = M;
-      shape[i] = ClassShape{M, t, occ};
-      key[i] = ((long long)m_slot(M) * 4096 + t) * 32 + occ;
-    }
+      shape[i] = ClassShape{M, t};
+      key[i] = (long long)m_slot(M) * 4096 + t;
+    });
     std::vector<long long> keys(key);
     std::sort(keys.begin(), keys.end());
     keys.erase(std::unique(keys.begin(), keys.end()), keys.end());
     a.cls.resize(n);
     a.shapes.resize(keys.size());
-    a.max_live.assign(keys.size(), 0);
     for (size_t i = 0; i < n; ++i) {
       const int c = (int)(std::lower_bound(keys.begin(), keys.end(), key[i]) - keys.begin());
       a.cls[i] = c;
       a.shapes[c] = shape[i];
-      a.max_live[c] = std::max(a.max_live[c], schedule_at(i, a.M[i]).max_live);
     }
     return a;
   }
 
   // The member's schedule at M words per item (built once per plan).
-  const Schedule& schedule_at(size_t i, int m) {
+  Schedule& schedule_at(size_t i, int m) {
     MemberCache& c = cache[i];
     const int sl = m_slot(m);
     if (!c.has[sl]) {
@@ -809,29 +779,28 @@ struct fsimb_batch {
   }
 
   // Explicit shape: every member at words_per_item (or the largest smaller
-  // value that fits), one class per words-per-item value.
+  // value that fits), one class per words-per-item value; without a CTA size
+  // the one its largest member would take.
   BatchAssign fixed_assign(int M, int threads, int occ) {
     BatchAssign a;
     a.M = schedules(M ? M : 8, smem_share(occ));
     a.cls.resize(members.size());
     for (int m : {8, 4, 2, 1}) {
-      std::vector<uint32_t> w;
-      bool any = false;
+      uint32_t t = 0;
       for (size_t i = 0; i < members.size(); ++i)
         if (a.M[i] == m) {
           a.cls[i] = (int)a.shapes.size();
-          level_widths(i, w);
-          any = true;
+          t = std::max(t, pick_sweep_threads(schedule_at(i, m), m));
         }
-      if (!any) continue;
-      a.shapes.push_back(ClassShape{m, threads ? threads : (int)pick_sweep_threads(w, m), occ});
+      if (!t) continue;
+      a.shapes.push_back(ClassShape{m, (int)std::min<uint32_t>(threads ? threads : t, sweep_max_threads(m))});
     }
     return a;
   }
 
   std::vector<BatchJob> jobs_for(const std::vector<size_t>& idx, const BatchAssign& a) {
     std::vector<BatchJob> js(idx.size());
-    for (size_t k = 0; k < idx.size(); ++k) {
+    parallel_for(idx.size(), [&](size_t k) {
       const size_t i = idx[k];
       fsimb_handle* h = members[i];
       BatchJob& j = js[k];
@@ -841,8 +810,10 @@ struct fsimb_batch {
       j.F = h->faults.size();
       j.M = a.M[i];
       j.cls = a.cls[i];
-      j.sched = &cache[i].sched[m_slot(a.M[i])];
-    }
+      Schedule& sc = schedule_at(i, a.M[i]);
+      pack_schedule(sc, (uint32_t)a.shapes[a.cls[i]].threads);
+      j.sched = &sc;
+    });
     return js;
   }
 
@@ -859,9 +830,6 @@ struct fsimb_batch {
       CK(cudaEventSynchronize(e1));
       float x = 0;
       CK(cudaEventElapsedTime(&x, e0, e1));
-      int kerr = 0;
-      CK(cudaMemcpy(&kerr, tx.d_ctl.p, sizeof(int), cudaMemcpyDeviceToHost));
-      if (kerr) throw CudaError{"a sweep kernel reached its wait limit during tuning"};
       if (rep >= 0) ms = std::min(ms, x);
     }
     return ms;
@@ -908,38 +876,36 @@ struct fsimb_batch {
       const ClassShape def = a.shapes[a.cls[i]];
       const size_t share1 = smem_share(1);
       auto fits_M = [&](int M) {
-        if (sweep_vals_bytes(P.max_live, M) > share1) return false;
+        if (sweep_vals_bytes(P.net_live, M) > share1) return false;
         const Schedule& sc = schedule_at(i, M);
         return sc.max_live <= kMaxSlots && sweep_vals_bytes(sc.max_live, M) <= share1;
       };
-      // A one-circuit layout of `plan` at M, with its first tile's good machine.
-      auto lay = [&](BatchExec& tx, const Plan& plan, int M) {
+      // Times shape sh on `plan`: a one-circuit layout with its first
+      // tile's good machine.  Negative if the shape does not run.
+      BatchExec tx;
+      tx.n_sms = n_sms;
+      tx.smem_optin = smem_optin;
+      tx.smem_per_sm = smem_per_sm;
+      auto time_shape = [&](const Plan& plan, const ClassShape& sh, int runs) {
+        Schedule& sc = schedule_at(i, sh.M);
+        pack_schedule(sc, (uint32_t)sh.threads);
         BatchJob j;
         j.nl = &members[i]->nl;
         j.plan = &plan;
-        j.sched = &schedule_at(i, M);
+        j.sched = &sc;
         j.pats = &members[i]->pats;
         j.F = members[i]->faults.size();
-        j.M = M;
+        j.M = sh.M;
         j.cls = 0;
-        tx.n_sms = n_sms;
-        tx.smem_optin = smem_optin;
-        tx.smem_per_sm = smem_per_sm;
-        tx.layout({j}, {ClassShape{M, 256, 1}}, true, s);
-        tx.enqueue(s, true, false, nullptr);
-      };
-      // Sizes class 0 of tx at sh; false if the shape does not run as asked.
-      auto usable = [&](BatchExec& tx, const ClassShape& sh) {
-        if (sweep_vals_bytes(schedule_at(i, sh.M).max_live, sh.M) > smem_share(sh.occ)) return false;
-        SweepClass& kc = tx.classes[0];
         try {
-          tx.size_class(kc, sh);
+          tx.layout({j}, {sh}, true, s);
         } catch (const LimitError&) {
-          return false;
+          return -1.0f;
         }
-        if (sh.occ > 1 && kc.rec_buf < std::min<uint32_t>(kc.widest, 64)) return false;
-        // fewer CTAs per SM than asked: the same as a smaller shape
-        return kc.blocks >= (int)std::min<unsigned long long>((unsigned long long)n_sms * sh.occ, kc.n_items);
+        tx.enqueue(s, true, false, nullptr);
+        const float ms = time_class0(tx, warm, s, runs);
+        warm = false;
+        return ms;
       };
       // Stage 1: every candidate once on the coarse sample.
       struct Timed {
@@ -949,16 +915,11 @@ struct fsimb_batch {
       std::vector<Timed> t1;
       for (int M : {8, 4, 2, 1}) {
         if (!fits_M(M)) continue;
-        BatchExec tx;
-        lay(tx, coarse, M);
-        for (int occ : {1, 2, 3, 4})
-          for (int T : {256, 384, 512, 768, 1024}) {
-            const ClassShape sh{M, T, occ};
-            if (T > (int)sweep_max_threads(M) || T * occ > 2048 || !usable(tx, sh)) continue;
-            t1.push_back(Timed{time_class0(tx, warm, s, 1), sh});
-            warm = false;
-          }
-        tx.release();
+        for (int T : {32, 64, 128, 256, 384, 512, 768, 1024}) {
+          if (T > (int)sweep_max_threads(M)) continue;
+          const float ms = time_shape(coarse, ClassShape{M, T}, 1);
+          if (ms >= 0) t1.push_back(Timed{ms, ClassShape{M, T}});
+        }
       }
       std::sort(t1.begin(), t1.end(), [](const Timed& x, const Timed& y) { return x.ms < y.ms; });
       // Stage 2: the default and the three fastest, twice each on the fine
@@ -966,30 +927,22 @@ struct fsimb_batch {
       std::vector<ClassShape> fin{def};
       for (const Timed& t : t1) {
         if (fin.size() >= 4) break;
-        if (!(t.sh.M == def.M && t.sh.occ == def.occ && t.sh.threads == def.threads)) fin.push_back(t.sh);
+        if (!(t.sh.M == def.M && t.sh.threads == def.threads)) fin.push_back(t.sh);
       }
       ClassShape best = def;
       float best_ms = 1e30f;
       bool best_is_default = false;
-      for (int M : {8, 4, 2, 1}) {
-        bool any = false;
-        for (const ClassShape& sh : fin) any |= sh.M == M;
-        if (!any || !fits_M(M)) continue;
-        BatchExec tx;
-        lay(tx, fine, M);
-        for (const ClassShape& sh : fin) {
-          if (sh.M != M || !usable(tx, sh)) continue;
-          const float ms = time_class0(tx, warm, s, 2);
-          warm = false;
-          const bool is_default = sh.M == def.M && sh.occ == def.occ && sh.threads == def.threads;
-          if (is_default || ms < (best_is_default ? 0.98f : 1.0f) * best_ms) {
-            best_ms = ms;
-            best = sh;
-            best_is_default = is_default;
-          }
+      for (const ClassShape& sh : fin) {
+        const float ms = time_shape(fine, sh, 2);
+        if (ms < 0) continue;
+        const bool is_default = sh.M == def.M && sh.threads == def.threads;
+        if (is_default || ms < (best_is_default ? 0.98f : 1.0f) * best_ms) {
+          best_ms = ms;
+          best = sh;
+          best_is_default = is_default;
         }
-        tx.release();
       }
+      tx.release();
       chosen[d] = best;
     }
 
@@ -1017,29 +970,29 @@ struct fsimb_batch {
       b.shapes.push_back(chosen[d]);
       fixed.push_back(1);
     }
-    b.max_live.assign(b.shapes.size(), 0);
-    for (size_t i = 0; i < n; ++i)
-      b.max_live[b.cls[i]] = std::max(b.max_live[b.cls[i]], schedule_at(i, b.M[i]).max_live);
     a = std::move(b);
     return fixed;
   }
 
-  // Times candidate shapes per class (CTAs per SM x CTA size, words per item
-  // fixed) on the first tile of a spread of the class's circuits (about 3%
-  // of its sweep work); the default shape stays unless beaten by 2%.
+  // Times CTA sizes per class (words per item fixed) on the first tile of a
+  // spread of the class's circuits (about 3% of its sweep work); the default
+  // shape stays unless beaten by 2%.
   void autotune(BatchAssign& a, cudaStream_t s, const std::vector<char>& fixed) {
     const size_t n = members.size();
-    const size_t n_cls = a.shapes.size();
     std::vector<double> w1(n), wall(n);
     for (size_t i = 0; i < n; ++i) {
       const uint64_t tiles = std::max<uint64_t>(1, (members[i]->pats.W + kTileWords - 1) / kTileWords);
       w1[i] = (double)members[i]->plan.dense_sweep_gates + 1.0;
       wall[i] = w1[i] * tiles;
     }
-    std::vector<size_t> sample;
-    for (size_t c = 0; c < n_cls; ++c) {
+    BatchExec tx;
+    tx.n_sms = n_sms;
+    tx.smem_optin = smem_optin;
+    tx.smem_per_sm = smem_per_sm;
+    bool warm = true;
+    for (size_t c = 0; c < a.shapes.size(); ++c) {
       if (fixed[c]) continue;  // tuned on its own already
-      std::vector<size_t> in;
+      std::vector<size_t> in, sample;
       double total = 0, t0 = 0;
       for (size_t i = 0; i < n; ++i)
         if (a.cls[i] == (int)c) {
@@ -1049,75 +1002,36 @@ struct fsimb_batch {
         }
       std::sort(in.begin(), in.end(), [&](size_t x, size_t y) { return w1[x] < w1[y]; });
       const size_t k = std::max<size_t>(1, (size_t)(t0 / (0.03 * total)));
-      size_t picked = 0;
-      for (size_t q = k / 2; q < in.size(); q += k, ++picked) sample.push_back(in[q]);
-      if (!picked && !in.empty()) sample.push_back(in.back());
-    }
-    std::sort(sample.begin(), sample.end());
-    if (sample.empty()) return;
+      for (size_t q = k / 2; q < in.size(); q += k) sample.push_back(in[q]);
+      if (sample.empty() && !in.empty()) sample.push_back(in.back());
+      bool swept = false;
+      for (size_t i : sample) swept |= !members[i]->plan.sweeps.empty();
+      if (!swept) continue;
 
-    BatchExec tx;
-    tx.n_sms = n_sms;
-    tx.smem_optin = smem_optin;
-    tx.smem_per_sm = smem_per_sm;
-    std::vector<BatchJob> js = jobs_for(sample, a);
-    tx.layout(js, a.shapes, true, s);
-    tx.enqueue(s, true, false, nullptr);  // good machine of the sampled tiles
-    cudaEvent_t e0 = ev(0), e1 = ev(1);
-    std::vector<ClassShape> cur = a.shapes;
-    for (size_t c = 0; c < n_cls; ++c) {
-      SweepClass* kc = nullptr;
-      for (SweepClass& k : tx.classes)
-        if (k.id == (int)c) kc = &k;
-      if (!kc) continue;  // no sampled circuit in this class
       const ClassShape def = a.shapes[c];
-      const int M = def.M;
       std::vector<ClassShape> cands{def};
-      for (int occ : {1, 2, 3, 4})
-        for (int T : {128, 256, 384, 512, 768, 1024})
-          if (T <= (int)sweep_max_threads(M) && T * occ <= 2048 && !(occ == def.occ && T == def.threads))
-            cands.push_back(ClassShape{M, T, occ});
+      for (int T : {32, 64, 128, 256, 384, 512, 768, 1024})
+        if (T <= (int)sweep_max_threads(def.M) && T != def.threads) cands.push_back(ClassShape{def.M, T});
       float best_ms = 1e30f;
       ClassShape best = def;
       bool best_is_default = false;
       for (const ClassShape& sh : cands) {
-        // every member of the class, not only the sampled ones, must fit
-        if (sweep_vals_bytes(a.max_live[c], M) > smem_share(sh.occ)) continue;
-        try {
-          tx.size_class(*kc, sh);
-        } catch (const LimitError&) {
-          continue;  // slots do not fit this many CTAs per SM
-        }
-        if (kc->blocks < (int)std::min<unsigned long long>((unsigned long long)n_sms * sh.occ, kc->n_items))
-          continue;  // fewer CTAs per SM than asked: the same as a smaller shape
-        // an untimed run of the first candidate warms the GPU up; then the
-        // fastest of two timed runs counts
-        float ms = 1e30f;
-        for (int rep = (&sh == &cands[0]) ? -1 : 0; rep < 2; ++rep) {
-          CK(cudaMemsetAsync(tx.d_ctl.p, 0, tx.ctl_bytes, s));
-          CK(cudaEventRecord(e0, s));
-          tx.enqueue_sweeps(s, (int)c);
-          CK(cudaEventRecord(e1, s));
-          CK(cudaEventSynchronize(e1));
-          float x = 0;
-          CK(cudaEventElapsedTime(&x, e0, e1));
-          int kerr = 0;
-          CK(cudaMemcpy(&kerr, tx.d_ctl.p, sizeof(int), cudaMemcpyDeviceToHost));
-          if (kerr) throw CudaError{"a sweep kernel reached its wait limit during tuning"};
-          if (rep >= 0) ms = std::min(ms, x);
-        }
-        // the default shape stays unless a candidate beats it by 2%
-        const bool is_default = sh.occ == def.occ && sh.threads == def.threads;
+        a.shapes[c] = sh;
+        std::vector<BatchJob> js = jobs_for(sample, a);
+        for (BatchJob& j : js) j.cls = 0;
+        tx.layout(js, {sh}, true, s);
+        tx.enqueue(s, true, false, nullptr);  // good machine of the sampled tiles
+        const float ms = time_class0(tx, warm, s, 2);
+        warm = false;
+        const bool is_default = sh.threads == def.threads;
         if (is_default || ms < (best_is_default ? 0.98f : 1.0f) * best_ms) {
           best_ms = ms;
           best = sh;
           best_is_default = is_default;
         }
       }
-      tx.size_class(*kc, best);
-      cur[c] = best;
+      a.shapes[c] = best;
     }
-    a.shapes = cur;
     tx.release();
   }
 
@@ -1210,11 +1124,9 @@ void fsimb_batch::run(const fsimb_batch_opts* opts) {
     exec.class_events = nullptr;
   }
   CK(cudaEventRecord(e2, s));
-  int kerr = 0;
-  exec.fetch(s, &kerr);
+  exec.fetch(s);
   CK(cudaEventRecord(e3, s));
   CK(cudaEventSynchronize(e3));
-  if (kerr) throw CudaError{"a sweep kernel reached its wait limit for a record copy; results discarded"};
 
   const std::vector<BatchJob> js = jobs_for(all, a);
   for (size_t i = 0; i < members.size(); ++i) {
@@ -1268,7 +1180,7 @@ void fsimb_batch::run(const fsimb_batch_opts* opts) {
     for (const SweepClass& k : exec.classes)
       if (k.n_items > big->n_items) big = &k;
     stats.words_per_item = (uint32_t)big->shape.M;
-    stats.block_threads = (uint32_t)big->threads;
+    stats.block_threads = (uint32_t)big->shape.threads;
     stats.blocks = (uint32_t)big->blocks;
     stats.smem_bytes = (uint32_t)big->smem;
     stats.ctas_per_sm = (uint32_t)(big->blocks / std::max(1, n_sms));
@@ -1365,7 +1277,7 @@ int fsimb_batch_class_stats(const fsimb_batch* b, uint32_t i, fsimb_batch_class*
   const SweepClass& k = b->exec.classes[i];
   *out = fsimb_batch_class{};
   out->words_per_item = (uint32_t)k.shape.M;
-  out->block_threads = (uint32_t)k.threads;
+  out->block_threads = (uint32_t)k.shape.threads;
   out->blocks = (uint32_t)k.blocks;
   out->smem_bytes = (uint32_t)k.smem;
   out->n_circuits = k.circ_ids.size();

@@ -16,24 +16,23 @@
 
 namespace fsimb {
 
-// Sweep launch shape: words per item, CTA size, target CTAs per SM.
+// Sweep launch shape: words per item and CTA size.
 struct ClassShape {
   int M;
   int threads;
-  int occ;
 };
 
 // One job of a batch.
 struct BatchJob {
   const Netlist* nl = nullptr;
   const Plan* plan = nullptr;
-  const Schedule* sched = nullptr;  // schedule at M
+  const Schedule* sched = nullptr;  // schedule at M, packed for the class's CTA size
   const Patterns* pats = nullptr;
   uint64_t F = 0;
   int M = 4;
   int cls = 0;      // sweep class (index into the layout's shapes)
   // resident: the circuit arrays (type, fi_off, fi_idx, level, lvl, blob,
-  // li_off, li) are dev's, already on the device.  good_resident:
+  // li) are dev's, already on the device.  good_resident:
   // dev.good holds the job's good-machine tiles; no patterns are uploaded and
   // no good machine runs for it.
   bool resident = false;
@@ -48,16 +47,15 @@ struct WaveBytes {
 
 struct SweepClass {
   int id = 0;  // index into the layout's shapes
-  ClassShape shape{0, 0, 0};
+  ClassShape shape{0, 0};
   std::vector<uint32_t> circ_ids;   // members, in launch order
-  uint32_t queue_base = 0;          // their work counters: d_ctl words 1 + queue_base + j
+  uint32_t queue_base = 0;          // their work counters: d_ctl words queue_base + j
   unsigned long long n_items = 0;
   double work = 0;        // gate-words its sweeps evaluate (launch order)
   uint32_t max_live = 0;  // slots of the largest schedule in the class
-  uint32_t widest = 0;    // largest level block of gate records in the class, 16-byte units
-  uint32_t vals_bytes = 0, rec_buf = 0;
+  uint32_t widest = 0;    // records of the widest level in the class
   size_t smem = 0;
-  int threads = 0, blocks = 0;
+  int occ = 0, blocks = 0;  // CTAs per SM, CTAs launched
 };
 
 // Device bytes of a job's work arena: good values (unless resident), sweep
@@ -77,7 +75,7 @@ class BatchExec {
   size_t smem_optin = 0, smem_per_sm = 0;
 
   DevBuf d_static, d_desc, d_work, d_res;
-  DevBuf d_ctl;  // [0]: error flag; then one work counter per swept circuit
+  DevBuf d_ctl;  // one work counter per swept circuit
   PinnedBuf h_static, h_desc, h_res;
 
   std::vector<BatchCirc> circs;
@@ -93,7 +91,7 @@ class BatchExec {
   uint32_t n_circ = 0;
   bool tile0 = false;
   uint64_t static_bytes = 0, desc_bytes = 0;
-  uint64_t ctl_bytes = 256;  // error flag + one work counter per swept circuit
+  uint64_t ctl_bytes = 256;  // one work counter per swept circuit
   BatchSweepParams params{};  // launch parameters being built (32 KB)
   size_t smem_attr[4] = {0, 0, 0, 0};  // dynamic smem limit set per words-per-item kernel
   cudaEvent_t* class_events = nullptr;  // direct launches: recorded after each class
@@ -128,9 +126,7 @@ class BatchExec {
   // to the device (the layout's pointers stay valid: same jobs, same sizes).
   // Returns the bytes copied.
   uint64_t upload_static(const std::vector<BatchJob>& jobs, cudaStream_t s);
-  // New CTA size / CTAs per SM for the laid-out classes.
-  void relaunch_shapes(const std::vector<ClassShape>& shapes);
-  // Record buffer, shared memory, CTA size and grid of a class for a shape.
+  // Shared memory and grid of a class for a shape.
   void size_class(SweepClass& k, const ClassShape& sh);
   // Sets each class's dynamic shared-memory limit on its kernel (a
   // per-kernel attribute other launch sequences may have changed).
@@ -146,11 +142,10 @@ class BatchExec {
   // Captures the sequence on capture_stream once, then launches the graph on s.
   uint64_t run_graph(cudaStream_t capture_stream, cudaStream_t s);
   void invalidate_graph();
-  // Copies the per-fault counters and the error flag to the host (synchronises s).
-  void fetch(cudaStream_t s, int* kerr);
-  // The same copies, queued on s without waiting; read_err() once they ran.
+  // Copies the per-fault counters to the host (synchronises s).
+  void fetch(cudaStream_t s);
+  // The same copies, queued on s without waiting.
   void fetch_async(cudaStream_t s);
-  int read_err() const;
   void results(size_t i, const BatchJob& j, fsimb_fault_result* out) const;
   uint64_t items() const;
 };

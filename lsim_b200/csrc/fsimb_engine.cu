@@ -56,79 +56,92 @@ std::string read_file(const char* path) {
 // --------------------------------------------------------------------------
 static int m_slot(int M) { return M == 1 ? 0 : M == 2 ? 1 : M == 4 ? 2 : 3; }
 
-const Schedule& fsimb_handle::cached_schedule(int M) {
+Schedule& fsimb_handle::cached_schedule(int M) {
   const int sl = m_slot(M);
   if (sched_cache_gen[sl] != plan_gen) {
-    if (sched_M == M) {
-      sched_cache[sl] = sched;
-    } else {
-      build_schedule(nl, plan, 16u / (uint32_t)M, sched_cache[sl]);
-    }
+    build_schedule(nl, plan, 16u / (uint32_t)M, sched_cache[sl]);
     sched_cache_gen[sl] = plan_gen;
   }
   return sched_cache[sl];
 }
 
-void fsimb_handle::use_schedule(int M) {
-  if (sched_M == M) return;
-  sched = cached_schedule(M);
+const Schedule& fsimb_handle::use_schedule(int M, int T, cudaStream_t s) {
+  Schedule& sc = cached_schedule(M);
+  if (sched_M == M && sched_T == T) return sc;
+  sched_M = 0;
+  pack_schedule(sc, (uint32_t)T);
+  upload(d_recs, sc.blob, s);
+  upload(d_lvl, sc.lvl, s);
+  upload(d_li, sc.li, s);
   sched_M = M;
-  sched_uploaded = false;
+  sched_T = T;
+  return sc;
 }
 
 namespace fsimb {
 
+// The default shape minimises a model of one SM's time per pattern word.  A
+// level of a CTA's sweep takes a latency (barrier, record, operands, store)
+// of kLevel cycles plus kRound for each further round, and the shared-memory
+// and issue time of all the SM's CTAs: kWarp[M] cycles for a warp's records,
+// kPad for a warp of padding.  Fitted to shape sweeps on a B200; best of the
+// sweep against this choice: 2,000 gates 0.129 / 0.138 ms, 6,586 gates 2.34 /
+// 2.36, 20,000 gates with MUX 8.00 / 8.14, 30,000 gates 31.5 / 33.6, 50,000
+// gates 52.2 / 54.9, 200,000 gates 339 / 347 ms.
 void default_sweep_shape(const Plan& plan, const std::function<const Schedule&(int)>& sched_at,
-                         const std::function<int(int, int, size_t)>& occupancy,
-                         std::vector<uint32_t> widths, uint32_t words, size_t smem_optin,
-                         size_t smem_per_sm, int& M, int& occ, int& threads) {
-  // Words beyond the pattern block are work for nothing: no more words per
-  // item than the block has, rounded up to a power of two.
-  int most = 1;
-  while (most < 8 && (uint32_t)most < words) most *= 2;
+                         uint32_t words, size_t smem_optin, size_t smem_per_sm, int& M, int& threads) {
+  constexpr double kLevel = 1100, kRound = 300, kPad = 4;
   const size_t share1 = sweep_smem_share(smem_optin, smem_per_sm, 1);
-  const size_t share2 = sweep_smem_share(smem_optin, smem_per_sm, 2);
-  for (int m : {8, 4}) {
-    if (m > most) continue;
-    // plan.max_live (no bank constraints) bounds every schedule's slots from below
-    if (plan.max_live > kMaxSlots || sweep_vals_bytes(plan.max_live, m) + 64 * 32 > share2) continue;
-    const Schedule& sc = sched_at(m);
-    if (sc.max_live > kMaxSlots) continue;
-    const uint32_t vals = sweep_vals_bytes(sc.max_live, m);
-    const uint32_t blk = std::max<uint32_t>(sc.max_block16, 1);
-    if (vals + std::min<uint32_t>(blk, 64) * 32 > share2) continue;
-    const size_t smem = vals + std::min<size_t>(blk, (share2 - vals) / 32) * 32;
-    int t = (int)std::min<uint32_t>(pick_sweep_threads(widths, m), sweep_max_threads(m));
-    while (t > 64 && occupancy(m, t, smem) < 2) t -= 32;
-    M = m;
-    occ = 2;
-    threads = t;
-    return;
+  const uint32_t w = std::max<uint32_t>(1, std::min<uint32_t>(words, kTileWords));
+  auto cost = [&](int m, uint32_t t, size_t vals) {
+    const double warp = m == 8 ? 61 : m == 4 ? 31 : m == 2 ? 18 : 15;
+    const uint32_t ctas = (uint32_t)std::min<size_t>({smem_per_sm / (vals + 1024 + 256), 1024 / t, 32});
+    if (ctas < 1) return 1e300;
+    double cycles = 0;
+    for (uint32_t n : plan.net.level_recs) {
+      if (!n) continue;
+      const uint32_t rounds = (n + t - 1) / t, full = (n + 31) / 32, all = rounds * (t / 32);
+      cycles += kLevel + kRound * (rounds - 1) + ctas * (full * warp + (all - full) * kPad);
+    }
+    return cycles / ctas * ((w + m - 1) / m);
+  };
+  // Slots are about the peak of live values until a schedule says more.
+  size_t vals[4] = {0, 0, 0, 0};
+  bool exact[4] = {false, false, false, false};
+  for (int i = 0; i < 4; ++i) vals[i] = sweep_vals_bytes(plan.net_live + plan.net_live / 64 + 16, 1 << i);
+  for (;;) {
+    double best = 1e300;
+    int bi = 0;
+    threads = 64;
+    for (int i = 3; i >= 0; --i) {
+      if (i > 0 && vals[i] > share1) continue;
+      for (uint32_t t = 32; t <= 1024; t += 32) {
+        const double c = cost(1 << i, t, vals[i]);
+        if (c < best * 0.99) {
+          best = c;
+          bi = i;
+          threads = (int)t;
+        }
+      }
+    }
+    M = 1 << bi;
+    if (exact[bi]) break;
+    const Schedule& sc = sched_at(M);
+    exact[bi] = true;
+    vals[bi] = sc.max_live > kMaxSlots ? share1 + 1 : sweep_vals_bytes(sc.max_live, M);
   }
-  M = most;
-  while (M > 1 && sweep_vals_bytes(plan.max_live, M) > share1) M /= 2;
-  while (M > 1 && (sched_at(M).max_live > kMaxSlots || sweep_vals_bytes(sched_at(M).max_live, M) > share1))
-    M /= 2;
-  occ = 1;
-  threads = (int)std::min<uint32_t>(pick_sweep_threads(widths, M), sweep_max_threads(M));
+  threads = std::min<int>(threads, (int)sweep_max_threads(M));
 }
 
 }  // namespace fsimb
 
-void fsimb_handle::default_shape(std::vector<uint32_t> widths, int& M, int& occ, int& threads) {
+void fsimb_handle::default_shape(int& M, int& threads) {
   default_sweep_shape(
       plan, [&](int m) -> const Schedule& { return cached_schedule(m); },
-      [&](int m, int t, size_t smem) {
-        CK(sweep_set_smem(m, smem));
-        int got = 0;
-        CK(sweep_occupancy(m, t, smem, &got));
-        return got;
-      },
-      std::move(widths), (uint32_t)std::min<uint64_t>(pats.W, kTileWords), smem_optin, smem_per_sm, M, occ,
-      threads);
+      (uint32_t)std::min<uint64_t>(pats.W, kTileWords), smem_optin, smem_per_sm, M, threads);
 }
 
-void fsimb_handle::tune_shape(cudaStream_t s, const std::vector<uint32_t>& widths) {
+void fsimb_handle::tune_shape(cudaStream_t s) {
   const uint32_t N = plan.N;
   const uint32_t n_sweeps = (uint32_t)plan.sweeps.size();
   for (auto& e : tune_ev)
@@ -158,60 +171,43 @@ void fsimb_handle::tune_shape(cudaStream_t s, const std::vector<uint32_t>& width
   for (uint32_t i = 0; i < n_sweeps; i += stride) list.push_back(i);
   upload(d_tune_list, list, s);
   float best_ms = 1e30f;
-  int bM = 0, bT = 0, bocc = 1;
+  int bM = 0, bT = 0;
   // The default shape is the incumbent: a candidate replaces it only when
   // faster by more than 2% on the sample (the sample favours no shape, but
   // its time carries a few percent of noise).
-  int dM = 0, docc = 1, dT = 0;
-  default_shape(widths, dM, docc, dT);
+  int dM = 0, dT = 0;
+  default_shape(dM, dT);
   float default_ms = -1;
   struct Cand {
-    int M, occ, T;
+    int M, T;
   };
-  std::vector<Cand> cands{{dM, docc, dT}};
+  std::vector<Cand> cands{{dM, dT}};
   for (int M : {8, 4, 2, 1})
-    for (int occ : {1, 2, 3, 4})
-      for (int T : {128, 256, 384, 512, 768, 1024})
-        if (!(M == dM && occ == docc && T == dT)) cands.push_back({M, occ, T});
-  int cur_M = 0;
+    for (int T : {32, 64, 128, 192, 256, 384, 512, 768, 1024})
+      if (!(M == dM && T == dT)) cands.push_back({M, T});
+  const size_t share1 = sweep_smem_share(smem_optin, smem_per_sm, 1);
   for (const Cand& cd : cands) {
-    const int M = cd.M, occ = cd.occ, T = cd.T;
-    const size_t share1 = sweep_smem_share(smem_optin, smem_per_sm, 1);
-    if (plan.max_live > kMaxSlots || sweep_vals_bytes(plan.max_live, M) > share1) continue;
-    const Schedule& sc = cached_schedule(M);
-    if (sc.max_live > kMaxSlots || sweep_vals_bytes(sc.max_live, M) > share1) continue;
-    if (cur_M != M) {
-      upload(d_recs, sc.blob, s);
-      upload(d_lvl, sc.lvl, s);
-      upload(d_li_off, sc.li_off, s);
-      upload(d_li, sc.li, s);
-      sched_uploaded = false;
-      cur_M = M;
-    }
-    const uint32_t vals = sweep_vals_bytes(sc.max_live, M);
-    const size_t share = sweep_smem_share(smem_optin, smem_per_sm, occ);
-    if (vals > share) continue;
-    const uint32_t blk = std::max<uint32_t>(sc.max_block16, 1);
-    const uint32_t rec_buf = (uint32_t)std::min<size_t>(blk, (share - vals) / 32);
-    if (occ > 1 && rec_buf < std::min<uint32_t>(blk, 64)) continue;
-    const size_t smem = std::max<size_t>(16, vals + (size_t)rec_buf * 32);
-    if (T > (int)sweep_max_threads(M) || T * occ > 2048) continue;
+    const int M = cd.M, T = cd.T;
+    if (T > (int)sweep_max_threads(M)) continue;
+    if (plan.net_live > kMaxSlots || sweep_vals_bytes(plan.net_live, M) > share1) continue;
+    if (cached_schedule(M).max_live > kMaxSlots || sweep_vals_bytes(cached_schedule(M).max_live, M) > share1)
+      continue;
+    const Schedule& sc = use_schedule(M, T, s);
+    const size_t smem = std::max<size_t>(16, sweep_vals_bytes(sc.max_live, M));
     CK(sweep_set_smem(M, smem));
     int got = 0;
     CK(sweep_occupancy(M, T, smem, &got));
-    if (got < occ) continue;  // the same as a shape with fewer CTAs per SM
+    if (got < 1) continue;
     SweepArgs sa{};
     sa.blob = d_recs.as<uint4>();
     sa.lvl = d_lvl.as<uint4>();
     sa.level = d_level.as<uint32_t>();
-    sa.li_off = d_li_off.as<uint32_t>();
     sa.li = d_li.as<uint32_t>();
     sa.fi_off = d_fi_off.as<uint32_t>();
     sa.fi_idx = d_fi_idx.as<uint32_t>();
     sa.type = d_type.as<uint8_t>();
     sa.inj = d_inj.as<InjRec>();
     sa.list = d_tune_list.as<uint32_t>();
-    sa.wait_ns = kWaitLimitNs;
     sa.n_list = (uint32_t)list.size();
     sa.n_words = tile_words(pats.W, 0);
     sa.max_gate_level = plan.max_gate_level;
@@ -219,8 +215,10 @@ void fsimb_handle::tune_shape(cudaStream_t s, const std::vector<uint32_t>& width
     sa.good = d_good.as<uint64_t>();
     sa.out = d_out.as<uint64_t>();
     sa.queue = d_queue.as<int>();
-    sa.vals_bytes = vals;
-    sa.rec_buf = rec_buf;
+    sa.stream_recs = sc.stream_recs;
+    sa.fix0 = sc.fix0;
+    sa.inj_slot = sc.max_live - 1;
+    sa.split = sc.split;
     sa.err = d_err.as<int>();
     const int nb = (int)std::min<uint64_t>((uint64_t)n_sms * got, (uint64_t)sa.n_list * ((sa.n_words + M - 1) / M));
     // an untimed run of the first candidate warms the GPU up; then the
@@ -228,35 +226,28 @@ void fsimb_handle::tune_shape(cudaStream_t s, const std::vector<uint32_t>& width
     float ms = 1e30f;
     for (int rep = (&cd == &cands[0]) ? -1 : 0; rep < 2; ++rep) {
       CK(cudaMemsetAsync(d_queue.p, 0, sizeof(int), s));
-      CK(cudaMemsetAsync(d_err.p, 0, sizeof(int), s));
       CK(cudaEventRecord(tune_ev[0], s));
       CK(launch_sweep(M, T, nb, smem, sa, s));
       CK(cudaEventRecord(tune_ev[1], s));
       CK(cudaEventSynchronize(tune_ev[1]));
-      int kerr = 0;
-      CK(cudaMemcpy(&kerr, d_err.p, sizeof(int), cudaMemcpyDeviceToHost));
-      if (kerr) throw CudaError{"a sweep kernel reached its wait limit during tuning"};
       float x = 0;
       CK(cudaEventElapsedTime(&x, tune_ev[0], tune_ev[1]));
       if (rep >= 0) ms = std::min(ms, x);
     }
-    if (default_ms < 0 && M == dM && occ == docc && T == dT) {
+    if (default_ms < 0 && M == dM && T == dT) {
       default_ms = ms;
       best_ms = ms;
       bM = M;
       bT = T;
-      bocc = occ;
-    } else if (ms < (default_ms > 0 && bM == dM && bT == dT && bocc == docc ? 0.98f : 1.0f) * best_ms) {
+    } else if (ms < (default_ms > 0 && bM == dM && bT == dT ? 0.98f : 1.0f) * best_ms) {
       best_ms = ms;
       bM = M;
       bT = T;
-      bocc = occ;
     }
   }
   if (!bM) throw LimitError{"no sweep shape fits this circuit"};
   tuned_M = bM;
   tuned_T = bT;
-  tuned_occ = bocc;
   tuned_gen = plan_gen;
 }
 
@@ -289,7 +280,6 @@ void fsimb_handle::run(const fsimb_opts* opts) {
     plan_valid = true;
     plan_uploaded = false;
     sched_M = 0;
-    sched_uploaded = false;
   }
   const uint32_t N = plan.N;
   const uint64_t F = faults.size();
@@ -302,16 +292,13 @@ void fsimb_handle::run(const fsimb_opts* opts) {
   if (W_pad > (1ull << 31) || tiles * (uint64_t)N * kTileWords > (1ull << 40))
     throw LimitError{"pattern block too large"};
 
-  std::vector<uint32_t> widths;
-  for (uint32_t l = 1; l <= plan.max_gate_level && l < plan.n_levels; ++l)
-    widths.push_back(plan.level_off[l + 1] - plan.level_off[l]);
   cudaEvent_t e0 = ev(0), e1 = ev(1), e2 = ev(2), e3 = ev(3);
   CK(cudaEventRecord(e0, s));
   if (!plan_uploaded) {
     upload(d_type, nl.type, s);
     upload(d_fi_off, nl.fi_off, s);
     upload(d_fi_idx, nl.fi_idx, s);
-    upload(d_level, nl.level, s);
+    upload(d_level, plan.net.lev_up, s);
     upload(d_level_off, plan.level_off, s);
     upload(d_roots, plan.roots, s);
     upload(d_members, plan.members, s);
@@ -345,67 +332,56 @@ void fsimb_handle::run(const fsimb_opts* opts) {
   }
 
   // Sweep shape: explicit options, the autotuned shape of this plan, or the
-  // default (the largest words per item that fits; two CTAs per SM when 8
-  // or 4 words per item leave room for them).  Circuits whose live values
-  // do not fit in shared memory take the global-memory sweep.
+  // default.  Circuits whose live values do not fit in shared memory take
+  // the global-memory sweep.
   double tune_ms_now = 0;
-  int M = 0, occ = 1, threads = 0;
+  int M = 0, threads = 0;
   bool wide = o.sweep_variant == 2;
-  size_t vals_bytes = 0, smem = 0;
-  uint32_t rec_buf = 0;
+  size_t smem = 0;
+  const Schedule* sched = nullptr;
   const size_t share1 = sweep_smem_share(smem_optin, smem_per_sm, 1);
-  if (!wide && o.sweep_variant == 0 && n_sweeps &&
-      (plan.max_live > kMaxSlots || sweep_vals_bytes(plan.max_live, 1) > share1))
-    wide = true;  // no schedule can fit: skip building them
+  // The documented limit counts every gate's live value (the schedules fold
+  // some of them away): levels beyond it keep to the global-memory sweep,
+  // and explicit shapes beyond it stay refused.
+  auto gates_fit = [&](int m, size_t bytes) {
+    return plan.max_live <= kMaxSlots && sweep_vals_bytes(plan.max_live, m) <= bytes;
+  };
+  auto no_room = [&](uint32_t live, int m, size_t bytes, int ctas) {
+    return LimitError{"a sweep needs " + std::to_string(live) + " live values; shared memory holds " +
+                      std::to_string(bytes / (8 * m)) + " at " + std::to_string(m) + " word(s) per item and " +
+                      std::to_string(ctas) + " CTA(s) per SM"};
+  };
+  if (!wide && n_sweeps && !gates_fit(1, share1)) {
+    if (o.sweep_variant == 1) throw no_room(plan.max_live, 1, share1, 1);
+    wide = true;
+  }
   const bool explicit_shape = o.words_per_item || o.block_threads || o.ctas_per_sm;
   if (!wide && n_sweeps) {
-    try {
-      if (explicit_shape) {
-        M = (int)o.words_per_item;
-        occ = o.ctas_per_sm ? (int)o.ctas_per_sm : 1;
-        threads = (int)o.block_threads;
-      } else if (o.tune && tiles) {
-        if (tuned_gen != plan_gen) {
-          const auto t0 = std::chrono::steady_clock::now();
-          tune_shape(s, widths);
-          tune_ms_now =
-              std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-        }
-        M = tuned_M;
-        occ = tuned_occ;
-        threads = tuned_T;
-      } else {
-        default_shape(widths, M, occ, threads);
+    if (explicit_shape) {
+      const int ctas = o.ctas_per_sm ? (int)o.ctas_per_sm : 1;
+      const size_t budget = sweep_smem_share(smem_optin, smem_per_sm, ctas);
+      M = o.words_per_item ? (int)o.words_per_item : 8;
+      for (;; M /= 2) {
+        if (gates_fit(M, budget) && cached_schedule(M).max_live <= kMaxSlots &&
+            sweep_vals_bytes(cached_schedule(M).max_live, M) <= budget)
+          break;
+        if (o.words_per_item || M == 1)
+          throw no_room(std::max(plan.max_live, cached_schedule(M).max_live), M, budget, ctas);
       }
-      const size_t budget = sweep_smem_share(smem_optin, smem_per_sm, occ);
-      const bool fixed_M = M != 0;
-      if (!M) {
-        M = 8;
-        while (M > 1 && sweep_vals_bytes(plan.max_live, M) > budget) M /= 2;
+      threads = o.block_threads ? (int)o.block_threads : (int)pick_sweep_threads(cached_schedule(M), M);
+    } else if (o.tune && tiles) {
+      if (tuned_gen != plan_gen) {
+        const auto t0 = std::chrono::steady_clock::now();
+        tune_shape(s);
+        tune_ms_now =
+            std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
       }
-      for (;;) {
-        use_schedule(M);
-        const bool fits = sched.max_live <= kMaxSlots && sweep_vals_bytes(sched.max_live, M) <= budget;
-        if (fits) break;
-        if (fixed_M || M == 1)
-          throw LimitError{"a sweep needs " + std::to_string(sched.max_live) +
-                           " live values; shared memory holds " + std::to_string(budget / (8 * M)) +
-                           " at " + std::to_string(M) + " word(s) per item and " + std::to_string(occ) +
-                           " CTA(s) per SM"};
-        M /= 2;
-      }
-      vals_bytes = sweep_vals_bytes(sched.max_live, M);
-      rec_buf = (uint32_t)std::min<size_t>(std::max<uint32_t>(sched.max_block16, 1),
-                                           (budget - vals_bytes) / 32);
-      smem = std::max<size_t>(16, vals_bytes + (size_t)rec_buf * 32);
-      if (!threads) threads = (int)pick_sweep_threads(widths, M);
-      threads = std::min<int>(threads, (int)sweep_max_threads(M));
-    } catch (const LimitError&) {
-      // an explicit shape that does not fit stays an error; without one, the
-      // circuit does not fit shared memory at any shape
-      if (o.sweep_variant == 1 || explicit_shape) throw;
-      wide = true;
+      M = tuned_M;
+      threads = tuned_T;
+    } else {
+      default_shape(M, threads);
     }
+    threads = std::min<int>(threads, (int)sweep_max_threads(M));
   }
   int blocks = 0, occ_got = 0;
   if (wide) {
@@ -414,7 +390,7 @@ void fsimb_handle::run(const fsimb_opts* opts) {
     if (!eflag_uploaded) {
       std::vector<uint8_t> fl(N, 0);
       for (uint32_t e = plan.n_pi; e < N; ++e)
-        fl[e] = (uint8_t)((plan.gate_fo[e] || plan.po_drv[e]) ? 1 : 0) | (uint8_t)(plan.po_drv[e] ? 2 : 0);
+        fl[e] = (uint8_t)((plan.net.live[e] && nl.type[e] != G_PO) ? 1 : 0) | (uint8_t)(plan.po_drv[e] ? 2 : 0);
       upload(d_eflag, fl, s);
       eflag_uploaded = true;
     }
@@ -424,13 +400,8 @@ void fsimb_handle::run(const fsimb_opts* opts) {
     blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)n_sms * std::max(occ_got, 1), cap));
     if (n_sweeps) d_gvals.ensure((size_t)blocks * per_block);
   } else if (n_sweeps) {
-    if (!sched_uploaded) {
-      upload(d_recs, sched.blob, s);
-      upload(d_lvl, sched.lvl, s);
-      upload(d_li_off, sched.li_off, s);
-      upload(d_li, sched.li, s);
-      sched_uploaded = true;
-    }
+    sched = &use_schedule(M, threads, s);
+    smem = std::max<size_t>(16, sweep_vals_bytes(sched->max_live, M));
   }
   CK(cudaMemsetAsync(d_queue.p, 0, std::max<uint64_t>(tiles, 1) * sizeof(int), s));
   CK(cudaMemsetAsync(d_err.p, 0, sizeof(int), s));
@@ -509,7 +480,6 @@ void fsimb_handle::run(const fsimb_opts* opts) {
         sa.blob = d_recs.as<uint4>();
         sa.lvl = d_lvl.as<uint4>();
         sa.level = d_level.as<uint32_t>();
-        sa.li_off = d_li_off.as<uint32_t>();
         sa.li = d_li.as<uint32_t>();
         sa.fi_off = d_fi_off.as<uint32_t>();
         sa.fi_idx = d_fi_idx.as<uint32_t>();
@@ -523,10 +493,12 @@ void fsimb_handle::run(const fsimb_opts* opts) {
         sa.good = good_t;
         sa.out = d_out.as<uint64_t>();
         sa.queue = d_queue.as<int>() + t;
-        sa.vals_bytes = (uint32_t)vals_bytes;
-        sa.rec_buf = rec_buf;
+        sa.stream_recs = sched->stream_recs;
+        sa.fix0 = sched->fix0;
+        sa.inj_slot = sched->max_live - 1;
+        sa.split = sched->split;
         sa.err = d_err.as<int>();
-        sa.wait_ns = o.wait_test ? kWaitTestNs : kWaitLimitNs;
+        sa.wait_ns = kWaitTestNs;
         sa.wait_test = (o.wait_test && t == 0) ? 1u : 0u;
         CK(launch_sweep(M, threads, nb, smem, sa, s));
       }
@@ -540,7 +512,7 @@ void fsimb_handle::run(const fsimb_opts* opts) {
         CK(cudaMemcpyAsync(host_sw.data(), sw_list, n_sw * 4, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
         for (uint32_t si : host_sw) {
-          uint32_t L0 = nl.level[plan.sweeps[si].elem] + 1;
+          uint32_t L0 = nl.level[plan.sweeps[si].stored] + 1;
           if (L0 <= plan.max_gate_level) {
             dense += (uint64_t)(plan.eval_prefix[gates_end] - plan.eval_prefix[plan.level_off[L0]]) * subtiles * M;
             alg_bytes += (plan.nfp_prefix[gates_end] - plan.nfp_prefix[plan.level_off[L0]]) * subtiles * M;
@@ -700,12 +672,12 @@ void fsimb_handle::run(const fsimb_opts* opts) {
   CK(cudaEventElapsedTime(&x, e1, e3));
   stats.ms_compute = x;
   stats.good_gate_words = (uint64_t)(N - plan.n_pi) * W_pad;
-  stats.max_live = wide ? 0 : sched.max_live;
-  stats.bank_conflict_groups = wide ? 0 : sched.conflict_groups;
-  stats.bank_access_groups = wide ? 0 : sched.access_groups;
+  stats.max_live = sched ? sched->max_live : 0;
+  stats.bank_conflict_groups = sched ? sched->conflict_groups : 0;
+  stats.bank_access_groups = sched ? sched->access_groups : 0;
   stats.sweep_variant = wide ? 2 : 1;
   stats.hbm_bytes_per_tile = (uint64_t)N * kTileWords * 8 + (uint64_t)n_sweeps * (kTileWords * 8 + sizeof(InjRec)) +
-                             (wide ? (uint64_t)N * 10 + nl.fi_idx.size() * 4 : sched.bytes());
+                             (sched ? sched->bytes() : wide ? (uint64_t)N * 10 + nl.fi_idx.size() * 4 : 0);
   stats.ms_tune = tune_ms_now;
   stats.ctas_per_sm = (uint32_t)occ_got;
   stats.words_per_item = (uint32_t)M;
@@ -1002,7 +974,6 @@ int fsimb_fault_costs(fsimb_handle* h, uint64_t* group, uint64_t* cost, uint64_t
     h->plan_valid = true;
     h->plan_uploaded = false;
     h->sched_M = 0;
-    h->sched_uploaded = false;
   }
   const Plan& P = h->plan;
   const Netlist& nl = h->nl;
@@ -1014,7 +985,8 @@ int fsimb_fault_costs(fsimb_handle* h, uint64_t* group, uint64_t* cost, uint64_t
   // traced faults: one group per FFR root (its sweep, when it has one, plus
   // the tracing of its members); exact faults: one group each
   for (const RootRec& rr : P.roots) {
-    const uint64_t c = 1 + (rr.obs < kObsZero ? sweep_gates(rr.root) : 0) + (rr.mem_end - rr.mem_begin);
+    const bool swept = nl.type[rr.root] != G_PO && !P.po_drv[rr.root] && P.gate_fo[rr.root];
+    const uint64_t c = 1 + (swept ? sweep_gates(rr.root) : 0) + (rr.mem_end - rr.mem_begin);
     for (uint32_t i = rr.flt_begin; i < rr.flt_end; ++i) {
       const uint32_t f = P.traced[i].fault;
       if (group) group[f] = rr.root;

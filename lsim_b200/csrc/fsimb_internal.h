@@ -77,15 +77,17 @@ inline void upload(DevBuf& b, const std::vector<T>& v, cudaStream_t s) {
   if (!v.empty()) CK(cudaMemcpyAsync(b.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s));
 }
 
-// Largest sweep CTA for M words per item (the kernels' launch bounds).
-inline uint32_t sweep_max_threads(int M) { return M >= 8 ? 512 : (M >= 4 ? 768 : 1024); }
+// Largest sweep CTA for M words per item (the kernels' register caps).
+inline uint32_t sweep_max_threads(int) { return 1024; }
 
-// Sweep CTA size: one thread per gate of a level; the multiple of 32 that
-// splits the typical (90th percentile) level width into equal rounds, so no
-// thread idles long before the per-level barrier.  `widths` holds the gate
-// count of each swept level (reordered in place).
-inline uint32_t pick_sweep_threads(std::vector<uint32_t>& widths, int M) {
+// Sweep CTA size for one thread per record of a level: the multiple of 32
+// that splits the typical (90th percentile) level into equal rounds, so no
+// thread idles long before the per-level barrier.
+inline uint32_t pick_sweep_threads(const Schedule& sc, int M) {
   const uint32_t tmax = sweep_max_threads(M);
+  std::vector<uint32_t> widths;
+  for (size_t l = 0; l + 1 < sc.rec_off.size(); ++l)
+    if (sc.rec_off[l + 1] > sc.rec_off[l]) widths.push_back(sc.rec_off[l + 1] - sc.rec_off[l]);
   uint32_t w = 64;
   if (!widths.empty()) {
     std::nth_element(widths.begin(), widths.begin() + widths.size() * 9 / 10, widths.end());
@@ -154,17 +156,11 @@ struct PinnedBuf {
   }
 };
 
-// Default sweep shape of a circuit: two CTAs per SM at 8 or 4 words per
-// item when the value slots leave room for at least 64 staged records (the
-// CTA size then lowered until two fit), else the largest words per item
-// whose slots fit one CTA per SM, with the width heuristic's CTA size.
-// At most `words` words per item (rounded up to a power of two): the pattern
-// words a tile of the block has.  sched_at(M) returns the schedule at M;
-// occupancy(M, threads, smem) the sweep kernel's CTAs per SM.
+// Default sweep shape of a circuit.  At most `words` words per item (rounded
+// up to a power of two): the pattern words a tile of the block has.
+// sched_at(M) returns the schedule at M.
 void default_sweep_shape(const Plan& plan, const std::function<const Schedule&(int)>& sched_at,
-                         const std::function<int(int, int, size_t)>& occupancy,
-                         std::vector<uint32_t> widths, uint32_t words, size_t smem_optin,
-                         size_t smem_per_sm, int& M, int& occ, int& threads);
+                         uint32_t words, size_t smem_optin, size_t smem_per_sm, int& M, int& threads);
 
 // A fresh value for fsimb_handle::gen: every change of a handle's circuit,
 // faults or patterns gets a number no other state of any handle had.
@@ -191,22 +187,20 @@ struct fsimb_handle {
   fsimb::Plan plan;
   bool plan_valid = false;
   bool plan_uploaded = false;
-  fsimb::Schedule sched;          // for sched_M words per item
-  int sched_M = 0;
-  bool sched_uploaded = false;
   // Schedules built so far for this plan, per words per item (1, 2, 4, 8).
   fsimb::Schedule sched_cache[4];
+  int sched_M = 0, sched_T = 0;   // the one on the device, and its CTA size (0: none)
   uint64_t sched_cache_gen[4] = {0, 0, 0, 0};
   // Autotuned sweep shape of plan_gen (fsimb_opts.tune).
   uint64_t tuned_gen = 0;
-  int tuned_M = 0, tuned_T = 0, tuned_occ = 0;
+  int tuned_M = 0, tuned_T = 0;
   cudaEvent_t tune_ev[2] = {nullptr, nullptr};
   // Recorded after each fsimb_run's uploads, on the run's stream: work on
   // another stream that reads the circuit arrays waits for it.
   cudaEvent_t upload_ev = nullptr;
 
-  fsimb::DevBuf d_type, d_fi_off, d_fi_idx, d_recs, d_level, d_level_off, d_li_off, d_li;
-  fsimb::DevBuf d_lvl;     // schedule LevelDesc per level
+  fsimb::DevBuf d_type, d_fi_off, d_fi_idx, d_recs, d_level, d_level_off, d_li;
+  fsimb::DevBuf d_lvl;     // schedule: stream and live-in offsets per level
   fsimb::DevBuf d_eflag;   // wide-circuit sweep: per element, evaluated / drives a PO
   fsimb::DevBuf d_gvals;   // wide-circuit sweep: per-CTA value regions
   fsimb::DevBuf d_roots, d_members, d_traced, d_inj, d_exact;
@@ -226,7 +220,7 @@ struct fsimb_handle {
     if (device >= 0) {
       cudaSetDevice(device);
       for (fsimb::DevBuf* b : {&d_type, &d_fi_off, &d_fi_idx, &d_recs, &d_level, &d_level_off,
-                        &d_lvl, &d_eflag, &d_gvals, &d_li_off, &d_li, &d_roots, &d_members, &d_traced, &d_inj, &d_exact,
+                        &d_lvl, &d_eflag, &d_gvals, &d_li, &d_roots, &d_members, &d_traced, &d_inj, &d_exact,
                         &d_pwords, &d_good, &d_out, &d_sens, &d_count, &d_first, &d_lastflag,
                         &d_queue, &d_err, &d_root_list[0], &d_root_list[1], &d_sweep_list,
                         &d_exact_list[0], &d_exact_list[1], &d_nout, &d_tune_list})
@@ -251,7 +245,7 @@ struct fsimb_handle {
   uint64_t device_bytes() const {
     uint64_t s = 0;
     for (const fsimb::DevBuf* b : {&d_type, &d_fi_off, &d_fi_idx, &d_recs, &d_level, &d_level_off,
-                            &d_lvl, &d_eflag, &d_gvals, &d_li_off, &d_li, &d_roots, &d_members, &d_traced, &d_inj, &d_exact,
+                            &d_lvl, &d_eflag, &d_gvals, &d_li, &d_roots, &d_members, &d_traced, &d_inj, &d_exact,
                             &d_pwords, &d_good, &d_out, &d_sens, &d_count, &d_first, &d_lastflag,
                             &d_queue, &d_err, &d_root_list[0], &d_root_list[1], &d_sweep_list,
                             &d_exact_list[0], &d_exact_list[1], &d_nout, &d_tune_list})
@@ -265,7 +259,6 @@ struct fsimb_handle {
     plan_valid = false;
     plan_uploaded = false;
     sched_M = 0;
-    sched_uploaded = false;
     has_results = false;
     good_tiles = 0;
   }
@@ -331,15 +324,15 @@ struct fsimb_handle {
 
   void run(const fsimb_opts* opts);
   // The schedule at M words per item for the current plan (cached per M).
-  const fsimb::Schedule& cached_schedule(int M);
-  // Makes `sched` the schedule at M (re-uploaded before the next sweep).
-  void use_schedule(int M);
+  fsimb::Schedule& cached_schedule(int M);
+  // The schedule at M packed for T threads, uploaded unless it is there.
+  const fsimb::Schedule& use_schedule(int M, int T, cudaStream_t s);
   // default_sweep_shape for this circuit and the plain sweep kernel.
-  void default_shape(std::vector<uint32_t> widths, int& M, int& occ, int& threads);
+  void default_shape(int& M, int& threads);
   // Times candidate shapes on a strided sample of tile 0's sweeps and keeps
-  // the fastest in tuned_M / tuned_T / tuned_occ.  Needs the plan and the
+  // the fastest in tuned_M / tuned_T.  Needs the plan and the
   // patterns on the device.
-  void tune_shape(cudaStream_t s, const std::vector<uint32_t>& widths);
+  void tune_shape(cudaStream_t s);
 };
 
 // Wraps a C ABI body: exceptions become status codes and (h)->err.

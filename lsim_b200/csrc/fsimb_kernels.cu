@@ -6,9 +6,9 @@
 //   k_sweep<M>     persistent: each CTA pulls (sweep, M-word subtile) items from
 //                  a device work counter and re-simulates the levels above the
 //                  injection point with all live values in shared memory
-//                  (slots and a bank-conflict-free order chosen on the host;
-//                  gate records staged per level by TMA bulk copies).  Writes
-//                  the OR over POs of (faulty ^ good) per word.
+//                  (slots, a bank-conflict-free order and a stream of gate
+//                  records per CTA size laid out on the host).  Writes the OR
+//                  over POs of (faulty ^ good) per word.
 //   k_sweep_wide<M> the same sweep for circuits whose live values do not
 //                  fit in shared memory: values in a per-CTA region of global
 //                  memory indexed by element.
@@ -28,6 +28,7 @@
 #include "fsimb_kernels.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace fsimb {
 
@@ -96,27 +97,12 @@ __global__ void k_good_level(GoodArgs a) {
   }
 }
 
-// ---------------------------------------------------------------- TMA bulk staging
+// ---------------------------------------------------------------- bounded wait
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-// One thread arms the barrier for `bytes` and starts a bulk copy (no
-// multicast) of `bytes` from global to this CTA's shared memory.
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  if (bytes == 0) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-    return;
-  }
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-               : "memory");
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-          smem_u32(dst)),
-      "l"(src), "r"(bytes), "r"(smem_u32(bar))
-      : "memory");
 }
 __device__ __forceinline__ uint64_t global_ns() {
   uint64_t t;
@@ -159,238 +145,264 @@ __device__ __forceinline__ uint32_t find_prefix(const unsigned long long* prefix
 // ---------------------------------------------------------------- sweep
 // Per-circuit pointers a sweep item reads (one circuit, one tile).
 struct SweepView {
-  const uint4* blob;       // level blocks of gate records (fsimb_plan.h)
-  const uint4* lvl;        // LevelDesc per level
-  const uint32_t* level;   // element -> level
-  const uint32_t* li_off;
+  const uint4* blob;       // record stream for this CTA size (fsimb_plan.h)
+  const uint4* lvl;        // per level: its first record in the stream, its range in li
+  const uint32_t* level;   // element -> level, or kFolded | consumer
   const uint32_t* li;      // (element, slot) pairs
   const uint32_t* fi_off;
   const uint32_t* fi_idx;
   const uint8_t* type;
   const uint64_t* good;    // tile [N][32]
   uint32_t max_gate_level;
+  uint32_t stream_recs;
+  uint32_t fix0;           // 16-byte offset of the fix entries in blob
+  uint32_t inj_slot;       // the injection slot (the last one)
+  uint32_t split;          // levels are ordered by kind
 };
 
-// Faulty value of the injection element for word w of the tile.
+// Element x's word w of the tile with its input `pin` (any input that reads
+// `from` when pin < 0) at v; the other inputs hold their good values.
 template <class V>
-__device__ __forceinline__ uint64_t inj_value(const V& a, const InjRec& inj, uint32_t w) {
-  const uint32_t x = inj.elem;
-  if (!(inj.mode & kInjStuck)) return ~a.good[(uint64_t)x * 32 + w];
-  const uint64_t sv = inj.value ? ~0ull : 0ull;
-  if (inj.pin == 0) return sv;
+__device__ __forceinline__ uint64_t eval_with(const V& a, uint32_t x, int pin, uint32_t from, uint64_t v,
+                                              uint32_t w) {
   const uint8_t t = a.type[x];
   const uint32_t f0 = a.fi_off[x];
   uint32_t nf = a.fi_off[x + 1] - f0;
   if (t == G_INV || t == G_CLKBUF || t == G_PO) nf = 1;
   uint64_t in[4] = {0, 0, 0, 0};
 #pragma unroll
-  for (int k = 0; k < 4; ++k)
-    if ((uint32_t)k < nf) in[k] = a.good[(uint64_t)a.fi_idx[f0 + k] * 32 + w];
-  const uint32_t pk = inj.pin - 1;
-#pragma unroll
-  for (int k = 0; k < 4; ++k)
-    if ((uint32_t)k == pk) in[k] = sv;
+  for (int k = 0; k < 4; ++k) {
+    if ((uint32_t)k < nf) {
+      const uint32_t f = a.fi_idx[f0 + k];
+      in[k] = k == pin || (pin < 0 && f == from) ? v : a.good[(uint64_t)f * 32 + w];
+    }
+  }
   return eval_word(t, nf, in[0], in[1], in[2], in[3]);
 }
 
+// Word w of the injection's stored element with the fault: the faulty word
+// of inj.elem, taken up through the gates it is folded into (each has one
+// consumer, whose other inputs are good).
+template <class V>
+__device__ __forceinline__ uint64_t inj_value(const V& a, const InjRec& inj, uint32_t w) {
+  uint32_t x = inj.elem;
+  if (!(inj.mode & kInjStuck)) return ~a.good[(uint64_t)x * 32 + w];
+  const uint64_t sv = (inj.mode & kInjValue) ? ~0ull : 0ull;
+  const uint32_t pin = inj.mode >> kInjPinShift;
+  uint64_t v = pin ? eval_with(a, x, (int)pin - 1, 0u, sv, w) : sv;
+  for (uint32_t lv = a.level[x]; lv & kFolded; lv = a.level[x]) {
+    const uint32_t c = lv & ~kFolded;
+    v = eval_with(a, c, -1, x, v, w);
+    x = c;
+  }
+  return v;
+}
+
+// Chunk of a slot: 16 bytes, two words (one 8-byte word at M = 1), as 32-bit
+// registers so that inversion masks are one register each.
 template <int M>
-__device__ __forceinline__ void lds_chunk(const uint64_t* vals, uint32_t slot, int h, uint64_t (&v)[2]) {
+struct Chunk {
+  static constexpr int R = M == 1 ? 2 : 4;
+  uint32_t r[R];
+};
+template <int M>
+__device__ __forceinline__ Chunk<M> lds(uint32_t addr) {
+  Chunk<M> c;
+  if constexpr (M == 1)
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(c.r[0]), "=r"(c.r[1]) : "r"(addr));
+  else
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(c.r[0]), "=r"(c.r[1]), "=r"(c.r[2]), "=r"(c.r[3])
+                 : "r"(addr));
+  return c;
+}
+// The same for a literal that may be absent (has == 0: zeros), without a
+// branch: neighbouring records differ in their literal counts.
+template <int M>
+__device__ __forceinline__ Chunk<M> lds_if(uint32_t addr, uint32_t has) {
+  Chunk<M> c;
   if constexpr (M == 1) {
-    v[0] = vals[slot];
+    c.r[0] = c.r[1] = 0u;
+    asm volatile("{ .reg .pred p; setp.ne.u32 p, %3, 0; @p ld.shared.v2.u32 {%0, %1}, [%2]; }"
+                 : "+r"(c.r[0]), "+r"(c.r[1])
+                 : "r"(addr), "r"(has));
   } else {
-    const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(vals + (size_t)slot * M + 2 * h);
-    v[0] = q.x;
-    v[1] = q.y;
+    c.r[0] = c.r[1] = c.r[2] = c.r[3] = 0u;
+    asm volatile("{ .reg .pred p; setp.ne.u32 p, %5, 0; @p ld.shared.v4.u32 {%0, %1, %2, %3}, [%4]; }"
+                 : "+r"(c.r[0]), "+r"(c.r[1]), "+r"(c.r[2]), "+r"(c.r[3])
+                 : "r"(addr), "r"(has));
+  }
+  return c;
+}
+template <int M>
+__device__ __forceinline__ void sts(uint32_t addr, const Chunk<M>& c) {
+  if constexpr (M == 1)
+    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(addr), "r"(c.r[0]), "r"(c.r[1]) : "memory");
+  else
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(c.r[0]), "r"(c.r[1]), "r"(c.r[2]),
+                 "r"(c.r[3])
+                 : "memory");
+}
+// (a ^ i) & b, and x & y or x ^ y by the mask k: one LOP3 each.
+__device__ __forceinline__ uint32_t and_inv(uint32_t a, uint32_t i, uint32_t b) {
+  uint32_t r;
+  asm("lop3.b32 %0, %1, %2, %3, 0x28;" : "=r"(r) : "r"(a), "r"(i), "r"(b));
+  return r;
+}
+__device__ __forceinline__ uint32_t and_or_xor(uint32_t x, uint32_t y, uint32_t k) {
+  uint32_t r;
+  asm("lop3.b32 %0, %1, %2, %3, 0x68;" : "=r"(r) : "r"(x), "r"(y), "r"(k));
+  return r;
+}
+
+// A record (fsimb_plan.h RecKind): two words, four at one word per item.
+template <int M>
+using RecWords = typename std::conditional<M == 1, uint4, uint2>::type;
+
+// Byte offset of slot k of a record, to be masked by kOffMask: one shift.
+// Chunk c of a lane's order is the slot's chunk (first ^ c), its offset
+// (offset & mask) ^ (rot ^ 16c) with rot 16 bytes times the lane's first
+// chunk: one LOP3; the slots' base address is left to the load.
+template <int M>
+struct SlotBits {
+  static constexpr int kShift = M == 1 ? 3 : M == 2 ? 4 : M == 4 ? 5 : 6;  // 8 * M bytes a slot
+  static constexpr uint32_t kOffMask = kRecSlot << kShift;
+};
+template <int M>
+__device__ __forceinline__ uint32_t slot_off(const RecWords<M>& q, int k) {
+  const uint32_t w = k < 2 ? q.x : q.y;
+  if constexpr (M == 1) {
+    const uint32_t h = k < 2 ? q.z : q.w;
+    const int sh = 14 * (k & 1);
+    return ((w >> sh & kRecSlot) | (h >> sh & kRecSlot) << 14) * 8u;
+  } else {
+    return (k & 1) ? w >> (14 - SlotBits<M>::kShift) : w << SlotBits<M>::kShift;
   }
 }
-
 template <int M>
-__device__ __forceinline__ void sts_chunk(uint64_t* vals, uint32_t slot, int h, const uint64_t (&v)[2]) {
-  if constexpr (M == 1)
-    vals[slot] = v[0];
-  else
-    *reinterpret_cast<ulonglong2*>(vals + (size_t)slot * M + 2 * h) = make_ulonglong2(v[0], v[1]);
+__device__ __forceinline__ uint32_t chunk_at(uint32_t off, uint32_t rot, uint32_t c) {
+  if constexpr (M == 1) return off;
+  return (off & SlotBits<M>::kOffMask) ^ (rot ^ 16u * c);
 }
 
-template <int M>
-using PoAcc = uint64_t[(M >= 2) ? M / 2 : 1][(M >= 2) ? 2 : 1];
-
-// ---- plain records: one body per family and fan-in (fsimb_plan.h plain_body)
-// Slot chunk h of the value at byte offset `off` (slot * 8M).
-template <int M>
-__device__ __forceinline__ void ldo(const char* vb, uint32_t off, int h, uint64_t (&v)[2]) {
-  if constexpr (M == 1) {
-    v[0] = *reinterpret_cast<const uint64_t*>(vb + off);
-  } else {
-    const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(vb + off + 16 * h);
-    v[0] = q.x;
-    v[1] = q.y;
-  }
-}
-template <int M>
-__device__ __forceinline__ void sto(char* vb, uint32_t off, int h, const uint64_t (&v)[2]) {
-  if constexpr (M == 1)
-    *reinterpret_cast<uint64_t*>(vb + off) = v[0];
-  else
-    *reinterpret_cast<ulonglong2*>(vb + off + 16 * h) = make_ulonglong2(v[0], v[1]);
-}
-
-// A plain record (fsimb_plan.h plain_rec) of body B on all M words.  B = 0:
-// one input, io ^ a; 1 / 3: AND family with 2 / 3 inputs,
-// io ^ AND(in ^ ii); 2 / 4: XOR family with 2 / 3 inputs, io ^ XOR(in).
-// The inversions come from the class code: within the AND family the codes
-// run AND, NAND, OR, NOR, so ii is bit 1 of the offset and io the XOR of
-// its two bits; elsewhere io is bit 0 of the code.
-template <int M, int B>
-__device__ __forceinline__ void plain_body(char* vb, const uint2 r, int pl) {
+// A cluster record on all M words.  vb: shared address of the slots.  Two
+// chunks are in flight at a time.  KIND kRecNop: any AND or XOR, by masks.
+template <int M, int KIND>
+__device__ __forceinline__ void cluster_eval(uint32_t vb, uint32_t rot, const RecWords<M> q) {
   constexpr int C = (M >= 2) ? M / 2 : 1;
-  constexpr int VC = (M >= 2) ? 2 : 1;
-  constexpr int NF = B == 0 ? 1 : (B <= 2 ? 2 : 3);
-  constexpr uint32_t SB = 8u * M;
-  const uint32_t cls = r.y >> 28;
-  uint32_t io_bit, ii_bit = 0;
-  if constexpr (B == 1 || B == 3) {
-    const uint32_t rel = cls - (B == 1 ? (uint32_t)kPAnd2 : (uint32_t)kPAnd3);
-    ii_bit = (rel >> 1) & 1u;
-    io_bit = (rel ^ (rel >> 1)) & 1u;
-  } else {
-    io_bit = cls & 1u;
-  }
-  const uint64_t ii = 0ull - (uint64_t)ii_bit, io = 0ull - (uint64_t)io_bit;
-  const uint32_t o0 = (r.x & 0x7FFFu) * SB;
-  const uint32_t o1 = ((r.x >> 15) & 0x7FFFu) * SB;
-  const uint32_t o2 = (__funnelshift_r(r.x, r.y, 30) & 0x7FFFu) * SB;
-  const uint32_t oo = ((r.y >> 13) & 0x7FFFu) * SB;
+  constexpr int U = C >= 2 ? 2 : 1;
+  constexpr int R = Chunk<M>::R;
+  constexpr bool kAny = KIND == kRecNop;
+  constexpr bool kThree = KIND == kRecAnd3 || KIND == kRecXor3;
+  const uint32_t o0 = slot_off<M>(q, 0), o1 = slot_off<M>(q, 1), o2 = slot_off<M>(q, 2), oo = slot_off<M>(q, 3);
+  const uint32_t i0 = (uint32_t)((int32_t)q.x >> 31), i1 = (uint32_t)((int32_t)(q.x << 1) >> 31);
+  const uint32_t i2 = (uint32_t)((int32_t)(q.x << 2) >> 31), io = (uint32_t)((int32_t)(q.x << 3) >> 31);
+  const uint32_t kind = (q.y >> kRecKindShift) & 7u;
+  const uint32_t kx = kind >= kRecXor2 ? ~0u : 0u;
+  static_assert(kRecAnd3 % 2 == 0 && kRecXor3 % 2 == 0 && kRecAnd2 % 2 == 1 && kRecXor2 % 2 == 1, "third literal");
 #pragma unroll
-  for (int c = 0; c < C; ++c) {
-    const int h = (C == 1) ? 0 : (pl + c) % C;
-    uint64_t a[2], b[2] = {0, 0}, d[2] = {0, 0}, o[2];
-    ldo<M>(vb, o0, h, a);
-    if constexpr (NF > 1) ldo<M>(vb, o1, h, b);
-    if constexpr (NF > 2) ldo<M>(vb, o2, h, d);
+  for (int c = 0; c < C; c += U) {
+    Chunk<M> a[U], b[U], d[U];
 #pragma unroll
-    for (int v = 0; v < VC; ++v) {
-      if constexpr (B == 0)
-        o[v] = a[v] ^ io;
-      else if constexpr (B == 1)
-        o[v] = ((a[v] ^ ii) & (b[v] ^ ii)) ^ io;
-      else if constexpr (B == 2)
-        o[v] = a[v] ^ b[v] ^ io;
-      else if constexpr (B == 3)
-        o[v] = ((a[v] ^ ii) & (b[v] ^ ii) & (d[v] ^ ii)) ^ io;
-      else
-        o[v] = a[v] ^ b[v] ^ d[v] ^ io;
+    for (int u = 0; u < U; ++u) {
+      a[u] = lds<M>(vb + chunk_at<M>(o0, rot, c + u));
+      b[u] = lds<M>(vb + chunk_at<M>(o1, rot, c + u));
+      if constexpr (kThree) d[u] = lds<M>(vb + chunk_at<M>(o2, rot, c + u));
+      if constexpr (kAny) d[u] = lds_if<M>(vb + chunk_at<M>(o2, rot, c + u), ~kind & 1u);
     }
-    sto<M>(vb, oo, h, o);
-  }
-}
-
-template <int M>
-__device__ __forceinline__ void plain_dispatch(char* vb, const uint2 r, int pl) {
-  // Records are grouped by body on the host, so a warp mostly takes one
-  // path.  A chain of unsigned range tests on the class code, the
-  // three-input AND family first, costs fewer instructions per record than
-  // a switch over the classes.
-  const uint32_t cls = r.y >> 28;
-  if (cls - kPAnd3 < 4u)
-    plain_body<M, 3>(vb, r, pl);
-  else if (cls < kPAnd2)
-    plain_body<M, 0>(vb, r, pl);
-  else if (cls - kPAnd2 < 4u)
-    plain_body<M, 1>(vb, r, pl);
-  else if (cls - kPXor3 < 2u)
-    plain_body<M, 4>(vb, r, pl);
-  else if (cls - kPXor2 < 2u)
-    plain_body<M, 2>(vb, r, pl);  // else kPNop
-}
-
-// ---- wide records (PO drivers, MUX, four inputs): runtime type and masks
-// One gate of a known class (family F, fan-in NF) on all M words of the item:
-// loads of the fanin chunks, the gate function, the store and the PO
-// difference.  F = 0: io ^ AND(in ^ ii) covers AND, NAND, OR, NOR, INV and
-// CLKBUF; F = 1: io ^ XOR(in) covers XOR and XNOR; F = 2: MUX.
-template <int M, int F, int NF>
-__device__ __forceinline__ void gate_body(uint64_t* vals, const uint4 q, uint32_t meta, int pl,
-                                          const uint64_t* good_row, PoAcc<M>& pacc) {
-  constexpr int C = (M >= 2) ? M / 2 : 1;
-  constexpr int VC = (M >= 2) ? 2 : 1;
-  const uint64_t ii = (meta & kRecIi) ? ~0ull : 0ull;
-  const uint64_t io = (meta & kRecIo) ? ~0ull : 0ull;
 #pragma unroll
-  for (int c = 0; c < C; ++c) {
-    const int h = (pl + c) % C;
-    uint64_t i0[2], i1[2] = {0, 0}, i2[2] = {0, 0}, i3[2] = {0, 0};
-    lds_chunk<M>(vals, q.x & 0xFFFFu, h, i0);
-    if constexpr (NF > 1) lds_chunk<M>(vals, q.x >> 16, h, i1);
-    if constexpr (NF > 2) lds_chunk<M>(vals, q.y & 0xFFFFu, h, i2);
-    if constexpr (NF > 3) lds_chunk<M>(vals, q.y >> 16, h, i3);
-    uint64_t r[2];
+    for (int u = 0; u < U; ++u) {
 #pragma unroll
-    for (int v = 0; v < VC; ++v) {
-      uint64_t x;
-      if constexpr (F == 0) {
-        x = i0[v] ^ ii;
-        if constexpr (NF > 1) x &= i1[v] ^ ii;
-        if constexpr (NF > 2) x &= i2[v] ^ ii;
-        if constexpr (NF > 3) x &= i3[v] ^ ii;
-        x ^= io;
-      } else if constexpr (F == 1) {
-        x = i0[v];
-        if constexpr (NF > 1) x ^= i1[v];
-        if constexpr (NF > 2) x ^= i2[v];
-        if constexpr (NF > 3) x ^= i3[v];
-        x ^= io;
-      } else {
-        // (s & b) | (a & !s) with a logical not (fsim/simulation.cpp:1056)
-        x = (i2[v] & i1[v]) | (i0[v] & (uint64_t)(i2[v] == 0));
+      for (int r = 0; r < R; ++r) {
+        uint32_t x = a[u].r[r];
+        if constexpr (kAny) {
+          x = and_or_xor(and_or_xor(x ^ i0, b[u].r[r] ^ i1, kx), d[u].r[r] ^ i2, kx) ^ io;
+        } else if constexpr (KIND == kRecXor2) {
+          x = x ^ b[u].r[r] ^ io;
+        } else if constexpr (KIND == kRecXor3) {
+          x = x ^ b[u].r[r] ^ d[u].r[r];
+          x ^= io;
+        } else {
+          x = and_inv(b[u].r[r], i1, x ^ i0);
+          if constexpr (kThree) x = and_inv(d[u].r[r], i2, x);
+          x ^= io;
+        }
+        a[u].r[r] = x;
       }
-      r[v] = x;
-    }
-    if (meta & kRecHasSlot) sts_chunk<M>(vals, q.z & 0xFFFFu, h, r);
-    if (meta & kRecPo) {
-#pragma unroll
-      for (int v = 0; v < VC; ++v) pacc[c][v] |= r[v] ^ good_row[VC * h + v];
+      sts<M>(vb + chunk_at<M>(oo, rot, c + u), a[u]);
     }
   }
 }
 
-// Any other class (rare combinations): word-by-word generic evaluation.
+// (s & b) | (a & !s) with a logical not of the whole 64-bit select word
+// (fsim/simulation.cpp:1056).
 template <int M>
-__device__ __forceinline__ void gate_generic(uint64_t* vals, const uint4 q, uint32_t meta, int pl,
-                                             const uint64_t* good_row, PoAcc<M>& pacc) {
+__device__ __forceinline__ void mux_eval(uint32_t vb, uint32_t rot, const RecWords<M> q) {
+  constexpr int C = (M >= 2) ? M / 2 : 1;
+  const uint32_t o0 = slot_off<M>(q, 0), o1 = slot_off<M>(q, 1), o2 = slot_off<M>(q, 2), oo = slot_off<M>(q, 3);
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    Chunk<M> a = lds<M>(vb + chunk_at<M>(o0, rot, c));
+    const Chunk<M> b = lds<M>(vb + chunk_at<M>(o1, rot, c)), s = lds<M>(vb + chunk_at<M>(o2, rot, c));
+#pragma unroll
+    for (int r = 0; r < Chunk<M>::R; r += 2) {
+      const uint32_t not_s = (s.r[r] | s.r[r + 1]) == 0u;
+      a.r[r] = (s.r[r] & b.r[r]) | (a.r[r] & not_s);
+      a.r[r + 1] = s.r[r + 1] & b.r[r + 1];
+    }
+    sts<M>(vb + chunk_at<M>(oo, rot, c), a);
+  }
+}
+
+// A wide record: its description d, runtime type.
+template <int M>
+__device__ __forceinline__ void wide_eval(uint32_t vb, const uint4* d) {
   constexpr int C = (M >= 2) ? M / 2 : 1;
   constexpr int VC = (M >= 2) ? 2 : 1;
-  const uint32_t t = meta & kRecTypeMask;
-  const uint32_t nf = ((meta >> kRecNfShift) & 3u) + 1u;
+  const uint4 f = d[0], g = d[1];
+  const uint32_t t = g.y & 15u, nf = (g.y >> 4) & 15u;
+#pragma unroll 1
   for (int c = 0; c < C; ++c) {
-    const int h = (pl + c) % C;
-    uint64_t i0[2], i1[2] = {0, 0}, i2[2] = {0, 0}, i3[2] = {0, 0};
-    lds_chunk<M>(vals, q.x & 0xFFFFu, h, i0);
-    if (nf > 1) lds_chunk<M>(vals, q.x >> 16, h, i1);
-    if (nf > 2) lds_chunk<M>(vals, q.y & 0xFFFFu, h, i2);
-    if (nf > 3) lds_chunk<M>(vals, q.y >> 16, h, i3);
-    uint64_t r[2];
-    for (int v = 0; v < VC; ++v) r[v] = eval_word(t, nf, i0[v], i1[v], i2[v], i3[v]);
-    if (meta & kRecHasSlot) sts_chunk<M>(vals, q.z & 0xFFFFu, h, r);
-    if (meta & kRecPo)
-      for (int v = 0; v < VC; ++v) pacc[c][v] |= r[v] ^ good_row[VC * h + v];
+    const uint32_t vc = vb + 16u * c;
+    Chunk<M> x = lds<M>(vc + 8u * M * f.x);
+    const Chunk<M> i1 = lds_if<M>(vc + 8u * M * f.y, nf > 1), i2 = lds_if<M>(vc + 8u * M * f.z, nf > 2),
+                   i3 = lds_if<M>(vc + 8u * M * f.w, nf > 3);
+#pragma unroll
+    for (int v = 0; v < VC; ++v) {
+      auto word = [&](const Chunk<M>& k) { return (uint64_t)k.r[2 * v] | (uint64_t)k.r[2 * v + 1] << 32; };
+      const uint64_t r = eval_word(t, nf, word(x), word(i1), word(i2), word(i3));
+      x.r[2 * v] = (uint32_t)r;
+      x.r[2 * v + 1] = (uint32_t)(r >> 32);
+    }
+    sts<M>(vc + 8u * M * g.x, x);
   }
 }
 
+// A PO record: the driver's difference from its good words, to the CTA's
+// words in shared memory by one atomic per warp and 32-bit half (registers
+// for them would cost every other record).
 template <int M>
-__device__ __forceinline__ void gate_dispatch(uint64_t* vals, const uint4 q, int pl,
-                                              const uint64_t* good_row, PoAcc<M>& pacc) {
-  const uint32_t meta = q.z >> 16;
-  switch ((meta >> kRecClassShift) & 15u) {  // dense class index from the host (gate_class)
-    case 0: gate_body<M, 0, 1>(vals, q, meta, pl, good_row, pacc); break;
-    case 1: gate_body<M, 0, 2>(vals, q, meta, pl, good_row, pacc); break;
-    case 2: gate_body<M, 0, 3>(vals, q, meta, pl, good_row, pacc); break;
-    case 3: gate_body<M, 0, 4>(vals, q, meta, pl, good_row, pacc); break;
-    case 4: gate_body<M, 1, 2>(vals, q, meta, pl, good_row, pacc); break;
-    case 5: gate_body<M, 1, 3>(vals, q, meta, pl, good_row, pacc); break;
-    case 6: gate_body<M, 1, 4>(vals, q, meta, pl, good_row, pacc); break;
-    case 7: gate_body<M, 2, 3>(vals, q, meta, pl, good_row, pacc); break;
-    default: gate_generic<M>(vals, q, meta, pl, good_row, pacc); break;
+__device__ __forceinline__ void po_eval(uint32_t vb, const RecWords<M> q, const uint64_t* good_w0, uint32_t* acc) {
+  constexpr int C = (M >= 2) ? M / 2 : 1;
+  const unsigned lanes = __activemask();
+  const bool leader = (threadIdx.x & 31u) == (uint32_t)(__ffs(lanes) - 1);
+  const uint32_t o = slot_off<M>(q, 3);
+  const uint64_t* good_row = good_w0 + (uint64_t)q.x * 32;
+#pragma unroll
+  for (int c = 0; c < C; ++c) {  // every lane the same chunk: the lanes' words line up
+    Chunk<M> x = lds<M>(vb + chunk_at<M>(o, 0u, c)), g;
+    if constexpr (M == 1) {
+      const uint2 w = *reinterpret_cast<const uint2*>(good_row);
+      g.r[0] = w.x, g.r[1] = w.y;
+    } else {
+      const uint4 w = *reinterpret_cast<const uint4*>(good_row + 2 * c);
+      g.r[0] = w.x, g.r[1] = w.y, g.r[2] = w.z, g.r[3] = w.w;
+    }
+#pragma unroll
+    for (int r = 0; r < Chunk<M>::R; ++r) {
+      const uint32_t diff = __reduce_or_sync(lanes, x.r[r] ^ g.r[r]);
+      if (leader && diff) atomicOr(acc + 4 * c + r, diff);
+    }
   }
 }
 
@@ -404,107 +416,82 @@ __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
 }
 
-// M words per item, one thread per gate holding all M words.  Slots are
+template <int M>
+__device__ __forceinline__ void record_eval(uint32_t vb, uint32_t rot, bool split, const RecWords<M> q,
+                                            const uint4* blob, const uint64_t* good_w0, uint32_t* acc) {
+  const uint32_t kind = (q.y >> kRecKindShift) & 7u;
+  if (kind >= kRecMux) {
+    if (kind == kRecMux)
+      mux_eval<M>(vb, rot, q);
+    else if (kind == kRecPo)
+      po_eval<M>(vb, q, good_w0, acc);
+    else
+      wide_eval<M>(vb, blob + q.x);
+  } else if (kind == kRecNop) {  // padding
+  } else if (!split) {
+    cluster_eval<M, kRecNop>(vb, rot, q);
+  } else if (kind == kRecAnd3) {  // records are in kind order, so a warp mostly takes one path
+    cluster_eval<M, kRecAnd3>(vb, rot, q);
+  } else if (kind == kRecAnd2) {
+    cluster_eval<M, kRecAnd2>(vb, rot, q);
+  } else if (kind == kRecXor3) {
+    cluster_eval<M, kRecXor3>(vb, rot, q);
+  } else {
+    cluster_eval<M, kRecXor2>(vb, rot, q);
+  }
+}
+
+// A CTA of one warp needs no barrier between levels, only the warp's order.
+__device__ __forceinline__ void cta_sync() {
+  if (blockDim.x == 32)
+    __syncwarp();
+  else
+    __syncthreads();
+}
+
+// M words per item, one thread per record holding all M words.  Slots are
 // M*8 bytes; a thread reads a slot as C = M/2 16-byte chunks (one 8-byte word
 // for M = 1).  The host orders each level in groups of G = 16/M consecutive
-// positions whose slots have distinct residues mod G (for every fanin and the
-// output).  Within a phase of 8 lanes (16 for M = 1), lane l takes position
-// (l % C) * G + l / C and reads chunk (l + i) % C at step i, so the 8 chunks a
-// phase touches lie in 8 different bank quads: the loads and stores of a
-// sweep are free of bank conflicts wherever the host found such groups.
+// positions whose slots have distinct residues mod G (for every literal and
+// the output), and packs them so that within a phase of 8 lanes (16 for M =
+// 1) lane l takes position (l % C) * G + l / C; with chunk (l % C) ^ i at step
+// i the 8 chunks a phase touches lie in 8 different bank quads: the loads
+// and stores of a sweep are free of bank conflicts wherever the host found
+// such groups.
 //
-// Each level's block of gate records is staged into one of two shared-memory
-// buffers by a TMA bulk copy issued two levels ahead (one elected thread,
-// mbarrier completion, waits bounded in time); a block larger than a buffer
-// reads the rest from global memory.
-struct SweepCta {
-  uint64_t* vals;     // [max_live][M]
-  uint4* recbuf;      // [2][rec_buf]
-  uint64_t* bars;     // [3] mbarriers: two staging buffers, one for the wait test
-  unsigned long long* acc;
-  uint32_t rec_buf;   // 16-byte units per staging buffer
-  uint32_t uses;      // levels staged and consumed so far: use u goes through
-                      // buffer u & 1 and completes that barrier's phase u >> 1
-  uint64_t wait_ns;   // limit of one wait
-  uint32_t test_stall;
-};
-
-template <int M>
-__device__ __forceinline__ void sweep_cta_init(SweepCta& k, uint64_t* vals, uint32_t vals_bytes,
-                                               uint32_t rec_buf, uint64_t* bars, unsigned long long* acc,
-                                               uint64_t wait_ns, uint32_t test_stall) {
-  k.vals = vals;
-  k.recbuf = reinterpret_cast<uint4*>(reinterpret_cast<char*>(vals) + vals_bytes);
-  k.bars = bars;
-  k.acc = acc;
-  k.rec_buf = rec_buf;
-  k.uses = 0;
-  k.wait_ns = wait_ns;
-  k.test_stall = test_stall;
-  if (threadIdx.x == 0) {
-    mbar_init(&bars[0], 1);
-    mbar_init(&bars[1], 1);
-    mbar_init(&bars[2], 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-}
-
-// Thread 0 only: the block of level L into buffer b.
-__device__ __forceinline__ void sweep_stage(SweepCta& k, const SweepView& v, uint32_t L, int b) {
-  const uint4 d = v.lvl[L];
-  const uint32_t n = min(d.w, k.rec_buf);
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  bulk_load(k.recbuf + (size_t)b * k.rec_buf, v.blob + d.x, n * 16u, &k.bars[b]);
-}
-
-// Error path: thread 0 waits (bounded) for the n copies still in flight
-// into this CTA's shared memory (uses u, u + 1, ...), so none lands after
-// the CTA has exited.  A copy already waited for passes at once.
-__device__ __forceinline__ void sweep_drain(SweepCta& k, uint32_t u, uint32_t n) {
-  if (threadIdx.x == 0)
-    for (uint32_t i = 0; i < n; ++i) mbar_wait(&k.bars[(u + i) & 1u], ((u + i) >> 1) & 1u, k.wait_ns);
-  __syncthreads();
-}
-
+// A thread reads its records straight from global memory (L1 / L2), kPrefetch
+// rounds ahead: the stream is padded per level to rounds of one record per
+// thread, so the next address is one addition away and a level's end is a
+// bit of its last round's records.
+//
 // One item: the levels above the injection element for M words starting at
 // word w0 of the tile; writes the OR of PO differences to out_row[w0..w0+M).
-// Returns false (on every thread) if a bounded wait gave up.
 template <int M>
-__device__ __forceinline__ bool sweep_item(SweepCta& k, const SweepView& v, const InjRec inj, uint32_t w0,
-                                           uint64_t* out_row) {
+__device__ __forceinline__ void sweep_item(uint64_t* vals, unsigned long long* acc, const SweepView& v,
+                                           const InjRec inj, uint32_t w0, uint64_t* out_row) {
   constexpr int C = (M >= 2) ? M / 2 : 1;   // chunks per slot
-  constexpr int VC = (M >= 2) ? 2 : 1;      // words per chunk
-  constexpr int G = 16 / M;                 // residue group size
   constexpr int PH = (M == 1) ? 16 : 8;     // lanes per shared-memory phase
   const int tid = threadIdx.x, nth = blockDim.x;
   const int pl = tid & (PH - 1);
-  const uint32_t my_off = (uint32_t)((tid & ~(PH - 1)) + ((M >= 2) ? (pl % C) * G + pl / C : pl));
-  const uint32_t Lmax = v.max_gate_level;
-  uint64_t* vals = k.vals;
-  char* vb = reinterpret_cast<char*>(vals);
-  const uint32_t x = inj.elem;
-  const uint32_t L0 = v.level[x] + 1;
-  if (tid < M) k.acc[tid] = 0ull;
-  const uint32_t n_out = L0 > Lmax ? 0u : (L0 + 1 <= Lmax ? 2u : 1u);  // copies issued ahead
-  if (tid == 0) {
-    if (n_out > 0) sweep_stage(k, v, L0, (int)(k.uses & 1u));
-    if (n_out > 1) sweep_stage(k, v, L0 + 1, (int)((k.uses + 1) & 1u));
+  const uint32_t vb = smem_u32(vals), rot = 16u * ((uint32_t)pl % C);
+  const uint32_t x = inj.stored;
+  const uint4 lv = v.lvl[inj.level];
+  if (tid < M) {
+    acc[tid] = 0ull;
+    if (inj.mode & kInjReachesPo) acc[tid] = inj_value(v, inj, w0 + tid) ^ v.good[(uint64_t)x * 32 + w0 + tid];
   }
-  bool ok = true;
-  if (k.test_stall) {
-    // test hook: wait on a barrier that no copy completes, so the wait runs
-    // out and the item takes the error path
-    k.test_stall = 0;
-    if (tid == 0) ok = mbar_wait(&k.bars[2], 0, k.wait_ns);
-  }
-  if (L0 <= Lmax) {
+  const uint32_t first = inj.level <= v.max_gate_level ? lv.x : v.stream_recs;
+  if (first < v.stream_recs) {
+    const RecWords<M>* rp = reinterpret_cast<const RecWords<M>*>(v.blob) + first + tid;
+    RecWords<M> q[kPrefetch];
+#pragma unroll
+    for (int j = 0; j < (int)kPrefetch; ++j, rp += nth) q[j] = *rp;
     // Values live at the start level come from the good machine (copied
     // asynchronously, four list entries in flight per thread), except the
     // injection element itself.
-    const uint32_t i1 = v.li_off[L0 + 1];
+    const uint32_t i1 = lv.z;
     const uint2* li = reinterpret_cast<const uint2*>(v.li);
-    for (uint32_t i = v.li_off[L0] + tid; i < i1; i += 4 * nth) {
+    for (uint32_t i = lv.y + tid; i < i1; i += 4 * nth) {
       uint2 es[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) es[j] = (i + j * nth < i1) ? li[i + j * nth] : make_uint2(0xFFFFFFFFu, 0);
@@ -513,7 +500,7 @@ __device__ __forceinline__ bool sweep_item(SweepCta& k, const SweepView& v, cons
         if (es[j].x == 0xFFFFFFFFu) continue;
         uint64_t* dst = vals + (size_t)es[j].y * M;
         if (es[j].x == x) {
-#pragma unroll
+#pragma unroll 1
           for (int m = 0; m < M; ++m) dst[m] = inj_value(v, inj, w0 + m);
         } else {
           const uint64_t* src = v.good + (uint64_t)es[j].x * 32 + w0;
@@ -526,97 +513,95 @@ __device__ __forceinline__ bool sweep_item(SweepCta& k, const SweepView& v, cons
         }
       }
     }
+    // A flip of an alias goes to the injection slot, which the fix entries
+    // of its list read after their levels.
+    const uint4* fx = nullptr;
+    uint32_t fix_at = 0xFFFFFFFFu;
+    if (inj.fix) {
+      fx = v.blob + v.fix0 + 2 * (size_t)(inj.fix - 1);
+      fix_at = fx[1].x;
+      if (tid < M)
+        vals[(size_t)v.inj_slot * M + tid] =
+            inj_value(v, inj, w0 + tid) ^ ((inj.mode & kInjAliasInv) ? ~0ull : 0ull);
+    }
     cp_async_wait_all();
-  }
-  if (tid < M && (inj.mode & kInjReachesPo))
-    k.acc[tid] = inj_value(v, inj, w0 + tid) ^ v.good[(uint64_t)x * 32 + w0 + tid];
-  if (__syncthreads_or(!ok)) {
-    sweep_drain(k, k.uses, n_out);
-    return false;
-  }
-  PoAcc<M> pacc;
+    cta_sync();
+    const uint64_t* good_w0 = v.good + w0;
+    uint32_t* acc32 = reinterpret_cast<uint32_t*>(acc);
+    auto round = [&](const RecWords<M> q, uint32_t at) {
+      record_eval<M>(vb, rot, v.split, q, v.blob, good_w0, acc32);
+      if (q.y & kRecEnd) {
+        cta_sync();
+        if (at == fix_at) {
+          const uint32_t n = fx[1].y;
+          for (uint32_t i = tid; i < n; i += nth)
+            record_eval<M>(vb, rot, v.split, *reinterpret_cast<const RecWords<M>*>(fx + 2 * i), v.blob, good_w0,
+                           acc32);
+          fx += 2 * n;
+          fix_at = fx[1].x;
+          cta_sync();
+        }
+      }
+    };
+    // kPrefetch rounds a turn, so that a record's registers are loaded again
+    // only after its evaluation and nothing waits for a load early.
+    for (uint32_t at = first;;) {
 #pragma unroll
-  for (int c = 0; c < C; ++c)
-#pragma unroll
-    for (int q = 0; q < VC; ++q) pacc[c][q] = 0ull;
-  for (uint32_t L = L0; L <= Lmax; ++L) {
-    const uint32_t u = k.uses;
-    const int b = (int)(u & 1u);
-    const uint4 desc = v.lvl[L];  // issued before the wait, used after it
-    ok = mbar_wait(&k.bars[b], (u >> 1) & 1u, k.wait_ns);
-    if (ok) {
-      const char* sb = reinterpret_cast<const char*>(k.recbuf + (size_t)b * k.rec_buf);
-      const char* gb = reinterpret_cast<const char*>(v.blob + desc.x);
-      const uint32_t staged = min(desc.w, k.rec_buf) * 16u;
-      const uint32_t np = desc.y, n = desc.y + desc.z;
-      const uint32_t wide0 = (np + 1) / 2 * 16;
-      // Plain records from the staging buffer, then the rest of the plain
-      // part from global memory, then the wide records: three loops
-      // without a per-record choice of source cost fewer instructions than
-      // one loop that picks the source and the record kind per position.
-      const uint32_t ns = min(np, staged / 8u);
-      uint32_t p = my_off;
-      for (; p < ns; p += nth) plain_dispatch<M>(vb, *reinterpret_cast<const uint2*>(sb + (size_t)p * 8), pl);
-      for (; p < np; p += nth) plain_dispatch<M>(vb, *reinterpret_cast<const uint2*>(gb + (size_t)p * 8), pl);
-      for (; p < n; p += nth) {
-        const uint32_t byte = wide0 + (p - np) * 16;
-        uint4 q;
-        if (byte < staged)
-          q = *reinterpret_cast<const uint4*>(sb + byte);
-        else
-          q = *reinterpret_cast<const uint4*>(gb + byte);
-        gate_dispatch<M>(vals, q, pl, v.good + (uint64_t)q.w * 32 + w0, pacc);
+      for (int j = 0; j < (int)kPrefetch; ++j) {
+        round(q[j], at);
+        q[j] = *rp;
+        rp += nth;
+        at += nth;
+        if (at >= v.stream_recs) goto done;
       }
     }
-    if (__syncthreads_or(!ok)) {
-      sweep_drain(k, u, L + 1 <= Lmax ? 2u : 1u);
-      return false;
-    }
-    k.uses = u + 1;
-    if (L + 2 <= Lmax && tid == 0) sweep_stage(k, v, L + 2, b);
+  done:;
   }
-#pragma unroll
-  for (int c = 0; c < C; ++c) {
-    const int h = (pl + c) % C;
-#pragma unroll
-    for (int q = 0; q < VC; ++q)
-      if (pacc[c][q]) atomicOr(&k.acc[VC * h + q], (unsigned long long)pacc[c][q]);
-  }
-  __syncthreads();
-  if (tid < M) out_row[w0 + tid] = k.acc[tid];
-  return true;
+  cta_sync();
+  if (tid < M) out_row[w0 + tid] = acc[tid];
 }
 
-// Register caps: the CTA sizes up to sweep_max_threads(M) fit the register
-// file, and 56 at M = 2 lets three 384-thread CTAs share an SM.
+// Test hook: a wait on a barrier that nothing completes runs out and the
+// launch reports an error.
+__device__ __forceinline__ bool sweep_wait_test(uint64_t* bar, uint64_t wait_ns, int* err) {
+  if (threadIdx.x == 0) {
+    mbar_init(bar, 1);
+    if (!mbar_wait(bar, 0, wait_ns)) atomicExch(err, 1);
+  }
+  return false;
+}
+
+// Register caps: 1,024 threads an SM at up to 4 words per item.
 template <int M>
-__global__ void __maxnreg__(M >= 8 ? 120 : (M >= 4 ? 72 : (M >= 2 ? 56 : 64))) k_sweep(SweepArgs a) {
-  extern __shared__ __align__(16) uint64_t vals[];  // [max_live][M] | recbuf[2][rec_buf]
+__global__ void __maxnreg__(64) k_sweep(SweepArgs a) {
+  extern __shared__ __align__(128) uint64_t vals[];  // [max_live][M]
   __shared__ unsigned long long acc[M];
-  __shared__ __align__(8) uint64_t bars[3];
-  __shared__ int s_item;
-  SweepCta k;
-  sweep_cta_init<M>(k, vals, a.vals_bytes, a.rec_buf, bars, acc, a.wait_ns,
-                    (a.wait_test && blockIdx.x == 0) ? 1u : 0u);
-  const SweepView v{a.blob, a.lvl, a.level, a.li_off, a.li, a.fi_off, a.fi_idx, a.type, a.good,
-                    a.max_gate_level};
+  __shared__ __align__(8) uint64_t bar;
+  __shared__ uint32_t s_item;
+  if (a.wait_test && blockIdx.x == 0) {
+    sweep_wait_test(&bar, a.wait_ns, a.err);
+    return;
+  }
+  const SweepView v{a.blob, a.lvl, a.level, a.li, a.fi_off, a.fi_idx, a.type, a.good,
+                    a.max_gate_level, a.stream_recs, a.fix0, a.inj_slot, a.split};
   // Subtiles that hold pattern words: the last tile of a block is rarely full
   // (16 words of 32 for 1,000 patterns), and the tracing masks the others.
   const uint32_t subtiles = (a.n_words + M - 1) / M;
   const uint32_t n_items = a.n_list * subtiles;
+  // The next item's number is asked for while the current one runs.
+  uint32_t next = blockIdx.x;
   for (;;) {
-    if (threadIdx.x == 0) s_item = atomicAdd(a.queue, 1);
-    __syncthreads();
-    const uint32_t item = (uint32_t)s_item;
-    __syncthreads();  // s_item is rewritten for the next item only after all have read it
+    if (threadIdx.x == 0) {
+      s_item = next;
+      next = gridDim.x + (uint32_t)atomicAdd(a.queue, 1);
+    }
+    cta_sync();
+    const uint32_t item = s_item;
     if (item >= n_items) return;
     const uint32_t li = item / subtiles;
     const uint32_t w0 = (item % subtiles) * M;
     const uint32_t si = a.list ? a.list[li] : li;
-    if (!sweep_item<M>(k, v, a.inj[si], w0, a.out + (uint64_t)si * 32)) {
-      if (threadIdx.x == 0) atomicExch(a.err, 1);
-      return;
-    }
+    sweep_item<M>(vals, acc, v, a.inj[si], w0, a.out + (uint64_t)si * 32);
   }
 }
 
@@ -627,39 +612,36 @@ __global__ void __maxnreg__(M >= 8 ? 120 : (M >= 4 ? 72 : (M >= 2 ? 56 : 64))) k
 // circuit fields come from the kernel parameters: the compiler keeps the
 // pointers in uniform registers, as for k_sweep.
 template <int M>
-__global__ void __maxnreg__(M >= 8 ? 96 : (M >= 4 ? 72 : (M >= 2 ? 56 : 64)))
-    k_sweep_batch(const __grid_constant__ BatchSweepParams p) {
-  extern __shared__ __align__(16) uint64_t vals[];
+__global__ void __maxnreg__(64) k_sweep_batch(const __grid_constant__ BatchSweepParams p) {
+  extern __shared__ __align__(128) uint64_t vals[];
   __shared__ unsigned long long acc[M];
-  __shared__ __align__(8) uint64_t bars[3];
   __shared__ uint32_t s_item;
-  SweepCta k;
-  sweep_cta_init<M>(k, vals, p.vals_bytes, p.rec_buf, bars, acc, p.wait_ns, 0u);
   constexpr uint32_t subtiles = kTileWords / M;
   for (uint32_t ci = 0; ci < p.n_circ; ++ci) {
     const SweepCirc& c = p.c[ci];
     const uint32_t per_tile = c.n_sweeps * subtiles;
+    // The next item's number is asked for while the current one runs.
+    unsigned long long next = threadIdx.x == 0 ? atomicAdd(p.queue + ci, 1ull) : 0ull;
     for (;;) {
       if (threadIdx.x == 0) {
-        const unsigned long long it = atomicAdd(p.queue + ci, 1ull);
-        s_item = it < c.n_items ? (uint32_t)it : 0xFFFFFFFFu;
+        s_item = next < c.n_items ? (uint32_t)next : 0xFFFFFFFFu;
+        if (next < c.n_items) next = atomicAdd(p.queue + ci, 1ull);
       }
-      __syncthreads();
+      cta_sync();
       const uint32_t item = s_item;
-      __syncthreads();  // s_item is rewritten only after every thread read it
-      if (item == 0xFFFFFFFFu) break;
+      if (item == 0xFFFFFFFFu) {
+        cta_sync();  // s_item is written for the next circuit only after all have read it
+        break;
+      }
       // The last tile has items only for the subtiles that hold pattern words.
       const uint32_t tile = min(item / per_tile, c.tiles - 1);
       const uint32_t rem = item - tile * per_tile;
       const uint32_t sub = tile == c.tiles - 1 ? c.last_sub : subtiles;
       const uint32_t si = rem / sub;
       const uint32_t w0 = (rem % sub) * M;
-      const SweepView v{c.blob, c.lvl, c.level, c.li_off, c.li, c.fi_off, c.fi_idx, c.type,
-                        c.good + (uint64_t)tile * c.N * 32, c.max_gate_level};
-      if (!sweep_item<M>(k, v, c.inj[si], w0, c.out + ((uint64_t)tile * c.n_sweeps + si) * 32)) {
-        if (threadIdx.x == 0) atomicExch(p.err, 1);
-        return;
-      }
+      const SweepView v{c.blob, c.lvl, c.level, c.li, c.fi_off, c.fi_idx, c.type,
+                        c.good + (uint64_t)tile * c.N * 32, c.max_gate_level, c.stream_recs, c.fix0, c.inj_slot, c.split};
+      sweep_item<M>(vals, acc, v, c.inj[si], w0, c.out + ((uint64_t)tile * c.n_sweeps + si) * 32);
     }
   }
 }
@@ -692,7 +674,7 @@ __global__ void __launch_bounds__(256) k_sweep_wide(SweepWideArgs a) {
     const uint32_t w0 = (item % subtiles) * M;
     const uint32_t si = a.list ? a.list[li] : li;
     const InjRec inj = a.inj[si];
-    const uint32_t x = inj.elem;
+    const uint32_t x = inj.stored;
     const uint32_t L0 = a.level[x] + 1;
     const uint32_t lo0 = L0 <= a.max_gate_level ? a.level_off[L0] : 0;
     if (tid < M) {

@@ -22,10 +22,9 @@ struct GoodArgs {
 };
 
 struct SweepArgs {
-  const uint4* blob;       // level blocks of gate records (see fsimb_plan.h)
-  const uint4* lvl;        // LevelDesc per level
-  const uint32_t* level;   // element -> level
-  const uint32_t* li_off;
+  const uint4* blob;       // record stream for the launch's CTA size (see fsimb_plan.h)
+  const uint4* lvl;        // per level: its first record in the stream, its range in li
+  const uint32_t* level;   // element -> level, or kFolded | consumer
   const uint32_t* li;      // (element, slot) pairs
   const uint32_t* fi_off;
   const uint32_t* fi_idx;
@@ -39,11 +38,12 @@ struct SweepArgs {
   const uint64_t* good;    // this tile: [N][32]
   uint64_t* out;           // this tile: [n_sweeps][32] OR of PO differences
   int* queue;              // work counter for this launch
-  uint32_t vals_bytes;     // shared memory for values (multiple of 16)
-  uint32_t rec_buf;        // 16-byte units per staging buffer (2 buffers follow the values)
+  uint32_t stream_recs;    // records of the stream's rounds
+  uint32_t fix0, inj_slot; // fix entries in blob; the injection slot
+  uint32_t split;          // levels are ordered by record kind
   int* err;                // set to 1 if a bounded wait gave up
-  uint64_t wait_ns;        // time limit of one wait for a record copy
-  uint32_t wait_test;      // 1: the first CTA waits on a barrier no copy completes (test hook)
+  uint64_t wait_ns;        // time limit of that wait
+  uint32_t wait_test;      // 1: the first CTA waits on a barrier nothing completes (test hook)
 };
 
 // Sweep of circuits whose live values do not fit in shared memory.
@@ -127,7 +127,6 @@ struct BatchCirc {
   const uint4* blob;
   const uint4* lvl;
   const uint32_t* level;
-  const uint32_t* li_off;
   const uint32_t* li;
   const uint32_t* fi_off;
   const uint32_t* fi_idx;
@@ -149,7 +148,8 @@ struct BatchCirc {
   uint32_t N, n_pi, W, tiles;
   uint32_t n_sweeps, n_stem_sweeps, n_roots, n_exact;
   uint32_t max_gate_level, n_levels;
-  uint32_t n_slots, pad;         // sensitivity slots per tile
+  uint32_t n_slots;              // sensitivity slots per tile
+  uint32_t stream_recs, fix0, inj_slot, split;  // see SweepArgs
 };
 
 // What the batched sweep reads of one circuit.  A launch carries these in
@@ -158,7 +158,6 @@ struct SweepCirc {
   const uint4* blob;
   const uint4* lvl;
   const uint32_t* level;
-  const uint32_t* li_off;
   const uint32_t* li;
   const uint32_t* fi_off;
   const uint32_t* fi_idx;
@@ -169,17 +168,15 @@ struct SweepCirc {
   uint32_t N, n_sweeps, max_gate_level;
   uint32_t n_items;      // (tile, sweep, subtile), tile-major: n_sweeps * (32 / M) per tile,
                          // n_sweeps * last_sub for the last one
-  uint32_t tiles, last_sub;
+  uint32_t tiles, last_sub, stream_recs, fix0, inj_slot, split;
 };
 
-constexpr int kSweepCircsPerLaunch = 280;
+constexpr int kSweepCircsPerLaunch = 240;
 
 struct BatchSweepParams {
   SweepCirc c[kSweepCircsPerLaunch];
   unsigned long long* queue;  // [n_circ] work counters, zero before the launch
-  int* err;
-  uint64_t wait_ns;
-  uint32_t n_circ, vals_bytes, rec_buf;
+  uint32_t n_circ;
 };
 static_assert(sizeof(BatchSweepParams) <= 32000, "kernel parameters are limited to 32,764 bytes");
 
@@ -218,8 +215,7 @@ cudaError_t sweep_occupancy(int M, int threads, size_t smem, int* blocks_per_sm)
 // M in {1, 2}; 256 threads per CTA.
 cudaError_t launch_sweep_wide(int M, int blocks, const SweepWideArgs& a, cudaStream_t s);
 cudaError_t sweep_wide_occupancy(int M, int* blocks_per_sm);
-// Time limit of one wait for a record copy, and the shorter one of the wait test.
-constexpr uint64_t kWaitLimitNs = 2000000000ull;
+// Time limit of the wait test's wait.
 constexpr uint64_t kWaitTestNs = 20000000ull;
 void launch_ffr(const FfrArgs& a, cudaStream_t s);
 void launch_exact(const ExactArgs& a, cudaStream_t s);

@@ -3,8 +3,6 @@
 
 #include <algorithm>
 #include <array>
-#include <cstring>
-#include <functional>
 
 namespace fsimb {
 
@@ -21,41 +19,161 @@ uint32_t eff_fanin(const Netlist& nl, uint32_t e) {
 
 }  // namespace
 
-uint32_t gate_class(uint8_t type, uint32_t nf) {
-  const uint32_t fam = gate_family(type);
-  if (fam == 0 && nf >= 1 && nf <= 4) return nf - 1;
-  if (fam == 1 && nf >= 2 && nf <= 4) return 4 + nf - 2;
-  if (fam == 2 && nf == 3) return 7;
-  return kClassGeneric;
-}
-
-uint32_t plain_class(uint8_t t, uint32_t nf) {
-  if (nf == 1) {
-    switch (t) {
-      case G_AND: case G_OR: case G_XOR: case G_CLKBUF: return kPBuf;
-      case G_INV: case G_NAND: case G_NOR: case G_XNOR: return kPInv;
-      default: return kPlainClasses;
-    }
-  }
-  if (nf != 2 && nf != 3) return kPlainClasses;
-  const uint32_t base = nf == 2 ? kPAnd2 : kPAnd3;
-  switch (t) {
-    case G_AND: return base + 0;
-    case G_NAND: return base + 1;
-    case G_OR: return base + 2;
-    case G_NOR: return base + 3;
-    case G_XOR: return base + 4;
-    case G_XNOR: return base + 5;
-    default: return kPlainClasses;
-  }
-}
-
 uint32_t gate_family(uint8_t t) {
   switch (t) {
     case G_XOR:
     case G_XNOR: return 1;
     case G_MUX: return 2;
     default: return 0;
+  }
+}
+
+namespace {
+
+constexpr uint32_t kInvLit = 0x80000000u;
+
+// Adds the literals of `t`, inverted by `inv`, to cluster c.  False if the
+// result is not one AND or XOR of three literals.
+bool add_term(Cluster& c, const Cluster& t, uint32_t inv) {
+  const uint32_t tinv = t.inv ^ inv;
+  if (c.n + t.n > 3) return false;
+  if (t.n == 1) {  // a literal (its inversion is in the literal)
+    if (c.is_xor) {
+      c.lit[c.n++] = t.lit[0] & ~kInvLit;
+      c.inv ^= (uint8_t)(tinv ^ (t.lit[0] >> 31));
+    } else {
+      c.lit[c.n++] = t.lit[0] ^ (tinv ? kInvLit : 0u);
+    }
+    return true;
+  }
+  if (t.is_xor != c.is_xor || (!c.is_xor && tinv)) return false;
+  for (uint32_t k = 0; k < t.n; ++k) c.lit[c.n++] = t.lit[k];
+  if (c.is_xor) c.inv ^= (uint8_t)tinv;
+  return true;
+}
+
+}  // namespace
+
+void build_sweep_net(const Netlist& nl, const Plan& P, SweepNet& net) {
+  const uint32_t N = nl.N;
+  net = SweepNet();
+  // A PO is reached: the element is a PO, or a live element reads it.
+  net.live.assign(N, 0);
+  for (int64_t e = (int64_t)N - 1; e >= 0; --e) {
+    if (nl.type[e] == G_PO) net.live[e] = 1;
+    if (!net.live[e]) continue;
+    const uint32_t nf = eff_fanin(nl, (uint32_t)e);
+    for (uint32_t k = 0; k < nf; ++k) net.live[nl.fi_idx[nl.fi_off[e] + k]] = 1;
+  }
+  // Clusters of the gates that have one, bottom up.
+  std::vector<Cluster> form(N, Cluster{});  // n == 0: no cluster form
+  net.lev_up = nl.level;
+  const uint32_t g1 = P.n_pi + P.n_gates;
+  for (uint32_t e = P.n_pi; e < g1; ++e) {
+    const uint32_t nf = eff_fanin(nl, e);
+    const uint8_t t = nl.type[e];
+    if (!net.live[e] || t == G_MUX || nf < 1 || nf > 3) continue;
+    const uint32_t ii = nf > 1 && (t == G_OR || t == G_NOR);
+    const bool inverts = t == G_INV || t == G_NAND || t == G_NOR || t == G_XNOR;
+    const uint32_t io = inverts != (bool)ii;  // OR and NOR are ANDs of inverted inputs
+    const uint32_t* in = &nl.fi_idx[nl.fi_off[e]];
+    uint32_t may = 0;  // inputs that can be folded in
+    for (uint32_t k = 0; k < nf; ++k)
+      if (form[in[k]].n && nl.fo_off[in[k] + 1] - nl.fo_off[in[k]] == 1) may |= 1u << k;
+    // The subset of them that folds the most gates; of those one with the
+    // fewest literals.
+    Cluster best{};
+    int best_score = -1;
+    uint32_t best_set = 0;
+    for (uint32_t set = may;; set = (set - 1) & may) {
+      Cluster c{};
+      c.is_xor = gate_family(t) == 1 && nf > 1;
+      c.inv = (uint8_t)io;
+      bool ok = true;
+      for (uint32_t k = 0; k < nf && ok; ++k) {
+        const Cluster leaf{{in[k], 0, 0}, {0, 0, 0}, 1, 0, 0};
+        if (nf == 1 && set) {  // BUF / INV of a folded gate: that gate's form
+          c = form[in[0]];
+          c.inv ^= (uint8_t)io;
+        } else {
+          ok = add_term(c, (set >> k) & 1u ? form[in[k]] : leaf, ii);
+        }
+      }
+      const int score = __builtin_popcount(set) * 4 + 3 - c.n;
+      if (ok && score > best_score) {
+        best = c;
+        best_score = score;
+        best_set = set;
+      }
+      if (set == 0) break;
+    }
+    if (best.n == 1 && best.inv) {  // one literal takes the inversion
+      best.lit[0] ^= kInvLit;
+      best.inv = 0;
+    }
+    form[e] = best;
+    for (uint32_t k = 0; k < nf; ++k)
+      if ((best_set >> k) & 1u) net.lev_up[in[k]] = kFolded | e;
+  }
+  // Aliases: one literal, not folded away, and read by clusters only (every
+  // record a reader is folded into is a cluster's).
+  net.alias.assign(N, kNoSlot);
+  net.alias_of.assign(N, kNoSlot);
+  for (uint32_t e = P.n_pi; e < g1; ++e) {
+    if (form[e].n != 1 || (net.lev_up[e] & kFolded)) continue;
+    bool clusters_only = true;
+    for (uint32_t k = nl.fo_off[e]; k < nl.fo_off[e + 1] && clusters_only; ++k) {
+      const uint32_t c = nl.fo_idx[k];
+      clusters_only = form[c].n || !net.live[c] || nl.fo_pin[k] >= eff_fanin(nl, c);
+    }
+    if (!clusters_only) continue;
+    const uint32_t x = form[e].lit[0] & ~kInvLit, src = net.alias[x];
+    net.alias[e] = (src == kNoSlot ? x : src) ^ (form[e].lit[0] & kInvLit);
+    net.alias_of[e] = x;
+  }
+  // Records of the live elements that are neither folded away nor aliases.
+  net.cluster.assign(N, kNoSlot);
+  net.use_level.assign(N, 0);
+  net.fix_first.assign(N, kNoSlot);
+  std::vector<std::pair<uint32_t, uint32_t>> via;  // (alias, element whose record reads it)
+  for (uint32_t e = P.n_pi; e < g1; ++e) {
+    if (!net.live[e] || (net.lev_up[e] & kFolded) || net.alias[e] != kNoSlot) continue;
+    const uint32_t L = nl.level[e];
+    auto read = [&](uint32_t x) { net.use_level[x] = std::max(net.use_level[x], L); };
+    if (P.po_drv[e]) net.use_level[e] = L + 1;  // its PO record
+    Cluster c = form[e];
+    if (c.n) {
+      for (uint32_t k = 0; k < c.n; ++k) {
+        const uint32_t x = c.lit[k] & ~kInvLit;
+        c.via[k] = x;
+        // the literal's inversion goes to an XOR's output
+        if (net.alias[x] != kNoSlot) c.lit[k] = net.alias[x] ^ (c.lit[k] & kInvLit);
+        if (c.is_xor) {
+          c.inv ^= (uint8_t)(c.lit[k] >> 31);
+          c.lit[k] &= ~kInvLit;
+        }
+        read(c.lit[k] & ~kInvLit);
+        for (uint32_t y = x; net.alias[y] != kNoSlot; y = net.alias_of[y]) via.emplace_back(y, e);
+      }
+      net.cluster[e] = (uint32_t)net.clusters.size();
+      net.clusters.push_back(c);
+    } else {
+      const uint32_t nf = std::min<uint32_t>(eff_fanin(nl, e), 4);
+      for (uint32_t k = 0; k < nf; ++k) read(nl.fi_idx[nl.fi_off[e] + k]);
+    }
+  }
+  net.level_recs.assign(nl.n_levels, 0);
+  for (uint32_t e = P.n_pi; e < g1; ++e)
+    if (net.live[e] && !(net.lev_up[e] & kFolded) && net.alias[e] == kNoSlot) net.level_recs[nl.level[e]]++;
+  for (uint32_t e = 0; e < g1; ++e)
+    if (P.po_drv[e]) net.level_recs[nl.level[e] + 1]++;
+  // Fix lists (elements ascending, so by level).
+  std::sort(via.begin(), via.end());
+  via.erase(std::unique(via.begin(), via.end()), via.end());
+  for (size_t i = 0; i < via.size(); ++i) {
+    if (i == 0 || via[i].first != via[i - 1].first) net.fix_first[via[i].first] = (uint32_t)net.fixes.size();
+    net.fixes.push_back(via[i].second);
+    if (i + 1 == via.size() || via[i + 1].first != via[i].first) net.fixes.push_back(kNoSlot);
   }
 }
 
@@ -78,7 +196,7 @@ void build_circuit_plan(const Netlist& nl, CircuitPlan& C) {
   C.mux_below.assign(N, 0);
   P.po_drv.assign(N, 0);
   P.gate_fo.assign(N, 0);
-  P.maxfo_level.assign(N, 0);
+  std::vector<uint32_t> maxfo_level(N, 0);  // highest non-PO consumer level (0 if none)
   for (uint32_t e = 0; e < N; ++e) {
     for (uint32_t k = nl.fo_off[e]; k < nl.fo_off[e + 1]; ++k) {
       uint32_t c = nl.fo_idx[k];
@@ -86,7 +204,7 @@ void build_circuit_plan(const Netlist& nl, CircuitPlan& C) {
         P.po_drv[e] = 1;
       } else {
         P.gate_fo[e] = 1;
-        P.maxfo_level[e] = std::max(P.maxfo_level[e], nl.level[c]);
+        maxfo_level[e] = std::max(maxfo_level[e], nl.level[c]);
       }
     }
     P.has_mux |= nl.type[e] == G_MUX;
@@ -100,20 +218,24 @@ void build_circuit_plan(const Netlist& nl, CircuitPlan& C) {
     C.mux_below[e] = hb;
   }
 
-  // Peak number of live values (interval graph of [level, highest consumer
-  // level]); the schedule may need a few more to honour slot residues.
+  // What sweeps evaluate, and the peak number of live values (interval graph
+  // of [level, highest reading level]), over all gates and over the stored
+  // ones; a schedule may need a few more slots to honour residues.
+  build_sweep_net(nl, P, P.net);
   {
-    std::vector<int64_t> delta(nl.n_levels + 2, 0);
-    for (uint32_t e = 0; e < N; ++e)
-      if (P.gate_fo[e]) {
-        delta[nl.level[e]]++;
-        delta[P.maxfo_level[e] + 1]--;
-      }
-    int64_t live = 0;
-    for (uint32_t l = 0; l < nl.n_levels; ++l) {
-      live += delta[l];
-      P.max_live = std::max<uint32_t>(P.max_live, (uint32_t)live);
-    }
+    auto peak = [&](const std::vector<uint32_t>& last) {
+      std::vector<int64_t> delta(nl.n_levels + 2, 0);
+      for (uint32_t e = 0; e < N; ++e)
+        if (last[e]) {
+          delta[nl.level[e]]++;
+          delta[last[e] + 1]--;
+        }
+      int64_t live = 0, most = 0;
+      for (uint32_t l = 0; l < nl.n_levels; ++l) most = std::max(most, live += delta[l]);
+      return (uint32_t)most;
+    };
+    P.max_live = peak(maxfo_level);
+    P.net_live = peak(P.net.use_level);
   }
 
   // FFR roots: an element with exactly one consumer belongs to the FFR of that
@@ -169,9 +291,20 @@ void build_fault_plan(const Netlist& nl, const CircuitPlan& C, const std::vector
   P.max_gate_level = B.max_gate_level;
   P.max_level_width = B.max_level_width;
   P.max_live = B.max_live;
+  P.net_live = B.net_live;
   P.has_mux = B.has_mux;
   auto reaches_po = [&](uint32_t x) {
     return (nl.type[x] == G_PO || B.po_drv[x]) ? kInjReachesPo : 0u;
+  };
+  auto stored = [&](uint32_t x) {
+    while (B.net.lev_up[x] & kFolded) x = B.net.lev_up[x] & ~kFolded;
+    return x;
+  };
+  auto inject = [&](uint32_t x, uint32_t v, uint32_t mode) {
+    const uint32_t a = B.net.alias[v];
+    const uint32_t L = nl.level[v] + 1;
+    if (a == kNoSlot) return InjRec{x, v, mode, 0, L, {0, 0, 0}};
+    return InjRec{x, v, mode | ((a & kInvLit) ? kInjAliasInv : 0u), B.net.fix_first[v] + 1, L, {0, 0, 0}};
   };
   auto is_exact = [&](const Fault& ft) {
     return ft.pin == 0 ? (bool)C.mux_below[ft.site]
@@ -194,11 +327,11 @@ void build_fault_plan(const Netlist& nl, const CircuitPlan& C, const std::vector
     rr.root = r;
     if (nl.type[r] == G_PO || B.po_drv[r])
       rr.obs = kObsOne;
-    else if (!B.gate_fo[r])
+    else if (!B.net.live[r])
       rr.obs = kObsZero;
     else {
       rr.obs = (uint32_t)P.sweeps.size();
-      P.sweeps.push_back(InjRec{r, 0, reaches_po(r), 0});
+      P.sweeps.push_back(inject(r, r, reaches_po(r)));
       P.sweep_root.push_back((uint32_t)P.roots.size());
     }
     rr.mem_begin = (uint32_t)P.members.size();
@@ -234,13 +367,16 @@ void build_fault_plan(const Netlist& nl, const CircuitPlan& C, const std::vector
   for (uint32_t f = 0; f < faults.size(); ++f) {
     const Fault& ft = faults[f];
     if (!is_exact(ft)) continue;
-    P.sweeps.push_back(InjRec{ft.site, ft.pin, kInjStuck | reaches_po(ft.site), ft.value});
+    const uint32_t v = stored(ft.site);
+    P.sweeps.push_back(inject(ft.site, v,
+                              kInjStuck | reaches_po(v) | (ft.value ? kInjValue : 0u) |
+                                  ((uint32_t)ft.pin << kInjPinShift)));
     P.exact_fault.push_back(f);
   }
 
   const uint32_t gates_end = nl.level_off[std::min(P.max_gate_level + 1, nl.n_levels)];
   for (auto& s : P.sweeps) {
-    uint32_t L0 = nl.level[s.elem] + 1;
+    uint32_t L0 = nl.level[s.stored] + 1;
     if (L0 <= P.max_gate_level) {
       P.dense_sweep_gates += B.eval_prefix[gates_end] - B.eval_prefix[nl.level_off[L0]];
       P.dense_sweep_bytes += B.nfp_prefix[gates_end] - B.nfp_prefix[nl.level_off[L0]];
@@ -252,7 +388,7 @@ void build_plan(const Netlist& nl, const std::vector<Fault>& faults, Plan& P) {
   CircuitPlan C;
   build_circuit_plan(nl, C);
   build_fault_plan(nl, C, faults, P);
-  P.maxfo_level = std::move(C.base.maxfo_level);
+  P.net = std::move(C.base.net);
   P.gate_fo = std::move(C.base.gate_fo);
   P.po_drv = std::move(C.base.po_drv);
   P.nfp_prefix = std::move(C.base.nfp_prefix);
@@ -285,215 +421,179 @@ void build_schedule(const Netlist& nl, const Plan& P, uint32_t G, Schedule& S) {
   S = Schedule();
   S.G = G;
   const uint32_t N = nl.N;
+  const SweepNet& net = P.net;
   std::vector<uint32_t> slot(N, kNoSlot);
   SlotPool pool(G);
   std::vector<std::vector<uint32_t>> release(nl.n_levels + 2);
   // PIs: residues round robin.
   uint32_t rr = 0;
   for (uint32_t e = nl.level_off[0]; e < nl.level_off[1]; ++e) {
-    if (!P.gate_fo[e]) continue;
+    if (!net.use_level[e]) continue;
     slot[e] = pool.alloc(rr++ % G);
-    release[P.maxfo_level[e] + 1].push_back(slot[e]);
+    release[net.use_level[e] + 1].push_back(slot[e]);
   }
-  auto nf_of = [&](uint32_t e) { return std::min<uint32_t>(eff_fanin(nl, e), 4); };
-  // Classes by (gate family, fan-in): a warp runs one code path.  The AND
-  // family (AND, NAND, OR, NOR, INV, CLKBUF) is io ^ AND(in ^ ii), the XOR
-  // family io ^ XOR(in); MUX is its own family.
-  auto cls_of = [&](uint32_t e) { return gate_family(nl.type[e]) * 8 + nf_of(e); };
-  // Record position k of element e reads its fanin perm[e][k]: the AND and
-  // XOR families are commutative, so the grouper may reorder their fanins
-  // (pin faults and FFR tracing use the netlist's pin order, not the
-  // records); MUX keeps its order.
-  std::vector<std::array<uint8_t, 4>> perm(N, std::array<uint8_t, 4>{0, 1, 2, 3});
-  auto res_in = [&](uint32_t e, uint32_t k) { return slot[nl.fi_idx[nl.fi_off[e] + k]] % G; };
-  // permutations of 2, 3 and 4 inputs
-  static const uint8_t kPerm2[2][4] = {{0, 1, 2, 3}, {1, 0, 2, 3}};
-  static const uint8_t kPerm3[6][4] = {{0, 1, 2, 3}, {0, 2, 1, 3}, {1, 0, 2, 3},
-                                       {1, 2, 0, 3}, {2, 0, 1, 3}, {2, 1, 0, 3}};
-  uint8_t perm4[24][4];
-  {
-    uint8_t a[4] = {0, 1, 2, 3};
-    int n = 0;
-    do {
-      for (int k = 0; k < 4; ++k) perm4[n][k] = a[k];
-      ++n;
-    } while (std::next_permutation(a, a + 4));
+  // A record's literals, and its kind.
+  auto has_record = [&](uint32_t e) {
+    return net.live[e] && !(net.lev_up[e] & kFolded) && net.alias[e] == kNoSlot;
+  };
+  uint64_t n_recs = 0, n_lev = 0;
+  for (uint32_t n : net.level_recs) {
+    n_recs += n;
+    n_lev += n > 0;
   }
-  // Cost of element e in a group with residue masks used[]: repeated
-  // residues over its fanin positions, for the best order of its fanins
-  // (written to *best_p).
-  auto place_cost = [&](uint32_t e, const uint32_t (&used)[4], const uint8_t** best_p) {
-    const uint32_t nf = nf_of(e);
-    const bool comm = gate_family(nl.type[e]) != 2;
-    const uint8_t(*list)[4] = kPerm2;
-    int np = 1;
-    if (comm && nf == 2) {
-      list = kPerm2;
-      np = 2;
-    } else if (comm && nf == 3) {
-      list = kPerm3;
-      np = 6;
-    } else if (comm && nf == 4) {
-      list = perm4;
-      np = 24;
-    }
-    int best = 1 << 30;
-    for (int q = 0; q < np; ++q) {
-      int cost = 0;
-      for (uint32_t k = 0; k < nf; ++k) cost += (used[k] >> res_in(e, list[q][k])) & 1u;
-      if (cost < best) {
-        best = cost;
-        *best_p = list[q];
-        if (cost == 0) break;
-      }
-    }
-    return best;
+  // Levels with fewer records than kSplitRecords on average are not ordered
+  // by kind: a warp would run several bodies on most of its rounds, so there
+  // the sweep runs one body for all ANDs and XORs.
+  S.split = n_recs >= kSplitRecords * n_lev;
+  auto order_key = [&](uint32_t kind) { return S.split || kind >= kRecMux ? kind : (uint32_t)kRecAnd2; };
+  struct Rec {
+    uint32_t e, kind, n;
+    uint32_t lit[4], via[4];
+    uint8_t res[4];   // slot residues
+    bool taken;
   };
-  std::vector<uint32_t> order, leftover;
-  // Groups of G consecutive positions inside one class.  Each member is the
-  // candidate (with its best fanin order) adding the fewest repeated
-  // residues per fanin position to the group, none if possible; only the
-  // last, partial group of a class goes to a mixed tail at the end of the
-  // level.
-  auto make_groups = [&](std::vector<uint32_t>& pool_in, bool tail) {
-    std::vector<uint8_t> taken(pool_in.size(), 0);
-    size_t left = pool_in.size(), first_free = 0;
-    while (left >= G || (tail && left > 0)) {
-      uint32_t used[4] = {0, 0, 0, 0};
-      size_t n_grp = 0;
-      while (n_grp < G && left > 0) {
-        size_t best = SIZE_MAX;
-        int best_cost = 1 << 30;
-        const uint8_t* best_perm = kPerm2[0];
-        size_t scanned = 0;
-        while (first_free < pool_in.size() && taken[first_free]) ++first_free;
-        for (size_t c = first_free; c < pool_in.size() && scanned < 256; ++c) {
-          if (taken[c]) continue;
-          ++scanned;
-          const uint8_t* pp = kPerm2[0];
-          const int cost = place_cost(pool_in[c], used, &pp);
-          if (cost < best_cost) {
-            best_cost = cost;
-            best = c;
-            best_perm = pp;
-            if (cost == 0) break;
-          }
-        }
-        if (best == SIZE_MAX) break;  // unreachable: left > 0 leaves a candidate
-        const uint32_t e = pool_in[best];
-        taken[best] = 1;
-        --left;
-        for (uint32_t k = 0; k < 4; ++k) perm[e][k] = best_perm[k];
-        for (uint32_t k = 0; k < nf_of(e); ++k) used[k] |= 1u << res_in(e, perm[e][k]);
-        order.push_back(e);
-        ++n_grp;
+  auto rec_of = [&](uint32_t e) {
+    Rec r{};
+    r.e = e;
+    if (net.cluster[e] != kNoSlot) {
+      const Cluster& c = net.clusters[net.cluster[e]];
+      r.n = std::max<uint32_t>(c.n, 2);
+      r.kind = (c.is_xor ? kRecXor2 : kRecAnd2) + r.n - 2;
+      for (uint32_t k = 0; k < r.n; ++k) {
+        r.lit[k] = c.lit[k % c.n];
+        r.via[k] = c.via[k % c.n];
       }
+    } else {
+      r.n = std::min<uint32_t>(eff_fanin(nl, e), 4);
+      r.kind = nl.type[e] == G_MUX && r.n == 3 ? kRecMux : kRecWide;
+      for (uint32_t k = 0; k < r.n; ++k) r.lit[k] = nl.fi_idx[nl.fi_off[e] + k];
     }
-    if (!tail)
-      for (size_t c = 0; c < pool_in.size(); ++c)
-        if (!taken[c]) leftover.push_back(pool_in[c]);
+    for (uint32_t k = 0; k < r.n; ++k) r.res[k] = (uint8_t)(slot[r.lit[k] & ~kInvLit] % G);
+    return r;
   };
-  S.lvl.assign(nl.n_levels + 1, LevelDesc{0, 0, 0, 0});
-  std::vector<uint64_t>& blob = S.blob;
-  std::vector<uint32_t> plain, wide;
-  for (uint32_t L = 1; L <= P.max_gate_level && L < nl.n_levels; ++L) {
-    for (uint32_t s : release[L]) pool.release(s);
-    const uint32_t lo = nl.level_off[L], hi = nl.level_off[L + 1];
-    // Gates that feed a gate or a PO; a plain record holds a gate that feeds
-    // gates only, with a compile-time class.
-    plain.clear();
-    wide.clear();
-    for (uint32_t e = lo; e < hi; ++e) {
-      if (!P.gate_fo[e] && !P.po_drv[e]) continue;
-      if (!P.po_drv[e] && plain_class(nl.type[e], nf_of(e)) < kPlainClasses)
-        plain.push_back(e);
-      else
-        wide.push_back(e);
-    }
+  auto po_rec = [&](uint32_t e) {
+    Rec r{};
+    r.e = e;
+    r.kind = kRecPo;
+    r.n = 1;
+    r.lit[0] = e;
+    r.res[0] = (uint8_t)(slot[e] % G);
+    return r;
+  };
+  // Permutations of 1 to 4 literals; the order of a MUX's is fixed.
+  std::vector<std::array<uint8_t, 4>> perms[5];
+  for (uint32_t n = 1; n <= 4; ++n) {
+    std::array<uint8_t, 4> a{0, 1, 2, 3};
+    do perms[n].push_back(a);
+    while (std::next_permutation(a.begin(), a.begin() + n));
+  }
+  // Orders a level's records in groups of G consecutive positions.  Each
+  // member is the candidate (with its best literal order) adding the fewest
+  // repeated residues per literal position to the group, none if possible,
+  // among the next 256 of the first one's kind; a group that runs out of a
+  // kind's candidates goes on with the next kind's.
+  std::vector<Rec> recs, order;
+  auto make_groups = [&] {
     order.clear();
-    // Groups of G inside each class, then the classes' partial groups as a
-    // mixed tail (grouped too); `key` orders the classes.
-    auto part = [&](std::vector<uint32_t>& elems, const std::function<uint32_t(uint32_t)>& key) {
-      std::stable_sort(elems.begin(), elems.end(), [&](uint32_t a, uint32_t b) { return key(a) < key(b); });
-      leftover.clear();
-      for (size_t i = 0; i < elems.size();) {
-        size_t j = i;
-        while (j < elems.size() && key(elems[j]) == key(elems[i])) ++j;
-        std::vector<uint32_t> cls(elems.begin() + i, elems.begin() + j);
-        make_groups(cls, false);
-        i = j;
+    size_t first = 0, left = recs.size();
+    while (left > 0) {
+      uint32_t used[4] = {0, 0, 0, 0};
+      for (size_t n_grp = 0; n_grp < G && left > 0; ++n_grp) {
+        while (recs[first].taken) ++first;
+        size_t best = first, scanned = 0;
+        int best_cost = 1 << 30;
+        const std::array<uint8_t, 4>* best_perm = &perms[1][0];
+        for (size_t c = first; c < recs.size() && scanned < 256 &&
+                               order_key(recs[c].kind) == order_key(recs[first].kind); ++c) {
+          const Rec& r = recs[c];
+          if (r.taken) continue;
+          ++scanned;
+          for (const auto& q : perms[r.n]) {
+            int cost = 0;
+            for (uint32_t k = 0; k < r.n; ++k) cost += (used[k] >> r.res[q[k]]) & 1u;
+            if (cost < best_cost) {
+              best_cost = cost;
+              best = c;
+              best_perm = &q;
+            }
+            if (best_cost == 0 || r.kind >= kRecMux) break;
+          }
+          if (best_cost == 0) break;
+        }
+        Rec& b = recs[best];
+        b.taken = true;
+        --left;
+        Rec o = b;
+        for (uint32_t k = 0; k < b.n; ++k) {
+          o.lit[k] = b.lit[(*best_perm)[k]];
+          o.via[k] = b.via[(*best_perm)[k]];
+          used[k] |= 1u << b.res[(*best_perm)[k]];
+        }
+        order.push_back(o);
       }
-      std::stable_sort(leftover.begin(), leftover.end(), [&](uint32_t a, uint32_t b) { return key(a) < key(b); });
-      make_groups(leftover, true);
-    };
-    part(plain, [&](uint32_t e) { return plain_body(plain_class(nl.type[e], nf_of(e))); });
-    uint32_t n_plain = (uint32_t)order.size();
-    // the wide part starts on a group boundary: pad with no-op records
-    const uint32_t n_pad = wide.empty() ? 0 : (G - n_plain % G) % G;
-    part(wide, [&](uint32_t e) { return cls_of(e); });
-    const uint32_t n_wide = (uint32_t)order.size() - n_plain;
-    // Level block: plain records (8 bytes), padded to 16 bytes, then wide
-    // records (16 bytes).
-    while (blob.size() % 2) blob.push_back(0);
-    LevelDesc& d = S.lvl[L];
-    d.off16 = (uint32_t)(blob.size() / 2);
-    d.n_plain = n_plain + n_pad;
-    d.n_wide = n_wide;
-    const size_t plain_base = blob.size();
-    blob.resize(plain_base + ((size_t)d.n_plain + 1) / 2 * 2 + 2ull * n_wide, 0);
-    for (uint32_t k = 0; k < n_pad; ++k) blob[plain_base + n_plain + k] = plain_rec(0, 0, 0, 0, kPNop);
-    const size_t wide_base = plain_base + ((size_t)d.n_plain + 1) / 2 * 2;
-    d.n16 = (uint32_t)((blob.size() - plain_base) / 2);
-    S.max_block16 = std::max(S.max_block16, d.n16);
-    // Positions, output slots (residue = position mod G) and records.
-    std::vector<uint32_t> pos_slot[5];
-    for (auto& v : pos_slot) v.assign(order.size() + n_pad, kNoSlot);
-    for (uint32_t o = 0; o < order.size(); ++o) {
-      const uint32_t e = order[o];
-      const uint32_t pos = o < n_plain ? o : o + n_pad;
-      const uint32_t nf = nf_of(e);
-      uint32_t fs[4] = {0, 0, 0, 0};
-      for (uint32_t k = 0; k < nf; ++k) {
-        fs[k] = slot[nl.fi_idx[nl.fi_off[e] + perm[e][k]]];
-        pos_slot[k][pos] = fs[k];
-      }
-      uint32_t out = 0;
-      if (P.gate_fo[e]) {
-        slot[e] = pool.alloc(pos % G);
-        release[P.maxfo_level[e] + 1].push_back(slot[e]);
-        out = slot[e];
-        pos_slot[4][pos] = out;
-      }
-      const uint8_t t = nl.type[e];
-      if (o < n_plain) {
-        blob[plain_base + o] = plain_rec(fs[0], fs[1], fs[2], out, plain_class(t, nf));
+    }
+  };
+  S.rec_off.assign(nl.n_levels + 1, 0);
+  // A slot at bit 14 * (k & 1) of word k / 2, its high bits in word 2 + k / 2.
+  auto put_slot = [](std::array<uint32_t, 4>& w, uint32_t k, uint32_t sl) {
+    const uint32_t sh = 14 * (k & 1u);
+    w[k / 2] = (w[k / 2] & ~(kRecSlot << sh)) | (sl & kRecSlot) << sh;
+    w[2 + k / 2] = (w[2 + k / 2] & ~(kRecSlot << sh)) | (sl >> 14) << sh;
+  };
+  std::vector<std::array<uint32_t, 4>> fix_rec(net.fixes.empty() ? 0 : N);  // per element: record index, via
+  std::vector<std::array<uint32_t, 5>> pos_slot;
+  for (uint32_t L = 1; L <= P.max_gate_level + 1 && L < nl.n_levels; ++L) {
+    for (uint32_t s : release[L]) pool.release(s);
+    recs.clear();
+    for (uint32_t e = nl.level_off[L]; e < nl.level_off[L + 1] && nl.type[e] != G_PO; ++e)
+      if (has_record(e)) recs.push_back(rec_of(e));
+    for (uint32_t e = nl.level_off[L - 1]; e < nl.level_off[L]; ++e)
+      if (P.po_drv[e] && slot[e] != kNoSlot) recs.push_back(po_rec(e));
+    std::stable_sort(recs.begin(), recs.end(), [&](const Rec& a, const Rec& b) { return order_key(a.kind) > order_key(b.kind); });
+    make_groups();
+    // Output slots (residue = position mod G) and records.
+    S.rec_off[L] = (uint32_t)S.recs.size();
+    pos_slot.assign(order.size(), std::array<uint32_t, 5>{kNoSlot, kNoSlot, kNoSlot, kNoSlot, kNoSlot});
+    for (uint32_t pos = 0; pos < order.size(); ++pos) {
+      const Rec& r = order[pos];
+      const uint32_t e = r.e;
+      for (uint32_t k = 0; k < r.n; ++k) pos_slot[pos][k] = slot[r.lit[k] & ~kInvLit];
+      if (r.kind == kRecPo) {
+        std::array<uint32_t, 4> w{0, (uint32_t)kRecPo << kRecKindShift, 0, 0};
+        put_slot(w, 3, slot[e]);
+        w[0] = e;
+        S.recs.push_back(w);
         continue;
       }
-      SweepRec r{};
-      for (uint32_t k = 0; k < nf; ++k) r.fs[k] = (uint16_t)fs[k];
-      uint32_t meta = (uint32_t)t & kRecTypeMask;
-      meta |= ((nf ? nf - 1 : 0) & 3u) << kRecNfShift;
-      meta |= gate_class(t, nf) << kRecClassShift;
-      if (t == G_OR || t == G_NOR) meta |= kRecIi;
-      if (t == G_INV || t == G_OR || t == G_NAND || t == G_XNOR) meta |= kRecIo;
-      if (P.po_drv[e]) meta |= kRecPo;
-      if (P.gate_fo[e]) {
-        meta |= kRecHasSlot;
-        r.slot = (uint16_t)out;
+      const uint32_t out = slot[e] = pool.alloc(pos % G);  // every record is read
+      release[net.use_level[e] + 1].push_back(out);
+      pos_slot[pos][4] = out;
+      if (r.kind == kRecWide) {
+        std::array<uint32_t, 8> d{0, 0, 0, 0, out, (uint32_t)nl.type[e] | r.n << 4, 0, 0};
+        for (uint32_t k = 0; k < r.n; ++k) d[k] = pos_slot[pos][k];
+        S.recs.push_back({(uint32_t)S.wides.size(), (uint32_t)kRecWide << kRecKindShift, 0, 0});
+        S.wides.push_back(d);
+        continue;
       }
-      r.meta = (uint16_t)meta;
-      r.elem = e;
-      std::memcpy(&blob[wide_base + 2ull * (o - n_plain)], &r, sizeof r);
+      std::array<uint32_t, 4> w{0, r.kind << kRecKindShift, 0, 0};
+      for (uint32_t k = 0; k < r.n; ++k) {
+        put_slot(w, k, pos_slot[pos][k]);
+        w[0] |= (r.lit[k] >> 31) << (31 - k);
+      }
+      put_slot(w, 3, out);
+      if (r.kind == kRecAnd2) w[0] |= 1u << 29;  // an absent literal reads as inverted zeros
+      if (r.kind != kRecMux) w[0] |= (uint32_t)net.clusters[net.cluster[e]].inv << 28;
+      if (!fix_rec.empty()) fix_rec[e] = {(uint32_t)S.recs.size(), r.via[0], r.via[1], r.via[2]};
+      S.recs.push_back(w);
     }
     // Bank-conflict accounting per aligned group of G positions.
-    const uint32_t n_pos = (uint32_t)order.size() + n_pad;
-    for (uint32_t g0 = 0; g0 < n_pos; g0 += G) {
-      const uint32_t g1 = std::min<uint32_t>(g0 + G, n_pos);
+    for (uint32_t g0 = 0; g0 < order.size(); g0 += G) {
+      const uint32_t g_end = std::min<uint32_t>(g0 + G, (uint32_t)order.size());
       for (uint32_t k = 0; k < 5; ++k) {
         uint32_t seen = 0, any = 0;
         bool conflict = false;
-        for (uint32_t o = g0; o < g1; ++o) {
-          const uint32_t sl = pos_slot[k][o];
+        for (uint32_t o = g0; o < g_end; ++o) {
+          const uint32_t sl = pos_slot[o][k];
           if (sl == kNoSlot) continue;
           any = 1;
           conflict |= (seen >> (sl % G)) & 1u;
@@ -504,27 +604,96 @@ void build_schedule(const Netlist& nl, const Plan& P, uint32_t G, Schedule& S) {
       }
     }
   }
-  S.max_live = pool.next_block * G;
+  for (uint32_t L = std::min(P.max_gate_level + 2, nl.n_levels); L <= nl.n_levels; ++L)
+    S.rec_off[L] = (uint32_t)S.recs.size();
+  S.max_live = pool.next_block * G + (net.fixes.empty() ? 0 : 1);
   if (S.max_live > kMaxSlots) {
-    S.blob.clear();
+    S.recs.clear();
+    S.wides.clear();
     return;
+  }
+  // Fix entries: the record of a reader of alias y, with the literals that
+  // name y, or an alias of y, on the injection slot.
+  S.fixes.resize(net.fixes.size(), std::array<uint32_t, 4>{0, 0, 0, 0});
+  S.fix_level.assign(net.fixes.size(), kNoSlot);
+  for (uint32_t y = 0; y < N && !net.fixes.empty(); ++y) {
+    if (net.fix_first[y] == kNoSlot) continue;
+    for (uint32_t i = net.fix_first[y]; net.fixes[i] != kNoSlot; ++i) {
+      const auto& fr = fix_rec[net.fixes[i]];
+      std::array<uint32_t, 4> w = S.recs[fr[0]];
+      const uint32_t n = std::max<uint32_t>(net.clusters[net.cluster[net.fixes[i]]].n, 2);
+      for (uint32_t k = 0; k < n; ++k) {
+        uint32_t x = fr[1 + k];
+        while (x != y && net.alias[x] != kNoSlot) x = net.alias_of[x];
+        if (x == y) put_slot(w, k, S.max_live - 1);
+      }
+      S.fixes[i] = w;
+      S.fix_level[i] = nl.level[net.fixes[i]];
+    }
   }
   // Live-in sets as (element, slot) pairs.
   std::vector<uint32_t> cnt(nl.n_levels + 2, 0);
   for (uint32_t e = 0; e < N; ++e)
     if (slot[e] != kNoSlot)
-      for (uint32_t l = nl.level[e] + 1; l <= P.maxfo_level[e]; ++l) cnt[l]++;
+      for (uint32_t l = nl.level[e] + 1; l <= net.use_level[e]; ++l) cnt[l]++;
   S.li_off.assign(nl.n_levels + 1, 0);
   for (uint32_t l = 0; l < nl.n_levels; ++l) S.li_off[l + 1] = S.li_off[l] + cnt[l];
   S.li.assign(2ull * S.li_off[nl.n_levels], 0);
   std::vector<uint32_t> fill(S.li_off.begin(), S.li_off.end() - 1);
   for (uint32_t e = 0; e < N; ++e)
     if (slot[e] != kNoSlot)
-      for (uint32_t l = nl.level[e] + 1; l <= P.maxfo_level[e]; ++l) {
+      for (uint32_t l = nl.level[e] + 1; l <= net.use_level[e]; ++l) {
         const uint32_t i = fill[l]++;
         S.li[2 * i] = e;
         S.li[2 * i + 1] = slot[e];
       }
+}
+
+void pack_schedule(Schedule& S, uint32_t T) {
+  if (S.T == T) return;
+  S.T = T;
+  S.blob.clear();
+  const uint32_t n_levels = (uint32_t)S.rec_off.size() - 1, nw = S.rec_words();
+  S.lvl.assign(n_levels + 1, std::array<uint32_t, 4>{0, 0, 0, 0});
+  // Lane l of a shared-memory phase (8 lanes; 16 at one word per item, where
+  // a phase is one group) takes position (l % C) * G + l / C of the phase's
+  // groups, C = 16-byte chunks per slot: with chunk (l % C) ^ i at step i the
+  // phase's chunks lie in different banks wherever the group's slots do.
+  const uint32_t C = 8 / S.G ? 8 / S.G : 1, ph = S.G == 16 ? 16 : 8;
+  uint32_t n = 0;  // records so far
+  std::vector<uint32_t> wide_at;
+  for (uint32_t L = 0; L < n_levels; ++L) {
+    S.lvl[L] = {n, S.li_off[L], S.li_off[L + 1], 0};
+    const uint32_t lo = S.rec_off[L], n_lev = S.rec_off[L + 1] - lo;
+    const uint32_t rounds = (n_lev + T - 1) / T;
+    S.blob.resize((size_t)(n + rounds * T) * nw, 0);
+    for (uint32_t i = 0; i < rounds * T; ++i) {
+      const uint32_t l = i % ph;
+      const uint32_t pos = i - l + (S.G == 16 ? l : (l % C) * S.G + l / C);
+      uint32_t* w = &S.blob[(size_t)(n + i) * nw];
+      if (pos < n_lev) {
+        std::copy_n(S.recs[lo + pos].begin(), nw, w);
+        if (((w[1] >> kRecKindShift) & 7u) == kRecWide) wide_at.push_back(n + i);
+      }
+      if (i >= (rounds - 1) * T) w[1] |= kRecEnd;
+    }
+    n += rounds * T;
+  }
+  S.lvl[n_levels][0] = S.stream_recs = n;
+  S.blob.resize((size_t)(n + kPrefetch * T) * nw, 0);
+  const uint32_t wide0 = (uint32_t)(S.blob.size() / 4);
+  for (uint32_t i : wide_at) S.blob[(size_t)i * nw] = wide0 + 2 * S.blob[(size_t)i * nw];
+  for (const auto& d : S.wides) S.blob.insert(S.blob.end(), d.begin(), d.end());
+  S.fix0 = (uint32_t)(S.blob.size() / 4);
+  for (size_t i = 0; i < S.fixes.size(); ++i) {
+    uint32_t at = kNoSlot, same = 0;
+    if (S.fix_level[i] != kNoSlot) {
+      at = S.lvl[S.fix_level[i] + 1][0] - T;
+      while (S.fix_level[i + same] == S.fix_level[i]) ++same;  // a list ends with kNoSlot
+    }
+    S.blob.insert(S.blob.end(), S.fixes[i].begin(), S.fixes[i].end());
+    S.blob.insert(S.blob.end(), {at, same, 0u, 0u});
+  }
 }
 
 }  // namespace fsimb

@@ -4,23 +4,32 @@
 // Layout in HBM (all arrays indexed by the reference's topological index):
 //   type[N]            u8 gate type
 //   fi_off[N+1], fi_idx[E]   fanin CSR in pin order (good-machine kernel)
-//   sweep blocks       per level one block of gate records (the level's
-//                      order of evaluation), 16-byte aligned:
-//                        plain records, 8 bytes: 15-bit shared-memory slots
-//                        of up to three fanins and of the output, and a
-//                        4-bit gate class (PlainClass) -- every non-MUX gate
-//                        with 1-3 inputs that feeds other gates and no PO;
-//                        wide records, 16 bytes (SweepRec): everything else
-//                        that must be evaluated (PO drivers, MUX, 4 inputs).
-//                      Gates that feed nothing are left out.  Within each
-//                      part the order is by class, and every group of G
-//                      consecutive positions has pairwise different slot
-//                      residues mod G for each fanin and for the output
-//                      wherever the host found such groups, so the group's
-//                      shared-memory accesses hit distinct banks
-//   lvl[L]             (block offset in 16-byte units, plain count, wide
-//                      count, block size in 16-byte units)
-//   li_off[L+1], li[]  (element, slot) pairs live when a sweep starts at
+//   blob[]             the sweep's record stream, 8 bytes a record, level
+//                      after level in order of evaluation.  A record is a
+//                      cluster: a gate together with single-consumer gates
+//                      folded into it, an AND or XOR of up to three literals
+//                      in all.  The inner values are never stored, because a
+//                      sweep flips multi-consumer elements only.  MUX gates
+//                      have records of their own kind; gates of four inputs
+//                      ("wide" records) are described in 32 bytes each
+//                      behind the stream.  A PO driver's value is compared
+//                      with the good one by a record one level above it.
+//                      Elements from which no PO is reached are left out.
+//                      A level is padded to rounds of T records, T the sweep
+//                      CTA's threads: thread t of round r reads record
+//                      r * T + t, and the last round of a level carries
+//                      kRecEnd, so a sweep needs no other table of levels.
+//                      Within a level the order is by kind, and every
+//                      group of G consecutive positions has pairwise
+//                      different slot residues mod G for each literal and
+//                      for the output wherever the host found such groups,
+//                      so the group's shared-memory accesses hit distinct
+//                      banks
+//   lvl[L]             of a sweep that starts at level L: record offset in the
+//                      stream of its first round, and its range in li
+//   level[e]           level of a stored element; kFolded | consumer for an
+//                      element folded into its consumer's cluster
+//   li[]               (element, slot) pairs live when a sweep starts at
 //                      level L (read from the good values at start)
 //   good[tile][N][32]  u64 good-machine words, 32 words (2048 patterns) per tile
 //
@@ -36,6 +45,7 @@
 //     logical not (fsim/simulation.cpp:1056) that is not bitwise.
 #pragma once
 
+#include <array>
 #include <cstdint>
 #include <vector>
 
@@ -47,65 +57,42 @@ constexpr uint32_t kTileWords = 32;  // words per tile = lanes of a warp
 constexpr uint32_t kNoSlot = 0xFFFFFFFFu;
 constexpr uint32_t kMaxSlots = 32767;   // slots are 15-bit in the plain gate records
 
-// Plain gate records: classes of the gate function (a compile-time body in
-// the sweep kernel each).  One-input gates are BUF (AND, OR, XOR, CLKBUF) or
-// INV (INV, NAND, NOR, XNOR).  kPNop pads a level's plain part to a group
-// boundary and does nothing.
-enum PlainClass : uint32_t {
-  kPBuf = 0, kPInv, kPAnd2, kPNand2, kPOr2, kPNor2, kPXor2, kPXnor2,
-  kPAnd3, kPNand3, kPOr3, kPNor3, kPXor3, kPXnor3, kPlainClasses, kPNop = 15
-};
-// Classes that share one sweep body, which reads the class's input and
-// output inversions from the class code at run time: one input, AND family
-// (AND, NAND, OR, NOR) with two and with three inputs, XOR family with two
-// and with three inputs.  The host groups records by body, not by class:
-// larger groups leave fewer repeated bank residues and fewer class
-// boundaries inside a warp.
-inline uint32_t plain_body(uint32_t cls) {
-  return cls < kPAnd2 ? 0u : cls < kPXor2 ? 1u : cls < kPAnd3 ? 2u : cls < kPXor3 ? 3u : 4u;
-}
-// Bits [0,15) fanin 0, [15,30) fanin 1, [30,45) fanin 2, [45,60) output
-// slot, [60,64) class.
-inline uint64_t plain_rec(uint32_t f0, uint32_t f1, uint32_t f2, uint32_t out, uint32_t cls) {
-  return (uint64_t)f0 | ((uint64_t)f1 << 15) | ((uint64_t)f2 << 30) | ((uint64_t)out << 45) |
-         ((uint64_t)cls << 60);
-}
+constexpr uint32_t kFolded = 0x80000000u;  // level[]: the element is folded; low bits: its consumer
 
-// One level of the sweep order (see "sweep blocks" above).
-struct LevelDesc {
-  uint32_t off16;    // block offset in 16-byte units
-  uint32_t n_plain;  // plain records (8 bytes each, first)
-  uint32_t n_wide;   // wide records (16 bytes each, after the plain part padded to 16 bytes)
-  uint32_t n16;      // block size in 16-byte units
+// A record is two 32-bit words.  Word 0: slots of literals 0 and 1 in bits
+// 0-13 and 14-27; word 1: slots of literal 2 and of the output.  The top four
+// bits of word 0 are inversions (literals 0, 1, 2 from bit 31 down, then the
+// output's), those of word 1 the end-of-level bit and the kind.  At one word
+// per item, where up to 28,000 slots fit shared memory, a record is four
+// words, one slot each in bits 0-13 and 14-27 (low and high half): word 2 the
+// high halves of literals 0 and 1, word 3 those of literal 2 and the output.
+// A cluster of one literal is the AND of it with itself.  A MUX record has
+// its three inputs in pin order.  A wide record's word 0 is the offset of its
+// description from the stream's start, in 16-byte units.  A PO record has the
+// driver's slot in the output's place and the driver in word 0.
+enum RecKind : uint32_t {
+  kRecNop = 0,  // padding
+  kRecAnd2, kRecAnd3, kRecXor2, kRecXor3,
+  kRecMux,
+  kRecWide,
+  kRecPo
 };
-
-// SweepRec::meta bit fields
-constexpr uint32_t kRecTypeMask = 15u;     // bits 0-3: gate type
-constexpr int kRecNfShift = 4;             // bits 4-5: fan-in - 1
-constexpr uint32_t kRecPo = 1u << 6;       // drives a PO
-constexpr uint32_t kRecHasSlot = 1u << 7;  // has gate consumers (value stored)
-constexpr int kRecClassShift = 8;          // bits 8-11: gate class (sweep code path)
-constexpr uint32_t kRecIi = 1u << 12;      // invert inputs (OR, NOR)
-constexpr uint32_t kRecIo = 1u << 13;      // invert output (INV, OR, NAND, XNOR)
-// Gate classes: 0-3 AND family with 1-4 inputs, 4-6 XOR family with 2-4
-// inputs, 7 MUX with 3 inputs, 8 any other combination (generic path).
-constexpr uint32_t kClassGeneric = 8;
+constexpr int kRecKindShift = 28;  // word 1, three bits
+constexpr uint32_t kRecEnd = 1u << 31;  // word 1: the last round of the level
+constexpr uint32_t kRecSlot = 0x3FFFu;
+// A wide record's description, eight words: slots of up to four inputs, of
+// the output, and type | fan-in << 4.
 
 // InjRec::mode bit fields
 constexpr uint32_t kInjStuck = 1u;      // 0: flip the element's word, 1: stuck value
-constexpr uint32_t kInjReachesPo = 2u;  // the element is, or drives, a PO
+constexpr uint32_t kInjReachesPo = 2u;  // the stored element is, or drives, a PO
+constexpr uint32_t kInjValue = 4u;      // the stuck value
+constexpr uint32_t kInjAliasInv = 8u;   // the stored element is an inverting alias
+constexpr int kInjPinShift = 4;         // exact faults: 0 output, k input; flips: 0
 
 // Observability source of an FFR root.
 constexpr uint32_t kObsZero = 0xFFFFFFFEu;  // root reaches no PO
 constexpr uint32_t kObsOne = 0xFFFFFFFFu;   // root is / drives a PO
-
-struct SweepRec {  // wide gate record
-  uint16_t fs[4];  // fanin slots
-  uint16_t slot;   // own slot (valid with kRecHasSlot)
-  uint16_t meta;
-  uint32_t elem;   // topological index
-};
-static_assert(sizeof(SweepRec) == 16, "SweepRec is one 16-byte load");
 
 struct RootRec {
   uint32_t root;
@@ -134,16 +121,47 @@ struct TracedRec {  // one traced fault
 
 struct InjRec {     // sweep injection: flip (stem) or stuck (exact fault)
   uint32_t elem;
-  uint32_t pin;     // exact faults: 0 output, k input; flips: 0
-  uint32_t mode;    // kInjStuck | kInjReachesPo
-  uint32_t value;
+  uint32_t stored;  // the stored element whose word the sweep replaces: elem, or the
+                    // element whose cluster it is folded into
+  uint32_t mode;    // kInjStuck | kInjReachesPo | kInjValue | kInjAliasInv | pin << kInjPinShift
+  uint32_t fix;     // stored is an alias: its first fix entry + 1; else 0
+  uint32_t level;   // the sweep's first level: one above stored
+  uint32_t pad[3];
+};
+
+// What a sweep evaluates and stores (independent of the fault list).
+struct Cluster {
+  uint32_t lit[3];  // stored element | inversion << 31
+  uint32_t via[3];  // the element the literal names in the netlist: the same, or an alias of it
+  uint8_t n;        // literals
+  uint8_t is_xor;
+  uint8_t inv;      // the output inverted
+};
+struct SweepNet {
+  std::vector<uint32_t> lev_up;     // [N] level, or kFolded | consumer
+  std::vector<uint32_t> use_level;  // [N] highest level of a record that reads it (0: none, no slot)
+  std::vector<uint32_t> cluster;    // [N] index into clusters; kNoSlot: no cluster record
+  // BUF and INV gates that only clusters read have no record and no slot:
+  // their readers take the source's slot, inverted or not.  A sweep that
+  // injects at such an alias runs the level as it is and then evaluates the
+  // records that read it again, on an extra slot with the faulty value.
+  std::vector<uint32_t> alias;      // [N] stored source | inversion << 31; kNoSlot: not an alias
+  std::vector<uint32_t> alias_of;   // [N] an alias's direct source, maybe an alias itself
+  std::vector<uint32_t> fix_first;  // [N] an alias's first entry in fixes; kNoSlot: none
+  std::vector<uint32_t> fixes;      // per alias, by level: elements whose records read it, then kNoSlot
+  std::vector<uint8_t> live;        // [N] a PO is reached from it
+  std::vector<Cluster> clusters;
+  std::vector<uint32_t> level_recs; // [n_levels] records a sweep evaluates on each level
 };
 
 struct Plan {
   uint32_t N = 0, n_pi = 0, n_gates = 0, n_po = 0;
   uint32_t n_levels = 0;
   uint32_t max_gate_level = 0;       // highest level holding a non-PO element
-  uint32_t max_live = 0;             // slots needed without residue constraints
+  // Peak of live gate outputs, every gate counted: the documented limit of
+  // the shared-memory sweep and of explicit shapes.
+  uint32_t max_live = 0;
+  uint32_t net_live = 0;             // peak of stored values: slots needed without residue constraints
   uint32_t max_level_width = 0;
   uint64_t dense_sweep_gates = 0;    // sum over sweeps of gates evaluated
   uint64_t dense_sweep_bytes = 0;    // sum over sweeps of 8*(fanin+1) per evaluated gate, per word
@@ -152,7 +170,7 @@ struct Plan {
   std::vector<uint64_t> nfp_prefix;
   std::vector<uint32_t> eval_prefix; // [N+1] prefix counts of those elements
   std::vector<uint32_t> level_off;   // [n_levels+1]
-  std::vector<uint32_t> maxfo_level; // [N] highest non-PO consumer level (0 if none)
+  SweepNet net;
   std::vector<uint8_t> gate_fo;      // [N] has a non-PO consumer
   std::vector<uint8_t> po_drv;       // [N] drives a PO
   // traced faults
@@ -182,38 +200,56 @@ struct CircuitPlan {
   std::vector<uint32_t> ffr_local;  // [N] position of a member within its FFR's list
 };
 
-// Per-level evaluation order and shared-memory slots for one residue group
-// size G (16 / words per item).
+// Evaluation order and shared-memory slots for one residue group size G
+// (16 / words per item), and the record stream packed for a CTA size.
 struct Schedule {
   uint32_t G = 0;
-  uint32_t max_live = 0;             // slots (multiple of G)
-  std::vector<uint64_t> blob;        // level blocks (8-byte units; each block 16-byte aligned)
-  std::vector<LevelDesc> lvl;        // [n_levels+1]; levels 1..max_gate_level used
-  uint32_t max_block16 = 0;          // largest level block, 16-byte units
-  std::vector<uint32_t> li_off;      // [n_levels+1]
+  uint32_t max_live = 0;             // slots, the injection slot among them
+  bool split = false;                // levels are ordered by kind
+  std::vector<std::array<uint32_t, 4>> recs;  // records in position order, level after level
+                                     // (a wide one's word 0: its index in wides)
+  std::vector<std::array<uint32_t, 8>> wides;
+  std::vector<uint32_t> rec_off;     // [n_levels+1] first record of each level
+  std::vector<uint32_t> li_off;      // [n_levels+1] first pair of each level in li
   std::vector<uint32_t> li;          // pairs (element, slot)
+  std::vector<std::array<uint32_t, 4>> fixes;  // per net.fixes entry: its record, reading the
+                                     // injection slot (the last one) in the alias's place
+  std::vector<uint32_t> fix_level;   // level of each entry; kNoSlot ends a list
   uint64_t conflict_groups = 0;      // group accesses whose slots repeat a residue
   uint64_t access_groups = 0;        // group accesses (fanin loads + stores)
-  uint64_t bytes() const {
-    return blob.size() * 8 + lvl.size() * sizeof(LevelDesc) + li_off.size() * 4 + li.size() * 4;
-  }
+  // pack_schedule
+  uint32_t T = 0;                    // CTA threads the stream is packed for
+  uint32_t stream_recs = 0;          // records of all rounds
+  uint32_t fix0 = 0;                 // offset of the fix entries in blob, 16-byte units
+  // The rounds (rec_words() words a record), kPrefetch rounds of padding, the
+  // wide descriptions, and eight words per fix entry: the record (four
+  // words), then stream offset of its level's last round and entries of the
+  // list on that level; ~0 ends a list.
+  std::vector<uint32_t> blob;
+  uint32_t rec_words() const { return G == 16 ? 4 : 2; }
+  std::vector<std::array<uint32_t, 4>> lvl;  // [n_levels+1] first record, li begin, li end, 0
+  uint64_t bytes() const { return blob.size() * 4 + lvl.size() * 16 + li.size() * 4; }
 };
+constexpr uint32_t kPrefetch = 2;  // rounds a sweep reads ahead
+constexpr uint64_t kSplitRecords = 256;  // records a level from which ANDs and XORs have kinds of their own
 
 // 0: AND family (AND, NAND, OR, NOR, INV, CLKBUF, PO), 1: XOR family, 2: MUX.
 uint32_t gate_family(uint8_t type);
-uint32_t gate_class(uint8_t type, uint32_t fanin);
 void build_plan(const Netlist& nl, const std::vector<Fault>& faults, Plan& plan);
 void build_circuit_plan(const Netlist& nl, CircuitPlan& cplan);
 // Roots, members, traced faults and sweeps of a fault list; the circuit's
-// per-element vectors (maxfo_level, gate_fo, po_drv, nfp_prefix) stay in
+// per-element vectors (net, gate_fo, po_drv, nfp_prefix) stay in
 // cplan.base and are left empty in `plan`.  Costs O(faults log faults +
 // members of the FFRs the faults touch).
 void build_fault_plan(const Netlist& nl, const CircuitPlan& cplan, const std::vector<Fault>& faults,
                       Plan& plan);
-// Class of a plain record, or kPlainClasses when the gate needs a wide one.
-uint32_t plain_class(uint8_t type, uint32_t eff_fanin);
+// Folds single-consumer gates into their consumers.
+void build_sweep_net(const Netlist& nl, const Plan& plan, SweepNet& net);
 // G in {2, 4, 8, 16}.  A schedule that needs more than kMaxSlots slots
-// reports max_live > kMaxSlots and leaves blob and li empty.
+// reports max_live > kMaxSlots and leaves recs and li empty.
 void build_schedule(const Netlist& nl, const Plan& plan, uint32_t G, Schedule& out);
+// Packs the schedule's records into the stream of a T-thread CTA (T a
+// multiple of 32); nothing to do if it is packed for T already.
+void pack_schedule(Schedule& s, uint32_t T);
 
 }  // namespace fsimb

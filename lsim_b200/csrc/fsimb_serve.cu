@@ -57,21 +57,21 @@ struct ResidentCircuit {
   Netlist nl;
   CircuitPlan cp;
   Schedule sched;
-  ClassShape shape{4, 256, 1};
+  ClassShape shape{4, 256};
   Patterns block;  // resident pattern block (host copy of its words)
   uint64_t block_tiles = 0;
-  // d_level_off holds the schedule's level descriptors, d_recs its record blocks
-  DevBuf d_type, d_fi_off, d_fi_idx, d_level, d_level_off, d_recs, d_li_off, d_li, d_pwords, d_good;
+  // d_recs holds the schedule's record stream
+  DevBuf d_type, d_fi_off, d_fi_idx, d_level, d_lvl, d_recs, d_li, d_pwords, d_good;
   BatchCirc dev{};
   uint64_t device_bytes() const {
     uint64_t s = 0;
-    for (const DevBuf* b : {&d_type, &d_fi_off, &d_fi_idx, &d_level, &d_level_off, &d_recs, &d_li_off,
-                            &d_li, &d_pwords, &d_good})
+    for (const DevBuf* b : {&d_type, &d_fi_off, &d_fi_idx, &d_level, &d_lvl, &d_recs, &d_li,
+                            &d_pwords, &d_good})
       s += b->n;
     return s;
   }
   void release() {
-    for (DevBuf* b : {&d_type, &d_fi_off, &d_fi_idx, &d_level, &d_level_off, &d_recs, &d_li_off, &d_li,
+    for (DevBuf* b : {&d_type, &d_fi_off, &d_fi_idx, &d_level, &d_lvl, &d_recs, &d_li,
                       &d_pwords, &d_good})
       b->release();
   }
@@ -264,10 +264,7 @@ struct fsimb_server {
     if (words) c->block.words.assign(words, words + c->block.W * nl.n_pi);
     build_circuit_plan(nl, c->cp);
     // the default shape, for the batch kernel
-    std::vector<uint32_t> widths;
     const Plan& B = c->cp.base;
-    for (uint32_t l = 1; l <= B.max_gate_level && l < B.n_levels; ++l)
-      widths.push_back(B.level_off[l + 1] - B.level_off[l]);
     Schedule sc[4];
     bool has[4] = {false, false, false, false};
     auto sched_at = [&](int m) -> const Schedule& {
@@ -278,28 +275,16 @@ struct fsimb_server {
       }
       return sc[sl];
     };
-    // the schedules the default shape looks at first, before taking the lock
-    for (int m : {8, 4})
-      if (sweep_vals_bytes(B.max_live, m) <= sweep_smem_share(smem_optin, smem_per_sm, 2)) sched_at(m);
-    int M = 0, occ = 1, T = 0;
-    {
-      std::lock_guard<std::mutex> g(attr_mu);
-      default_sweep_shape(
-          B, sched_at,
-          [&](int m, int th, size_t smem) {
-            CK(sweep_batch_set_smem(m, smem));
-            int got = 0;
-            CK(sweep_batch_occupancy(m, th, smem, &got));
-            return got;
-          },
-          widths, kTileWords, smem_optin, smem_per_sm, M, occ, T);
-    }
-    const Schedule& chosen = sched_at(M);
-    if (chosen.max_live > kMaxSlots ||
-        sweep_vals_bytes(chosen.max_live, M) > sweep_smem_share(smem_optin, smem_per_sm, occ))
+    const size_t share = sweep_smem_share(smem_optin, smem_per_sm, 1);
+    if (B.max_live > kMaxSlots || sweep_vals_bytes(B.max_live, 1) > share)
       throw LimitError{"the circuit has more live values than shared memory holds at 1 word per item"};
-    c->sched = chosen;
-    c->shape = ClassShape{M, T, occ};
+    int M = 0, T = 0;
+    default_sweep_shape(B, sched_at, kTileWords, smem_optin, smem_per_sm, M, T);
+    if (sched_at(M).max_live > kMaxSlots || sweep_vals_bytes(sched_at(M).max_live, M) > share)
+      throw LimitError{"the circuit has more live values than shared memory holds at 1 word per item"};
+    pack_schedule(sc[m_slot_s(M)], (uint32_t)T);
+    c->sched = std::move(sc[m_slot_s(M)]);
+    c->shape = ClassShape{M, T};
 
     // resident device data
     CK(cudaSetDevice(device));
@@ -309,10 +294,9 @@ struct fsimb_server {
       upload(c->d_type, nl.type, s);
       upload(c->d_fi_off, nl.fi_off, s);
       upload(c->d_fi_idx, nl.fi_idx, s);
-      upload(c->d_level, nl.level, s);
-      upload(c->d_level_off, c->sched.lvl, s);
+      upload(c->d_level, B.net.lev_up, s);
+      upload(c->d_lvl, c->sched.lvl, s);
       upload(c->d_recs, c->sched.blob, s);
-      upload(c->d_li_off, c->sched.li_off, s);
       upload(c->d_li, c->sched.li, s);
       c->block_tiles = (c->block.W + kTileWords - 1) / kTileWords;
       if (c->block.W) {
@@ -346,9 +330,8 @@ struct fsimb_server {
     c->dev.fi_off = c->d_fi_off.as<uint32_t>();
     c->dev.fi_idx = c->d_fi_idx.as<uint32_t>();
     c->dev.level = c->d_level.as<uint32_t>();
-    c->dev.lvl = c->d_level_off.as<uint4>();
+    c->dev.lvl = c->d_lvl.as<uint4>();
     c->dev.blob = c->d_recs.as<uint4>();
-    c->dev.li_off = c->d_li_off.as<uint32_t>();
     c->dev.li = c->d_li.as<uint32_t>();
     std::lock_guard<std::mutex> g(circuits_mu);
     circuits.push_back(std::move(c));
@@ -479,7 +462,7 @@ struct fsimb_server {
       ResidentCircuit& c = circuit(r->circuit);
       int cls = -1;
       for (size_t k = 0; k < shapes.size(); ++k)
-        if (shapes[k].M == c.shape.M && shapes[k].threads == c.shape.threads && shapes[k].occ == c.shape.occ)
+        if (shapes[k].M == c.shape.M && shapes[k].threads == c.shape.threads)
           cls = (int)k;
       if (cls < 0) {
         cls = (int)shapes.size();
@@ -501,7 +484,6 @@ struct fsimb_server {
   // Takes the results of slot s's finished wave (mu held).
   void finish(Slot& s) {
     const auto now = Clock::now();
-    int kerr = s.exec.read_err();
     float gpu = 0;
     cudaEventElapsedTime(&gpu, s.e0, s.e1);
     stat_busy_ms += gpu;
@@ -510,19 +492,13 @@ struct fsimb_server {
     if (gpu > 1.0f && work > 0) gwe_per_ms = 0.8 * gwe_per_ms + 0.2 * (work / gpu);
     for (size_t i = 0; i < s.wave.size(); ++i) {
       Request* r = s.wave[i];
-      if (kerr) {
-        r->status = FSIMB_ERR_CUDA;
-        r->error = "a sweep kernel reached its wait limit for a record copy; results discarded";
-        ++stat_failed;
-      } else {
-        r->results.resize(r->job.F);
-        s.exec.results(i, s.jobs[i], r->results.data());
-        ++stat_completed;
-        stat_fault_patterns += (double)r->job.F * (double)r->pats.P;
-        lat_ms.push_back(ms_between(r->t_submit, now));
-        queue_ms.push_back(ms_between(r->t_submit, r->t_launch));
-        gpu_ms.push_back(gpu);
-      }
+      r->results.resize(r->job.F);
+      s.exec.results(i, s.jobs[i], r->results.data());
+      ++stat_completed;
+      stat_fault_patterns += (double)r->job.F * (double)r->pats.P;
+      lat_ms.push_back(ms_between(r->t_submit, now));
+      queue_ms.push_back(ms_between(r->t_submit, r->t_launch));
+      gpu_ms.push_back(gpu);
       r->t_done = now;
       r->done = true;
       // the plan is no longer needed
@@ -655,14 +631,6 @@ void BatchExec::fetch_async(cudaStream_t s) {
     CK(cudaMemcpyAsync(hb + Fp * 8, d_first, F_total * 8, cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(hb + Fp * 16, d_lastflag, F_total, cudaMemcpyDeviceToHost, s));
   }
-  CK(cudaMemcpyAsync(hb + Fp * 17, d_ctl.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-}
-
-int BatchExec::read_err() const {
-  const uint64_t Fp = std::max<uint64_t>(F_total, 1);
-  int kerr = 0;
-  std::memcpy(&kerr, h_res.as<char>() + Fp * 17, sizeof(int));
-  return kerr;
 }
 
 }  // namespace fsimb

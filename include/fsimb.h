@@ -244,10 +244,10 @@ int fsimb_good_po_noalloc(fsimb_handle* h, const uint64_t* d_pattern_words, uint
  * Many circuits, each with its own fault list and pattern block, simulated
  * together.  No counterpart in the reference, whose drivers simulate one
  * circuit per process (main/simple.cpp:21-39, main/MA_partition.cu:40-63).
- * One run launches, for all members at once: the good machine one launch per
- * level index, the sweeps as one persistent launch per words-per-item class
- * pulling (circuit, tile, sweep, subtile) items from a device work counter,
- * and one launch each for FFR tracing and exact faults.  The sequence is
+ * One run launches, for all members at once: the good machine, the sweeps as
+ * one persistent launch per words-per-item class pulling (circuit, tile,
+ * sweep, subtile) items from a device work counter, and one launch each for
+ * FFR tracing and exact faults.  The sequence is
  * captured into a CUDA graph and replayed while the membership stays the same.
  * Members are handles loaded with circuit, faults and patterns; host-only
  * handles (device -1) are enough.  The batch borrows them until

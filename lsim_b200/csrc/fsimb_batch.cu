@@ -3,8 +3,7 @@
 //
 // One run is a fixed launch sequence over all member circuits at once:
 //   * results init: one launch over the faults of every circuit;
-//   * good machine: one k_good_batch launch per level index, holding the
-//     elements of that level of every circuit, all tiles of each;
+//   * good machine: one k_good_batch launch, a CTA per few words of a circuit;
 //   * sweeps: one persistent k_sweep_batch launch per words-per-item class,
 //     its CTAs pulling (circuit, tile, sweep, subtile) items from one device
 //     counter, so circuits of very different sizes share the SMs;
@@ -108,6 +107,8 @@ uint64_t batch_job_static_bytes(const BatchJob& j) {
     t(nl.fi_off.size() * 4);
     t(nl.fi_idx.size() * 4);
     t(p.net.lev_up.size() * 4);
+    t(nl.level_off.size() * 4);
+    t(p.net.gates.size() * sizeof(GateRec));
     t(sc.lvl.size() * 16);
     t(sc.blob.size() * 4);
     t(sc.li.size() * 4);
@@ -122,26 +123,18 @@ uint64_t batch_job_static_bytes(const BatchJob& j) {
   return b;
 }
 
-uint32_t batch_job_good_segments(const BatchJob& j) {
-  if (j.good_resident) return 0;
-  uint32_t n = 0;
-  for (uint32_t l = 0; l < j.nl->n_levels; ++l) n += j.nl->level_off[l + 1] > j.nl->level_off[l];
-  return n;
-}
-
 WaveBytes batch_wave_bytes(const std::vector<BatchJob>& jobs, bool first_tile_only) {
   WaveBytes w;
-  uint64_t F = 0, segs = 0, swept = 0;
+  uint64_t F = 0, swept = 0;
   for (const BatchJob& j : jobs) {
     w.stat += batch_job_static_bytes(j);
     w.work += batch_job_work_bytes(j, first_tile_only);
     F += j.F;
-    segs += batch_job_good_segments(j);
     swept += j.plan->sweeps.empty() ? 0 : 1;
   }
   const uint64_t n = jobs.size();
   w.res = std::max<uint64_t>(F, 1) * 17 + 512;
-  w.desc = align256(n * sizeof(BatchCirc)) + align256(segs * sizeof(BatchGoodSeg)) + 2 * align256((n + 1) * 8);
+  w.desc = align256(n * sizeof(BatchCirc)) + 3 * align256((n + 1) * 8);
   w.ctl = align256((swept + 1) * 8);
   return w;
 }
@@ -151,7 +144,7 @@ WaveBytes batch_job_bytes(const BatchJob& j, bool first_tile_only) {
   w.stat = batch_job_static_bytes(j);
   w.work = batch_job_work_bytes(j, first_tile_only);
   w.res = 17 * j.F;
-  w.desc = sizeof(BatchCirc) + batch_job_good_segments(j) * sizeof(BatchGoodSeg) + 16;
+  w.desc = sizeof(BatchCirc) + 24;
   w.ctl = 8;
   return w;
 }
@@ -195,6 +188,8 @@ uint64_t BatchExec::upload_static(const std::vector<BatchJob>& jobs, cudaStream_
       c.fi_off = j.dev.fi_off;
       c.fi_idx = j.dev.fi_idx;
       c.level = j.dev.level;
+      c.level_off = j.dev.level_off;
+      c.gates = j.dev.gates;
       c.lvl = j.dev.lvl;
       c.blob = j.dev.blob;
       c.li = j.dev.li;
@@ -204,6 +199,8 @@ uint64_t BatchExec::upload_static(const std::vector<BatchJob>& jobs, cudaStream_
       c.fi_off = (const uint32_t*)put(nl.fi_off.data(), nl.fi_off.size() * 4);
       c.fi_idx = (const uint32_t*)put(nl.fi_idx.data(), nl.fi_idx.size() * 4);
       c.level = (const uint32_t*)put(p.net.lev_up.data(), p.net.lev_up.size() * 4);
+      c.level_off = (const uint32_t*)put(nl.level_off.data(), nl.level_off.size() * 4);
+      c.gates = (const uint4*)put(p.net.gates.data(), p.net.gates.size() * sizeof(GateRec));
       c.lvl = (const uint4*)put(sc.lvl.data(), sc.lvl.size() * 16);
       c.blob = (const uint4*)put(sc.blob.data(), sc.blob.size() * 4);
       c.li = (const uint32_t*)put(sc.li.data(), sc.li.size() * 4);
@@ -303,29 +300,6 @@ void BatchExec::layout(const std::vector<BatchJob>& jobs, const std::vector<Clas
   }
 
   // Launch tables.
-  // Good machine: per level index, segments (circuit, element range).
-  segs.clear();
-  level_first_seg.clear();
-  level_units.clear();
-  uint32_t max_levels = 0;
-  for (const BatchJob& j : jobs) max_levels = std::max(max_levels, j.nl->n_levels);
-  good_units = 0;
-  for (uint32_t l = 0; l < max_levels; ++l) {
-    level_first_seg.push_back((uint32_t)segs.size());
-    unsigned long long u = 0;
-    for (size_t i = 0; i < n; ++i) {
-      const Netlist& nl = *jobs[i].nl;
-      if (jobs[i].good_resident || l >= nl.n_levels) continue;
-      const uint32_t lo = nl.level_off[l], hi = nl.level_off[l + 1];
-      if (hi <= lo) continue;
-      segs.push_back(BatchGoodSeg{(uint32_t)i, lo, hi, 0, u});
-      u += (unsigned long long)(hi - lo) * circs[i].tiles;
-    }
-    level_units.push_back(u);
-    good_units += u;
-  }
-  level_first_seg.push_back((uint32_t)segs.size());
-
   // Sweep classes: shapes[c] runs the jobs with cls == c.
   classes.clear();
   uint32_t n_counters = 0;
@@ -363,6 +337,13 @@ void BatchExec::layout(const std::vector<BatchJob>& jobs, const std::vector<Clas
   }
 
   // FFR / exact units: (circuit, tile, root) and (circuit, tile, exact fault).
+  // Good machine units: kGoodBatchWords words of a circuit.
+  good_prefix.assign(n + 1, 0);
+  for (size_t i = 0; i < n; ++i) {
+    const uint32_t words = jobs[i].good_resident ? 0 : std::min<uint32_t>(circs[i].W, circs[i].tiles * kTileWords);
+    good_prefix[i + 1] = good_prefix[i] + (words + kGoodBatchWords - 1) / kGoodBatchWords;
+  }
+  good_units = good_prefix[n];
   ffr_prefix.assign(n + 1, 0);
   exact_prefix.assign(n + 1, 0);
   for (size_t i = 0; i < n; ++i) {
@@ -372,7 +353,7 @@ void BatchExec::layout(const std::vector<BatchJob>& jobs, const std::vector<Clas
   ffr_units = ffr_prefix[n];
   exact_units = exact_prefix[n];
 
-  // Descriptor block: circuits, good segments, class tables, unit prefixes.
+  // Descriptor block: circuits and unit prefixes.
   d_desc.ensure(wb_need.desc);
   h_desc.ensure(wb_need.desc);
   {
@@ -386,7 +367,7 @@ void BatchExec::layout(const std::vector<BatchJob>& jobs, const std::vector<Clas
       return db + o;
     };
     dd_circs = (const BatchCirc*)put(circs.data(), n * sizeof(BatchCirc));
-    dd_segs = (const BatchGoodSeg*)put(segs.data(), segs.size() * sizeof(BatchGoodSeg));
+    dd_good_prefix = (const unsigned long long*)put(good_prefix.data(), (n + 1) * 8);
     dd_ffr_prefix = (const unsigned long long*)put(ffr_prefix.data(), (n + 1) * 8);
     dd_exact_prefix = (const unsigned long long*)put(exact_prefix.data(), (n + 1) * 8);
     CK(cudaMemcpyAsync(d_desc.p, h_desc.p, at, cudaMemcpyHostToDevice, s));
@@ -431,12 +412,8 @@ uint64_t BatchExec::enqueue(cudaStream_t s, bool good_only, bool with_events, cu
     launch_init_results_batch(d_count, d_first, d_lastflag, F_total, s);
     launches += F_total ? 1 : 0;
   }
-  for (size_t l = 0; l + 1 < level_first_seg.size(); ++l) {
-    const uint32_t s0 = level_first_seg[l], s1 = level_first_seg[l + 1];
-    if (s1 == s0) continue;
-    launch_good_batch(dd_circs, dd_segs + s0, s1 - s0, level_units[l], s);
-    ++launches;
-  }
+  launch_good_batch(BatchUnits{dd_circs, dd_good_prefix, n_circ}, good_units, s);
+  launches += good_units ? 1 : 0;
   CK(cudaGetLastError());
   if (with_events) CK(cudaEventRecord(ev[0], s));
   if (good_only) return launches;

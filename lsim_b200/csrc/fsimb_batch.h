@@ -80,10 +80,7 @@ class BatchExec {
 
   std::vector<BatchCirc> circs;
   std::vector<uint64_t> res_off;
-  std::vector<BatchGoodSeg> segs;
-  std::vector<uint32_t> level_first_seg;
-  std::vector<unsigned long long> level_units;
-  std::vector<unsigned long long> ffr_prefix, exact_prefix;
+  std::vector<unsigned long long> good_prefix, ffr_prefix, exact_prefix;
   std::vector<SweepClass> classes;
   unsigned long long ffr_units = 0, exact_units = 0, good_units = 0;
   uint64_t F_total = 0, fault_patterns = 0, dense_gate_words = 0, sweep_alg_bytes = 0,
@@ -103,7 +100,7 @@ class BatchExec {
   cudaEvent_t fork_ev = nullptr;
 
   const BatchCirc* dd_circs = nullptr;
-  const BatchGoodSeg* dd_segs = nullptr;
+  const unsigned long long* dd_good_prefix = nullptr;
   const unsigned long long* dd_ffr_prefix = nullptr;
   const unsigned long long* dd_exact_prefix = nullptr;
   unsigned long long* d_count = nullptr;

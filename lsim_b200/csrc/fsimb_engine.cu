@@ -141,28 +141,17 @@ void fsimb_handle::default_shape(int& M, int& threads) {
       (uint32_t)std::min<uint64_t>(pats.W, kTileWords), smem_optin, smem_per_sm, M, threads);
 }
 
+GoodView fsimb_handle::good_view(uint32_t W) const {
+  return GoodView{d_gates.as<uint4>(), d_level_off.as<uint32_t>(), d_pwords.as<uint64_t>(),
+                  d_good.as<uint64_t>(), (uint32_t)nl.n_pi, nl.N, nl.n_levels, W};
+}
+
 void fsimb_handle::tune_shape(cudaStream_t s) {
   const uint32_t N = plan.N;
   const uint32_t n_sweeps = (uint32_t)plan.sweeps.size();
   for (auto& e : tune_ev)
     if (!e) CK(cudaEventCreate(&e));
-  // good machine of tile 0
-  for (uint32_t l = 0; l < nl.n_levels; ++l) {
-    GoodArgs g{};
-    g.type = d_type.as<uint8_t>();
-    g.fi_off = d_fi_off.as<uint32_t>();
-    g.fi_idx = d_fi_idx.as<uint32_t>();
-    g.pwords = d_pwords.as<uint64_t>();
-    g.good = d_good.as<uint64_t>();
-    g.n_pi = (uint32_t)nl.n_pi;
-    g.N = N;
-    g.lo = nl.level_off[l];
-    g.hi = nl.level_off[l + 1];
-    g.W = (uint32_t)pats.W;
-    g.W_pad = kTileWords;
-    launch_good_level(g, s);
-  }
-  CK(cudaGetLastError());
+  launch_good(good_view(tile_words(pats.W, 0)), nl.level_off.data(), n_sms, s);  // tile 0
   // every stride-th sweep: at most 1 in 16 and about 4,096 of them, so a
   // candidate's run stays short on large circuits
   const uint32_t stride =
@@ -299,6 +288,7 @@ void fsimb_handle::run(const fsimb_opts* opts) {
     upload(d_fi_off, nl.fi_off, s);
     upload(d_fi_idx, nl.fi_idx, s);
     upload(d_level, plan.net.lev_up, s);
+    upload(d_gates, plan.net.gates, s);
     upload(d_level_off, plan.level_off, s);
     upload(d_roots, plan.roots, s);
     upload(d_members, plan.members, s);
@@ -410,22 +400,7 @@ void fsimb_handle::run(const fsimb_opts* opts) {
   CK(cudaEventRecord(e1, s));
 
   // 2. good machine
-  for (uint32_t l = 0; l < nl.n_levels; ++l) {
-    GoodArgs g{};
-    g.type = d_type.as<uint8_t>();
-    g.fi_off = d_fi_off.as<uint32_t>();
-    g.fi_idx = d_fi_idx.as<uint32_t>();
-    g.pwords = d_pwords.as<uint64_t>();
-    g.good = d_good.as<uint64_t>();
-    g.n_pi = (uint32_t)nl.n_pi;
-    g.N = N;
-    g.lo = nl.level_off[l];
-    g.hi = nl.level_off[l + 1];
-    g.W = (uint32_t)W;
-    g.W_pad = (uint32_t)W_pad;
-    launch_good_level(g, s);
-    launches += (g.hi > g.lo) ? 1 : 0;
-  }
+  launches += launch_good(good_view((uint32_t)W), nl.level_off.data(), n_sms, s);
   CK(cudaGetLastError());
   good_tiles = tiles;
   good_P = pats.P;

@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../include/fsimb.h"
+#include "fsimb_kernels.cuh"
 #include "fsimb_loader.h"
 #include "fsimb_netlist.h"
 #include "fsimb_plan.h"
@@ -199,7 +200,7 @@ struct fsimb_handle {
   // another stream that reads the circuit arrays waits for it.
   cudaEvent_t upload_ev = nullptr;
 
-  fsimb::DevBuf d_type, d_fi_off, d_fi_idx, d_recs, d_level, d_level_off, d_li;
+  fsimb::DevBuf d_type, d_fi_off, d_fi_idx, d_recs, d_level, d_level_off, d_gates, d_li;
   fsimb::DevBuf d_lvl;     // schedule: stream and live-in offsets per level
   fsimb::DevBuf d_eflag;   // wide-circuit sweep: per element, evaluated / drives a PO
   fsimb::DevBuf d_gvals;   // wide-circuit sweep: per-CTA value regions
@@ -219,7 +220,7 @@ struct fsimb_handle {
   ~fsimb_handle() {
     if (device >= 0) {
       cudaSetDevice(device);
-      for (fsimb::DevBuf* b : {&d_type, &d_fi_off, &d_fi_idx, &d_recs, &d_level, &d_level_off,
+      for (fsimb::DevBuf* b : {&d_type, &d_fi_off, &d_fi_idx, &d_recs, &d_level, &d_level_off, &d_gates,
                         &d_lvl, &d_eflag, &d_gvals, &d_li, &d_roots, &d_members, &d_traced, &d_inj, &d_exact,
                         &d_pwords, &d_good, &d_out, &d_sens, &d_count, &d_first, &d_lastflag,
                         &d_queue, &d_err, &d_root_list[0], &d_root_list[1], &d_sweep_list,
@@ -244,7 +245,7 @@ struct fsimb_handle {
 
   uint64_t device_bytes() const {
     uint64_t s = 0;
-    for (const fsimb::DevBuf* b : {&d_type, &d_fi_off, &d_fi_idx, &d_recs, &d_level, &d_level_off,
+    for (const fsimb::DevBuf* b : {&d_type, &d_fi_off, &d_fi_idx, &d_recs, &d_level, &d_level_off, &d_gates,
                             &d_lvl, &d_eflag, &d_gvals, &d_li, &d_roots, &d_members, &d_traced, &d_inj, &d_exact,
                             &d_pwords, &d_good, &d_out, &d_sens, &d_count, &d_first, &d_lastflag,
                             &d_queue, &d_err, &d_root_list[0], &d_root_list[1], &d_sweep_list,
@@ -327,6 +328,8 @@ struct fsimb_handle {
   fsimb::Schedule& cached_schedule(int M);
   // The schedule at M packed for T threads, uploaded unless it is there.
   const fsimb::Schedule& use_schedule(int M, int T, cudaStream_t s);
+  // The circuit's good machine on the device for the first W pattern words.
+  fsimb::GoodView good_view(uint32_t W) const;
   // default_sweep_shape for this circuit and the plain sweep kernel.
   void default_shape(int& M, int& threads);
   // Times candidate shapes on a strided sample of tile 0's sweeps and keeps

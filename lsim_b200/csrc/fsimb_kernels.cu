@@ -1,8 +1,7 @@
 // B200 (sm_100a) kernels of the stuck-at fault simulator.
 //
-//   k_good_level   good machine, one launch per level, one thread per
-//                  (element, word); warps cover the 32 words of a tile so every
-//                  fanin read is one coalesced 256-byte segment.
+//   k_good         good machine: a CTA takes a few words through all levels.
+//   k_good_level   the same, one launch per level, for very wide levels.
 //   k_sweep<M>     persistent: each CTA pulls (sweep, M-word subtile) items from
 //                  a device work counter and re-simulates the levels above the
 //                  injection point with all live values in shared memory
@@ -70,30 +69,153 @@ __device__ __forceinline__ uint64_t bits_mask(uint32_t bits) {
   return bits >= 64 ? ~0ull : ((1ull << bits) - 1ull);
 }
 
+// (a ^ i) & b, and x & y or x ^ y by the mask k: one LOP3 each.
+__device__ __forceinline__ uint32_t and_inv(uint32_t a, uint32_t i, uint32_t b) {
+  uint32_t r;
+  asm("lop3.b32 %0, %1, %2, %3, 0x28;" : "=r"(r) : "r"(a), "r"(i), "r"(b));
+  return r;
+}
+__device__ __forceinline__ uint32_t and_or_xor(uint32_t x, uint32_t y, uint32_t k) {
+  uint32_t r;
+  asm("lop3.b32 %0, %1, %2, %3, 0x68;" : "=r"(r) : "r"(x), "r"(y), "r"(k));
+  return r;
+}
+
 // ---------------------------------------------------------------- good
-__global__ void k_good_level(GoodArgs a) {
-  const uint64_t n = (uint64_t)(a.hi - a.lo) * a.W_pad;
+// V consecutive words (1 or 2) of a gate.
+template <int V>
+struct GoodWords {
+  uint64_t v[4][V];
+};
+__device__ __forceinline__ uint32_t gate_type(const uint4& r) {
+  return r.x >> 31 | r.y >> 31 << 1 | r.z >> 31 << 2 | r.w >> 31 << 3;
+}
+template <int V>
+__device__ __forceinline__ GoodWords<V> good_inputs(const uint4& r, const uint64_t* g) {
+  GoodWords<V> x;
+  const uint32_t in[4] = {r.x & kNoInput, r.y & kNoInput, r.z & kNoInput, r.w & kNoInput};
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const uint64_t* p = g + (uint64_t)in[k] * 32;
+    const bool has = in[k] != kNoInput;
+    if constexpr (V == 2) {
+      const ulonglong2 q = has ? *reinterpret_cast<const ulonglong2*>(p) : make_ulonglong2(0, 0);
+      x.v[k][0] = q.x;
+      x.v[k][1] = q.y;
+    } else {
+      x.v[k][0] = has ? *p : 0ull;
+    }
+  }
+  return x;
+}
+// AND and XOR families by masks, as 32-bit halves: a missing input is zeros,
+// inverted in an AND; MUX by its own rule.
+template <int V>
+__device__ __forceinline__ void good_store(const uint4& r, const GoodWords<V>& x, uint64_t* p) {
+  const uint32_t t = gate_type(r);
+  uint64_t o[V];
+  if (t == G_MUX) {
+#pragma unroll
+    for (int j = 0; j < V; ++j) o[j] = eval_word(t, 3, x.v[0][j], x.v[1][j], x.v[2][j], 0ull);
+  } else {
+    const uint32_t ii = 0u - ((kIiMask >> t) & 1u), io = 0u - ((kIoMask >> t) & 1u), kx = 0u - ((kXfMask >> t) & 1u);
+    const uint32_t i1 = (r.y & kNoInput) == kNoInput ? ~kx : ii, i2 = (r.z & kNoInput) == kNoInput ? ~kx : ii,
+                   i3 = (r.w & kNoInput) == kNoInput ? ~kx : ii;
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      uint32_t h[2];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        auto half = [&](int k) { return (uint32_t)(x.v[k][j] >> (32 * q)); };
+        uint32_t y = and_or_xor(half(0) ^ ii, half(1) ^ i1, kx);
+        y = and_or_xor(y, half(2) ^ i2, kx);
+        h[q] = and_or_xor(y, half(3) ^ i3, kx) ^ io;
+      }
+      o[j] = (uint64_t)h[0] | (uint64_t)h[1] << 32;
+    }
+  }
+  if constexpr (V == 2)
+    *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(o[0], o[1]);
+  else
+    *p = o[0];
+}
+
+// All levels of the words [w0, w0 + P) by one CTA: words are independent, so
+// a level needs a barrier, not a launch.  A thread takes two words (one at P
+// = 1) of an element, so P / 2 consecutive lanes share an element; a word
+// beyond the patterns that shares a thread with the last one is computed
+// from its zeros.  200,000 gates, 150 levels: 1,024 words 2.18 -> 0.95 ms (P =
+// 8); 6,586 gates, 157 words 270 -> 57 us; 400 gates, one word 67 -> 14 us
+// (P = 1), against one launch per level.
+template <int P>
+__device__ __forceinline__ void good_words(const GoodView& a, uint32_t w0) {
+  constexpr int V = P == 1 ? 1 : 2, L = P / V;  // words per thread, lanes per element
+  const uint32_t t = threadIdx.x / L, step = blockDim.x / L, w = w0 + threadIdx.x % L * V;
+  const bool on = w < a.W;
+  uint64_t* g = a.good + ((uint64_t)(w >> 5) * a.N) * 32 + (w & 31u);
+  if (on)
+    for (uint32_t e = t; e < a.n_pi; e += step)
+#pragma unroll
+      for (int j = 0; j < V; ++j) g[(uint64_t)e * 32 + j] = w + j < a.W ? a.pwords[(uint64_t)(w + j) * a.n_pi + e] : 0ull;
+  __syncthreads();
+  // Steps of U elements a thread: the next step's gate records (and the next
+  // level's bound) are loaded before this step's words are waited for, so a
+  // level costs the words' latency and a barrier.
+  constexpr int U = 2;
+  const uint4 none = make_uint4(kNoInput, kNoInput, kNoInput, kNoInput);
+  auto bound = [&](uint32_t level) { return a.level_off[min(level, a.n_levels - 1) + 1]; };
+  uint32_t l = 1, hi = bound(1), e = a.level_off[1] + t, hi1 = bound(2), hi2 = bound(3);
+  uint4 q[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) q[u] = e + u * step < hi ? a.gates[e + u * step] : none;
+  while (l < a.n_levels) {
+    // the step after this one: (level, element) and its bound
+    const bool last = e - t + U * step >= hi;  // the same for every thread of the CTA
+    const uint32_t ne = last ? hi + t : e + U * step, nh = last ? hi1 : hi;
+    if (last) {
+      hi1 = hi2;
+      hi2 = bound(l + 3);
+    }
+    uint4 nq[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) nq[u] = ne + u * step < nh ? a.gates[ne + u * step] : none;
+    if (on && e < hi) {
+      GoodWords<V> x[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) x[u] = good_inputs<V>(q[u], g);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (e + u * step < hi) good_store<V>(q[u], x[u], g + (uint64_t)(e + u * step) * 32);
+    }
+    if (last) {
+      __syncthreads();
+      ++l;
+    }
+    hi = nh;
+    e = ne;
+#pragma unroll
+    for (int u = 0; u < U; ++u) q[u] = nq[u];
+  }
+}
+
+template <int P>
+__global__ void __launch_bounds__(1024) k_good(GoodView a) { good_words<P>(a, blockIdx.x * P); }
+
+// One level of all words, for circuits whose levels are too wide for the
+// words' CTAs to cover (launch_good): one thread per (element, word).
+__global__ void k_good_level(GoodView a, uint32_t lo, uint32_t hi) {
+  const uint64_t n = (uint64_t)(hi - lo) * a.W;
   for (uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n;
        idx += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t w = (uint32_t)(idx % a.W_pad);
-    const uint32_t e = a.lo + (uint32_t)(idx / a.W_pad);
-    const uint32_t tile = w >> 5, lane = w & 31u;
-    const uint64_t base = (uint64_t)tile * a.N;
-    const uint8_t t = a.type[e];
-    uint64_t v;
-    if (t == G_PI) {
-      v = (w < a.W) ? a.pwords[(uint64_t)w * a.n_pi + e] : 0ull;
+    const uint32_t w = (uint32_t)(idx % a.W);
+    const uint32_t e = lo + (uint32_t)(idx / a.W);
+    uint64_t* g = a.good + ((uint64_t)(w >> 5) * a.N) * 32 + (w & 31u);
+    if (e < a.n_pi) {
+      g[(uint64_t)e * 32] = a.pwords[(uint64_t)w * a.n_pi + e];
     } else {
-      const uint32_t f0 = a.fi_off[e];
-      uint32_t nf = a.fi_off[e + 1] - f0;
-      if (t == G_INV || t == G_CLKBUF || t == G_PO) nf = 1;
-      uint64_t in[4] = {0, 0, 0, 0};
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if ((uint32_t)k < nf) in[k] = a.good[(base + a.fi_idx[f0 + k]) * 32 + lane];
-      v = eval_word(t, nf, in[0], in[1], in[2], in[3]);
+      const uint4 q = a.gates[e];
+      good_store<1>(q, good_inputs<1>(q, g), g + (uint64_t)e * 32);
     }
-    a.good[(base + e) * 32 + lane] = v;
   }
 }
 
@@ -243,18 +365,6 @@ __device__ __forceinline__ void sts(uint32_t addr, const Chunk<M>& c) {
                  "r"(c.r[3])
                  : "memory");
 }
-// (a ^ i) & b, and x & y or x ^ y by the mask k: one LOP3 each.
-__device__ __forceinline__ uint32_t and_inv(uint32_t a, uint32_t i, uint32_t b) {
-  uint32_t r;
-  asm("lop3.b32 %0, %1, %2, %3, 0x28;" : "=r"(r) : "r"(a), "r"(i), "r"(b));
-  return r;
-}
-__device__ __forceinline__ uint32_t and_or_xor(uint32_t x, uint32_t y, uint32_t k) {
-  uint32_t r;
-  asm("lop3.b32 %0, %1, %2, %3, 0x68;" : "=r"(r) : "r"(x), "r"(y), "r"(k));
-  return r;
-}
-
 // A record (fsimb_plan.h RecKind): two words, four at one word per item.
 template <int M>
 using RecWords = typename std::conditional<M == 1, uint4, uint2>::type;
@@ -817,39 +927,13 @@ struct TileView {
   const uint64_t* good;
 };
 
-// One warp per (element, tile) of a level, over the circuits of the batch.
-__global__ void __launch_bounds__(256) k_good_batch(const BatchCirc* circs, const BatchGoodSeg* segs,
-                                                    uint32_t n_segs, unsigned long long n_units) {
-  const uint32_t lane = threadIdx.x & 31u;
-  const unsigned long long unit = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (unit >= n_units) return;
-  uint32_t lo = 0, hi = n_segs;
-  while (hi - lo > 1) {
-    const uint32_t mid = (lo + hi) / 2;
-    if (segs[mid].unit0 <= unit) lo = mid; else hi = mid;
-  }
-  const BatchGoodSeg sg = segs[lo];
-  const BatchCirc& c = circs[sg.circ];
-  const unsigned long long local = unit - sg.unit0;
-  const uint32_t e = sg.lo + (uint32_t)(local / c.tiles);
-  const uint32_t tile = (uint32_t)(local % c.tiles);
-  const uint32_t w = tile * 32 + lane;
-  const uint64_t base = (uint64_t)tile * c.N;
-  const uint8_t t = c.type[e];
-  uint64_t v;
-  if (t == G_PI) {
-    v = (w < c.W) ? c.pwords[(uint64_t)w * c.n_pi + e] : 0ull;
-  } else {
-    const uint32_t f0 = c.fi_off[e];
-    uint32_t nf = c.fi_off[e + 1] - f0;
-    if (t == G_INV || t == G_CLKBUF || t == G_PO) nf = 1;
-    uint64_t in[4] = {0, 0, 0, 0};
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-      if ((uint32_t)k < nf) in[k] = c.good[(base + c.fi_idx[f0 + k]) * 32 + lane];
-    v = eval_word(t, nf, in[0], in[1], in[2], in[3]);
-  }
-  c.good[(base + e) * 32 + lane] = v;
+// One CTA per (circuit, kGoodBatchWords words) of the batch.
+__global__ void __launch_bounds__(256) k_good_batch(BatchUnits u) {
+  const uint32_t ci = find_prefix(u.unit_prefix, u.n_circ, blockIdx.x);
+  const BatchCirc& c = u.circs[ci];
+  const GoodView v{c.gates, c.level_off, c.pwords, c.good, c.n_pi, c.N, c.n_levels,
+                   min(c.W, c.tiles * kTileWords)};
+  good_words<kGoodBatchWords>(v, (uint32_t)(blockIdx.x - u.unit_prefix[ci]) * kGoodBatchWords);
 }
 
 // One warp per (circuit, tile, root): the k_ffr body on that circuit's tile.
@@ -960,10 +1044,9 @@ __global__ void k_drop(DropArgs a) {
 
 }  // namespace
 
-void launch_good_batch(const BatchCirc* circs, const BatchGoodSeg* segs, uint32_t n_segs,
-                       unsigned long long n_units, cudaStream_t s) {
+void launch_good_batch(const BatchUnits& u, unsigned long long n_units, cudaStream_t s) {
   if (!n_units) return;
-  k_good_batch<<<(unsigned)((n_units * 32 + 255) / 256), 256, 0, s>>>(circs, segs, n_segs, n_units);
+  k_good_batch<<<(unsigned)n_units, 256, 0, s>>>(u);
 }
 
 void launch_ffr_batch(const BatchUnits& u, unsigned long long n_units, cudaStream_t s) {
@@ -1013,13 +1096,47 @@ cudaError_t launch_sweep_batch(int M, int threads, int blocks, size_t smem, cons
   return cudaGetLastError();
 }
 
-void launch_good_level(const GoodArgs& a, cudaStream_t s) {
-  const uint64_t n = (uint64_t)(a.hi - a.lo) * a.W_pad;
-  if (n == 0) return;
-  const int threads = 256;
-  uint64_t blocks = (n + threads - 1) / threads;
-  if (blocks > 148ull * 64) blocks = 148ull * 64;
-  k_good_level<<<(unsigned)blocks, threads, 0, s>>>(a);
+uint32_t launch_good(const GoodView& a, const uint32_t* level_off, int n_sms, cudaStream_t s) {
+  if (!a.W || !a.N) return 0;
+  // Words per CTA: as few as leave at most one CTA an SM.
+  uint32_t p = 1;
+  while (p < 8 && (a.W + p - 1) / p > (uint32_t)n_sms) p *= 2;
+  // Time by levels, us: a barrier, latency and the elements' share for the
+  // words' CTAs against a launch and all words' share of the chip.  Measured
+  // us a level: 32 words at 1,333 gates 3.2 against 4.5, at 5,000 11.6 against
+  // 5.2, at 50,000 105 against 15; 1,024 words at 1,333 gates 6.2 against 13,
+  // at 50,000 197 against 279.
+  const uint32_t waves = ((a.W + p - 1) / p + (uint32_t)n_sms - 1) / (uint32_t)n_sms;
+  const double per_elem = (p == 8 ? 3.9e-3 : p == 4 ? 2.6e-3 : 2.1e-3) * waves;
+  double by_words = 0, by_levels = 0;
+  for (uint32_t l = 1; l < a.n_levels; ++l) {
+    const double n = level_off[l + 1] - level_off[l];
+    by_words += 1 + n * per_elem;
+    by_levels += 4.5 + n * a.W * 5.4e-6;
+  }
+  if (by_words > by_levels) {
+    uint32_t launches = 0;
+    for (uint32_t l = 0; l < a.n_levels; ++l) {
+      const uint64_t n = (uint64_t)(level_off[l + 1] - level_off[l]) * a.W;
+      if (!n) continue;
+      const uint64_t blocks = std::min<uint64_t>((n + 255) / 256, 148ull * 64);
+      k_good_level<<<(unsigned)blocks, 256, 0, s>>>(a, level_off[l], level_off[l + 1]);
+      ++launches;
+    }
+    return launches;
+  }
+  // A thread per element of a typical level and pair of words: more would
+  // only run the loop's overhead.
+  const uint64_t lanes = (uint64_t)(a.N - a.n_pi) / std::max<uint32_t>(a.n_levels - 1, 1) * 5 / 4 * std::max(p / 2, 1u);
+  const unsigned threads = (unsigned)std::min<uint64_t>(1024, std::max<uint64_t>(64, (lanes + 31) / 32 * 32));
+  const unsigned blocks = (a.W + p - 1) / p;
+  switch (p) {
+    case 1: k_good<1><<<blocks, threads, 0, s>>>(a); break;
+    case 2: k_good<2><<<blocks, threads, 0, s>>>(a); break;
+    case 4: k_good<4><<<blocks, threads, 0, s>>>(a); break;
+    default: k_good<8><<<blocks, threads, 0, s>>>(a); break;
+  }
+  return 1;
 }
 
 cudaError_t sweep_set_smem(int M, size_t smem) {

@@ -10,15 +10,13 @@
 
 namespace fsimb {
 
-struct GoodArgs {
-  const uint8_t* type;
-  const uint32_t* fi_off;
-  const uint32_t* fi_idx;
-  const uint64_t* pwords;  // [W][n_pi]
-  uint64_t* good;          // [tiles][N][32]
-  uint32_t n_pi, N;
-  uint32_t lo, hi;         // element range of one level
-  uint32_t W, W_pad;       // real and padded word counts
+struct GoodView {
+  const uint4* gates;         // GateRec per element
+  const uint32_t* level_off;  // [n_levels + 1]
+  const uint64_t* pwords;     // [W][n_pi]
+  uint64_t* good;             // [tiles][N][32]; words at and beyond W are left as they are
+  uint32_t n_pi, N, n_levels;
+  uint32_t W;
 };
 
 struct SweepArgs {
@@ -127,6 +125,8 @@ struct BatchCirc {
   const uint4* blob;
   const uint4* lvl;
   const uint32_t* level;
+  const uint32_t* level_off;
+  const uint4* gates;
   const uint32_t* li;
   const uint32_t* fi_off;
   const uint32_t* fi_idx;
@@ -180,23 +180,18 @@ struct BatchSweepParams {
 };
 static_assert(sizeof(BatchSweepParams) <= 32000, "kernel parameters are limited to 32,764 bytes");
 
-// A level of the batched good machine: segments (circuit, element range)
-// with one warp per (element, tile).
-struct BatchGoodSeg {
-  uint32_t circ, lo, hi, pad;
-  unsigned long long unit0;  // first unit of the segment
-};
+constexpr int kGoodBatchWords = 4;  // words per CTA of the batched good machine
 
-// Units of the batched tracing kernels: one warp per (circuit, tile, root)
-// or (circuit, tile, exact fault); prefix over circuits.
+// Units of the batched kernels: one warp per (circuit, tile, root) or
+// (circuit, tile, exact fault), one CTA per (circuit, words); prefix over
+// circuits.
 struct BatchUnits {
   const BatchCirc* circs;
   const unsigned long long* unit_prefix;  // [n_circ + 1]
   uint32_t n_circ;
 };
 
-void launch_good_batch(const BatchCirc* circs, const BatchGoodSeg* segs, uint32_t n_segs,
-                       unsigned long long n_units, cudaStream_t s);
+void launch_good_batch(const BatchUnits& u, unsigned long long n_units, cudaStream_t s);
 cudaError_t launch_sweep_batch(int M, int threads, int blocks, size_t smem, const BatchSweepParams& p,
                                cudaStream_t s);
 cudaError_t sweep_batch_set_smem(int M, size_t smem);
@@ -206,7 +201,9 @@ void launch_exact_batch(const BatchUnits& u, unsigned long long n_units, cudaStr
 void launch_init_results_batch(unsigned long long* count, unsigned long long* first, uint8_t* lastflag,
                                uint64_t F, cudaStream_t s);
 
-void launch_good_level(const GoodArgs& a, cudaStream_t s);
+// The good machine of all words; level_off is the host's copy.  Returns the
+// kernels launched.
+uint32_t launch_good(const GoodView& a, const uint32_t* level_off, int n_sms, cudaStream_t s);
 // Returns cudaErrorInvalidValue when M is unsupported.
 cudaError_t launch_sweep(int M, int threads, int blocks, size_t smem, const SweepArgs& a,
                          cudaStream_t s);

@@ -57,6 +57,12 @@ bool add_term(Cluster& c, const Cluster& t, uint32_t inv) {
 void build_sweep_net(const Netlist& nl, const Plan& P, SweepNet& net) {
   const uint32_t N = nl.N;
   net = SweepNet();
+  net.gates.resize(N);
+  for (uint32_t e = 0; e < N; ++e) {
+    const uint32_t nf = std::min<uint32_t>(eff_fanin(nl, e), 4);
+    for (uint32_t k = 0; k < 4; ++k)
+      net.gates[e][k] = (k < nf ? nl.fi_idx[nl.fi_off[e] + k] : kNoInput) | (nl.type[e] >> k & 1u) << 31;
+  }
   // A PO is reached: the element is a PO, or a live element reads it.
   net.live.assign(N, 0);
   for (int64_t e = (int64_t)N - 1; e >= 0; --e) {

@@ -3,6 +3,7 @@
 //
 // Layout in HBM (all arrays indexed by the reference's topological index):
 //   type[N]            u8 gate type
+//   gates[N]           inputs and type of each gate in one record (GateRec)
 //   fi_off[N+1], fi_idx[E]   fanin CSR in pin order (good-machine kernel)
 //   blob[]             the sweep's record stream, 8 bytes a record, level
 //                      after level in order of evaluation.  A record is a
@@ -137,7 +138,14 @@ struct Cluster {
   uint8_t is_xor;
   uint8_t inv;      // the output inverted
 };
+// A gate for the good machine, one 16-byte load: its inputs' indices, the
+// bits of the type in the top bits (bit k of the type in word k); an input
+// it does not have, or does not read, is kNoInput.
+using GateRec = std::array<uint32_t, 4>;
+constexpr uint32_t kNoInput = 0x7FFFFFFFu;
+
 struct SweepNet {
+  std::vector<GateRec> gates;       // [N]
   std::vector<uint32_t> lev_up;     // [N] level, or kFolded | consumer
   std::vector<uint32_t> use_level;  // [N] highest level of a record that reads it (0: none, no slot)
   std::vector<uint32_t> cluster;    // [N] index into clusters; kNoSlot: no cluster record

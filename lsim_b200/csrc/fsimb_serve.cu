@@ -61,17 +61,17 @@ struct ResidentCircuit {
   Patterns block;  // resident pattern block (host copy of its words)
   uint64_t block_tiles = 0;
   // d_recs holds the schedule's record stream
-  DevBuf d_type, d_fi_off, d_fi_idx, d_level, d_lvl, d_recs, d_li, d_pwords, d_good;
+  DevBuf d_type, d_fi_off, d_fi_idx, d_level, d_level_off, d_gates, d_lvl, d_recs, d_li, d_pwords, d_good;
   BatchCirc dev{};
   uint64_t device_bytes() const {
     uint64_t s = 0;
-    for (const DevBuf* b : {&d_type, &d_fi_off, &d_fi_idx, &d_level, &d_lvl, &d_recs, &d_li,
+    for (const DevBuf* b : {&d_type, &d_fi_off, &d_fi_idx, &d_level, &d_level_off, &d_gates, &d_lvl, &d_recs, &d_li,
                             &d_pwords, &d_good})
       s += b->n;
     return s;
   }
   void release() {
-    for (DevBuf* b : {&d_type, &d_fi_off, &d_fi_idx, &d_level, &d_lvl, &d_recs, &d_li,
+    for (DevBuf* b : {&d_type, &d_fi_off, &d_fi_idx, &d_level, &d_level_off, &d_gates, &d_lvl, &d_recs, &d_li,
                       &d_pwords, &d_good})
       b->release();
   }
@@ -295,6 +295,8 @@ struct fsimb_server {
       upload(c->d_fi_off, nl.fi_off, s);
       upload(c->d_fi_idx, nl.fi_idx, s);
       upload(c->d_level, B.net.lev_up, s);
+      upload(c->d_level_off, nl.level_off, s);
+      upload(c->d_gates, B.net.gates, s);
       upload(c->d_lvl, c->sched.lvl, s);
       upload(c->d_recs, c->sched.blob, s);
       upload(c->d_li, c->sched.li, s);
@@ -302,21 +304,9 @@ struct fsimb_server {
       if (c->block.W) {
         upload(c->d_pwords, c->block.words, s);
         c->d_good.ensure(c->block_tiles * nl.N * kTileWords * 8);
-        for (uint32_t l = 0; l < nl.n_levels; ++l) {
-          GoodArgs g{};
-          g.type = c->d_type.as<uint8_t>();
-          g.fi_off = c->d_fi_off.as<uint32_t>();
-          g.fi_idx = c->d_fi_idx.as<uint32_t>();
-          g.pwords = c->d_pwords.as<uint64_t>();
-          g.good = c->d_good.as<uint64_t>();
-          g.n_pi = (uint32_t)nl.n_pi;
-          g.N = nl.N;
-          g.lo = nl.level_off[l];
-          g.hi = nl.level_off[l + 1];
-          g.W = (uint32_t)c->block.W;
-          g.W_pad = (uint32_t)(c->block_tiles * kTileWords);
-          launch_good_level(g, s);
-        }
+        launch_good(GoodView{c->d_gates.as<uint4>(), c->d_level_off.as<uint32_t>(), c->d_pwords.as<uint64_t>(),
+                             c->d_good.as<uint64_t>(), (uint32_t)nl.n_pi, nl.N, nl.n_levels, (uint32_t)c->block.W},
+                    nl.level_off.data(), n_sms, s);
         CK(cudaGetLastError());
       }
       CK(cudaStreamSynchronize(s));
@@ -330,6 +320,8 @@ struct fsimb_server {
     c->dev.fi_off = c->d_fi_off.as<uint32_t>();
     c->dev.fi_idx = c->d_fi_idx.as<uint32_t>();
     c->dev.level = c->d_level.as<uint32_t>();
+    c->dev.level_off = c->d_level_off.as<uint32_t>();
+    c->dev.gates = c->d_gates.as<uint4>();
     c->dev.lvl = c->d_lvl.as<uint4>();
     c->dev.blob = c->d_recs.as<uint4>();
     c->dev.li = c->d_li.as<uint32_t>();

@@ -51,3 +51,19 @@ def test_batch_of_all_sizes():
             b.run(words_per_item=m)
             for s, ref in zip(sims, refs):
                 _same(s.results(), ref)
+
+
+@pytest.mark.parametrize("n_words", [1, 2, 147, 148, 149, 296, 297, 592, 593, 1200])
+@pytest.mark.parametrize("gates,levels", [(300, 12), (9000, 3)])
+def test_good_machine_word_counts(n_words, gates, levels):
+    """Good-machine values at the edges of the words per CTA, narrow levels
+    (all levels in one launch) and wide ones, against the oracle."""
+    P = 64 * n_words - 5
+    w = gen.generate(n_gates=gates, n_pi=20, n_po=15, n_levels=levels, n_patterns=P, seed=n_words,
+                     type_mask=gen.ALL_TYPES)
+    sim = Simulator(0)
+    sim.read_text(w["ckt"], "0\n", w["ptn"])
+    sim.run()
+    ref = Oracle(w["ckt"], "0\n", w["ptn"])
+    for rd in sorted({0, n_words // 2, n_words - 1}):
+        assert np.array_equal(sim.good_values(rd), ref.good_values(rd)), rd

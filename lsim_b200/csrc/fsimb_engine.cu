@@ -377,7 +377,7 @@ void fsimb_handle::run(const fsimb_opts* opts) {
   if (wide) {
     M = o.words_per_item == 1 || (!o.words_per_item && W == 1) ? 1 : 2;
     threads = 256;
-    if (!eflag_uploaded) {
+    if (!eflag_uploaded && n_sweeps) {
       std::vector<uint8_t> fl(N, 0);
       for (uint32_t e = plan.n_pi; e < N; ++e)
         fl[e] = (uint8_t)((plan.net.live[e] && nl.type[e] != G_PO) ? 1 : 0) | (uint8_t)(plan.po_drv[e] ? 2 : 0);

@@ -32,18 +32,27 @@ namespace {
 
 constexpr uint32_t kInvLit = 0x80000000u;
 
+// A cluster while clusters are formed, over netlist elements.
+struct Form {
+  uint32_t lit[3];
+  uint8_t n, is_xor, inv, pad;
+};
+
+inline void add_literal(Form& c, uint32_t lit) {
+  if (c.is_xor) {  // its inversion turns the output
+    c.inv ^= (uint8_t)(lit >> 31);
+    lit &= ~kInvLit;
+  }
+  c.lit[c.n++] = lit;
+}
+
 // Adds the literals of `t`, inverted by `inv`, to cluster c.  False if the
 // result is not one AND or XOR of three literals.
-bool add_term(Cluster& c, const Cluster& t, uint32_t inv) {
+bool add_term(Form& c, const Form& t, uint32_t inv) {
   const uint32_t tinv = t.inv ^ inv;
   if (c.n + t.n > 3) return false;
   if (t.n == 1) {  // a literal (its inversion is in the literal)
-    if (c.is_xor) {
-      c.lit[c.n++] = t.lit[0] & ~kInvLit;
-      c.inv ^= (uint8_t)(tinv ^ (t.lit[0] >> 31));
-    } else {
-      c.lit[c.n++] = t.lit[0] ^ (tinv ? kInvLit : 0u);
-    }
+    add_literal(c, t.lit[0] ^ (tinv ? kInvLit : 0u));
     return true;
   }
   if (t.is_xor != c.is_xor || (!c.is_xor && tinv)) return false;
@@ -54,15 +63,17 @@ bool add_term(Cluster& c, const Cluster& t, uint32_t inv) {
 
 }  // namespace
 
-void build_sweep_net(const Netlist& nl, const Plan& P, SweepNet& net) {
-  const uint32_t N = nl.N;
-  net = SweepNet();
-  net.gates.resize(N);
-  for (uint32_t e = 0; e < N; ++e) {
+static void build_gate_recs(const Netlist& nl, std::vector<GateRec>& gates) {
+  gates.resize(nl.N);
+  for (uint32_t e = 0; e < nl.N; ++e) {
     const uint32_t nf = std::min<uint32_t>(eff_fanin(nl, e), 4);
     for (uint32_t k = 0; k < 4; ++k)
-      net.gates[e][k] = (k < nf ? nl.fi_idx[nl.fi_off[e] + k] : kNoInput) | (nl.type[e] >> k & 1u) << 31;
+      gates[e][k] = (k < nf ? nl.fi_idx[nl.fi_off[e] + k] : kNoInput) | (nl.type[e] >> k & 1u) << 31;
   }
+}
+
+void build_sweep_net(const Netlist& nl, const Plan& P, SweepNet& net) {
+  const uint32_t N = nl.N;
   // A PO is reached: the element is a PO, or a live element reads it.
   net.live.assign(N, 0);
   for (int64_t e = (int64_t)N - 1; e >= 0; --e) {
@@ -72,7 +83,7 @@ void build_sweep_net(const Netlist& nl, const Plan& P, SweepNet& net) {
     for (uint32_t k = 0; k < nf; ++k) net.live[nl.fi_idx[nl.fi_off[e] + k]] = 1;
   }
   // Clusters of the gates that have one, bottom up.
-  std::vector<Cluster> form(N, Cluster{});  // n == 0: no cluster form
+  std::vector<Form> form(N, Form{});  // n == 0: no cluster form
   net.lev_up = nl.level;
   const uint32_t g1 = P.n_pi + P.n_gates;
   for (uint32_t e = P.n_pi; e < g1; ++e) {
@@ -83,26 +94,27 @@ void build_sweep_net(const Netlist& nl, const Plan& P, SweepNet& net) {
     const bool inverts = t == G_INV || t == G_NAND || t == G_NOR || t == G_XNOR;
     const uint32_t io = inverts != (bool)ii;  // OR and NOR are ANDs of inverted inputs
     const uint32_t* in = &nl.fi_idx[nl.fi_off[e]];
+    const Form empty{{0, 0, 0}, 0, (uint8_t)(gate_family(t) == 1 && nf > 1), (uint8_t)io, 0};
     uint32_t may = 0;  // inputs that can be folded in
     for (uint32_t k = 0; k < nf; ++k)
       if (form[in[k]].n && nl.fo_off[in[k] + 1] - nl.fo_off[in[k]] == 1) may |= 1u << k;
     // The subset of them that folds the most gates; of those one with the
     // fewest literals.
-    Cluster best{};
+    Form best = empty;
     int best_score = -1;
     uint32_t best_set = 0;
-    for (uint32_t set = may;; set = (set - 1) & may) {
-      Cluster c{};
-      c.is_xor = gate_family(t) == 1 && nf > 1;
-      c.inv = (uint8_t)io;
+    for (uint32_t set = may; set; set = (set - 1) & may) {
+      Form c = empty;
       bool ok = true;
-      for (uint32_t k = 0; k < nf && ok; ++k) {
-        const Cluster leaf{{in[k], 0, 0}, {0, 0, 0}, 1, 0, 0};
-        if (nf == 1 && set) {  // BUF / INV of a folded gate: that gate's form
-          c = form[in[0]];
-          c.inv ^= (uint8_t)io;
-        } else {
-          ok = add_term(c, (set >> k) & 1u ? form[in[k]] : leaf, ii);
+      if (nf == 1) {  // BUF / INV of a folded gate: that gate's form
+        c = form[in[0]];
+        c.inv ^= (uint8_t)io;
+      } else {
+        for (uint32_t k = 0; k < nf && ok; ++k) {
+          if ((set >> k) & 1u)
+            ok = add_term(c, form[in[k]], ii);
+          else if ((ok = c.n < 3))
+            add_literal(c, in[k] | ii << 31);
         }
       }
       const int score = __builtin_popcount(set) * 4 + 3 - c.n;
@@ -111,8 +123,9 @@ void build_sweep_net(const Netlist& nl, const Plan& P, SweepNet& net) {
         best_score = score;
         best_set = set;
       }
-      if (set == 0) break;
     }
+    if (!best_set)
+      for (uint32_t k = 0; k < nf; ++k) add_literal(best, in[k] | ii << 31);
     if (best.n == 1 && best.inv) {  // one literal takes the inversion
       best.lit[0] ^= kInvLit;
       best.inv = 0;
@@ -141,28 +154,36 @@ void build_sweep_net(const Netlist& nl, const Plan& P, SweepNet& net) {
   net.cluster.assign(N, kNoSlot);
   net.use_level.assign(N, 0);
   net.fix_first.assign(N, kNoSlot);
-  std::vector<std::pair<uint32_t, uint32_t>> via;  // (alias, element whose record reads it)
+  std::vector<std::pair<uint32_t, uint32_t>> via;  // (alias, element whose record reads it), once each
+  std::vector<uint32_t> last_via(N, kNoSlot);
+  net.clusters.reserve(P.n_gates);
   for (uint32_t e = P.n_pi; e < g1; ++e) {
     if (!net.live[e] || (net.lev_up[e] & kFolded) || net.alias[e] != kNoSlot) continue;
     const uint32_t L = nl.level[e];
     auto read = [&](uint32_t x) { net.use_level[x] = std::max(net.use_level[x], L); };
     if (P.po_drv[e]) net.use_level[e] = L + 1;  // its PO record
-    Cluster c = form[e];
-    if (c.n) {
+    const Form& f = form[e];
+    if (f.n) {
+      net.cluster[e] = (uint32_t)net.clusters.size();
+      net.clusters.push_back(Cluster{{f.lit[0], f.lit[1], f.lit[2]}, {0, 0, 0}, f.n, f.is_xor, f.inv});
+      Cluster& c = net.clusters.back();
       for (uint32_t k = 0; k < c.n; ++k) {
         const uint32_t x = c.lit[k] & ~kInvLit;
         c.via[k] = x;
-        // the literal's inversion goes to an XOR's output
-        if (net.alias[x] != kNoSlot) c.lit[k] = net.alias[x] ^ (c.lit[k] & kInvLit);
-        if (c.is_xor) {
-          c.inv ^= (uint8_t)(c.lit[k] >> 31);
-          c.lit[k] &= ~kInvLit;
+        if (net.alias[x] != kNoSlot) {
+          c.lit[k] = net.alias[x] ^ (c.lit[k] & kInvLit);
+          if (c.is_xor) {  // the alias's inversion goes to the output
+            c.inv ^= (uint8_t)(c.lit[k] >> 31);
+            c.lit[k] &= ~kInvLit;
+          }
+          for (uint32_t y = x; net.alias[y] != kNoSlot; y = net.alias_of[y])
+            if (last_via[y] != e) {
+              last_via[y] = e;
+              via.emplace_back(y, e);
+            }
         }
         read(c.lit[k] & ~kInvLit);
-        for (uint32_t y = x; net.alias[y] != kNoSlot; y = net.alias_of[y]) via.emplace_back(y, e);
       }
-      net.cluster[e] = (uint32_t)net.clusters.size();
-      net.clusters.push_back(c);
     } else {
       const uint32_t nf = std::min<uint32_t>(eff_fanin(nl, e), 4);
       for (uint32_t k = 0; k < nf; ++k) read(nl.fi_idx[nl.fi_off[e] + k]);
@@ -173,17 +194,22 @@ void build_sweep_net(const Netlist& nl, const Plan& P, SweepNet& net) {
     if (net.live[e] && !(net.lev_up[e] & kFolded) && net.alias[e] == kNoSlot) net.level_recs[nl.level[e]]++;
   for (uint32_t e = 0; e < g1; ++e)
     if (P.po_drv[e]) net.level_recs[nl.level[e] + 1]++;
-  // Fix lists (elements ascending, so by level).
-  std::sort(via.begin(), via.end());
-  via.erase(std::unique(via.begin(), via.end()), via.end());
-  for (size_t i = 0; i < via.size(); ++i) {
-    if (i == 0 || via[i].first != via[i - 1].first) net.fix_first[via[i].first] = (uint32_t)net.fixes.size();
-    net.fixes.push_back(via[i].second);
-    if (i + 1 == via.size() || via[i + 1].first != via[i].first) net.fixes.push_back(kNoSlot);
-  }
+  // Fix lists: by alias, elements ascending and so by level.
+  std::vector<uint32_t> count(N, 0);
+  for (const auto& v : via) ++count[v.first];
+  uint32_t at = 0;
+  for (uint32_t e = 0; e < N; ++e)
+    if (count[e]) {
+      net.fix_first[e] = at;
+      at += count[e] + 1;
+    }
+  net.fixes.assign(at, kNoSlot);
+  for (const auto& v : via) net.fixes[net.fix_first[v.first]++] = v.second;
+  for (uint32_t e = 0; e < N; ++e)
+    if (count[e]) net.fix_first[e] -= count[e];
 }
 
-void build_circuit_plan(const Netlist& nl, CircuitPlan& C) {
+void build_circuit_plan(const Netlist& nl, CircuitPlan& C, bool sweeps) {
   C = CircuitPlan();
   Plan& P = C.base;
   const uint32_t N = nl.N;
@@ -227,8 +253,9 @@ void build_circuit_plan(const Netlist& nl, CircuitPlan& C) {
   // What sweeps evaluate, and the peak number of live values (interval graph
   // of [level, highest reading level]), over all gates and over the stored
   // ones; a schedule may need a few more slots to honour residues.
-  build_sweep_net(nl, P, P.net);
-  {
+  build_gate_recs(nl, P.net.gates);
+  if (sweeps) build_sweep_net(nl, P, P.net);
+  if (sweeps) {
     auto peak = [&](const std::vector<uint32_t>& last) {
       std::vector<int64_t> delta(nl.n_levels + 2, 0);
       for (uint32_t e = 0; e < N; ++e)
@@ -392,7 +419,7 @@ void build_fault_plan(const Netlist& nl, const CircuitPlan& C, const std::vector
 
 void build_plan(const Netlist& nl, const std::vector<Fault>& faults, Plan& P) {
   CircuitPlan C;
-  build_circuit_plan(nl, C);
+  build_circuit_plan(nl, C, !faults.empty());
   build_fault_plan(nl, C, faults, P);
   P.net = std::move(C.base.net);
   P.gate_fo = std::move(C.base.gate_fo);
@@ -428,6 +455,9 @@ void build_schedule(const Netlist& nl, const Plan& P, uint32_t G, Schedule& S) {
   S.G = G;
   const uint32_t N = nl.N;
   const SweepNet& net = P.net;
+  S.rec_off.assign(nl.n_levels + 1, 0);
+  S.li_off.assign(nl.n_levels + 1, 0);
+  if (net.use_level.empty()) return;  // no fault will be simulated: no sweeps
   std::vector<uint32_t> slot(N, kNoSlot);
   SlotPool pool(G);
   std::vector<std::vector<uint32_t>> release(nl.n_levels + 2);
@@ -539,7 +569,6 @@ void build_schedule(const Netlist& nl, const Plan& P, uint32_t G, Schedule& S) {
       }
     }
   };
-  S.rec_off.assign(nl.n_levels + 1, 0);
   // A slot at bit 14 * (k & 1) of word k / 2, its high bits in word 2 + k / 2.
   auto put_slot = [](std::array<uint32_t, 4>& w, uint32_t k, uint32_t sl) {
     const uint32_t sh = 14 * (k & 1u);
@@ -642,7 +671,6 @@ void build_schedule(const Netlist& nl, const Plan& P, uint32_t G, Schedule& S) {
   for (uint32_t e = 0; e < N; ++e)
     if (slot[e] != kNoSlot)
       for (uint32_t l = nl.level[e] + 1; l <= net.use_level[e]; ++l) cnt[l]++;
-  S.li_off.assign(nl.n_levels + 1, 0);
   for (uint32_t l = 0; l < nl.n_levels; ++l) S.li_off[l + 1] = S.li_off[l] + cnt[l];
   S.li.assign(2ull * S.li_off[nl.n_levels], 0);
   std::vector<uint32_t> fill(S.li_off.begin(), S.li_off.end() - 1);

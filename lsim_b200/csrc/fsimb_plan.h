@@ -244,14 +244,16 @@ constexpr uint64_t kSplitRecords = 256;  // records a level from which ANDs and 
 // 0: AND family (AND, NAND, OR, NOR, INV, CLKBUF, PO), 1: XOR family, 2: MUX.
 uint32_t gate_family(uint8_t type);
 void build_plan(const Netlist& nl, const std::vector<Fault>& faults, Plan& plan);
-void build_circuit_plan(const Netlist& nl, CircuitPlan& cplan);
+// Without `sweeps` (no fault will be simulated) base.net holds the gate
+// records only.
+void build_circuit_plan(const Netlist& nl, CircuitPlan& cplan, bool sweeps = true);
 // Roots, members, traced faults and sweeps of a fault list; the circuit's
 // per-element vectors (net, gate_fo, po_drv, nfp_prefix) stay in
 // cplan.base and are left empty in `plan`.  Costs O(faults log faults +
 // members of the FFRs the faults touch).
 void build_fault_plan(const Netlist& nl, const CircuitPlan& cplan, const std::vector<Fault>& faults,
                       Plan& plan);
-// Folds single-consumer gates into their consumers.
+// Folds single-consumer gates into their consumers (net.gates is left as it is).
 void build_sweep_net(const Netlist& nl, const Plan& plan, SweepNet& net);
 // G in {2, 4, 8, 16}.  A schedule that needs more than kMaxSlots slots
 // reports max_live > kMaxSlots and leaves recs and li empty.

@@ -15,6 +15,7 @@
 // atomicMax per edge gives that key; a per-wave count, scan and ordered
 // emit place the wave.  POs take no part in the waves: they never trigger
 // an element, and the reference moves them to the end in id order.
+#include <cub/block/block_scan.cuh>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
@@ -45,26 +46,69 @@ inline unsigned grid_for(uint64_t n) { return (unsigned)std::max<uint64_t>(1, st
 // Error bits a kernel sets when the input needs the host reader.
 enum : uint32_t { kBadSink = 1, kTooManyInputs = 2, kMuxInputs = 4, kNoInput = 8 };
 
-struct LoaderDev {
-  DevBuf a, line_src, line_k, line_off, line_eoff, types;
-  DevBuf indeg, wait, slot, esrc, outdeg, adj_off, line_key, line_key2, line_id, line_id2, line_ksorted,
-      line_rsorted, line_rank, adj, key, pos, lev, front[2], cnt, offs, ctl;
-  DevBuf tpg, order, type_t, level_t, fcount, fi_off, fi_idx, cons, fpin, fo_cnt, fo_off, fo_key,
-      fo_key2, fo_val, fo_val2, fo_idx, fo_pin, temp;
-  ~LoaderDev() {
-    for (DevBuf* b : {&a, &line_src, &line_k, &line_off, &line_eoff, &types, &indeg, &wait, &slot, &esrc,
-                      &outdeg, &adj_off, &line_key, &line_key2, &line_id, &line_id2, &line_ksorted,
-                      &line_rsorted, &line_rank, &adj, &key, &pos, &lev, &front[0], &front[1], &cnt,
-                      &offs, &ctl, &tpg, &order, &type_t, &level_t, &fcount, &fi_off, &fi_idx, &cons,
-                      &fpin, &fo_cnt, &fo_off, &fo_key, &fo_key2, &fo_val, &fo_val2, &fo_idx, &fo_pin, &temp})
-      b->release();
+// The loader's arrays share one device allocation (forty of their own cost
+// more in cudaMalloc and cudaFree than the kernels take: 200,000 gates, 11 of
+// 35 ms).
+struct Arena {
+  DevBuf block;
+  size_t at = 0;
+  void* take(size_t bytes) {
+    const size_t o = at;
+    at += (std::max<size_t>(bytes, 16) + 255) & ~(size_t)255;
+    if (at > block.n) throw CudaError{"loader arena of " + std::to_string(block.n) + " bytes is too small"};
+    return (char*)block.p + o;
+  }
+  ~Arena() { block.release(); }
+};
+struct Sub {
+  Arena* arena = nullptr;
+  void* p = nullptr;
+  size_t n = 0;
+  void ensure(size_t bytes) {
+    if (p && bytes <= n) return;
+    p = arena->take(bytes);
+    n = bytes;
+  }
+  template <class T>
+  T* as() const {
+    return reinterpret_cast<T*>(p);
   }
 };
 
-// ctl words: [0] error bits, [1] POs reached, [2] max gate level, [3] next
-// wave size, [4] levels not sorted.
+struct LoaderDev {
+  Arena arena;
+  Sub a, line_src, line_k, line_off, line_eoff, types;
+  Sub indeg, wait, slot, esrc, outdeg, adj_off, line_key, line_key2, line_id, line_id2, line_ksorted,
+      line_rsorted, line_rank, adj, key, pos, lev, front[2], offs, ctl;
+  Sub tpg, order, type_t, level_t, fcount, fi_off, fi_idx, cons, fpin, fo_cnt, fo_off, fo_key,
+      fo_key2, fo_val, fo_val2, fo_idx, fo_pin, temp;
+  // Room for tokens, N elements, W wire lines, E edges and cub's scratch.
+  LoaderDev(size_t tokens, size_t N, size_t W, size_t E) {
+    for (Sub* b : {&a, &line_src, &line_k, &line_off, &line_eoff, &types, &indeg, &wait, &slot, &esrc,
+                   &outdeg, &adj_off, &line_key, &line_key2, &line_id, &line_id2, &line_ksorted,
+                   &line_rsorted, &line_rank, &adj, &key, &pos, &lev, &front[0], &front[1],
+                   &offs, &ctl, &tpg, &order, &type_t, &level_t, &fcount, &fi_off, &fi_idx, &cons,
+                   &fpin, &fo_cnt, &fo_off, &fo_key, &fo_key2, &fo_val, &fo_val2, &fo_idx, &fo_pin, &temp})
+      b->arena = &arena;
+    size_t scratch = 0, bytes = 0;
+    uint32_t* u = nullptr;
+    auto most = [&](cudaError_t e) {
+      CK(e);
+      scratch = std::max(scratch, bytes);
+    };
+    const uint32_t M = (uint32_t)std::max({N, W, E, (size_t)1});
+    most(cub::DeviceScan::InclusiveSum(nullptr, bytes, u, u, M));
+    most(cub::DeviceRadixSort::SortPairs(nullptr, bytes, u, u, u, u, M));
+    most(cub::DeviceScan::ExclusiveSumByKey(nullptr, bytes, u, u, u, M, cub::Equality()));
+    arena.block.ensure(4 * tokens + 102 * N + 44 * W + 40 * E + scratch + 64 * 512);
+    temp.ensure(scratch);
+  }
+};
+
+// Error bits, POs reached, highest gate level, waves and their elements,
+// levels not sorted.
 struct Ctl {
-  uint32_t err, po_reached, max_level, next_n, unsorted;
+  uint32_t err, po_reached, max_level, waves, placed, unsorted;
 };
 
 struct Dims {
@@ -132,94 +176,138 @@ __global__ void k_adj(uint32_t W, const uint32_t* __restrict__ a, const uint32_t
   }
 }
 
-__global__ void k_init_pis(uint32_t nPI, uint32_t* __restrict__ front, uint32_t* __restrict__ pos,
-                           uint32_t* __restrict__ lev) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nPI; i += gridDim.x * blockDim.x) {
-    front[i] = i;
+// All waves in one launch: a cluster of kWaveCtas CTAs with hardware cluster
+// barriers, each CTA a contiguous share of the wave.  A launch sequence per
+// wave with a host read of the next wave's size took about 45 us a wave
+// (151 waves of 1,333 elements); this 13.  What other CTAs write is
+// read from L2 (__ldcg).
+constexpr int kWaveCtas = 8, kWaveThreads = 1024;
+constexpr uint32_t kWaveLanes = 4, kPass = kWaveThreads / kWaveLanes;
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__global__ void __cluster_dims__(kWaveCtas) __launch_bounds__(kWaveThreads)
+    k_waves(Dims d, const uint32_t* __restrict__ adj_off, const uint32_t* __restrict__ adj,
+            const uint32_t* __restrict__ indeg, const uint32_t* __restrict__ slot, const uint32_t* __restrict__ esrc,
+            const uint8_t* __restrict__ types, uint32_t* front0, uint32_t* front1, unsigned long long* key,
+            uint32_t* wait, uint32_t* offs, uint32_t* totals, uint32_t* pos, uint32_t* lev, Ctl* ctl) {
+  using Scan = cub::BlockScan<uint32_t, kWaveThreads>;
+  __shared__ typename Scan::TempStorage scan;
+  const uint32_t tid = threadIdx.x, cta = blockIdx.x, lane = tid % kWaveLanes;
+  const unsigned group = ((1u << kWaveLanes) - 1u) << (tid & 31u & ~(kWaveLanes - 1));  // this element's lanes
+  for (uint32_t i = cta * kWaveThreads + tid; i < d.nPI; i += kWaveCtas * kWaveThreads) {
+    front0[i] = i;
     pos[i] = i;
     lev[i] = 0;
   }
-}
-
-// Wave step 1: every edge out of the wave records its FIFO key at the sink
-// and takes one of the sink's pending inputs.
-__global__ void k_wave_push(uint32_t n, uint32_t base, const uint32_t* __restrict__ front,
-                            const uint32_t* __restrict__ adj_off, const uint32_t* __restrict__ adj,
-                            unsigned long long* key, uint32_t* wait) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const uint32_t u = front[i];
-    const uint64_t hi = (uint64_t)(base + i) << 32;
-    const uint32_t r0 = adj_off[u], r1 = adj_off[u + 1];
-    for (uint32_t r = r0; r < r1; ++r) {
-      const uint32_t v = adj[r];
-      atomicMax(key + v, (unsigned long long)(hi | (r - r0)));
-      atomicSub(wait + v, 1u);
+  cluster_sync();
+  uint32_t n = d.nPI, base = 0, waves = 0;
+  for (; n; ++waves) {
+    const uint32_t* front = (waves & 1u) ? front1 : front0;
+    uint32_t* next = (waves & 1u) ? front0 : front1;
+    const uint32_t share = (n + kWaveCtas - 1) / kWaveCtas;
+    const uint32_t i0 = min(cta * share, n), i1 = min(i0 + share, n);
+    // kWaveLanes lanes take an element's edges, in order; every pass of the
+    // CTA covers kPass elements.
+    auto edges = [&](uint32_t b, uint32_t& i, uint32_t& r0, uint32_t& r1) {
+      i = b + tid / kWaveLanes;
+      r0 = r1 = 0;
+      if (i >= i1) return;
+      const uint32_t u = __ldcg(front + i);
+      r0 = adj_off[u];
+      r1 = adj_off[u + 1];
+    };
+    // Every edge out of the wave records its FIFO key at the sink and takes
+    // one of the sink's pending inputs.
+    for (uint32_t b = i0; b < i1; b += kPass) {
+      uint32_t i, r0, r1;
+      edges(b, i, r0, r1);
+      for (uint32_t r = r0 + lane; r < r1; r += kWaveLanes) {
+        const uint32_t v = adj[r];
+        atomicMax(key + v, (unsigned long long)((uint64_t)(base + i) << 32 | (r - r0)));
+        atomicSub(wait + v, 1u);
+      }
     }
+    cluster_sync();
+    // Whether edge r of wave element i appends its sink v: it was the sink's
+    // last input.
+    auto appends = [&](uint32_t i, uint32_t r0, uint32_t r, uint32_t r1, uint32_t& v) {
+      if (r >= r1) return false;
+      v = adj[r];
+      const uint32_t pending = __ldcg(wait + v);
+      const unsigned long long k = __ldcg(key + v);
+      return pending == 0 && k == ((uint64_t)(base + i) << 32 | (r - r0));
+    };
+    // Per wave element, how many elements its edges append, and the sum of
+    // those before it in this CTA's share; POs are only counted as reached.
+    uint32_t total = 0, po_reached = 0;
+    for (uint32_t b = i0; b < i1; b += kPass) {
+      uint32_t i, r0, r1, c = 0;
+      edges(b, i, r0, r1);
+      for (uint32_t r = r0 + lane; __any_sync(~0u, r < r1); r += kWaveLanes) {
+        uint32_t v = 0;
+        const bool on = appends(i, r0, r, r1, v), po = on && is_po(d, v);
+        po_reached += po;
+        c += __popc(__ballot_sync(~0u, on && !po) & group);
+      }
+      uint32_t before, sum;
+      Scan(scan).ExclusiveSum(lane == 0 ? c : 0u, before, sum);
+      if (i < i1 && lane == 0) offs[i] = total + before;
+      total += sum;
+      __syncthreads();  // scan is used again
+    }
+    if (po_reached) atomicAdd(&ctl->po_reached, po_reached);
+    if (tid == 0) totals[cta] = total;
+    cluster_sync();
+    uint32_t at = 0, all = 0;
+    for (uint32_t b = 0; b < kWaveCtas; ++b) {
+      const uint32_t t = __ldcg(totals + b);
+      at += b < cta ? t : 0u;
+      all += t;
+    }
+    // The next wave in FIFO order, with positions and levels
+    // (fsim/simulation.cpp:882-893: 1 + the largest level over pin slots
+    // 1..count; an empty slot reads element 0).
+    const uint32_t nbase = base + n;
+    for (uint32_t b = i0; b < i1; b += kPass) {
+      uint32_t i, r0, r1;
+      edges(b, i, r0, r1);
+      uint32_t o = i < i1 ? at + __ldcg(offs + i) : 0u;
+      for (uint32_t r = r0 + lane; __any_sync(~0u, r < r1); r += kWaveLanes) {
+        uint32_t v = 0;
+        const bool on = appends(i, r0, r, r1, v) && !is_po(d, v);
+        const unsigned g = __ballot_sync(~0u, on) & group;
+        const uint32_t mine = o + __popc(g & ((1u << (tid & 31u)) - 1u));
+        o += __popc(g);
+        if (!on) continue;
+        next[mine] = v;
+        pos[v] = nbase + mine;
+        const uint32_t c = indeg[v];
+        if (c > 4) {
+          atomicOr(&ctl->err, kTooManyInputs);
+          continue;
+        }
+        const uint4 sl = reinterpret_cast<const uint4*>(slot)[v];
+        const uint32_t e[4] = {sl.x, sl.y, sl.z, sl.w};
+        uint32_t src[4], lv = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) src[j] = j < c && e[j] ? esrc[e[j] - 1] : 0u;
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j)
+          if (j < c) lv = max(lv, __ldcg(lev + src[j]) + 1);
+        lev[v] = lv;
+        atomicMax(&ctl->max_level, lv);
+        if (types[v - d.nPI - d.nPO] == G_MUX && c < 3) atomicOr(&ctl->err, kMuxInputs);
+      }
+    }
+    base = nbase;
+    n = all;
+    cluster_sync();
   }
-}
-
-// Wave step 2: per wave element, how many elements its edges append (their
-// last input was this edge); POs are only counted as reached.
-__global__ void k_wave_count(Dims d, uint32_t n, uint32_t base, const uint32_t* __restrict__ front,
-                             const uint32_t* __restrict__ adj_off, const uint32_t* __restrict__ adj,
-                             const unsigned long long* __restrict__ key, const uint32_t* __restrict__ wait,
-                             uint32_t* __restrict__ cnt, Ctl* ctl) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const uint32_t u = front[i];
-    const uint64_t hi = (uint64_t)(base + i) << 32;
-    const uint32_t r0 = adj_off[u], r1 = adj_off[u + 1];
-    uint32_t c = 0;
-    for (uint32_t r = r0; r < r1; ++r) {
-      const uint32_t v = adj[r];
-      if (wait[v] == 0 && key[v] == (hi | (r - r0))) {
-        if (is_po(d, v))
-          atomicAdd(&ctl->po_reached, 1u);
-        else
-          ++c;
-      }
-    }
-    cnt[i] = c;
-  }
-}
-
-// Wave step 3: the next wave in FIFO order, with positions and levels
-// (fsim/simulation.cpp:882-893: 1 + the largest level over pin slots
-// 1..count; an empty slot reads element 0).
-__global__ void k_wave_emit(Dims d, uint32_t n, uint32_t base, uint32_t nbase,
-                            const uint32_t* __restrict__ front, const uint32_t* __restrict__ adj_off,
-                            const uint32_t* __restrict__ adj, const unsigned long long* __restrict__ key,
-                            const uint32_t* __restrict__ wait, const uint32_t* __restrict__ cnt,
-                            const uint32_t* __restrict__ offs, const uint32_t* __restrict__ indeg,
-                            const uint32_t* __restrict__ slot, const uint32_t* __restrict__ esrc,
-                            const uint8_t* __restrict__ types, uint32_t* __restrict__ next,
-                            uint32_t* __restrict__ pos, uint32_t* lev, Ctl* ctl) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    if (i == n - 1) ctl->next_n = offs[i] + cnt[i];
-    const uint32_t u = front[i];
-    const uint64_t hi = (uint64_t)(base + i) << 32;
-    const uint32_t r0 = adj_off[u], r1 = adj_off[u + 1];
-    uint32_t o = offs[i];
-    for (uint32_t r = r0; r < r1; ++r) {
-      const uint32_t v = adj[r];
-      if (wait[v] != 0 || key[v] != (hi | (r - r0)) || is_po(d, v)) continue;
-      next[o] = v;
-      pos[v] = nbase + o;
-      ++o;
-      const uint32_t c = indeg[v];
-      if (c > 4) {
-        atomicOr(&ctl->err, kTooManyInputs);
-        continue;
-      }
-      uint32_t lv = 0;
-      for (uint32_t j = 0; j < c; ++j) {
-        const uint32_t e = slot[(size_t)v * 4 + j];
-        const uint32_t s = e ? esrc[e - 1] : 0u;
-        lv = max(lv, lev[s] + 1);
-      }
-      lev[v] = lv;
-      atomicMax(&ctl->max_level, lv);
-      if (types[v - d.nPI - d.nPO] == G_MUX && c < 3) atomicOr(&ctl->err, kMuxInputs);
-    }
+  if (cta == 0 && tid == 0) {
+    ctl->waves = waves;
+    ctl->placed = base;
   }
 }
 
@@ -290,19 +378,19 @@ __global__ void k_fanout(uint32_t E, const uint32_t* __restrict__ val, const uin
 }
 
 template <class T>
-void zero(DevBuf& b, size_t count, cudaStream_t s) {
+void zero(Sub& b, size_t count, cudaStream_t s) {
   b.ensure(count * sizeof(T));
   CK(cudaMemsetAsync(b.p, 0, count * sizeof(T), s));
 }
 
 template <class T>
-void put(DevBuf& b, const T* src, size_t count, cudaStream_t s) {
+void put(Sub& b, const T* src, size_t count, cudaStream_t s) {
   b.ensure(count * sizeof(T));
   if (count) CK(cudaMemcpyAsync(b.p, src, count * sizeof(T), cudaMemcpyHostToDevice, s));
 }
 
 template <class T>
-void get(std::vector<T>& v, const DevBuf& b, size_t count, cudaStream_t s) {
+void get(std::vector<T>& v, const Sub& b, size_t count, cudaStream_t s) {
   v.resize(count);
   if (count) CK(cudaMemcpyAsync(v.data(), b.p, count * sizeof(T), cudaMemcpyDeviceToHost, s));
 }
@@ -390,9 +478,9 @@ static bool tokenize(const char* text, size_t len, int threads, std::unique_ptr<
 bool parse_ckt_device(const char* text, size_t len, Netlist& nl, int device, cudaStream_t s, int threads,
                       LoadInfo& info) {
   const auto t0 = std::chrono::steady_clock::now();
-  if (threads <= 0) {  // the hardware threads, at most 32, at least 1 MiB each
+  if (threads <= 0) {  // the hardware threads, at most 32, at least 256 KiB each
     threads = (int)std::min<unsigned>(32, std::max(1u, std::thread::hardware_concurrency()));
-    threads = (int)std::max<size_t>(1, std::min<size_t>((size_t)threads, len / (1 << 20) + 1));
+    threads = (int)std::max<size_t>(1, std::min<size_t>((size_t)threads, len / (1 << 18) + 1));
   }
   threads = (int)std::max<size_t>(1, std::min<size_t>((size_t)threads, len));
   info = LoadInfo{};
@@ -432,7 +520,7 @@ bool parse_ckt_device(const char* text, size_t len, Netlist& nl, int device, cud
 
   const auto t1 = std::chrono::steady_clock::now();
   CK(cudaSetDevice(device));
-  LoaderDev D;
+  LoaderDev D(na, N, W, E);
   const Dims d{N, (uint32_t)nPI, (uint32_t)nPO, (uint32_t)nG};
   const uint32_t Wn = (uint32_t)W, En = (uint32_t)E;
   put(D.a, a, na, s);
@@ -500,7 +588,6 @@ bool parse_ckt_device(const char* text, size_t len, Netlist& nl, int device, cud
                                           D.adj.as<uint32_t>());
     CK(cudaGetLastError());
   }
-  D.a.release();
 
   // Waves.
   zero<unsigned long long>(D.key, N, s);
@@ -511,42 +598,17 @@ bool parse_ckt_device(const char* text, size_t len, Netlist& nl, int device, cud
   CK(cudaMemcpyAsync(D.wait.p, D.indeg.p, (size_t)N * 4, cudaMemcpyDeviceToDevice, s));
   D.front[0].ensure((size_t)N * 4);
   D.front[1].ensure((size_t)N * 4);
-  D.cnt.ensure((size_t)N * 4);
-  D.offs.ensure(((size_t)N + 1) * 4);
-  {
-    size_t bytes = 0;
-    CK(cub::DeviceScan::InclusiveSum(nullptr, bytes, D.cnt.as<uint32_t>(), D.offs.as<uint32_t>(), N, s));
-    D.temp.ensure(bytes);
-  }
-  k_init_pis<<<grid_for(nPI), kBlock, 0, s>>>((uint32_t)nPI, D.front[0].as<uint32_t>(), D.pos.as<uint32_t>(),
-                                               D.lev.as<uint32_t>());
+  D.offs.ensure(((size_t)N + kWaveCtas) * 4);
+  k_waves<<<kWaveCtas, kWaveThreads, 0, s>>>(
+      d, D.adj_off.as<uint32_t>(), D.adj.as<uint32_t>(), D.indeg.as<uint32_t>(), D.slot.as<uint32_t>(),
+      D.esrc.as<uint32_t>(), D.types.as<uint8_t>(), D.front[0].as<uint32_t>(), D.front[1].as<uint32_t>(),
+      D.key.as<unsigned long long>(), D.wait.as<uint32_t>(), D.offs.as<uint32_t>(), D.offs.as<uint32_t>() + N,
+      D.pos.as<uint32_t>(), D.lev.as<uint32_t>(), ctl);
   CK(cudaGetLastError());
-  uint32_t n = (uint32_t)nPI, base = 0, cur = 0, waves = 0;
-  while (n) {
-    const uint32_t nbase = base + n;
-    uint32_t* fr = D.front[cur].as<uint32_t>();
-    k_wave_push<<<grid_for(n), kBlock, 0, s>>>(n, base, fr, D.adj_off.as<uint32_t>(), D.adj.as<uint32_t>(),
-                                               D.key.as<unsigned long long>(), D.wait.as<uint32_t>());
-    k_wave_count<<<grid_for(n), kBlock, 0, s>>>(d, n, base, fr, D.adj_off.as<uint32_t>(), D.adj.as<uint32_t>(),
-                                                D.key.as<unsigned long long>(), D.wait.as<uint32_t>(),
-                                                D.cnt.as<uint32_t>(), ctl);
-    exclusive_sum(D, D.cnt.as<uint32_t>(), D.offs.as<uint32_t>(), n, s);
-    k_wave_emit<<<grid_for(n), kBlock, 0, s>>>(
-        d, n, base, nbase, fr, D.adj_off.as<uint32_t>(), D.adj.as<uint32_t>(), D.key.as<unsigned long long>(),
-        D.wait.as<uint32_t>(), D.cnt.as<uint32_t>(), D.offs.as<uint32_t>(), D.indeg.as<uint32_t>(),
-        D.slot.as<uint32_t>(), D.esrc.as<uint32_t>(), D.types.as<uint8_t>(), D.front[cur ^ 1].as<uint32_t>(),
-        D.pos.as<uint32_t>(), D.lev.as<uint32_t>(), ctl);
-    CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(&hc, ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    ++waves;
-    if (hc.err) return false;
-    base = nbase;
-    n = hc.next_n;
-    cur ^= 1;
-  }
-  info.waves = waves;
-  if (base != nPI + nG || hc.po_reached != nPO) return false;  // unreachable elements
+  CK(cudaMemcpyAsync(&hc, ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
+  CK(cudaStreamSynchronize(s));
+  info.waves = hc.waves;
+  if (hc.err || hc.placed != nPI + nG || hc.po_reached != nPO) return false;  // or unreachable elements
 
   // Topological arrays.
   D.tpg.ensure((size_t)N * 8);

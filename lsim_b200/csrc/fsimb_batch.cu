@@ -814,11 +814,11 @@ struct fsimb_batch {
 
   // Members that carry at least 1% of the batch's sweep work (the largest 64
   // at most) get a class of their own, tuned as the plain path tunes a
-  // circuit alone over words per item x CTAs per SM x CTA size (256-1,024
-  // threads), on strided samples of the first tile's sweeps: every
-  // candidate once on about 256 sweeps, then the default and the three
-  // fastest twice on about 1,024, the default kept unless beaten by 2%.  A shared class cannot give
-  // each of these circuits its own shape, and they carry most of the work.
+  // circuit alone over the likely shapes, on strided samples of the first
+  // tile's sweeps: every candidate once on about 256 sweeps, then the
+  // default and the three fastest twice on about 1,024, the default kept
+  // unless beaten by 2%.  A shared class cannot give each of these circuits
+  // its own shape, and they carry most of the work.
   // Returns, per class of the new assignment, whether its shape is final.
   std::vector<char> tune_singletons(BatchAssign& a, cudaStream_t s) {
     const size_t n = members.size();
@@ -890,13 +890,11 @@ struct fsimb_batch {
         ClassShape sh;
       };
       std::vector<Timed> t1;
-      for (int M : {8, 4, 2, 1}) {
-        if (!fits_M(M)) continue;
-        for (int T : {32, 64, 128, 256, 384, 512, 768, 1024}) {
-          if (T > (int)sweep_max_threads(M)) continue;
-          const float ms = time_shape(coarse, ClassShape{M, T}, 1);
-          if (ms >= 0) t1.push_back(Timed{ms, ClassShape{M, T}});
-        }
+      for (const ClassShape& sh : likely_shapes(P, (uint32_t)std::min<uint64_t>(members[i]->pats.W, kTileWords),
+                                                smem_optin, smem_per_sm, 10)) {
+        if (!fits_M(sh.M)) continue;
+        const float ms = time_shape(coarse, sh, 1);
+        if (ms >= 0) t1.push_back(Timed{ms, sh});
       }
       std::sort(t1.begin(), t1.end(), [](const Timed& x, const Timed& y) { return x.ms < y.ms; });
       // Stage 2: the default and the three fastest, twice each on the fine

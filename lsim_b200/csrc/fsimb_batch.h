@@ -16,11 +16,7 @@
 
 namespace fsimb {
 
-// Sweep launch shape: words per item and CTA size.
-struct ClassShape {
-  int M;
-  int threads;
-};
+using ClassShape = SweepShape;
 
 // One job of a batch.
 struct BatchJob {

@@ -80,31 +80,52 @@ const Schedule& fsimb_handle::use_schedule(int M, int T, cudaStream_t s) {
 
 namespace fsimb {
 
-// The default shape minimises a model of one SM's time per pattern word.  A
-// level of a CTA's sweep takes a latency (barrier, record, operands, store)
-// of kLevel cycles plus kRound for each further round, and the shared-memory
-// and issue time of all the SM's CTAs: kWarp[M] cycles for a warp's records,
-// kPad for a warp of padding.  Fitted to shape sweeps on a B200; best of the
-// sweep against this choice: 2,000 gates 0.129 / 0.138 ms, 6,586 gates 2.34 /
-// 2.36, 20,000 gates with MUX 8.00 / 8.14, 30,000 gates 31.5 / 33.6, 50,000
-// gates 52.2 / 54.9, 200,000 gates 339 / 347 ms.
+// A model of one SM's time per pattern word.  A level of a CTA's sweep takes
+// a latency (barrier, record, operands, store) of kLevel cycles plus kRound
+// for each further round, and the shared-memory and issue time of all the
+// SM's CTAs: a number of cycles by M for a warp's records, kPad for a warp of
+// padding.  Fitted to shape sweeps on a B200; best of the sweep against the
+// model's choice: 2,000 gates 0.129 / 0.138 ms, 6,586 gates 2.34 / 2.36, 20,000
+// gates with MUX 8.00 / 8.14, 30,000 gates 31.5 / 33.6, 50,000 gates 52.2 /
+// 54.9, 200,000 gates 339 / 347 ms.
+double sweep_shape_cost(const SweepNet& net, int m, uint32_t t, size_t vals, size_t smem_per_sm, uint32_t words) {
+  constexpr double kLevel = 1100, kRound = 300, kPad = 4;
+  const uint32_t w = std::max<uint32_t>(1, std::min<uint32_t>(words, kTileWords));
+  const double warp = m == 8 ? 61 : m == 4 ? 31 : m == 2 ? 18 : 15;
+  const uint32_t ctas = (uint32_t)std::min<size_t>({smem_per_sm / (vals + 1024 + 256), 1024 / t, 32});
+  if (ctas < 1) return 1e300;
+  double cycles = 0;
+  for (uint32_t n : net.level_recs) {
+    if (!n) continue;
+    const uint32_t rounds = (n + t - 1) / t, full = (n + 31) / 32, all = rounds * (t / 32);
+    cycles += kLevel + kRound * (rounds - 1) + ctas * (full * warp + (all - full) * kPad);
+  }
+  return cycles / ctas * ((w + m - 1) / m);
+}
+
+std::vector<SweepShape> likely_shapes(const Plan& plan, uint32_t words, size_t smem_optin, size_t smem_per_sm,
+                                      size_t most) {
+  struct Priced {
+    double cost;
+    SweepShape s;
+  };
+  std::vector<Priced> all;
+  for (int m : {8, 4, 2, 1}) {
+    const size_t vals = sweep_vals_bytes(plan.net_live, m);
+    if (plan.net_live > kMaxSlots || vals > sweep_smem_share(smem_optin, smem_per_sm, 1)) continue;
+    for (uint32_t t : {32, 64, 96, 128, 192, 256, 320, 384, 448, 512, 640, 768, 1024})
+      all.push_back({sweep_shape_cost(plan.net, m, t, vals, smem_per_sm, words), {m, (int)t}});
+  }
+  std::stable_sort(all.begin(), all.end(), [](const Priced& a, const Priced& b) { return a.cost < b.cost; });
+  std::vector<SweepShape> out;
+  for (const Priced& p : all)
+    if (out.size() < most && p.cost < 1.5 * all[0].cost) out.push_back(p.s);
+  return out;
+}
+
 void default_sweep_shape(const Plan& plan, const std::function<const Schedule&(int)>& sched_at,
                          uint32_t words, size_t smem_optin, size_t smem_per_sm, int& M, int& threads) {
-  constexpr double kLevel = 1100, kRound = 300, kPad = 4;
   const size_t share1 = sweep_smem_share(smem_optin, smem_per_sm, 1);
-  const uint32_t w = std::max<uint32_t>(1, std::min<uint32_t>(words, kTileWords));
-  auto cost = [&](int m, uint32_t t, size_t vals) {
-    const double warp = m == 8 ? 61 : m == 4 ? 31 : m == 2 ? 18 : 15;
-    const uint32_t ctas = (uint32_t)std::min<size_t>({smem_per_sm / (vals + 1024 + 256), 1024 / t, 32});
-    if (ctas < 1) return 1e300;
-    double cycles = 0;
-    for (uint32_t n : plan.net.level_recs) {
-      if (!n) continue;
-      const uint32_t rounds = (n + t - 1) / t, full = (n + 31) / 32, all = rounds * (t / 32);
-      cycles += kLevel + kRound * (rounds - 1) + ctas * (full * warp + (all - full) * kPad);
-    }
-    return cycles / ctas * ((w + m - 1) / m);
-  };
   // Slots are about the peak of live values until a schedule says more.
   size_t vals[4] = {0, 0, 0, 0};
   bool exact[4] = {false, false, false, false};
@@ -116,7 +137,7 @@ void default_sweep_shape(const Plan& plan, const std::function<const Schedule&(i
     for (int i = 3; i >= 0; --i) {
       if (i > 0 && vals[i] > share1) continue;
       for (uint32_t t = 32; t <= 1024; t += 32) {
-        const double c = cost(1 << i, t, vals[i]);
+        const double c = sweep_shape_cost(plan.net, 1 << i, t, vals[i], smem_per_sm, words);
         if (c < best * 0.99) {
           best = c;
           bi = i;
@@ -167,18 +188,13 @@ void fsimb_handle::tune_shape(cudaStream_t s) {
   int dM = 0, dT = 0;
   default_shape(dM, dT);
   float default_ms = -1;
-  struct Cand {
-    int M, T;
-  };
-  std::vector<Cand> cands{{dM, dT}};
-  for (int M : {8, 4, 2, 1})
-    for (int T : {32, 64, 128, 192, 256, 384, 512, 768, 1024})
-      if (!(M == dM && T == dT)) cands.push_back({M, T});
+  std::vector<SweepShape> cands{{dM, dT}};
+  for (const SweepShape& c :
+       likely_shapes(plan, (uint32_t)std::min<uint64_t>(pats.W, kTileWords), smem_optin, smem_per_sm, 10))
+    if (!(c.M == dM && c.threads == dT)) cands.push_back(c);
   const size_t share1 = sweep_smem_share(smem_optin, smem_per_sm, 1);
-  for (const Cand& cd : cands) {
-    const int M = cd.M, T = cd.T;
-    if (T > (int)sweep_max_threads(M)) continue;
-    if (plan.net_live > kMaxSlots || sweep_vals_bytes(plan.net_live, M) > share1) continue;
+  for (const SweepShape& cd : cands) {
+    const int M = cd.M, T = cd.threads;
     if (cached_schedule(M).max_live > kMaxSlots || sweep_vals_bytes(cached_schedule(M).max_live, M) > share1)
       continue;
     const Schedule& sc = use_schedule(M, T, s);

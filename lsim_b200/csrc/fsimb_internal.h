@@ -157,9 +157,22 @@ struct PinnedBuf {
   }
 };
 
-// Default sweep shape of a circuit.  At most `words` words per item (rounded
-// up to a power of two): the pattern words a tile of the block has.
-// sched_at(M) returns the schedule at M.
+// Sweep launch shape: words per item and CTA size.
+struct SweepShape {
+  int M;
+  int threads;
+};
+
+// Modelled cost of a sweep shape (cycles of an SM per tile of `words` pattern
+// words and sweep) with `vals` bytes of slots; the shapes within 1.5x of the
+// cheapest, cheapest first, at most `most` of them.
+double sweep_shape_cost(const SweepNet& net, int M, uint32_t threads, size_t vals, size_t smem_per_sm,
+                        uint32_t words);
+std::vector<SweepShape> likely_shapes(const Plan& plan, uint32_t words, size_t smem_optin, size_t smem_per_sm,
+                                      size_t most);
+
+// Default sweep shape of a circuit: the cheapest for a tile of `words` pattern
+// words.  sched_at(M) returns the schedule at M.
 void default_sweep_shape(const Plan& plan, const std::function<const Schedule&(int)>& sched_at,
                          uint32_t words, size_t smem_optin, size_t smem_per_sm, int& M, int& threads);
 

@@ -224,7 +224,6 @@ void fsimb_handle::tune_shape(cudaStream_t s) {
     sa.fix0 = sc.fix0;
     sa.inj_slot = sc.max_live - 1;
     sa.split = sc.split;
-    sa.err = d_err.as<int>();
     const int nb = (int)std::min<uint64_t>((uint64_t)n_sms * got, (uint64_t)sa.n_list * ((sa.n_words + M - 1) / M));
     // an untimed run of the first candidate warms the GPU up; then the
     // fastest of two timed runs counts
@@ -326,8 +325,9 @@ void fsimb_handle::run(const fsimb_opts* opts) {
   d_count.ensure(std::max<uint64_t>(F, 1) * 8);
   d_first.ensure(std::max<uint64_t>(F, 1) * 8);
   d_lastflag.ensure(std::max<uint64_t>(F, 1));
-  d_queue.ensure(std::max<uint64_t>(tiles, 1) * sizeof(int));
-  d_err.ensure(sizeof(int));
+  d_queue.ensure((tiles + 1) * sizeof(int));
+  d_records.ensure(F * sizeof(fsimb_fault_result) + 16);
+  h_records.ensure(F * sizeof(fsimb_fault_result) + 16);
   if (o.drop) {
     d_root_list[0].ensure(std::max<uint32_t>(n_roots, 1) * 4);
     d_root_list[1].ensure(std::max<uint32_t>(n_roots, 1) * 4);
@@ -409,10 +409,11 @@ void fsimb_handle::run(const fsimb_opts* opts) {
     sched = &use_schedule(M, threads, s);
     smem = std::max<size_t>(16, sweep_vals_bytes(sched->max_live, M));
   }
-  CK(cudaMemsetAsync(d_queue.p, 0, std::max<uint64_t>(tiles, 1) * sizeof(int), s));
-  CK(cudaMemsetAsync(d_err.p, 0, sizeof(int), s));
+  // control words: the error word, then a work counter per tile
+  int* err_word = d_queue.as<int>();
+  int* queue = err_word + 1;
   launch_init_results(d_count.as<unsigned long long>(), d_first.as<unsigned long long>(),
-                      d_lastflag.as<uint8_t>(), (uint32_t)F, s);
+                      d_lastflag.as<uint8_t>(), (uint32_t)F, err_word, (uint32_t)tiles + 1, s);
   CK(cudaEventRecord(e1, s));
 
   // 2. good machine
@@ -463,7 +464,7 @@ void fsimb_handle::run(const fsimb_opts* opts) {
         wa.N = N;
         wa.good = good_t;
         wa.out = d_out.as<uint64_t>();
-        wa.queue = d_queue.as<int>() + t;
+        wa.queue = queue + t;
         wa.gvals = d_gvals.as<uint64_t>();
         CK(launch_sweep_wide(M, nb, wa, s));
       } else {
@@ -483,12 +484,12 @@ void fsimb_handle::run(const fsimb_opts* opts) {
         sa.N = N;
         sa.good = good_t;
         sa.out = d_out.as<uint64_t>();
-        sa.queue = d_queue.as<int>() + t;
+        sa.queue = queue + t;
         sa.stream_recs = sched->stream_recs;
         sa.fix0 = sched->fix0;
         sa.inj_slot = sched->max_live - 1;
         sa.split = sched->split;
-        sa.err = d_err.as<int>();
+        sa.err = err_word;
         sa.wait_ns = kWaitTestNs;
         sa.wait_test = (o.wait_test && t == 0) ? 1u : 0u;
         CK(launch_sweep(M, threads, nb, smem, sa, s));
@@ -605,18 +606,20 @@ void fsimb_handle::run(const fsimb_opts* opts) {
   CK(cudaEventRecord(e3, s));
 
   // 4. results
-  std::vector<unsigned long long> cnt(F), fst(F);
-  std::vector<uint8_t> lf(F);
-  int kerr = 0;
+  const uint64_t last_rd = W ? W - 1 : 0;
+  launch_results(ResultArgs{d_count.as<unsigned long long>(), d_first.as<unsigned long long>(),
+                            d_lastflag.as<uint8_t>(), err_word, d_records.as<ulonglong2>(), last_rd, (uint32_t)F,
+                            W ? 1u : 0u},
+                 s);
+  ++launches;
+  CK(cudaGetLastError());
+  const size_t record_bytes = F * sizeof(fsimb_fault_result);
   cudaEvent_t e4 = ev(4 + 3 * tiles + 1);
-  CK(cudaMemcpyAsync(&kerr, d_err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-  if (F) {
-    CK(cudaMemcpyAsync(cnt.data(), d_count.p, F * 8, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(fst.data(), d_first.p, F * 8, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(lf.data(), d_lastflag.p, F, cudaMemcpyDeviceToHost, s));
-  }
+  CK(cudaMemcpyAsync(h_records.p, d_records.p, record_bytes + 16, cudaMemcpyDeviceToHost, s));
   CK(cudaEventRecord(e4, s));
   CK(cudaStreamSynchronize(s));
+  uint64_t kerr = 0;
+  std::memcpy(&kerr, h_records.as<char>() + record_bytes, sizeof kerr);
   if (kerr) throw CudaError{"a sweep kernel reached its time limit waiting for a record copy; results discarded"};
   if (!o.drop) {
     for (uint64_t t = 0; t < tiles; ++t) {
@@ -627,16 +630,9 @@ void fsimb_handle::run(const fsimb_opts* opts) {
       ms_ffr += x;
     }
   }
-  results.assign(F, fsimb_fault_result{});
-  const uint64_t last_rd = W ? W - 1 : 0;
-  for (uint64_t f = 0; f < F; ++f) {
-    fsimb_fault_result& r = results[f];
-    r.count = cnt[f];
-    r.detected = cnt[f] > 0;
-    r.first_pattern = (fst[f] == ~0ull) ? -1 : (int64_t)fst[f];
-    r.ref_last_round_flag = W ? lf[f] : 0;
-    r.ref_last_rd = last_rd;
-  }
+  static_assert(sizeof(fsimb_fault_result) == 32, "k_results writes two 16-byte halves");
+  records = h_records.as<fsimb_fault_result>();
+  n_records = F;
   has_results = true;
 
   float x = 0;
@@ -796,11 +792,17 @@ int fsimb_set_patterns(fsimb_handle* h, const uint64_t* words, uint64_t num_patt
   const uint64_t W = (num_patterns + 63) / 64;
   if (W && !words) throw ArgError{"null pattern words"};
   if (W * h->nl.n_pi > (1ull << 36)) throw LimitError{"pattern block too large"};
-  Patterns p;
-  p.P = num_patterns;
-  p.W = W;
-  p.words.assign(words, words + W * h->nl.n_pi);
-  h->pats = std::move(p);
+  if (h->pats.words.capacity() >= W * h->nl.n_pi) {  // into the room the last patterns had
+    h->pats.words.assign(words, words + W * h->nl.n_pi);
+    h->pats.P = num_patterns;
+    h->pats.W = W;
+  } else {
+    Patterns p;
+    p.P = num_patterns;
+    p.W = W;
+    p.words.assign(words, words + W * h->nl.n_pi);
+    h->pats = std::move(p);
+  }
   h->has_pats = true;
   h->gen = next_generation();
   h->has_results = false;
@@ -819,8 +821,8 @@ int fsimb_results(const fsimb_handle* hc, fsimb_fault_result* out, uint64_t n) {
   fsimb_handle* h = const_cast<fsimb_handle*>(hc);
   API_BEGIN(h)
   if (!h->has_results) throw StateError{"no results: call fsimb_run first"};
-  if (n != h->results.size() || (n && !out)) throw ArgError{"result buffer size must equal the fault count"};
-  std::memcpy(out, h->results.data(), n * sizeof(fsimb_fault_result));
+  if (n != h->n_records || (n && !out)) throw ArgError{"result buffer size must equal the fault count"};
+  if (n) std::memcpy(out, h->records, n * sizeof(fsimb_fault_result));
   API_END(h)
 }
 
@@ -828,10 +830,10 @@ int fsimb_found_fault_to_pattern(const fsimb_handle* hc, uint64_t* out, uint64_t
   fsimb_handle* h = const_cast<fsimb_handle*>(hc);
   API_BEGIN(h)
   if (!h->has_results) throw StateError{"no results: call fsimb_run first"};
-  if (n != 2 * h->results.size() || (n && !out)) throw ArgError{"buffer size must be 2 * faults"};
-  for (size_t f = 0; f < h->results.size(); ++f) {
-    out[2 * f] = h->results[f].ref_last_round_flag;
-    out[2 * f + 1] = h->results[f].ref_last_rd;
+  if (n != 2 * h->n_records || (n && !out)) throw ArgError{"buffer size must be 2 * faults"};
+  for (size_t f = 0; f < h->n_records; ++f) {
+    out[2 * f] = h->records[f].ref_last_round_flag;
+    out[2 * f + 1] = h->records[f].ref_last_rd;
   }
   API_END(h)
 }
@@ -844,12 +846,13 @@ int fsimb_good_values(const fsimb_handle* hc, uint64_t round, uint64_t* out, uin
   if (n != h->nl.N || !out) throw ArgError{"buffer size must equal the element count"};
   CK(cudaSetDevice(h->device));
   const uint64_t tile = round / kTileWords, lane = round % kTileWords;
-  const uint64_t* src = h->d_good.as<uint64_t>() + (tile * h->nl.N) * kTileWords + lane;
-  CK(cudaMemcpy2DAsync(out, 8, src, kTileWords * 8, 8, h->nl.N, cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaStreamSynchronize(h->stream));
   const uint32_t bits = h->pats.bits(round);
-  const uint64_t mask = bits >= 64 ? ~0ull : ((1ull << bits) - 1);
-  for (uint64_t i = 0; i < n; ++i) out[i] &= mask;
+  h->d_round.ensure(n * 8);
+  launch_round(h->d_good.as<uint64_t>() + (tile * h->nl.N) * kTileWords + lane, h->nl.N,
+               bits >= 64 ? ~0ull : ((1ull << bits) - 1), h->d_round.as<uint64_t>(), h->stream);
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(out, h->d_round.p, n * 8, cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaStreamSynchronize(h->stream));
   API_END(h)
 }
 

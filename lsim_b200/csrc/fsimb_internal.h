@@ -218,14 +218,20 @@ struct fsimb_handle {
   fsimb::DevBuf d_eflag;   // wide-circuit sweep: per element, evaluated / drives a PO
   fsimb::DevBuf d_gvals;   // wide-circuit sweep: per-CTA value regions
   fsimb::DevBuf d_roots, d_members, d_traced, d_inj, d_exact;
-  fsimb::DevBuf d_pwords, d_good, d_out, d_sens, d_count, d_first, d_lastflag, d_queue, d_err;
+  fsimb::DevBuf d_pwords, d_good, d_out, d_sens, d_count, d_first, d_lastflag, d_queue;
   fsimb::DevBuf d_root_list[2], d_sweep_list, d_exact_list[2], d_nout, d_tune_list;
   uint64_t good_tiles = 0;  // tiles held in d_good
   uint64_t good_P = 0;
   bool pats_uploaded = false;  // d_pwords holds the current patterns
   bool eflag_uploaded = false; // d_eflag holds the current plan's element flags
 
-  std::vector<fsimb_fault_result> results;
+  // The last run's records: in h_records after fsimb_run, in batch_results
+  // after a batch's run.
+  fsimb::DevBuf d_records, d_round;
+  fsimb::PinnedBuf h_records;
+  std::vector<fsimb_fault_result> batch_results;
+  const fsimb_fault_result* records = nullptr;
+  uint64_t n_records = 0;
   bool has_results = false;
   fsimb_stats stats{};
   std::vector<cudaEvent_t> events;
@@ -236,9 +242,10 @@ struct fsimb_handle {
       for (fsimb::DevBuf* b : {&d_type, &d_fi_off, &d_fi_idx, &d_recs, &d_level, &d_level_off, &d_gates,
                         &d_lvl, &d_eflag, &d_gvals, &d_li, &d_roots, &d_members, &d_traced, &d_inj, &d_exact,
                         &d_pwords, &d_good, &d_out, &d_sens, &d_count, &d_first, &d_lastflag,
-                        &d_queue, &d_err, &d_root_list[0], &d_root_list[1], &d_sweep_list,
-                        &d_exact_list[0], &d_exact_list[1], &d_nout, &d_tune_list})
+                        &d_queue, &d_root_list[0], &d_root_list[1], &d_sweep_list,
+                        &d_exact_list[0], &d_exact_list[1], &d_nout, &d_tune_list, &d_records, &d_round})
         b->release();
+      h_records.release();
       for (auto e : events) cudaEventDestroy(e);
       for (auto e : tune_ev)
         if (e) cudaEventDestroy(e);
@@ -261,8 +268,8 @@ struct fsimb_handle {
     for (const fsimb::DevBuf* b : {&d_type, &d_fi_off, &d_fi_idx, &d_recs, &d_level, &d_level_off, &d_gates,
                             &d_lvl, &d_eflag, &d_gvals, &d_li, &d_roots, &d_members, &d_traced, &d_inj, &d_exact,
                             &d_pwords, &d_good, &d_out, &d_sens, &d_count, &d_first, &d_lastflag,
-                            &d_queue, &d_err, &d_root_list[0], &d_root_list[1], &d_sweep_list,
-                            &d_exact_list[0], &d_exact_list[1], &d_nout, &d_tune_list})
+                            &d_queue, &d_root_list[0], &d_root_list[1], &d_sweep_list,
+                            &d_exact_list[0], &d_exact_list[1], &d_nout, &d_tune_list, &d_records, &d_round})
       s += b->n;
     return s;
   }

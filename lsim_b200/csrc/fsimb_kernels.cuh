@@ -100,6 +100,16 @@ struct ExactArgs {
   uint8_t* lastflag;
 };
 
+struct ResultArgs {
+  const unsigned long long* count;
+  const unsigned long long* first;
+  const uint8_t* lastflag;
+  const int* err;
+  ulonglong2* out;           // [F] records of two, then the error word
+  unsigned long long last_rd;
+  uint32_t F, any_rounds;    // 0: no pattern rounds
+};
+
 // Threads [0, n_in_pad) handle roots, the rest exact faults.
 struct DropArgs {
   const RootRec* roots;
@@ -216,8 +226,12 @@ cudaError_t sweep_wide_occupancy(int M, int* blocks_per_sm);
 constexpr uint64_t kWaitTestNs = 20000000ull;
 void launch_ffr(const FfrArgs& a, cudaStream_t s);
 void launch_exact(const ExactArgs& a, cudaStream_t s);
+// Also zeroes n_zero control words.
 void launch_init_results(unsigned long long* count, unsigned long long* first, uint8_t* lastflag,
-                         uint32_t F, cudaStream_t s);
+                         uint32_t F, int* zero, uint32_t n_zero, cudaStream_t s);
+void launch_results(const ResultArgs& a, cudaStream_t s);
+// good: the round's word of element 0 in its tile.
+void launch_round(const uint64_t* good, uint32_t N, uint64_t mask, uint64_t* out, cudaStream_t s);
 void launch_drop(const DropArgs& a, cudaStream_t s);
 
 }  // namespace fsimb

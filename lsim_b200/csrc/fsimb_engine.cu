@@ -214,6 +214,8 @@ void fsimb_handle::tune_shape(cudaStream_t s) {
     sa.inj = d_inj.as<InjRec>();
     sa.list = d_tune_list.as<uint32_t>();
     sa.n_list = (uint32_t)list.size();
+    sa.n_tiles = 1;
+    sa.n_sweeps = n_sweeps;
     sa.n_words = tile_words(pats.W, 0);
     sa.max_gate_level = plan.max_gate_level;
     sa.N = N;
@@ -308,6 +310,7 @@ void fsimb_handle::run(const fsimb_opts* opts) {
     upload(d_roots, plan.roots, s);
     upload(d_members, plan.members, s);
     upload(d_traced, plan.traced, s);
+    upload(d_traced_slot, plan.traced_slot, s);
     upload(d_inj, plan.sweeps, s);
     upload(d_exact, plan.exact_fault, s);
     eflag_uploaded = false;
@@ -320,8 +323,29 @@ void fsimb_handle::run(const fsimb_opts* opts) {
   CK(cudaEventRecord(upload_ev, s));
   uint64_t launches = 1;  // results init
   d_good.ensure(tiles * N * kTileWords * 8);
-  d_sens.ensure((size_t)N * kTileWords * 8);
-  d_out.ensure((size_t)std::max<uint32_t>(n_sweeps, 1) * kTileWords * 8);
+  const size_t share1 = sweep_smem_share(smem_optin, smem_per_sm, 1);
+  // The documented limit counts every gate's live value (the schedules fold
+  // some of them away): levels beyond it keep to the global-memory sweep,
+  // and explicit shapes beyond it stay refused.
+  auto gates_fit = [&](int m, size_t bytes) {
+    return plan.max_live <= kMaxSlots && sweep_vals_bytes(plan.max_live, m) <= bytes;
+  };
+  // Tiles of one launch: in count mode as many as kTileScratch bytes hold the
+  // sweep outputs and sensitivities of (and fewer than 2^31 sweep items), so
+  // that a run of few tiles has one sweep launch and one tracing launch and
+  // their last CTAs run dry once; drop mode compacts after every tile.
+  // 6,586 gates, 5 tiles: 2.36 + 0.14 -> 2.23 + 0.04 ms; 2,000 gates, 2 tiles: 0.132 +
+  // 0.044 -> 0.113 + 0.023 ms.
+  constexpr uint64_t kTileScratch = 512ull << 20;
+  const uint32_t n_slots = (uint32_t)(plan.members.size() + plan.roots.size());
+  const uint64_t tile_bytes = ((uint64_t)n_sweeps + n_slots + 1) * kTileWords * 8;
+  uint64_t group = 1;
+  if (!o.drop && o.sweep_variant != 2 && gates_fit(1, share1)) {
+    const uint64_t by_items = (1ull << 31) / ((uint64_t)std::max(n_sweeps, 1u) * kTileWords);
+    group = std::max<uint64_t>(1, std::min(tiles, std::min(kTileScratch / tile_bytes, by_items)));
+  }
+  d_sens.ensure(group * std::max<uint32_t>(n_slots, 1) * kTileWords * 8);
+  d_out.ensure(group * std::max<uint32_t>(n_sweeps, 1) * kTileWords * 8);
   d_count.ensure(std::max<uint64_t>(F, 1) * 8);
   d_first.ensure(std::max<uint64_t>(F, 1) * 8);
   d_lastflag.ensure(std::max<uint64_t>(F, 1));
@@ -345,13 +369,6 @@ void fsimb_handle::run(const fsimb_opts* opts) {
   bool wide = o.sweep_variant == 2;
   size_t smem = 0;
   const Schedule* sched = nullptr;
-  const size_t share1 = sweep_smem_share(smem_optin, smem_per_sm, 1);
-  // The documented limit counts every gate's live value (the schedules fold
-  // some of them away): levels beyond it keep to the global-memory sweep,
-  // and explicit shapes beyond it stay refused.
-  auto gates_fit = [&](int m, size_t bytes) {
-    return plan.max_live <= kMaxSlots && sweep_vals_bytes(plan.max_live, m) <= bytes;
-  };
   auto no_room = [&](uint32_t live, int m, size_t bytes, int ctas) {
     return LimitError{"a sweep needs " + std::to_string(live) + " live values; shared memory holds " +
                       std::to_string(bytes / (8 * m)) + " at " + std::to_string(m) + " word(s) per item and " +
@@ -391,6 +408,7 @@ void fsimb_handle::run(const fsimb_opts* opts) {
   }
   int blocks = 0, occ_got = 0;
   if (wide) {
+    group = 1;
     M = o.words_per_item == 1 || (!o.words_per_item && W == 1) ? 1 : 2;
     threads = 256;
     if (!eflag_uploaded && n_sweeps) {
@@ -440,14 +458,16 @@ void fsimb_handle::run(const fsimb_opts* opts) {
   float ms_sweep = 0, ms_ffr = 0;
   const uint32_t gates_end = plan.level_off[std::min(plan.max_gate_level + 1, plan.n_levels)];
   std::vector<uint32_t> host_sw;  // only for the dense-work counter in drop mode
-  for (uint64_t t = 0; t < tiles; ++t) {
+  uint64_t n_groups = 0;
+  for (uint64_t t = 0; t < tiles; t += group, ++n_groups) {
+    const uint32_t n_tiles = (uint32_t)std::min(group, tiles - t);
     const uint64_t* good_t = d_good.as<uint64_t>() + t * (uint64_t)N * kTileWords;
-    cudaEvent_t a0 = ev(4 + 3 * t), a1 = ev(5 + 3 * t), a2 = ev(6 + 3 * t);
+    cudaEvent_t a0 = ev(5 + 3 * n_groups), a1 = ev(6 + 3 * n_groups), a2 = ev(7 + 3 * n_groups);
     CK(cudaEventRecord(a0, s));
     if (n_sw) {
-      const uint32_t n_words = tile_words(W, t);
-      const uint32_t subtiles = (n_words + M - 1) / M;
-      const int nb = (int)std::min<uint64_t>((uint64_t)blocks, (uint64_t)n_sw * subtiles);
+      const uint32_t n_words = tile_words(W, t + n_tiles - 1);
+      const uint64_t subtiles = (uint64_t)(n_tiles - 1) * (kTileWords / M) + (n_words + M - 1) / M;
+      const int nb = (int)std::min<uint64_t>((uint64_t)blocks, n_sw * subtiles);
       if (wide) {
         SweepWideArgs wa{};
         wa.level = d_level.as<uint32_t>();
@@ -479,6 +499,8 @@ void fsimb_handle::run(const fsimb_opts* opts) {
         sa.inj = d_inj.as<InjRec>();
         sa.list = sw_list;
         sa.n_list = n_sw;
+        sa.n_tiles = n_tiles;
+        sa.n_sweeps = n_sweeps;
         sa.n_words = n_words;
         sa.max_gate_level = plan.max_gate_level;
         sa.N = N;
@@ -519,6 +541,11 @@ void fsimb_handle::run(const fsimb_opts* opts) {
     fa.n_list = n_rt;
     fa.members = d_members.as<MemberRec>();
     fa.traced = d_traced.as<TracedRec>();
+    fa.traced_slot = d_traced_slot.as<uint32_t>();
+    fa.N = N;
+    fa.n_sweeps = n_sweeps;
+    fa.n_slots = n_slots;
+    fa.n_tiles = n_tiles;
     fa.fi_off = d_fi_off.as<uint32_t>();
     fa.fi_idx = d_fi_idx.as<uint32_t>();
     fa.type = d_type.as<uint8_t>();
@@ -541,6 +568,8 @@ void fsimb_handle::run(const fsimb_opts* opts) {
     xa.n_exact = n_ex;
     xa.first_sweep = plan.n_stem_sweeps;
     xa.out = d_out.as<uint64_t>();
+    xa.n_sweeps = n_sweeps;
+    xa.n_tiles = n_tiles;
     xa.tile = (uint32_t)t;
     xa.W = (uint32_t)W;
     xa.P = pats.P;
@@ -614,7 +643,7 @@ void fsimb_handle::run(const fsimb_opts* opts) {
   ++launches;
   CK(cudaGetLastError());
   const size_t record_bytes = F * sizeof(fsimb_fault_result);
-  cudaEvent_t e4 = ev(4 + 3 * tiles + 1);
+  cudaEvent_t e4 = ev(4);
   CK(cudaMemcpyAsync(h_records.p, d_records.p, record_bytes + 16, cudaMemcpyDeviceToHost, s));
   CK(cudaEventRecord(e4, s));
   CK(cudaStreamSynchronize(s));
@@ -622,11 +651,11 @@ void fsimb_handle::run(const fsimb_opts* opts) {
   std::memcpy(&kerr, h_records.as<char>() + record_bytes, sizeof kerr);
   if (kerr) throw CudaError{"a sweep kernel reached its time limit waiting for a record copy; results discarded"};
   if (!o.drop) {
-    for (uint64_t t = 0; t < tiles; ++t) {
+    for (uint64_t g = 0; g < n_groups; ++g) {
       float x = 0;
-      CK(cudaEventElapsedTime(&x, ev(4 + 3 * t), ev(5 + 3 * t)));
+      CK(cudaEventElapsedTime(&x, ev(5 + 3 * g), ev(6 + 3 * g)));
       ms_sweep += x;
-      CK(cudaEventElapsedTime(&x, ev(5 + 3 * t), ev(6 + 3 * t)));
+      CK(cudaEventElapsedTime(&x, ev(6 + 3 * g), ev(7 + 3 * g)));
       ms_ffr += x;
     }
   }

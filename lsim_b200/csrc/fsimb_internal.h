@@ -217,7 +217,7 @@ struct fsimb_handle {
   fsimb::DevBuf d_lvl;     // schedule: stream and live-in offsets per level
   fsimb::DevBuf d_eflag;   // wide-circuit sweep: per element, evaluated / drives a PO
   fsimb::DevBuf d_gvals;   // wide-circuit sweep: per-CTA value regions
-  fsimb::DevBuf d_roots, d_members, d_traced, d_inj, d_exact;
+  fsimb::DevBuf d_roots, d_members, d_traced, d_traced_slot, d_inj, d_exact;
   fsimb::DevBuf d_pwords, d_good, d_out, d_sens, d_count, d_first, d_lastflag, d_queue;
   fsimb::DevBuf d_root_list[2], d_sweep_list, d_exact_list[2], d_nout, d_tune_list;
   uint64_t good_tiles = 0;  // tiles held in d_good
@@ -240,7 +240,7 @@ struct fsimb_handle {
     if (device >= 0) {
       cudaSetDevice(device);
       for (fsimb::DevBuf* b : {&d_type, &d_fi_off, &d_fi_idx, &d_recs, &d_level, &d_level_off, &d_gates,
-                        &d_lvl, &d_eflag, &d_gvals, &d_li, &d_roots, &d_members, &d_traced, &d_inj, &d_exact,
+                        &d_lvl, &d_eflag, &d_gvals, &d_li, &d_roots, &d_members, &d_traced, &d_traced_slot, &d_inj, &d_exact,
                         &d_pwords, &d_good, &d_out, &d_sens, &d_count, &d_first, &d_lastflag,
                         &d_queue, &d_root_list[0], &d_root_list[1], &d_sweep_list,
                         &d_exact_list[0], &d_exact_list[1], &d_nout, &d_tune_list, &d_records, &d_round})
@@ -266,7 +266,7 @@ struct fsimb_handle {
   uint64_t device_bytes() const {
     uint64_t s = 0;
     for (const fsimb::DevBuf* b : {&d_type, &d_fi_off, &d_fi_idx, &d_recs, &d_level, &d_level_off, &d_gates,
-                            &d_lvl, &d_eflag, &d_gvals, &d_li, &d_roots, &d_members, &d_traced, &d_inj, &d_exact,
+                            &d_lvl, &d_eflag, &d_gvals, &d_li, &d_roots, &d_members, &d_traced, &d_traced_slot, &d_inj, &d_exact,
                             &d_pwords, &d_good, &d_out, &d_sens, &d_count, &d_first, &d_lastflag,
                             &d_queue, &d_root_list[0], &d_root_list[1], &d_sweep_list,
                             &d_exact_list[0], &d_exact_list[1], &d_nout, &d_tune_list, &d_records, &d_round})

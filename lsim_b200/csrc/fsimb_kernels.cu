@@ -692,12 +692,13 @@ __global__ void __maxnreg__(64) k_sweep(SweepArgs a) {
     sweep_wait_test(&bar, a.wait_ns, a.err);
     return;
   }
-  const SweepView v{a.blob, a.lvl, a.level, a.li, a.fi_off, a.fi_idx, a.type, a.good,
-                    a.max_gate_level, a.stream_recs, a.fix0, a.inj_slot, a.split};
-  // Subtiles that hold pattern words: the last tile of a block is rarely full
-  // (16 words of 32 for 1,000 patterns), and the tracing masks the others.
-  const uint32_t subtiles = (a.n_words + M - 1) / M;
-  const uint32_t n_items = a.n_list * subtiles;
+  // Items are (tile, sweep, subtile), tile-major.  Only subtiles that hold
+  // pattern words: the last tile of a block is rarely full (16 words of 32
+  // for 1,000 patterns), and the tracing masks the others.
+  constexpr uint32_t subtiles = kTileWords / M;
+  const uint32_t last_sub = (a.n_words + M - 1) / M;
+  const uint32_t per_tile = a.n_list * subtiles;
+  const uint32_t n_items = (a.n_tiles - 1) * per_tile + a.n_list * last_sub;
   // The next item's number is asked for while the current one runs.
   uint32_t next = blockIdx.x;
   for (;;) {
@@ -708,10 +709,16 @@ __global__ void __maxnreg__(64) k_sweep(SweepArgs a) {
     cta_sync();
     const uint32_t item = s_item;
     if (item >= n_items) return;
-    const uint32_t li = item / subtiles;
-    const uint32_t w0 = (item % subtiles) * M;
+    const uint32_t tile = min(item / per_tile, a.n_tiles - 1);
+    const uint32_t rem = item - tile * per_tile;
+    const uint32_t sub = tile == a.n_tiles - 1 ? last_sub : subtiles;
+    const uint32_t li = rem / sub;
+    const uint32_t w0 = (rem % sub) * M;
     const uint32_t si = a.list ? a.list[li] : li;
-    sweep_item<M>(vals, acc, v, a.inj[si], w0, a.out + (uint64_t)si * 32);
+    const SweepView v{a.blob, a.lvl, a.level, a.li, a.fi_off, a.fi_idx, a.type,
+                      a.good + (uint64_t)tile * a.N * 32,
+                      a.max_gate_level, a.stream_recs, a.fix0, a.inj_slot, a.split};
+    sweep_item<M>(vals, acc, v, a.inj[si], w0, a.out + ((uint64_t)tile * a.n_sweeps + si) * 32);
   }
 }
 
@@ -770,9 +777,7 @@ __global__ void __launch_bounds__(256) k_sweep_wide(SweepWideArgs a) {
   uint64_t* gv = a.gvals + (size_t)blockIdx.x * a.N * M;
   const uint32_t tid = threadIdx.x, nth = blockDim.x;
   const uint32_t m = tid % M, step = nth / M;
-  // Subtiles that hold pattern words: the last tile of a block is rarely full
-  // (16 words of 32 for 1,000 patterns), and the tracing masks the others.
-  const uint32_t subtiles = (a.n_words + M - 1) / M;
+  const uint32_t subtiles = (a.n_words + M - 1) / M;  // those that hold pattern words
   const uint32_t n_items = a.n_list * subtiles;
   for (;;) {
     if (tid == 0) s_item = atomicAdd(a.queue, 1);
@@ -862,71 +867,80 @@ __device__ __forceinline__ void record(unsigned long long* count, unsigned long 
   if (w == W - 1) lastflag[f] = D != 0ull;
 }
 
-__global__ void __launch_bounds__(256) k_ffr(FfrArgs a) {
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t n = a.n_list;
-  if (warp >= n) return;
-  const uint32_t ri = a.list ? a.list[warp] : warp;
-  const RootRec rr = a.roots[ri];
+// What tracing reads of one circuit's tile.
+struct FfrView {
+  const MemberRec* members;
+  const TracedRec* traced;
+  const uint32_t* traced_slot;
+  const uint32_t* fi_off;
+  const uint32_t* fi_idx;
+  const uint8_t* type;
+  const uint64_t* good;      // tile [N][32]
+  const uint64_t* obs;       // tile [n_sweeps][32]
+  uint64_t* sens;            // tile [n_slots][32]: slot i = members[i], then the roots
+  unsigned long long* count;
+  unsigned long long* first;
+  uint8_t* lastflag;
+  uint64_t P;
+  uint32_t W, tile;
+  uint32_t drop_at;          // skip faults whose count reached this (0: none)
+};
+
+// One FFR on one tile by one warp, lanes = words.
+__device__ __forceinline__ void ffr_root(const FfrView& a, const RootRec& rr, uint32_t lane) {
   const uint32_t w = a.tile * 32 + lane;
   const uint32_t bits = round_bits(a.P, a.W, w);
-  const uint64_t mask = bits_mask(bits);
-  uint64_t obs;
-  if (rr.obs == kObsOne)
-    obs = ~0ull;
-  else if (rr.obs == kObsZero)
-    obs = 0ull;
-  else
-    obs = a.obs[(uint64_t)rr.obs * 32 + lane];
-  obs &= mask;
-  a.sens[(uint64_t)rr.root * 32 + lane] = ~0ull;
+  uint64_t obs = rr.obs == kObsOne ? ~0ull : rr.obs == kObsZero ? 0ull : a.obs[(uint64_t)rr.obs * 32 + lane];
+  obs &= bits_mask(bits);
+  a.sens[(uint64_t)rr.slot * 32 + lane] = ~0ull;
   for (uint32_t i = rr.mem_begin; i < rr.mem_end; ++i) {
     const MemberRec m = a.members[i];
-    const uint64_t sp = a.sens[(uint64_t)m.p * 32 + lane];
-    a.sens[(uint64_t)m.e * 32 + lane] = sp & local_sens(a, m.p, m.pin, lane);
+    a.sens[(uint64_t)i * 32 + lane] = a.sens[(uint64_t)m.p_slot * 32 + lane] & local_sens(a, m.p, m.pin, lane);
   }
   for (uint32_t i = rr.flt_begin; i < rr.flt_end; ++i) {
     const TracedRec tr = a.traced[i];
-    if (a.drop && a.count[tr.fault] >= a.n_detect) continue;  // dropped after an earlier tile
-    uint64_t s, gv;
+    if (a.drop_at && a.count[tr.fault] >= a.drop_at) continue;  // dropped after an earlier tile
+    uint64_t s = a.sens[(uint64_t)a.traced_slot[i] * 32 + lane], gv;
     if (tr.pin == 0) {
-      s = a.sens[(uint64_t)tr.elem * 32 + lane];
       gv = a.good[(uint64_t)tr.elem * 32 + lane];
     } else {
-      s = a.sens[(uint64_t)tr.elem * 32 + lane] & local_sens(a, tr.elem, tr.pin - 1, lane);
+      s &= local_sens(a, tr.elem, tr.pin - 1, lane);
       gv = a.good[(uint64_t)a.fi_idx[a.fi_off[tr.elem] + tr.pin - 1] * 32 + lane];
     }
-    const uint64_t sv = tr.value ? ~0ull : 0ull;
-    const uint64_t D = s & (gv ^ sv) & obs;
+    const uint64_t D = s & (gv ^ (tr.value ? ~0ull : 0ull)) & obs;
     record(a.count, a.first, a.lastflag, tr.fault, D, w, bits, a.W, lane);
   }
 }
 
+// One warp per (tile, root).
+__global__ void __launch_bounds__(256) k_ffr(FfrArgs a) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint64_t unit = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (unit >= (uint64_t)a.n_list * a.n_tiles) return;
+  const uint32_t t = (uint32_t)(unit / a.n_list), i = (uint32_t)(unit % a.n_list);
+  const FfrView v{a.members, a.traced, a.traced_slot, a.fi_off, a.fi_idx, a.type,
+                  a.good + (uint64_t)t * a.N * 32, a.obs + (uint64_t)t * a.n_sweeps * 32,
+                  a.sens + (uint64_t)t * a.n_slots * 32, a.count, a.first, a.lastflag, a.P, a.W, a.tile + t,
+                  a.drop ? a.n_detect : 0u};
+  ffr_root(v, a.roots[a.list ? a.list[i] : i], lane);
+}
+
+// One warp per (tile, exact fault).
 __global__ void __launch_bounds__(256) k_exact(ExactArgs a) {
   const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (warp >= a.n_exact) return;
-  const uint32_t j = a.list ? a.list[warp] : warp;
+  const uint64_t unit = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (unit >= (uint64_t)a.n_exact * a.n_tiles) return;
+  const uint32_t t = (uint32_t)(unit / a.n_exact), i = (uint32_t)(unit % a.n_exact);
+  const uint32_t j = a.list ? a.list[i] : i;
   const uint32_t f = a.exact_fault[j];
   if (a.drop && a.count[f] >= a.n_detect) return;  // dropped after an earlier tile
-  const uint32_t w = a.tile * 32 + lane;
+  const uint32_t w = (a.tile + t) * 32 + lane;
   const uint32_t bits = round_bits(a.P, a.W, w);
-  const uint64_t mask = bits_mask(bits);
-  const uint64_t D = a.out[(uint64_t)(a.first_sweep + j) * 32 + lane] & mask;
+  const uint64_t D = a.out[((uint64_t)t * a.n_sweeps + a.first_sweep + j) * 32 + lane] & bits_mask(bits);
   record(a.count, a.first, a.lastflag, f, D, w, bits, a.W, lane);
 }
 
 // ---------------------------------------------------------------- batches
-// The good-machine words and scratch of one circuit's tile, for the batched
-// tracing kernels.
-struct TileView {
-  const uint8_t* type;
-  const uint32_t* fi_off;
-  const uint32_t* fi_idx;
-  const uint64_t* good;
-};
-
 // One CTA per (circuit, kGoodBatchWords words) of the batch.
 __global__ void __launch_bounds__(256) k_good_batch(BatchUnits u) {
   const uint32_t ci = find_prefix(u.unit_prefix, u.n_circ, blockIdx.x);
@@ -936,7 +950,7 @@ __global__ void __launch_bounds__(256) k_good_batch(BatchUnits u) {
   good_words<kGoodBatchWords>(v, (uint32_t)(blockIdx.x - u.unit_prefix[ci]) * kGoodBatchWords);
 }
 
-// One warp per (circuit, tile, root): the k_ffr body on that circuit's tile.
+// One warp per (circuit, tile, root).
 __global__ void __launch_bounds__(256) k_ffr_batch(BatchUnits u, unsigned long long n_units) {
   const uint32_t lane = threadIdx.x & 31u;
   const unsigned long long unit = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -945,35 +959,10 @@ __global__ void __launch_bounds__(256) k_ffr_batch(BatchUnits u, unsigned long l
   const BatchCirc& c = u.circs[ci];
   const unsigned long long local = unit - u.unit_prefix[ci];
   const uint32_t tile = (uint32_t)(local / c.n_roots);
-  const uint32_t ri = (uint32_t)(local % c.n_roots);
-  const TileView tv{c.type, c.fi_off, c.fi_idx, c.good + (uint64_t)tile * c.N * 32};
-  // compact sensitivities: slot i = members[i], slot n_members + r = root r
-  uint64_t* sens = c.sens + (uint64_t)tile * c.n_slots * 32;
-  const uint64_t* obsv = c.out + (uint64_t)tile * c.n_sweeps * 32;
-  const RootRec rr = c.roots[ri];
-  const uint32_t w = tile * 32 + lane;
-  const uint32_t bits = round_bits(c.P, c.W, w);
-  uint64_t obs = rr.obs == kObsOne ? ~0ull : rr.obs == kObsZero ? 0ull : obsv[(uint64_t)rr.obs * 32 + lane];
-  obs &= bits_mask(bits);
-  sens[(uint64_t)rr.slot * 32 + lane] = ~0ull;
-  for (uint32_t i = rr.mem_begin; i < rr.mem_end; ++i) {
-    const MemberRec m = c.members[i];
-    sens[(uint64_t)i * 32 + lane] = sens[(uint64_t)m.p_slot * 32 + lane] & local_sens(tv, m.p, m.pin, lane);
-  }
-  for (uint32_t i = rr.flt_begin; i < rr.flt_end; ++i) {
-    const TracedRec tr = c.traced[i];
-    const uint64_t st = sens[(uint64_t)c.traced_slot[i] * 32 + lane];
-    uint64_t sv, gv;
-    if (tr.pin == 0) {
-      sv = st;
-      gv = tv.good[(uint64_t)tr.elem * 32 + lane];
-    } else {
-      sv = st & local_sens(tv, tr.elem, tr.pin - 1, lane);
-      gv = tv.good[(uint64_t)c.fi_idx[c.fi_off[tr.elem] + tr.pin - 1] * 32 + lane];
-    }
-    const uint64_t D = sv & (gv ^ (tr.value ? ~0ull : 0ull)) & obs;
-    record(c.count, c.first, c.lastflag, tr.fault, D, w, bits, c.W, lane);
-  }
+  const FfrView v{c.members, c.traced, c.traced_slot, c.fi_off, c.fi_idx, c.type,
+                  c.good + (uint64_t)tile * c.N * 32, c.out + (uint64_t)tile * c.n_sweeps * 32,
+                  c.sens + (uint64_t)tile * c.n_slots * 32, c.count, c.first, c.lastflag, c.P, c.W, tile, 0u};
+  ffr_root(v, c.roots[(uint32_t)(local % c.n_roots)], lane);
 }
 
 // One warp per (circuit, tile, exact fault).
@@ -1219,14 +1208,14 @@ cudaError_t sweep_wide_occupancy(int M, int* blocks_per_sm) {
 void launch_ffr(const FfrArgs& a, cudaStream_t s) {
   if (a.n_list == 0) return;
   const int threads = 256;
-  const uint64_t blocks = ((uint64_t)a.n_list * 32 + threads - 1) / threads;
+  const uint64_t blocks = ((uint64_t)a.n_list * a.n_tiles * 32 + threads - 1) / threads;
   k_ffr<<<(unsigned)blocks, threads, 0, s>>>(a);
 }
 
 void launch_exact(const ExactArgs& a, cudaStream_t s) {
   if (a.n_exact == 0) return;
   const int threads = 256;
-  const uint64_t blocks = ((uint64_t)a.n_exact * 32 + threads - 1) / threads;
+  const uint64_t blocks = ((uint64_t)a.n_exact * a.n_tiles * 32 + threads - 1) / threads;
   k_exact<<<(unsigned)blocks, threads, 0, s>>>(a);
 }
 

@@ -30,11 +30,12 @@ struct SweepArgs {
   const InjRec* inj;
   const uint32_t* list;    // sweep indices to run (nullptr: 0..n_list-1)
   uint32_t n_list;
-  uint32_t n_words;        // pattern words of this tile (1..32): the others are not swept
+  uint32_t n_tiles, n_sweeps;
+  uint32_t n_words;        // pattern words of the last tile (1..32): the others are not swept
   uint32_t max_gate_level;
   uint32_t N;
-  const uint64_t* good;    // this tile: [N][32]
-  uint64_t* out;           // this tile: [n_sweeps][32] OR of PO differences
+  const uint64_t* good;    // first tile: [n_tiles][N][32]
+  uint64_t* out;           // [n_tiles][n_sweeps][32] OR of PO differences
   int* queue;              // work counter for this launch
   uint32_t stream_recs;    // records of the stream's rounds
   uint32_t fix0, inj_slot; // fix entries in blob; the injection slot
@@ -70,13 +71,16 @@ struct FfrArgs {
   uint32_t n_list;
   const MemberRec* members;
   const TracedRec* traced;
+  const uint32_t* traced_slot;
   const uint32_t* fi_off;
   const uint32_t* fi_idx;
   const uint8_t* type;
-  const uint64_t* good;    // tile [N][32]
-  const uint64_t* obs;     // tile [n_sweeps][32]
-  uint64_t* sens;          // scratch [N][32]
-  uint32_t tile, W;
+  const uint64_t* good;    // first tile: [n_tiles][N][32]
+  const uint64_t* obs;     // [n_tiles][n_sweeps][32]
+  uint64_t* sens;          // scratch [n_tiles][n_slots][32]: members, then roots
+  uint32_t N, n_sweeps, n_slots;
+  uint32_t n_tiles;
+  uint32_t tile, W;        // first tile
   uint64_t P;
   int drop;                // skip faults whose count reached n_detect in an earlier tile
   uint32_t n_detect;       // >= 1
@@ -90,8 +94,9 @@ struct ExactArgs {
   const uint32_t* list;    // exact indices to process (nullptr: all)
   uint32_t n_exact;
   uint32_t first_sweep;    // index of the first exact sweep
-  const uint64_t* out;     // tile [n_sweeps][32]
-  uint32_t tile, W;
+  const uint64_t* out;     // [n_tiles][n_sweeps][32]
+  uint32_t n_sweeps, n_tiles;
+  uint32_t tile, W;        // first tile
   uint64_t P;
   int drop;
   uint32_t n_detect;

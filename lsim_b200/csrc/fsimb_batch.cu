@@ -1106,9 +1106,9 @@ void fsimb_batch::run(const fsimb_batch_opts* opts) {
   const std::vector<BatchJob> js = jobs_for(all, a);
   for (size_t i = 0; i < members.size(); ++i) {
     fsimb_handle* h = members[i];
-    h->batch_results.resize(js[i].F);
-    exec.results(i, js[i], h->batch_results.data());
-    h->records = h->batch_results.data();
+    h->host_records.resize(js[i].F);
+    exec.results(i, js[i], h->host_records.data());
+    h->records = h->host_records.data();
     h->n_records = js[i].F;
     h->has_results = true;
   }

@@ -146,6 +146,14 @@ struct PinnedBuf {
     }
     n = bytes;
   }
+  // As ensure(); false, with nothing held, where the memory cannot be locked.
+  bool try_ensure(size_t bytes) {
+    try {
+      ensure(bytes);
+    } catch (const CudaError&) {
+    }
+    return p != nullptr;
+  }
   void release() {
     if (p) cudaFreeHost(p);
     p = nullptr;
@@ -225,11 +233,11 @@ struct fsimb_handle {
   bool pats_uploaded = false;  // d_pwords holds the current patterns
   bool eflag_uploaded = false; // d_eflag holds the current plan's element flags
 
-  // The last run's records: in h_records after fsimb_run, in batch_results
-  // after a batch's run.
+  // The last run's records: in host_records or h_records after fsimb_run, in
+  // host_records after a batch's run.
   fsimb::DevBuf d_records, d_round;
   fsimb::PinnedBuf h_records;
-  std::vector<fsimb_fault_result> batch_results;
+  std::vector<fsimb_fault_result> host_records;
   const fsimb_fault_result* records = nullptr;
   uint64_t n_records = 0;
   bool has_results = false;

@@ -84,10 +84,13 @@ namespace fsimb {
 // a latency (barrier, record, operands, store) of kLevel cycles plus kRound
 // for each further round, and the shared-memory and issue time of all the
 // SM's CTAs: a number of cycles by M for a warp's records, kPad for a warp of
-// padding.  Fitted to shape sweeps on a B200; best of the sweep against the
-// model's choice: 2,000 gates 0.129 / 0.138 ms, 6,586 gates 2.34 / 2.36, 20,000
-// gates with MUX 8.00 / 8.14, 30,000 gates 31.5 / 33.6, 50,000 gates 52.2 /
-// 54.9, 200,000 gates 339 / 347 ms.
+// padding.  A CTA alone on its SM has nothing to fill its barriers with: a
+// fifth more.  Fitted to shape sweeps on a B200; best of the nine cheapest
+// against the model's choice: 2,000 gates 0.113 / 0.113 ms, 6,586 gates 2.25 /
+// 2.25, 20,000 gates with MUX 8.14 / 8.04, 30,000 gates 2.87 / 2.96, 60,000
+// gates 6.12 / 6.12; two CTAs of 512 threads and 4 words against one of 1,024
+// and 8: 50,000 gates 52.7 / 54.6 ms, 100,000 gates 11.8 / 12.3, 200,000 gates
+// 342 / 344.
 double sweep_shape_cost(const SweepNet& net, int m, uint32_t t, size_t vals, size_t smem_per_sm, uint32_t words) {
   constexpr double kLevel = 1100, kRound = 300, kPad = 4;
   const uint32_t w = std::max<uint32_t>(1, std::min<uint32_t>(words, kTileWords));
@@ -100,7 +103,7 @@ double sweep_shape_cost(const SweepNet& net, int m, uint32_t t, size_t vals, siz
     const uint32_t rounds = (n + t - 1) / t, full = (n + 31) / 32, all = rounds * (t / 32);
     cycles += kLevel + kRound * (rounds - 1) + ctas * (full * warp + (all - full) * kPad);
   }
-  return cycles / ctas * ((w + m - 1) / m);
+  return (ctas == 1 ? 1.2 : 1.0) * cycles / ctas * ((w + m - 1) / m);
 }
 
 std::vector<SweepShape> likely_shapes(const Plan& plan, uint32_t words, size_t smem_optin, size_t smem_per_sm,

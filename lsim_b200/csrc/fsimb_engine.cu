@@ -87,14 +87,14 @@ namespace fsimb {
 // padding.  A CTA alone on its SM has nothing to fill its barriers with: a
 // fifth more.  Fitted to shape sweeps on a B200; best of the nine cheapest
 // against the model's choice: 2,000 gates 0.113 / 0.113 ms, 6,586 gates 2.25 /
-// 2.25, 20,000 gates with MUX 8.14 / 8.04, 30,000 gates 2.87 / 2.96, 60,000
+// 2.25, 20,000 gates with MUX 8.14 / 8.04, 30,000 gates 2.84 / 2.84, 60,000
 // gates 6.12 / 6.12; two CTAs of 512 threads and 4 words against one of 1,024
 // and 8: 50,000 gates 52.7 / 54.6 ms, 100,000 gates 11.8 / 12.3, 200,000 gates
 // 342 / 344.
 double sweep_shape_cost(const SweepNet& net, int m, uint32_t t, size_t vals, size_t smem_per_sm, uint32_t words) {
   constexpr double kLevel = 1100, kRound = 300, kPad = 4;
   const uint32_t w = std::max<uint32_t>(1, std::min<uint32_t>(words, kTileWords));
-  const double warp = m == 8 ? 61 : m == 4 ? 31 : m == 2 ? 18 : 15;
+  const double warp = m == 8 ? 61 : m == 4 ? 30 : m == 2 ? 18 : 15;
   const uint32_t ctas = (uint32_t)std::min<size_t>({smem_per_sm / (vals + 1024 + 256), 1024 / t, 32});
   if (ctas < 1) return 1e300;
   double cycles = 0;

@@ -569,7 +569,7 @@ __device__ __forceinline__ void cta_sync() {
 // and stores of a sweep are free of bank conflicts wherever the host found
 // such groups.
 //
-// A thread reads its records straight from global memory (L1 / L2), kPrefetch
+// A thread reads its records straight from global memory (L1 / L2), kAhead
 // rounds ahead: the stream is padded per level to rounds of one record per
 // thread, so the next address is one addition away and a level's end is a
 // bit of its last round's records.
@@ -593,9 +593,14 @@ __device__ __forceinline__ void sweep_item(uint64_t* vals, unsigned long long* a
   const uint32_t first = inj.level <= v.max_gate_level ? lv.x : v.stream_recs;
   if (first < v.stream_recs) {
     const RecWords<M>* rp = reinterpret_cast<const RecWords<M>*>(v.blob) + first + tid;
-    RecWords<M> q[kPrefetch];
+    // Three rounds at M = 4, the shape of large circuits: 100,000 gates 11.84 ->
+    // 11.75 ms, 200,000 gates 341.5 -> 336.4; four 11.67 and 335.3, but 30,000
+    // gates 2.90 -> 2.95.  At M = 8 three cost 6 % (6,586 gates) to 23 % (small).
+    constexpr int kAhead = M == 4 ? 3 : 2;
+    static_assert(kAhead <= (int)kPrefetch, "the stream's padding");
+    RecWords<M> q[kAhead];
 #pragma unroll
-    for (int j = 0; j < (int)kPrefetch; ++j, rp += nth) q[j] = *rp;
+    for (int j = 0; j < kAhead; ++j, rp += nth) q[j] = *rp;
     // Values live at the start level come from the good machine (copied
     // asynchronously, four list entries in flight per thread), except the
     // injection element itself.
@@ -653,11 +658,11 @@ __device__ __forceinline__ void sweep_item(uint64_t* vals, unsigned long long* a
         }
       }
     };
-    // kPrefetch rounds a turn, so that a record's registers are loaded again
+    // kAhead rounds a turn, so that a record's registers are loaded again
     // only after its evaluation and nothing waits for a load early.
     for (uint32_t at = first;;) {
 #pragma unroll
-      for (int j = 0; j < (int)kPrefetch; ++j) {
+      for (int j = 0; j < kAhead; ++j) {
         round(q[j], at);
         q[j] = *rp;
         rp += nth;

@@ -238,7 +238,7 @@ struct Schedule {
   std::vector<std::array<uint32_t, 4>> lvl;  // [n_levels+1] first record, li begin, li end, 0
   uint64_t bytes() const { return blob.size() * 4 + lvl.size() * 16 + li.size() * 4; }
 };
-constexpr uint32_t kPrefetch = 2;  // rounds a sweep reads ahead
+constexpr uint32_t kPrefetch = 3;  // rounds a sweep reads ahead at most
 constexpr uint64_t kSplitRecords = 256;  // records a level from which ANDs and XORs have kinds of their own
 
 // 0: AND family (AND, NAND, OR, NOR, INV, CLKBUF, PO), 1: XOR family, 2: MUX.

@@ -456,8 +456,8 @@ def _rooflines(launch_s, alg_bytes, st, clk):
     peak, peak_src = _peaks()
     prof = _profile_summary()
     traffic = prof.get("traffic_per_launch_bytes")
-    # compulsory DRAM bytes of one launch: the tile's good words, the gate
-    # records and live-in lists of the schedule, the sweep output rows
+    # compulsory DRAM bytes of one tile: its good words, the record stream and
+    # live-in lists of the schedule, the sweep output rows
     compulsory = st["hbm_bytes_per_tile"]
     hbm = compulsory / launch_s / 1e9 if launch_s > 0 else 0.0
     mhz = (clk or {}).get("sm_mhz") or 1965.0
@@ -468,9 +468,9 @@ def _rooflines(launch_s, alg_bytes, st, clk):
                      "frac": hbm / peak, "traffic": traffic, "kernel": "k_sweep",
                      "peak_source": peak_src,
                      "per_launch_bytes": compulsory, "per_launch_ms": launch_s * 1e3,
-                     "note": "achieved = compulsory DRAM bytes of one launch (good words of the "
-                             "tile, gate records, live-in lists, output rows) / its CUDA-event "
-                             "time; traffic = ncu dram bytes of one launch. Values stay in "
+                     "note": "achieved = compulsory DRAM bytes of one tile (good words, record "
+                             "stream, live-in lists, output rows) / its share of the CUDA-event "
+                             "time; traffic = ncu dram bytes per tile. Values stay in "
                              "shared memory, so HBM is not what binds this kernel (see onchip)"},
         "onchip": {"bound": "shared-memory bandwidth", "achieved": onchip, "peak": smem_peak,
                    "unit": "GB/s", "frac": onchip / smem_peak,

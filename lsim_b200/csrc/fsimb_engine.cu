@@ -2,11 +2,12 @@
 //
 // One run:
 //   1. upload the compiled plan (once per circuit + fault list) and patterns;
-//   2. good machine for all words, level by level (k_good_level);
-//   3. per 2048-pattern tile: stem / exact sweeps (k_sweep<M>), FFR tracing
-//      and per-fault accumulation (k_ffr, k_exact), and in drop mode the
-//      compaction of what is still undetected (k_drop);
-//   4. per-fault counters back to the host.
+//   2. good machine for all words (launch_good);
+//   3. per group of 2,048-pattern tiles: stem / exact sweeps (k_sweep<M>), FFR
+//      tracing and per-fault accumulation (k_ffr, k_exact); in drop mode a
+//      group is one tile, followed by the compaction of what is still
+//      undetected (k_drop);
+//   4. per-fault records back to the host (k_results).
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -776,7 +776,7 @@ __global__ void __maxnreg__(64) k_sweep_batch(const __grid_constant__ BatchSweep
 // good machine directly, so an item starts without copying live values.
 // Threads take (element, word) pairs of a level; one barrier per level.
 template <int M>
-__global__ void __launch_bounds__(256) k_sweep_wide(SweepWideArgs a) {
+__global__ void __launch_bounds__(1024) k_sweep_wide(SweepWideArgs a) {
   __shared__ unsigned long long acc[M];
   __shared__ uint32_t s_item;
   uint64_t* gv = a.gvals + (size_t)blockIdx.x * a.N * M;
@@ -1193,19 +1193,19 @@ cudaError_t launch_sweep(int M, int threads, int blocks, size_t smem, const Swee
   return cudaGetLastError();
 }
 
-cudaError_t launch_sweep_wide(int M, int blocks, const SweepWideArgs& a, cudaStream_t s) {
+cudaError_t launch_sweep_wide(int M, int threads, int blocks, const SweepWideArgs& a, cudaStream_t s) {
   switch (M) {
-    case 1: k_sweep_wide<1><<<blocks, 256, 0, s>>>(a); break;
-    case 2: k_sweep_wide<2><<<blocks, 256, 0, s>>>(a); break;
+    case 1: k_sweep_wide<1><<<blocks, threads, 0, s>>>(a); break;
+    case 2: k_sweep_wide<2><<<blocks, threads, 0, s>>>(a); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
 }
 
-cudaError_t sweep_wide_occupancy(int M, int* blocks_per_sm) {
+cudaError_t sweep_wide_occupancy(int M, int threads, int* blocks_per_sm) {
   switch (M) {
-    case 1: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_sweep_wide<1>, 256, 0);
-    case 2: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_sweep_wide<2>, 256, 0);
+    case 1: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_sweep_wide<1>, threads, 0);
+    case 2: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_sweep_wide<2>, threads, 0);
   }
   return cudaErrorInvalidValue;
 }

@@ -225,8 +225,8 @@ cudaError_t launch_sweep(int M, int threads, int blocks, size_t smem, const Swee
 cudaError_t sweep_set_smem(int M, size_t smem);
 cudaError_t sweep_occupancy(int M, int threads, size_t smem, int* blocks_per_sm);
 // M in {1, 2}; 256 threads per CTA.
-cudaError_t launch_sweep_wide(int M, int blocks, const SweepWideArgs& a, cudaStream_t s);
-cudaError_t sweep_wide_occupancy(int M, int* blocks_per_sm);
+cudaError_t launch_sweep_wide(int M, int threads, int blocks, const SweepWideArgs& a, cudaStream_t s);
+cudaError_t sweep_wide_occupancy(int M, int threads, int* blocks_per_sm);
 // Time limit of the wait test's wait.
 constexpr uint64_t kWaitTestNs = 20000000ull;
 void launch_ffr(const FfrArgs& a, cudaStream_t s);

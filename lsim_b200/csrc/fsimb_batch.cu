@@ -697,7 +697,7 @@ struct fsimb_batch {
       for (int m = M; m >= 1; m /= 2) {
         if (!gates_fit(i, share)) return;
         const Schedule& sc = schedule_at(i, m);
-        if (sc.max_live <= kMaxSlots && sweep_vals_bytes(sc.max_live, m) <= share) {
+        if (sched_fits(sc, m, share)) {
           got[i] = m;
           return;
         }
@@ -854,8 +854,7 @@ struct fsimb_batch {
       const size_t share1 = smem_share(1);
       auto fits_M = [&](int M) {
         if (sweep_vals_bytes(P.net_live, M) > share1) return false;
-        const Schedule& sc = schedule_at(i, M);
-        return sc.max_live <= kMaxSlots && sweep_vals_bytes(sc.max_live, M) <= share1;
+        return sched_fits(schedule_at(i, M), M, share1);
       };
       // Times shape sh on `plan`: a one-circuit layout with its first
       // tile's good machine.  Negative if the shape does not run.

@@ -153,7 +153,7 @@ void default_sweep_shape(const Plan& plan, const std::function<const Schedule&(i
     if (exact[bi]) break;
     const Schedule& sc = sched_at(M);
     exact[bi] = true;
-    vals[bi] = sc.max_live > kMaxSlots ? share1 + 1 : sweep_vals_bytes(sc.max_live, M);
+    vals[bi] = sched_fits(sc, M, share1) ? sweep_vals_bytes(sc.max_live, M) : share1 + 1;
   }
   threads = std::min<int>(threads, (int)sweep_max_threads(M));
 }
@@ -199,8 +199,7 @@ void fsimb_handle::tune_shape(cudaStream_t s) {
   const size_t share1 = sweep_smem_share(smem_optin, smem_per_sm, 1);
   for (const SweepShape& cd : cands) {
     const int M = cd.M, T = cd.threads;
-    if (cached_schedule(M).max_live > kMaxSlots || sweep_vals_bytes(cached_schedule(M).max_live, M) > share1)
-      continue;
+    if (!sched_fits(cached_schedule(M), M, share1)) continue;
     const Schedule& sc = use_schedule(M, T, s);
     const size_t smem = std::max<size_t>(16, sweep_vals_bytes(sc.max_live, M));
     CK(sweep_set_smem(M, smem));
@@ -388,9 +387,7 @@ void fsimb_handle::run(const fsimb_opts* opts) {
       const size_t budget = sweep_smem_share(smem_optin, smem_per_sm, ctas);
       M = o.words_per_item ? (int)o.words_per_item : 8;
       for (;; M /= 2) {
-        if (gates_fit(M, budget) && cached_schedule(M).max_live <= kMaxSlots &&
-            sweep_vals_bytes(cached_schedule(M).max_live, M) <= budget)
-          break;
+        if (gates_fit(M, budget) && sched_fits(cached_schedule(M), M, budget)) break;
         if (o.words_per_item || M == 1)
           throw no_room(std::max(plan.max_live, cached_schedule(M).max_live), M, budget, ctas);
       }

@@ -24,9 +24,6 @@ namespace fsimb {
 struct CudaError {
   std::string msg;
 };
-struct LimitError {
-  std::string msg;
-};
 struct StateError {
   std::string msg;
 };
@@ -128,6 +125,12 @@ inline uint32_t tile_words(uint64_t W, uint64_t t) {
 // Bytes of a sweep CTA's value slots: max_live slots of M words, 16-byte rounded.
 inline uint32_t sweep_vals_bytes(uint32_t max_live, int M) {
   return (uint32_t)(((size_t)max_live * M * 8 + 15) / 16 * 16);
+}
+
+// Whether the schedule at M words per item has its records and its slots fit
+// `bytes` of shared memory.
+inline bool sched_fits(const Schedule& sc, int M, size_t bytes) {
+  return sc.max_live <= max_slots(sc.G) && sweep_vals_bytes(sc.max_live, M) <= bytes;
 }
 
 // Page-locked host staging buffer.

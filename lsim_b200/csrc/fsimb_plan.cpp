@@ -642,9 +642,10 @@ void build_schedule(const Netlist& nl, const Plan& P, uint32_t G, Schedule& S) {
   for (uint32_t L = std::min(P.max_gate_level + 2, nl.n_levels); L <= nl.n_levels; ++L)
     S.rec_off[L] = (uint32_t)S.recs.size();
   S.max_live = pool.next_block * G + (net.fixes.empty() ? 0 : 1);
-  if (S.max_live > kMaxSlots) {
+  if (S.max_live > max_slots(G)) {
     S.recs.clear();
     S.wides.clear();
+    S.rec_off.assign(nl.n_levels + 1, 0);
     return;
   }
   // Fix entries: the record of a reader of alias y, with the literals that
@@ -685,6 +686,9 @@ void build_schedule(const Netlist& nl, const Plan& P, uint32_t G, Schedule& S) {
 
 void pack_schedule(Schedule& S, uint32_t T) {
   if (S.T == T) return;
+  if (S.max_live > max_slots(S.G))
+    throw LimitError{"a sweep needs " + std::to_string(S.max_live) + " live values; a schedule of this word count holds " +
+                     std::to_string(max_slots(S.G))};
   S.T = T;
   S.blob.clear();
   const uint32_t n_levels = (uint32_t)S.rec_off.size() - 1, nw = S.rec_words();

@@ -48,15 +48,25 @@
 
 #include <array>
 #include <cstdint>
+#include <string>
 #include <vector>
 
 #include "fsimb_netlist.h"
 
 namespace fsimb {
 
+// Thrown where a size is beyond what the code can hold; FSIMB_ERR_LIMIT at
+// the C ABI.
+struct LimitError {
+  std::string msg;
+};
+
 constexpr uint32_t kTileWords = 32;  // words per tile = lanes of a warp
 constexpr uint32_t kNoSlot = 0xFFFFFFFFu;
-constexpr uint32_t kMaxSlots = 32767;   // slots are 15-bit in the plain gate records
+// Slots a schedule may have: the documented limit, at one word per item more
+// than shared memory holds; the width of a record's slot field at more.
+constexpr uint32_t kMaxSlots = 32767;
+constexpr uint32_t max_slots(uint32_t G) { return G == 16 ? kMaxSlots : 1u << 14; }
 
 constexpr uint32_t kFolded = 0x80000000u;  // level[]: the element is folded; low bits: its consumer
 
@@ -255,11 +265,12 @@ void build_fault_plan(const Netlist& nl, const CircuitPlan& cplan, const std::ve
                       Plan& plan);
 // Folds single-consumer gates into their consumers (net.gates is left as it is).
 void build_sweep_net(const Netlist& nl, const Plan& plan, SweepNet& net);
-// G in {2, 4, 8, 16}.  A schedule that needs more than kMaxSlots slots
-// reports max_live > kMaxSlots and leaves recs and li empty.
+// G in {2, 4, 8, 16}.  A schedule that needs more than max_slots(G) slots
+// reports its max_live and holds no records, fix entries or live-in pairs.
 void build_schedule(const Netlist& nl, const Plan& plan, uint32_t G, Schedule& out);
 // Packs the schedule's records into the stream of a T-thread CTA (T a
-// multiple of 32); nothing to do if it is packed for T already.
+// multiple of 32); nothing to do if it is packed for T already.  LimitError
+// for a schedule of more than max_slots(G) slots.
 void pack_schedule(Schedule& s, uint32_t T);
 
 }  // namespace fsimb

@@ -280,7 +280,7 @@ struct fsimb_server {
       throw LimitError{"the circuit has more live values than shared memory holds at 1 word per item"};
     int M = 0, T = 0;
     default_sweep_shape(B, sched_at, kTileWords, smem_optin, smem_per_sm, M, T);
-    if (sched_at(M).max_live > kMaxSlots || sweep_vals_bytes(sched_at(M).max_live, M) > share)
+    if (!sched_fits(sched_at(M), M, share))
       throw LimitError{"the circuit has more live values than shared memory holds at 1 word per item"};
     pack_schedule(sc[m_slot_s(M)], (uint32_t)T);
     c->sched = std::move(sc[m_slot_s(M)]);

@@ -1,0 +1,62 @@
+"""Schedules at the limits of what the sweep's records can hold, on the CPU
+with the standard library's checks switched on."""
+import os
+import subprocess
+
+import pytest
+
+from lsim_b200 import build
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+MAX_SLOTS = {16: 32767, 8: 1 << 14, 4: 1 << 14, 2: 1 << 14}
+
+
+@pytest.fixture(scope="module")
+def check(tmp_path_factory):
+    exe = str(tmp_path_factory.mktemp("limits") / "sweep_limits_check")
+    src = [os.path.join(build.CSRC, f) for f in ("fsimb_netlist.cpp", "fsimb_plan.cpp")]
+    subprocess.check_call(["/usr/bin/g++", "-std=c++17", "-O2", "-D_GLIBCXX_ASSERTIONS",
+                           os.path.join(ROOT, "tests", "cpp", "sweep_limits_check.cpp")] + src + ["-o", exe])
+
+    def run(tmp_path, text):
+        path = tmp_path / "c.ckt"
+        path.write_text(text)
+        r = subprocess.run([exe, str(path)], capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stderr
+        lines = r.stdout.split("\n")
+        live = int(lines[0].split()[1])
+        return live, {int(g): (int(n), s if s == "refused" else int(s))
+                      for g, n, s in (x.split() for x in lines[1:] if x)}
+
+    return run
+
+
+def _two_rows(n):
+    """n XORs of neighbouring PIs (16 of them); n ANDs, each of two of the
+    XORs, each with a PO: every XOR is read twice, so all n live at once."""
+    pis = 16
+    g0 = pis + n
+    sinks = [[] for _ in range(g0 + 2 * n)]
+    for i in range(n):
+        sinks[i % pis].append((g0 + i, 1))
+        sinks[(i + 1 + i // pis % (pis - 1)) % pis].append((g0 + i, 2))
+        sinks[g0 + i].append((g0 + n + i, 1))
+        sinks[g0 + (i + 1) % n].append((g0 + n + i, 2))
+        sinks[g0 + n + i].append((pis + i, 1))
+    wires = ["%d 1 %d %s" % (e, len(s), " ".join("%d %d" % x for x in s)) for e, s in enumerate(sinks) if s]
+    return "%d %d %d %d\n%s\n%s\n" % (pis, n, 2 * n, len(wires), "\n".join(wires), "\n".join(["3"] * n + ["1"] * n))
+
+
+@pytest.mark.parametrize("n", [1000, 16000, 17000, 33000])
+def test_a_schedule_beyond_the_slot_fields_is_refused(check, tmp_path, n):
+    live, got = check(tmp_path, _two_rows(n))
+    assert live >= n
+    assert set(got) == set(MAX_SLOTS)
+    for g, (slots, packed) in got.items():
+        assert slots >= n
+        if slots > MAX_SLOTS[g]:
+            assert packed == "refused"
+        else:
+            assert packed >= 2 * n
+    if n == 33000:
+        assert all(packed == "refused" for _, packed in got.values())

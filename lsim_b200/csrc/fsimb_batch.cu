@@ -720,13 +720,13 @@ struct fsimb_batch {
     std::vector<ClassShape> shape(n);
     std::vector<long long> key(n);
     parallel_for(n, [&](size_t i) {
-      if (!gates_fit(i, smem_share(1)))
+      int M = 0, t = 0;
+      if (!gates_fit(i, smem_share(1)) ||
+          !default_sweep_shape(
+              members[i]->plan, [&](int m) -> const Schedule& { return schedule_at(i, m); },
+              (uint32_t)std::min<uint64_t>(members[i]->pats.W, kTileWords), smem_optin, smem_per_sm, M, t))
         throw LimitError{"batch member " + std::to_string(i) +
                          " has more live values than shared memory holds at 1 word per item"};
-      int M = 0, t = 0;
-      default_sweep_shape(
-          members[i]->plan, [&](int m) -> const Schedule& { return schedule_at(i, m); },
-          (uint32_t)std::min<uint64_t>(members[i]->pats.W, kTileWords), smem_optin, smem_per_sm, M, t);
       a.M[i] = M;
       shape[i] = ClassShape{M, t};
       key[i] = (long long)m_slot(M) * 4096 + t;

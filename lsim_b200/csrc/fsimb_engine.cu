@@ -127,7 +127,7 @@ std::vector<SweepShape> likely_shapes(const Plan& plan, uint32_t words, size_t s
   return out;
 }
 
-void default_sweep_shape(const Plan& plan, const std::function<const Schedule&(int)>& sched_at,
+bool default_sweep_shape(const Plan& plan, const std::function<const Schedule&(int)>& sched_at,
                          uint32_t words, size_t smem_optin, size_t smem_per_sm, int& M, int& threads) {
   const size_t share1 = sweep_smem_share(smem_optin, smem_per_sm, 1);
   // Slots are about the peak of live values until a schedule says more.
@@ -136,10 +136,9 @@ void default_sweep_shape(const Plan& plan, const std::function<const Schedule&(i
   for (int i = 0; i < 4; ++i) vals[i] = sweep_vals_bytes(plan.net_live + plan.net_live / 64 + 16, 1 << i);
   for (;;) {
     double best = 1e300;
-    int bi = 0;
-    threads = 64;
+    int bi = -1;
     for (int i = 3; i >= 0; --i) {
-      if (i > 0 && vals[i] > share1) continue;
+      if (vals[i] > share1) continue;
       for (uint32_t t = 32; t <= 1024; t += 32) {
         const double c = sweep_shape_cost(plan.net, 1 << i, t, vals[i], smem_per_sm, words);
         if (c < best * 0.99) {
@@ -149,6 +148,8 @@ void default_sweep_shape(const Plan& plan, const std::function<const Schedule&(i
         }
       }
     }
+    if (bi < 0 && !exact[0]) bi = 0;  // the estimate may be too high: ask the schedule
+    if (bi < 0) return false;
     M = 1 << bi;
     if (exact[bi]) break;
     const Schedule& sc = sched_at(M);
@@ -156,12 +157,13 @@ void default_sweep_shape(const Plan& plan, const std::function<const Schedule&(i
     vals[bi] = sched_fits(sc, M, share1) ? sweep_vals_bytes(sc.max_live, M) : share1 + 1;
   }
   threads = std::min<int>(threads, (int)sweep_max_threads(M));
+  return true;
 }
 
 }  // namespace fsimb
 
-void fsimb_handle::default_shape(int& M, int& threads) {
-  default_sweep_shape(
+bool fsimb_handle::default_shape(int& M, int& threads) {
+  return default_sweep_shape(
       plan, [&](int m) -> const Schedule& { return cached_schedule(m); },
       (uint32_t)std::min<uint64_t>(pats.W, kTileWords), smem_optin, smem_per_sm, M, threads);
 }
@@ -190,7 +192,11 @@ void fsimb_handle::tune_shape(cudaStream_t s) {
   // faster by more than 2% on the sample (the sample favours no shape, but
   // its time carries a few percent of noise).
   int dM = 0, dT = 0;
-  default_shape(dM, dT);
+  if (!default_shape(dM, dT)) {
+    tuned_M = tuned_T = 0;
+    tuned_gen = plan_gen;
+    return;
+  }
   float default_ms = -1;
   std::vector<SweepShape> cands{{dM, dT}};
   for (const SweepShape& c :
@@ -254,7 +260,6 @@ void fsimb_handle::tune_shape(cudaStream_t s) {
       bT = T;
     }
   }
-  if (!bM) throw LimitError{"no sweep shape fits this circuit"};
   tuned_M = bM;
   tuned_T = bT;
   tuned_gen = plan_gen;
@@ -401,10 +406,14 @@ void fsimb_handle::run(const fsimb_opts* opts) {
       }
       M = tuned_M;
       threads = tuned_T;
-    } else {
-      default_shape(M, threads);
+    } else if (!default_shape(M, threads)) {
+      M = 0;
     }
     threads = std::min<int>(threads, (int)sweep_max_threads(M));
+    if (!M) {  // no schedule fits: the global-memory sweep
+      if (o.sweep_variant == 1) throw no_room(cached_schedule(1).max_live, 1, share1, 1);
+      wide = true;
+    }
   }
   int blocks = 0, occ_got = 0;
   if (wide) {

@@ -183,8 +183,9 @@ std::vector<SweepShape> likely_shapes(const Plan& plan, uint32_t words, size_t s
                                       size_t most);
 
 // Default sweep shape of a circuit: the cheapest for a tile of `words` pattern
-// words.  sched_at(M) returns the schedule at M.
-void default_sweep_shape(const Plan& plan, const std::function<const Schedule&(int)>& sched_at,
+// words.  sched_at(M) returns the schedule at M.  False if no schedule fits
+// shared memory, not even at one word per item.
+bool default_sweep_shape(const Plan& plan, const std::function<const Schedule&(int)>& sched_at,
                          uint32_t words, size_t smem_optin, size_t smem_per_sm, int& M, int& threads);
 
 // A fresh value for fsimb_handle::gen: every change of a handle's circuit,
@@ -362,10 +363,10 @@ struct fsimb_handle {
   // The circuit's good machine on the device for the first W pattern words.
   fsimb::GoodView good_view(uint32_t W) const;
   // default_sweep_shape for this circuit and the plain sweep kernel.
-  void default_shape(int& M, int& threads);
+  bool default_shape(int& M, int& threads);
   // Times candidate shapes on a strided sample of tile 0's sweeps and keeps
-  // the fastest in tuned_M / tuned_T.  Needs the plan and the
-  // patterns on the device.
+  // the fastest in tuned_M / tuned_T (0: none fits shared memory).  Needs the
+  // plan and the patterns on the device.
   void tune_shape(cudaStream_t s);
 };
 

@@ -276,11 +276,9 @@ struct fsimb_server {
       return sc[sl];
     };
     const size_t share = sweep_smem_share(smem_optin, smem_per_sm, 1);
-    if (B.max_live > kMaxSlots || sweep_vals_bytes(B.max_live, 1) > share)
-      throw LimitError{"the circuit has more live values than shared memory holds at 1 word per item"};
     int M = 0, T = 0;
-    default_sweep_shape(B, sched_at, kTileWords, smem_optin, smem_per_sm, M, T);
-    if (!sched_fits(sched_at(M), M, share))
+    if (B.max_live > kMaxSlots || sweep_vals_bytes(B.max_live, 1) > share ||
+        !default_sweep_shape(B, sched_at, kTileWords, smem_optin, smem_per_sm, M, T))
       throw LimitError{"the circuit has more live values than shared memory holds at 1 word per item"};
     pack_schedule(sc[m_slot_s(M)], (uint32_t)T);
     c->sched = std::move(sc[m_slot_s(M)]);

@@ -60,3 +60,39 @@ def test_a_schedule_beyond_the_slot_fields_is_refused(check, tmp_path, n):
             assert packed >= 2 * n
     if n == 33000:
         assert all(packed == "refused" for _, packed in got.values())
+
+
+@pytest.fixture(scope="module")
+def shape(tmp_path_factory):
+    exe = str(tmp_path_factory.mktemp("shape") / "sweep_shape_check")
+    lib = build.build()
+    subprocess.check_call(["/usr/bin/g++", "-std=c++17", "-O2", "-I/usr/local/cuda/include",
+                           os.path.join(ROOT, "tests", "cpp", "sweep_shape_check.cpp"), lib,
+                           "-Wl,-rpath," + os.path.dirname(lib), "-o", exe])
+
+    def run(tmp_path, text, smem, words):
+        path = tmp_path / "c.ckt"
+        path.write_text(text)
+        r = subprocess.run([exe, str(path), str(smem), str(words)], capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stderr
+        lines = [[int(x) for x in s.split()] for s in r.stdout.split("\n") if s and s != "none"]
+        return (None if r.stdout.startswith("none") else lines[0]), lines[0 if r.stdout.startswith("none") else 1:]
+
+    return run
+
+
+@pytest.mark.parametrize("n", [1000, 17000, 33000])
+@pytest.mark.parametrize("smem", [16 << 10, 64 << 10, 227 << 10])
+@pytest.mark.parametrize("words", [1, 32])
+def test_the_default_shape_fits_or_there_is_none(shape, tmp_path, n, smem, words):
+    got, likely = shape(tmp_path, _two_rows(n), smem, words)
+    room = smem - 1536  # what the launch's own use leaves
+    if got is None:
+        assert (2 * n + 16) * 8 > room  # not one word of every gate's value
+    else:
+        m, threads, slots = got
+        assert slots * m * 8 <= room and slots <= MAX_SLOTS[16 // m]
+        assert 32 <= threads <= 1024 and threads % 32 == 0
+    for m, _ in likely:
+        assert n * m * 8 <= room
+    assert n != 33000 or got is None

@@ -34,11 +34,15 @@ struct IoError {
   std::string msg;
 };
 
+// The error is cleared: left as the thread's last error, the next launch
+// check, of any handle, would take it for its own.
 #define CK(call)                                                                            \
   do {                                                                                      \
     cudaError_t e_ = (call);                                                                \
-    if (e_ != cudaSuccess)                                                                  \
+    if (e_ != cudaSuccess) {                                                                \
+      cudaGetLastError();                                                                   \
       throw ::fsimb::CudaError{std::string(#call) + ": " + cudaGetErrorString(e_)};         \
+    }                                                                                       \
   } while (0)
 
 struct DevBuf {

@@ -303,7 +303,7 @@ void BatchExec::layout(const std::vector<BatchJob>& jobs, const std::vector<Clas
   // Sweep classes: shapes[c] runs the jobs with cls == c.
   classes.clear();
   uint32_t n_counters = 0;
-  for (int a = 0; a < 4; ++a) smem_attr[a] = 0;
+  for (size_t& a : smem_attr) a = 0;
   for (size_t ci = 0; ci < shapes.size(); ++ci) {
     const ClassShape& sh = shapes[ci];
     SweepClass k;
@@ -323,6 +323,7 @@ void BatchExec::layout(const std::vector<BatchJob>& jobs, const std::vector<Clas
       items += ci_items;
       k.work += (double)jobs[i].plan->dense_sweep_gates * circs[i].tiles;
       max_live = std::max(max_live, jobs[i].sched->max_live);
+      k.direct |= jobs[i].sched->direct;
       const std::vector<uint32_t>& ro = jobs[i].sched->rec_off;
       for (size_t l = 0; l + 1 < ro.size(); ++l) widest = std::max(widest, ro[l + 1] - ro[l]);
     }
@@ -391,18 +392,19 @@ void BatchExec::size_class(SweepClass& k, const ClassShape& sh) {
                      std::to_string(sh.M) + " word(s) per item; shared memory holds " +
                      std::to_string(share / (8 * sh.M))};
   k.smem = std::max<size_t>(16, vals);
-  size_t& attr = smem_attr[m_slot(sh.M)];
+  size_t& attr = smem_attr[m_slot(sh.M) + 4 * k.direct];
   attr = std::max(attr, k.smem);
-  CK(sweep_batch_set_smem(sh.M, attr));
+  CK(sweep_batch_set_smem(sh.M, k.direct, attr));
   k.occ = 0;
-  CK(sweep_batch_occupancy(sh.M, sh.threads, k.smem, &k.occ));
+  CK(sweep_batch_occupancy(sh.M, k.direct, sh.threads, k.smem, &k.occ));
   if (k.occ < 1) throw LimitError{"batch sweep kernel does not fit on an SM with this shape"};
   k.blocks = (int)std::min<unsigned long long>((unsigned long long)n_sms * k.occ, k.n_items);
 }
 
 void BatchExec::apply_attributes() {
   for (int M : {1, 2, 4, 8})
-    if (smem_attr[m_slot(M)]) CK(sweep_batch_set_smem(M, smem_attr[m_slot(M)]));
+    for (bool direct : {false, true})
+      if (const size_t a = smem_attr[m_slot(M) + 4 * direct]) CK(sweep_batch_set_smem(M, direct, a));
 }
 
 uint64_t BatchExec::enqueue(cudaStream_t s, bool good_only, bool with_events, cudaEvent_t* ev) {
@@ -511,7 +513,7 @@ uint64_t BatchExec::enqueue_sweeps(cudaStream_t s, int only) {
       }
       params.queue = d_ctl.as<unsigned long long>() + k.queue_base + j0;
       const int blocks = (int)std::min<unsigned long long>((unsigned long long)k.blocks, chunk_items);
-      CK(launch_sweep_batch(k.shape.M, k.shape.threads, std::max(blocks, 1), k.smem, params, s));
+      CK(launch_sweep_batch(k.shape.M, k.direct, k.shape.threads, std::max(blocks, 1), k.smem, params, s));
       ++launches;
     }
   }

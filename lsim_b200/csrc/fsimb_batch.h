@@ -48,6 +48,7 @@ struct SweepClass {
   uint32_t queue_base = 0;          // their work counters: d_ctl words queue_base + j
   unsigned long long n_items = 0;
   double work = 0;        // gate-words its sweeps evaluate (launch order)
+  bool direct = false;    // a circuit's schedule has direct PO records
   uint32_t max_live = 0;  // slots of the largest schedule in the class
   uint32_t widest = 0;    // records of the widest level in the class
   size_t smem = 0;
@@ -86,7 +87,8 @@ class BatchExec {
   uint64_t static_bytes = 0, desc_bytes = 0;
   uint64_t ctl_bytes = 256;  // one work counter per swept circuit
   BatchSweepParams params{};  // launch parameters being built (32 KB)
-  size_t smem_attr[4] = {0, 0, 0, 0};  // dynamic smem limit set per words-per-item kernel
+  // dynamic smem limit set per words-per-item kernel, without and with direct records
+  size_t smem_attr[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   cudaEvent_t* class_events = nullptr;  // direct launches: recorded after each class
   // Classes run as concurrent branches (one stream each), so CTAs of small
   // circuits can share SMs with the CTAs of large ones.

@@ -130,10 +130,14 @@ std::vector<SweepShape> likely_shapes(const Plan& plan, uint32_t words, size_t s
 bool default_sweep_shape(const Plan& plan, const std::function<const Schedule&(int)>& sched_at,
                          uint32_t words, size_t smem_optin, size_t smem_per_sm, int& M, int& threads) {
   const size_t share1 = sweep_smem_share(smem_optin, smem_per_sm, 1);
-  // Slots are about the peak of live values until a schedule says more.
+  // Slots are about the peak of live values until a schedule says more, and
+  // at most the plan's cap.
   size_t vals[4] = {0, 0, 0, 0};
   bool exact[4] = {false, false, false, false};
-  for (int i = 0; i < 4; ++i) vals[i] = sweep_vals_bytes(plan.net_live + plan.net_live / 64 + 16, 1 << i);
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t about = plan.net_live + plan.net_live / 64 + 16;
+    vals[i] = sweep_vals_bytes(std::min(about, plan.slot_cap(16u >> i)), 1 << i);
+  }
   for (;;) {
     double best = 1e300;
     int bi = -1;
@@ -208,9 +212,9 @@ void fsimb_handle::tune_shape(cudaStream_t s) {
     if (!sched_fits(cached_schedule(M), M, share1)) continue;
     const Schedule& sc = use_schedule(M, T, s);
     const size_t smem = std::max<size_t>(16, sweep_vals_bytes(sc.max_live, M));
-    CK(sweep_set_smem(M, smem));
+    CK(sweep_set_smem(M, sc.direct, smem));
     int got = 0;
-    CK(sweep_occupancy(M, T, smem, &got));
+    CK(sweep_occupancy(M, sc.direct, T, smem, &got));
     if (got < 1) continue;
     SweepArgs sa{};
     sa.blob = d_recs.as<uint4>();
@@ -242,7 +246,7 @@ void fsimb_handle::tune_shape(cudaStream_t s) {
     for (int rep = (&cd == &cands[0]) ? -1 : 0; rep < 2; ++rep) {
       CK(cudaMemsetAsync(d_queue.p, 0, sizeof(int), s));
       CK(cudaEventRecord(tune_ev[0], s));
-      CK(launch_sweep(M, T, nb, smem, sa, s));
+      CK(launch_sweep(M, sc.direct, T, nb, smem, sa, s));
       CK(cudaEventRecord(tune_ev[1], s));
       CK(cudaEventSynchronize(tune_ev[1]));
       float x = 0;
@@ -456,8 +460,8 @@ void fsimb_handle::run(const fsimb_opts* opts) {
   CK(cudaEventRecord(e2, s));
 
   if (!wide && n_sweeps) {
-    CK(sweep_set_smem(M, smem));
-    CK(sweep_occupancy(M, threads, smem, &occ_got));
+    CK(sweep_set_smem(M, sched->direct, smem));
+    CK(sweep_occupancy(M, sched->direct, threads, smem, &occ_got));
     if (occ_got < 1) throw LimitError{"sweep kernel does not fit on an SM with this shape"};
     blocks = n_sms * occ_got;
   }
@@ -528,7 +532,7 @@ void fsimb_handle::run(const fsimb_opts* opts) {
         sa.err = err_word;
         sa.wait_ns = kWaitTestNs;
         sa.wait_test = (o.wait_test && t == 0) ? 1u : 0u;
-        CK(launch_sweep(M, threads, nb, smem, sa, s));
+        CK(launch_sweep(M, sched->direct, threads, nb, smem, sa, s));
       }
       ++launches;
       items += (uint64_t)n_sw * subtiles;

@@ -488,6 +488,57 @@ __device__ __forceinline__ void wide_eval(uint32_t vb, const uint4* d) {
   }
 }
 
+// A direct PO record: the driver's words from its inputs, by masks as in
+// good_store, against its good words.  A thread's chunk order is the
+// clusters' (the lanes of a phase read different banks), so the lanes'
+// words do not line up: each sets the bits that the CTA's words do not
+// have yet, which after a few records is nearly none.
+template <int M>
+__device__ __forceinline__ void direct_eval(uint32_t vb, uint32_t rot, const uint4* d, const uint64_t* good_w0,
+                                            uint32_t* acc) {
+  constexpr int C = (M >= 2) ? M / 2 : 1;
+  constexpr int R = Chunk<M>::R;
+  const uint4 f = d[0], g = d[1];
+  const uint32_t t = g.y & 15u, nf = (g.y >> 4) & 15u;
+  const uint32_t ii = 0u - ((kIiMask >> t) & 1u), io = 0u - ((kIoMask >> t) & 1u), kx = 0u - ((kXfMask >> t) & 1u);
+  const uint32_t i1 = nf > 1 ? ii : ~kx, i2 = nf > 2 ? ii : ~kx, i3 = nf > 3 ? ii : ~kx;
+  const uint64_t* good_row = good_w0 + (uint64_t)g.x * 32;
+#pragma unroll 1
+  for (int c = 0; c < C; ++c) {
+    const uint32_t o = M == 1 ? 0u : rot ^ 16u * c, vc = vb + o;  // o: the chunk's bytes in its slot
+    Chunk<M> w;
+    if constexpr (M == 1) {
+      const uint2 q = *reinterpret_cast<const uint2*>(good_row);
+      w.r[0] = q.x, w.r[1] = q.y;
+    } else {
+      const uint4 q = *reinterpret_cast<const uint4*>(good_row + o / 8);
+      w.r[0] = q.x, w.r[1] = q.y, w.r[2] = q.z, w.r[3] = q.w;
+    }
+    const Chunk<M> x0 = lds<M>(vc + 8u * M * f.x), x1 = lds_if<M>(vc + 8u * M * f.y, nf > 1),
+                   x2 = lds_if<M>(vc + 8u * M * f.z, nf > 2), x3 = lds_if<M>(vc + 8u * M * f.w, nf > 3);
+    uint32_t any = 0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      uint32_t x;
+      if (t == G_MUX) {
+        const uint32_t not_s = (x2.r[r & ~1] | x2.r[r | 1]) == 0u;
+        x = (x2.r[r] & x1.r[r]) | (r & 1 ? 0u : x0.r[r] & not_s);
+      } else {
+        x = and_or_xor(and_or_xor(x0.r[r] ^ ii, x1.r[r] ^ i1, kx), x2.r[r] ^ i2, kx);
+        x = and_or_xor(x, x3.r[r] ^ i3, kx) ^ io;
+      }
+      w.r[r] ^= x;
+      any |= w.r[r];
+    }
+    if (any) {
+      volatile uint32_t* at = acc + o / 4;
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (w.r[r] & ~at[r]) atomicOr(acc + o / 4 + r, w.r[r]);
+    }
+  }
+}
+
 // A PO record: the driver's difference from its good words, to the CTA's
 // words in shared memory by one atomic per warp and 32-bit half (registers
 // for them would cost every other record).
@@ -526,13 +577,15 @@ __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
 }
 
-template <int M>
+template <int M, bool D>
 __device__ __forceinline__ void record_eval(uint32_t vb, uint32_t rot, bool split, const RecWords<M> q,
                                             const uint4* blob, const uint64_t* good_w0, uint32_t* acc) {
   const uint32_t kind = (q.y >> kRecKindShift) & 7u;
   if (kind >= kRecMux) {
     if (kind == kRecMux)
       mux_eval<M>(vb, rot, q);
+    else if (D && kind == kRecPo && (q.x & kPoDirect))
+      direct_eval<M>(vb, rot, blob + (q.x & ~kPoDirect), good_w0, acc);
     else if (kind == kRecPo)
       po_eval<M>(vb, q, good_w0, acc);
     else
@@ -576,7 +629,7 @@ __device__ __forceinline__ void cta_sync() {
 //
 // One item: the levels above the injection element for M words starting at
 // word w0 of the tile; writes the OR of PO differences to out_row[w0..w0+M).
-template <int M>
+template <int M, bool D>
 __device__ __forceinline__ void sweep_item(uint64_t* vals, unsigned long long* acc, const SweepView& v,
                                            const InjRec inj, uint32_t w0, uint64_t* out_row) {
   constexpr int C = (M >= 2) ? M / 2 : 1;   // chunks per slot
@@ -644,13 +697,13 @@ __device__ __forceinline__ void sweep_item(uint64_t* vals, unsigned long long* a
     const uint64_t* good_w0 = v.good + w0;
     uint32_t* acc32 = reinterpret_cast<uint32_t*>(acc);
     auto round = [&](const RecWords<M> q, uint32_t at) {
-      record_eval<M>(vb, rot, v.split, q, v.blob, good_w0, acc32);
+      record_eval<M, D>(vb, rot, v.split, q, v.blob, good_w0, acc32);
       if (q.y & kRecEnd) {
         cta_sync();
         if (at == fix_at) {
           const uint32_t n = fx[1].y;
           for (uint32_t i = tid; i < n; i += nth)
-            record_eval<M>(vb, rot, v.split, *reinterpret_cast<const RecWords<M>*>(fx + 2 * i), v.blob, good_w0,
+            record_eval<M, D>(vb, rot, v.split, *reinterpret_cast<const RecWords<M>*>(fx + 2 * i), v.blob, good_w0,
                            acc32);
           fx += 2 * n;
           fix_at = fx[1].x;
@@ -686,8 +739,10 @@ __device__ __forceinline__ bool sweep_wait_test(uint64_t* bar, uint64_t wait_ns,
   return false;
 }
 
-// Register caps: 1,024 threads an SM at up to 4 words per item.
-template <int M>
+// Register caps: 1,024 threads an SM at up to 4 words per item.  D: the stream
+// has direct PO records (their code beside the others costs every sweep 1 to
+// 3 %: 50,000 gates 53.5 -> 55.1 ms).
+template <int M, bool D>
 __global__ void __maxnreg__(64) k_sweep(SweepArgs a) {
   extern __shared__ __align__(128) uint64_t vals[];  // [max_live][M]
   __shared__ unsigned long long acc[M];
@@ -723,7 +778,7 @@ __global__ void __maxnreg__(64) k_sweep(SweepArgs a) {
     const SweepView v{a.blob, a.lvl, a.level, a.li, a.fi_off, a.fi_idx, a.type,
                       a.good + (uint64_t)tile * a.N * 32,
                       a.max_gate_level, a.stream_recs, a.fix0, a.inj_slot, a.split};
-    sweep_item<M>(vals, acc, v, a.inj[si], w0, a.out + ((uint64_t)tile * a.n_sweeps + si) * 32);
+    sweep_item<M, D>(vals, acc, v, a.inj[si], w0, a.out + ((uint64_t)tile * a.n_sweeps + si) * 32);
   }
 }
 
@@ -733,7 +788,7 @@ __global__ void __maxnreg__(64) k_sweep(SweepArgs a) {
 // circuit order as from one queue.  The loop index is uniform and the
 // circuit fields come from the kernel parameters: the compiler keeps the
 // pointers in uniform registers, as for k_sweep.
-template <int M>
+template <int M, bool D>
 __global__ void __maxnreg__(64) k_sweep_batch(const __grid_constant__ BatchSweepParams p) {
   extern __shared__ __align__(128) uint64_t vals[];
   __shared__ unsigned long long acc[M];
@@ -763,7 +818,7 @@ __global__ void __maxnreg__(64) k_sweep_batch(const __grid_constant__ BatchSweep
       const uint32_t w0 = (rem % sub) * M;
       const SweepView v{c.blob, c.lvl, c.level, c.li, c.fi_off, c.fi_idx, c.type,
                         c.good + (uint64_t)tile * c.N * 32, c.max_gate_level, c.stream_recs, c.fix0, c.inj_slot, c.split};
-      sweep_item<M>(vals, acc, v, c.inj[si], w0, c.out + ((uint64_t)tile * c.n_sweeps + si) * 32);
+      sweep_item<M, D>(vals, acc, v, c.inj[si], w0, c.out + ((uint64_t)tile * c.n_sweeps + si) * 32);
     }
   }
 }
@@ -1088,34 +1143,56 @@ void launch_init_results_batch(unsigned long long* count, unsigned long long* fi
                                                   nullptr, 0);
 }
 
-#define FSIMB_SWEEP_BATCH_CASES(X) X(1) X(2) X(4) X(8)
-cudaError_t sweep_batch_set_smem(int M, size_t smem) {
+// The sweep kernels at M words per item, without and with direct records.
+using SweepFn = void (*)(SweepArgs);
+using SweepBatchFn = void (*)(BatchSweepParams);
+static SweepFn sweep_fn(int M, bool direct) {
   switch (M) {
-#define X(m) case m: return cudaFuncSetAttribute(k_sweep_batch<m>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    FSIMB_SWEEP_BATCH_CASES(X)
-#undef X
+    case 1: return direct ? k_sweep<1, true> : k_sweep<1, false>;
+    case 2: return direct ? k_sweep<2, true> : k_sweep<2, false>;
+    case 4: return direct ? k_sweep<4, true> : k_sweep<4, false>;
+    case 8: return direct ? k_sweep<8, true> : k_sweep<8, false>;
   }
-  return cudaErrorInvalidValue;
+  return nullptr;
 }
-
-cudaError_t sweep_batch_occupancy(int M, int threads, size_t smem, int* blocks_per_sm) {
+static SweepBatchFn sweep_batch_fn(int M, bool direct) {
   switch (M) {
-#define X(m) case m: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_sweep_batch<m>, threads, smem);
-    FSIMB_SWEEP_BATCH_CASES(X)
-#undef X
+    case 1: return direct ? k_sweep_batch<1, true> : k_sweep_batch<1, false>;
+    case 2: return direct ? k_sweep_batch<2, true> : k_sweep_batch<2, false>;
+    case 4: return direct ? k_sweep_batch<4, true> : k_sweep_batch<4, false>;
+    case 8: return direct ? k_sweep_batch<8, true> : k_sweep_batch<8, false>;
   }
-  return cudaErrorInvalidValue;
+  return nullptr;
 }
-
-cudaError_t launch_sweep_batch(int M, int threads, int blocks, size_t smem, const BatchSweepParams& p,
-                               cudaStream_t s) {
-  switch (M) {
-#define X(m) case m: k_sweep_batch<m><<<blocks, threads, smem, s>>>(p); break;
-    FSIMB_SWEEP_BATCH_CASES(X)
-#undef X
-    default: return cudaErrorInvalidValue;
-  }
+template <class Fn>
+static cudaError_t set_smem(Fn fn, size_t smem) {
+  return fn ? cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) : cudaErrorInvalidValue;
+}
+template <class Fn>
+static cudaError_t occupancy(Fn fn, int threads, size_t smem, int* blocks_per_sm) {
+  return fn ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, fn, threads, smem) : cudaErrorInvalidValue;
+}
+template <class Fn, class Args>
+static cudaError_t launch_fn(Fn fn, int threads, int blocks, size_t smem, const Args& a, cudaStream_t s) {
+  if (!fn) return cudaErrorInvalidValue;
+  fn<<<blocks, threads, smem, s>>>(a);
   return cudaGetLastError();
+}
+
+cudaError_t sweep_batch_set_smem(int M, bool direct, size_t smem) { return set_smem(sweep_batch_fn(M, direct), smem); }
+cudaError_t sweep_batch_occupancy(int M, bool direct, int threads, size_t smem, int* blocks_per_sm) {
+  return occupancy(sweep_batch_fn(M, direct), threads, smem, blocks_per_sm);
+}
+cudaError_t launch_sweep_batch(int M, bool direct, int threads, int blocks, size_t smem, const BatchSweepParams& p,
+                               cudaStream_t s) {
+  return launch_fn(sweep_batch_fn(M, direct), threads, blocks, smem, p, s);
+}
+cudaError_t sweep_set_smem(int M, bool direct, size_t smem) { return set_smem(sweep_fn(M, direct), smem); }
+cudaError_t sweep_occupancy(int M, bool direct, int threads, size_t smem, int* blocks_per_sm) {
+  return occupancy(sweep_fn(M, direct), threads, smem, blocks_per_sm);
+}
+cudaError_t launch_sweep(int M, bool direct, int threads, int blocks, size_t smem, const SweepArgs& a, cudaStream_t s) {
+  return launch_fn(sweep_fn(M, direct), threads, blocks, smem, a, s);
 }
 
 uint32_t launch_good(const GoodView& a, const uint32_t* level_off, int n_sms, cudaStream_t s) {
@@ -1159,38 +1236,6 @@ uint32_t launch_good(const GoodView& a, const uint32_t* level_off, int n_sms, cu
     default: k_good<8><<<blocks, threads, 0, s>>>(a); break;
   }
   return 1;
-}
-
-cudaError_t sweep_set_smem(int M, size_t smem) {
-  switch (M) {
-    case 1: return cudaFuncSetAttribute(k_sweep<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    case 2: return cudaFuncSetAttribute(k_sweep<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    case 4: return cudaFuncSetAttribute(k_sweep<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    case 8: return cudaFuncSetAttribute(k_sweep<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  }
-  return cudaErrorInvalidValue;
-}
-
-cudaError_t sweep_occupancy(int M, int threads, size_t smem, int* blocks_per_sm) {
-  switch (M) {
-    case 1: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_sweep<1>, threads, smem);
-    case 2: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_sweep<2>, threads, smem);
-    case 4: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_sweep<4>, threads, smem);
-    case 8: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_sweep<8>, threads, smem);
-  }
-  return cudaErrorInvalidValue;
-}
-
-cudaError_t launch_sweep(int M, int threads, int blocks, size_t smem, const SweepArgs& a,
-                         cudaStream_t s) {
-  switch (M) {
-    case 1: k_sweep<1><<<blocks, threads, smem, s>>>(a); break;
-    case 2: k_sweep<2><<<blocks, threads, smem, s>>>(a); break;
-    case 4: k_sweep<4><<<blocks, threads, smem, s>>>(a); break;
-    case 8: k_sweep<8><<<blocks, threads, smem, s>>>(a); break;
-    default: return cudaErrorInvalidValue;
-  }
-  return cudaGetLastError();
 }
 
 cudaError_t launch_sweep_wide(int M, int threads, int blocks, const SweepWideArgs& a, cudaStream_t s) {

@@ -207,10 +207,10 @@ struct BatchUnits {
 };
 
 void launch_good_batch(const BatchUnits& u, unsigned long long n_units, cudaStream_t s);
-cudaError_t launch_sweep_batch(int M, int threads, int blocks, size_t smem, const BatchSweepParams& p,
+cudaError_t launch_sweep_batch(int M, bool direct, int threads, int blocks, size_t smem, const BatchSweepParams& p,
                                cudaStream_t s);
-cudaError_t sweep_batch_set_smem(int M, size_t smem);
-cudaError_t sweep_batch_occupancy(int M, int threads, size_t smem, int* blocks_per_sm);
+cudaError_t sweep_batch_set_smem(int M, bool direct, size_t smem);
+cudaError_t sweep_batch_occupancy(int M, bool direct, int threads, size_t smem, int* blocks_per_sm);
 void launch_ffr_batch(const BatchUnits& u, unsigned long long n_units, cudaStream_t s);
 void launch_exact_batch(const BatchUnits& u, unsigned long long n_units, cudaStream_t s);
 void launch_init_results_batch(unsigned long long* count, unsigned long long* first, uint8_t* lastflag,
@@ -219,11 +219,12 @@ void launch_init_results_batch(unsigned long long* count, unsigned long long* fi
 // The good machine of all words; level_off is the host's copy.  Returns the
 // kernels launched.
 uint32_t launch_good(const GoodView& a, const uint32_t* level_off, int n_sms, cudaStream_t s);
-// Returns cudaErrorInvalidValue when M is unsupported.
-cudaError_t launch_sweep(int M, int threads, int blocks, size_t smem, const SweepArgs& a,
+// direct: the schedule (any of the launch's) has direct PO records.  Returns
+// cudaErrorInvalidValue when M is unsupported.
+cudaError_t launch_sweep(int M, bool direct, int threads, int blocks, size_t smem, const SweepArgs& a,
                          cudaStream_t s);
-cudaError_t sweep_set_smem(int M, size_t smem);
-cudaError_t sweep_occupancy(int M, int threads, size_t smem, int* blocks_per_sm);
+cudaError_t sweep_set_smem(int M, bool direct, size_t smem);
+cudaError_t sweep_occupancy(int M, bool direct, int threads, size_t smem, int* blocks_per_sm);
 // M in {1, 2}; 256 threads per CTA.
 cudaError_t launch_sweep_wide(int M, int threads, int blocks, const SweepWideArgs& a, cudaStream_t s);
 cudaError_t sweep_wide_occupancy(int M, int threads, int* blocks_per_sm);

@@ -72,8 +72,9 @@ static void build_gate_recs(const Netlist& nl, std::vector<GateRec>& gates) {
   }
 }
 
-void build_sweep_net(const Netlist& nl, const Plan& P, SweepNet& net) {
+void build_sweep_net(const Netlist& nl, const Plan& P, NetForm net_form, SweepNet& net) {
   const uint32_t N = nl.N;
+  const bool fold = net_form != kNetPlain;
   // A PO is reached: the element is a PO, or a live element reads it.
   net.live.assign(N, 0);
   for (int64_t e = (int64_t)N - 1; e >= 0; --e) {
@@ -82,14 +83,25 @@ void build_sweep_net(const Netlist& nl, const Plan& P, SweepNet& net) {
     const uint32_t nf = eff_fanin(nl, (uint32_t)e);
     for (uint32_t k = 0; k < nf; ++k) net.live[nl.fi_idx[nl.fi_off[e] + k]] = 1;
   }
+  const uint32_t g1 = P.n_pi + P.n_gates;
+  // PO drivers that no gate's record reads.
+  net.direct.assign(N, 0);
+  for (uint32_t e = P.n_pi; e < g1 && net_form != kNetFolded; ++e) {
+    if (!P.po_drv[e]) continue;
+    bool read = false;
+    for (uint32_t k = nl.fo_off[e]; k < nl.fo_off[e + 1] && !read; ++k) {
+      const uint32_t c = nl.fo_idx[k];
+      read = nl.type[c] != G_PO && net.live[c] && nl.fo_pin[k] < eff_fanin(nl, c);
+    }
+    net.direct[e] = !read;
+  }
   // Clusters of the gates that have one, bottom up.
   std::vector<Form> form(N, Form{});  // n == 0: no cluster form
   net.lev_up = nl.level;
-  const uint32_t g1 = P.n_pi + P.n_gates;
   for (uint32_t e = P.n_pi; e < g1; ++e) {
     const uint32_t nf = eff_fanin(nl, e);
     const uint8_t t = nl.type[e];
-    if (!net.live[e] || t == G_MUX || nf < 1 || nf > 3) continue;
+    if (!net.live[e] || net.direct[e] || t == G_MUX || nf < 1 || nf > 3) continue;
     const uint32_t ii = nf > 1 && (t == G_OR || t == G_NOR);
     const bool inverts = t == G_INV || t == G_NAND || t == G_NOR || t == G_XNOR;
     const uint32_t io = inverts != (bool)ii;  // OR and NOR are ANDs of inverted inputs
@@ -97,7 +109,7 @@ void build_sweep_net(const Netlist& nl, const Plan& P, SweepNet& net) {
     const Form empty{{0, 0, 0}, 0, (uint8_t)(gate_family(t) == 1 && nf > 1), (uint8_t)io, 0};
     uint32_t may = 0;  // inputs that can be folded in
     for (uint32_t k = 0; k < nf; ++k)
-      if (form[in[k]].n && nl.fo_off[in[k] + 1] - nl.fo_off[in[k]] == 1) may |= 1u << k;
+      if (fold && form[in[k]].n && nl.fo_off[in[k] + 1] - nl.fo_off[in[k]] == 1) may |= 1u << k;
     // The subset of them that folds the most gates; of those one with the
     // fewest literals.
     Form best = empty;
@@ -138,7 +150,7 @@ void build_sweep_net(const Netlist& nl, const Plan& P, SweepNet& net) {
   // record a reader is folded into is a cluster's).
   net.alias.assign(N, kNoSlot);
   net.alias_of.assign(N, kNoSlot);
-  for (uint32_t e = P.n_pi; e < g1; ++e) {
+  for (uint32_t e = P.n_pi; e < g1 && fold; ++e) {
     if (form[e].n != 1 || (net.lev_up[e] & kFolded)) continue;
     bool clusters_only = true;
     for (uint32_t k = nl.fo_off[e]; k < nl.fo_off[e + 1] && clusters_only; ++k) {
@@ -161,7 +173,7 @@ void build_sweep_net(const Netlist& nl, const Plan& P, SweepNet& net) {
     if (!net.live[e] || (net.lev_up[e] & kFolded) || net.alias[e] != kNoSlot) continue;
     const uint32_t L = nl.level[e];
     auto read = [&](uint32_t x) { net.use_level[x] = std::max(net.use_level[x], L); };
-    if (P.po_drv[e]) net.use_level[e] = L + 1;  // its PO record
+    if (P.po_drv[e] && !net.direct[e]) net.use_level[e] = L + 1;  // its PO record
     const Form& f = form[e];
     if (f.n) {
       net.cluster[e] = (uint32_t)net.clusters.size();
@@ -193,7 +205,7 @@ void build_sweep_net(const Netlist& nl, const Plan& P, SweepNet& net) {
   for (uint32_t e = P.n_pi; e < g1; ++e)
     if (net.live[e] && !(net.lev_up[e] & kFolded) && net.alias[e] == kNoSlot) net.level_recs[nl.level[e]]++;
   for (uint32_t e = 0; e < g1; ++e)
-    if (P.po_drv[e]) net.level_recs[nl.level[e] + 1]++;
+    if (P.po_drv[e] && net.use_level[e]) net.level_recs[nl.level[e] + 1]++;
   // Fix lists: by alias, elements ascending and so by level.
   std::vector<uint32_t> count(N, 0);
   for (const auto& v : via) ++count[v.first];
@@ -254,7 +266,6 @@ void build_circuit_plan(const Netlist& nl, CircuitPlan& C, bool sweeps) {
   // of [level, highest reading level]), over all gates and over the stored
   // ones; a schedule may need a few more slots to honour residues.
   build_gate_recs(nl, P.net.gates);
-  if (sweeps) build_sweep_net(nl, P, P.net);
   if (sweeps) {
     auto peak = [&](const std::vector<uint32_t>& last) {
       std::vector<int64_t> delta(nl.n_levels + 2, 0);
@@ -268,7 +279,11 @@ void build_circuit_plan(const Netlist& nl, CircuitPlan& C, bool sweeps) {
       return (uint32_t)most;
     };
     P.max_live = peak(maxfo_level);
-    P.net_live = peak(P.net.use_level);
+    for (NetForm f : {kNetFolded, kNetDirectPos, kNetPlain}) {
+      build_sweep_net(nl, P, f, P.net);
+      P.net_live = peak(P.net.use_level);
+      if (P.net_live + !P.net.fixes.empty() <= std::max(P.max_live, kAnyShapeSlots)) break;
+    }
   }
 
   // FFR roots: an element with exactly one consumer belongs to the FFR of that
@@ -431,15 +446,20 @@ void build_plan(const Netlist& nl, const std::vector<Fault>& faults, Plan& P) {
 // ---------------------------------------------------------------- schedule
 namespace {
 
+// Slots by residue mod G, in blocks of one of each residue; at `cap` slots a
+// free one of another residue is taken instead of a new block.
 struct SlotPool {
-  uint32_t G;
-  uint32_t next_block = 0;
+  uint32_t G, cap;
+  uint32_t n = 0;  // slots so far
   std::vector<std::vector<uint32_t>> free;  // per residue
-  explicit SlotPool(uint32_t g) : G(g), free(g) {}
+  SlotPool(uint32_t g, uint32_t most) : G(g), cap(most), free(g) {}
   uint32_t alloc(uint32_t r) {
-    if (free[r].empty()) {
-      for (uint32_t q = 0; q < G; ++q) free[q].push_back(next_block * G + q);
-      ++next_block;
+    if (free[r].empty())
+      for (uint32_t q = 0; q < G && n < cap; ++q, ++n) free[n % G].push_back(n);
+    for (uint32_t q = 0; q < G && free[r].empty(); ++q) r = (r + 1) % G;
+    if (free[r].empty()) {  // more live values than the cap
+      r = n % G;
+      free[r].push_back(n++);
     }
     uint32_t s = free[r].back();
     free[r].pop_back();
@@ -459,7 +479,8 @@ void build_schedule(const Netlist& nl, const Plan& P, uint32_t G, Schedule& S) {
   S.li_off.assign(nl.n_levels + 1, 0);
   if (net.use_level.empty()) return;  // no fault will be simulated: no sweeps
   std::vector<uint32_t> slot(N, kNoSlot);
-  SlotPool pool(G);
+  const uint32_t inj_slots = net.fixes.empty() ? 0 : 1;
+  SlotPool pool(G, P.slot_cap(G) - inj_slots);
   std::vector<std::vector<uint32_t>> release(nl.n_levels + 2);
   // PIs: residues round robin.
   uint32_t rr = 0;
@@ -501,7 +522,7 @@ void build_schedule(const Netlist& nl, const Plan& P, uint32_t G, Schedule& S) {
       }
     } else {
       r.n = std::min<uint32_t>(eff_fanin(nl, e), 4);
-      r.kind = nl.type[e] == G_MUX && r.n == 3 ? kRecMux : kRecWide;
+      r.kind = net.direct[e] ? kRecPo : nl.type[e] == G_MUX && r.n == 3 ? kRecMux : kRecWide;
       for (uint32_t k = 0; k < r.n; ++k) r.lit[k] = nl.fi_idx[nl.fi_off[e] + k];
     }
     for (uint32_t k = 0; k < r.n; ++k) r.res[k] = (uint8_t)(slot[r.lit[k] & ~kInvLit] % G);
@@ -593,21 +614,25 @@ void build_schedule(const Netlist& nl, const Plan& P, uint32_t G, Schedule& S) {
       const Rec& r = order[pos];
       const uint32_t e = r.e;
       for (uint32_t k = 0; k < r.n; ++k) pos_slot[pos][k] = slot[r.lit[k] & ~kInvLit];
-      if (r.kind == kRecPo) {
+      if (r.kind == kRecPo && !net.direct[e]) {
         std::array<uint32_t, 4> w{0, (uint32_t)kRecPo << kRecKindShift, 0, 0};
         put_slot(w, 3, slot[e]);
         w[0] = e;
         S.recs.push_back(w);
         continue;
       }
-      const uint32_t out = slot[e] = pool.alloc(pos % G);  // every record is read
-      release[net.use_level[e] + 1].push_back(out);
-      pos_slot[pos][4] = out;
-      if (r.kind == kRecWide) {
+      uint32_t out = e;
+      if (!net.direct[e]) {
+        out = slot[e] = pool.alloc(pos % G);  // every such record is read
+        release[net.use_level[e] + 1].push_back(out);
+        pos_slot[pos][4] = out;
+      }
+      if (r.kind == kRecWide || r.kind == kRecPo) {
         std::array<uint32_t, 8> d{0, 0, 0, 0, out, (uint32_t)nl.type[e] | r.n << 4, 0, 0};
         for (uint32_t k = 0; k < r.n; ++k) d[k] = pos_slot[pos][k];
-        S.recs.push_back({(uint32_t)S.wides.size(), (uint32_t)kRecWide << kRecKindShift, 0, 0});
+        S.recs.push_back({(uint32_t)S.wides.size() | (net.direct[e] ? kPoDirect : 0u), r.kind << kRecKindShift, 0, 0});
         S.wides.push_back(d);
+        S.direct |= r.kind == kRecPo;
         continue;
       }
       std::array<uint32_t, 4> w{0, r.kind << kRecKindShift, 0, 0};
@@ -641,7 +666,7 @@ void build_schedule(const Netlist& nl, const Plan& P, uint32_t G, Schedule& S) {
   }
   for (uint32_t L = std::min(P.max_gate_level + 2, nl.n_levels); L <= nl.n_levels; ++L)
     S.rec_off[L] = (uint32_t)S.recs.size();
-  S.max_live = pool.next_block * G + (net.fixes.empty() ? 0 : 1);
+  S.max_live = pool.n + inj_slots;
   if (S.max_live > max_slots(G)) {
     S.recs.clear();
     S.wides.clear();
@@ -711,7 +736,8 @@ void pack_schedule(Schedule& S, uint32_t T) {
       uint32_t* w = &S.blob[(size_t)(n + i) * nw];
       if (pos < n_lev) {
         std::copy_n(S.recs[lo + pos].begin(), nw, w);
-        if (((w[1] >> kRecKindShift) & 7u) == kRecWide) wide_at.push_back(n + i);
+        const uint32_t kind = (w[1] >> kRecKindShift) & 7u;
+        if (kind == kRecWide || (kind == kRecPo && (w[0] & kPoDirect))) wide_at.push_back(n + i);
       }
       if (i >= (rounds - 1) * T) w[1] |= kRecEnd;
     }
@@ -720,7 +746,10 @@ void pack_schedule(Schedule& S, uint32_t T) {
   S.lvl[n_levels][0] = S.stream_recs = n;
   S.blob.resize((size_t)(n + kPrefetch * T) * nw, 0);
   const uint32_t wide0 = (uint32_t)(S.blob.size() / 4);
-  for (uint32_t i : wide_at) S.blob[(size_t)i * nw] = wide0 + 2 * S.blob[(size_t)i * nw];
+  for (uint32_t i : wide_at) {
+    uint32_t& w = S.blob[(size_t)i * nw];
+    w = (w & kPoDirect) | (wide0 + 2 * (w & ~kPoDirect));
+  }
   for (const auto& d : S.wides) S.blob.insert(S.blob.end(), d.begin(), d.end());
   S.fix0 = (uint32_t)(S.blob.size() / 4);
   for (size_t i = 0; i < S.fixes.size(); ++i) {

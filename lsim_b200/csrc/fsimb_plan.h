@@ -14,7 +14,9 @@
 //                      have records of their own kind; gates of four inputs
 //                      ("wide" records) are described in 32 bytes each
 //                      behind the stream.  A PO driver's value is compared
-//                      with the good one by a record one level above it.
+//                      with the good one by a record one level above it, or,
+//                      where the kept values would need more slots than the
+//                      gates alone, by a PO record that evaluates it.
 //                      Elements from which no PO is reached are left out.
 //                      A level is padded to rounds of T records, T the sweep
 //                      CTA's threads: thread t of round r reads record
@@ -92,7 +94,10 @@ constexpr int kRecKindShift = 28;  // word 1, three bits
 constexpr uint32_t kRecEnd = 1u << 31;  // word 1: the last round of the level
 constexpr uint32_t kRecSlot = 0x3FFFu;
 // A wide record's description, eight words: slots of up to four inputs, of
-// the output, and type | fan-in << 4.
+// the output, and type | fan-in << 4.  A direct PO record has kPoDirect and
+// the offset of such a description in word 0, the description the driver in
+// the output's place: the record evaluates the driver and compares it.
+constexpr uint32_t kPoDirect = 1u << 31;
 
 // InjRec::mode bit fields
 constexpr uint32_t kInjStuck = 1u;      // 0: flip the element's word, 1: stuck value
@@ -168,9 +173,24 @@ struct SweepNet {
   std::vector<uint32_t> fix_first;  // [N] an alias's first entry in fixes; kNoSlot: none
   std::vector<uint32_t> fixes;      // per alias, by level: elements whose records read it, then kNoSlot
   std::vector<uint8_t> live;        // [N] a PO is reached from it
+  std::vector<uint8_t> direct;      // [N] a PO driver compared by its own record: no slot
   std::vector<Cluster> clusters;
   std::vector<uint32_t> level_recs; // [n_levels] records a sweep evaluates on each level
 };
+
+// Forms of a sweep net, in the order they are tried.  What a circuit may ask
+// of shared memory is stated by its gates' live values (Plan::max_live), but
+// folding a gate keeps its inputs alive instead, and a PO driver that no gate
+// reads lives to the next level.  So a net that would keep more values than
+// the gates alone (and than kAnyShapeSlots) gives such PO drivers direct
+// records, and if that is not enough folds nothing and has no aliases, which
+// keeps at most the gates' live values.  Generated circuits of 400 to 200,000
+// gates keep 10 to 25 % less than their gates; 40,000 PO drivers on a level
+// kept 40,500 values against 927, and 930 slots with direct records.
+enum NetForm { kNetFolded, kNetDirectPos, kNetPlain };
+// Slots that every launch shape has room for (8 words an item, 8 CTAs an SM:
+// 431): below this, fewer slots allow nothing more.
+constexpr uint32_t kAnyShapeSlots = 384;
 
 struct Plan {
   uint32_t N = 0, n_pi = 0, n_gates = 0, n_po = 0;
@@ -202,6 +222,12 @@ struct Plan {
   std::vector<uint32_t> exact_fault;  // fault index of each exact sweep
   std::vector<uint32_t> sweep_root;   // root record of each stem sweep
   bool has_mux = false;
+  // The most slots a schedule of residue groups of G has: the gates' live
+  // values, rounded up to whole groups.
+  uint32_t slot_cap(uint32_t G) const {
+    const uint32_t n = max_live > kAnyShapeSlots ? max_live : kAnyShapeSlots;
+    return (n + G - 1) / G * G;
+  }
 };
 
 // The fault-independent part of a plan, built once per circuit: `base` holds
@@ -224,6 +250,7 @@ struct Schedule {
   uint32_t G = 0;
   uint32_t max_live = 0;             // slots, the injection slot among them
   bool split = false;                // levels are ordered by kind
+  bool direct = false;               // it has direct PO records
   std::vector<std::array<uint32_t, 4>> recs;  // records in position order, level after level
                                      // (a wide one's word 0: its index in wides)
   std::vector<std::array<uint32_t, 8>> wides;
@@ -263,8 +290,9 @@ void build_circuit_plan(const Netlist& nl, CircuitPlan& cplan, bool sweeps = tru
 // members of the FFRs the faults touch).
 void build_fault_plan(const Netlist& nl, const CircuitPlan& cplan, const std::vector<Fault>& faults,
                       Plan& plan);
-// Folds single-consumer gates into their consumers (net.gates is left as it is).
-void build_sweep_net(const Netlist& nl, const Plan& plan, SweepNet& net);
+// Folds single-consumer gates into their consumers, as `form` has it
+// (net.gates is left as it is).
+void build_sweep_net(const Netlist& nl, const Plan& plan, NetForm form, SweepNet& net);
 // G in {2, 4, 8, 16}.  A schedule that needs more than max_slots(G) slots
 // reports its max_live and holds no records, fix entries or live-in pairs.
 void build_schedule(const Netlist& nl, const Plan& plan, uint32_t G, Schedule& out);

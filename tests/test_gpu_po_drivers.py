@@ -3,7 +3,8 @@ beyond the level, against the oracle."""
 import numpy as np
 import pytest
 
-from lsim_b200 import Simulator, gen
+from lsim_b200 import Server, Simulator, gen
+from lsim_b200.batch import Batch
 from tests.oracle_lib import Oracle
 
 pytestmark = pytest.mark.gpu
@@ -67,3 +68,30 @@ def test_default_and_tuned_runs(drivers):
         sim.read_text(ckt, flst, ptn)
         sim.run(tune=tune)
         same(sim.results(), ref)
+
+
+@pytest.mark.parametrize("types", [(1, 2, 3, 4, 5, 6), (1, 3, 7)])
+@pytest.mark.parametrize("drivers", [4000, 29000, 40000])
+def test_every_shape_batches_and_servers(drivers, types):
+    """Shapes that the gates' live values (some 200 here) leave room for."""
+    patterns = 4500 if drivers == 4000 else 1100
+    ckt, flst, ptn = work(drivers, patterns, types=types)
+    ref = Oracle(ckt, flst, ptn).simulate()
+    sim = Simulator(0)
+    sim.read_text(ckt, flst, ptn)
+    for shape in [dict()] + [dict(words_per_item=m) for m in (1, 2, 4, 8)] + \
+            [dict(words_per_item=8, ctas_per_sm=2, block_threads=256), dict(sweep_variant="shared"),
+             dict(sweep_variant="global")]:
+        sim.run(**shape)
+        same(sim.results(), ref)
+    with Batch(0) as b:
+        host = Simulator(-1)
+        host.read_text(ckt, flst, ptn)
+        b.add(host)
+        for opts in (dict(), dict(tune=True), dict(words_per_item=8)):
+            b.run(**opts)
+            same(host.results(), ref)
+    site, pin, value = host.faults()
+    with Server(0, slot_bytes=1 << 30) as s:
+        cid = s.add_circuit(ckt, host.patterns(), patterns)
+        same(s.wait(s.submit(cid, site, value, pin, n_patterns=patterns)), ref)

@@ -63,7 +63,9 @@ typedef struct {
                                 values must leave room for that many */
   uint32_t tune;             /* 1, with the three above 0: on the first run of a circuit and
                                 fault list, time candidate sweep shapes on a strided sample
-                                of the first tile's sweeps and keep the fastest */
+                                of the first tile's sweeps and keep the fastest; again
+                                when a later run's tiles hold more pattern words (up to
+                                the next power of two) than those timed */
   void* stream;              /* cudaStream_t to run on; NULL: the handle's stream */
   uint32_t n_detect;         /* with drop = 1: detections after which a fault is dropped
                                 (N-detect); 0 or 1: the first detection */

@@ -198,6 +198,7 @@ void fsimb_handle::tune_shape(cudaStream_t s) {
   int dM = 0, dT = 0;
   if (!default_shape(dM, dT)) {
     tuned_M = tuned_T = 0;
+    tuned_words = kTileWords;  // of no tile
     tuned_gen = plan_gen;
     return;
   }
@@ -266,6 +267,7 @@ void fsimb_handle::tune_shape(cudaStream_t s) {
   }
   tuned_M = bM;
   tuned_T = bT;
+  tuned_words = tile_words(pats.W, 0);
   tuned_gen = plan_gen;
 }
 
@@ -402,7 +404,7 @@ void fsimb_handle::run(const fsimb_opts* opts) {
       }
       threads = o.block_threads ? (int)o.block_threads : (int)pick_sweep_threads(cached_schedule(M), M);
     } else if (o.tune && tiles) {
-      if (tuned_gen != plan_gen) {
+      if (!tuned_holds()) {
         const auto t0 = std::chrono::steady_clock::now();
         tune_shape(s);
         tune_ms_now =

@@ -221,8 +221,10 @@ struct fsimb_handle {
   fsimb::Schedule sched_cache[4];
   int sched_M = 0, sched_T = 0;   // the one on the device, and its CTA size (0: none)
   uint64_t sched_cache_gen[4] = {0, 0, 0, 0};
-  // Autotuned sweep shape of plan_gen (fsimb_opts.tune).
+  // Autotuned sweep shape of plan_gen (fsimb_opts.tune), timed on a tile of
+  // tuned_words pattern words.
   uint64_t tuned_gen = 0;
+  uint32_t tuned_words = 0;
   int tuned_M = 0, tuned_T = 0;
   cudaEvent_t tune_ev[2] = {nullptr, nullptr};
   // Recorded after each fsimb_run's uploads, on the run's stream: work on
@@ -368,6 +370,16 @@ struct fsimb_handle {
   fsimb::GoodView good_view(uint32_t W) const;
   // default_sweep_shape for this circuit and the plain sweep kernel.
   bool default_shape(int& M, int& threads);
+  // Whether the tuned shape holds for the current patterns: it was timed on
+  // this plan, and on no fewer words a tile, up to the next power of two (the
+  // words an item may take).  By the cost model a shape of one word takes 2.3
+  // (50,000 gates) to 3.1 (2,000 gates) times the best shape's time on a full
+  // tile.  For fewer words it is kept, so a plan is tuned six times at most.
+  bool tuned_holds() const {
+    uint32_t p = 1;  // tuned_words up to a power of two
+    while (p < tuned_words) p *= 2;
+    return tuned_gen == plan_gen && fsimb::tile_words(pats.W, 0) <= p;
+  }
   // Times candidate shapes on a strided sample of tile 0's sweeps and keeps
   // the fastest in tuned_M / tuned_T (0: none fits shared memory).  Needs the
   // plan and the patterns on the device.

@@ -349,17 +349,20 @@ void fsimb_handle::run(const fsimb_opts* opts) {
   // that a run of few tiles has one sweep launch and one tracing launch and
   // their last CTAs run dry once; drop mode compacts after every tile.
   // 6,586 gates, 5 tiles: 2.36 + 0.14 -> 2.23 + 0.04 ms; 2,000 gates, 2 tiles: 0.132 +
-  // 0.044 -> 0.113 + 0.023 ms.
+  // 0.044 -> 0.113 + 0.023 ms.  Their room is asked for last, and a device that
+  // does not have it runs one tile at a time.
   constexpr uint64_t kTileScratch = 512ull << 20;
   const uint32_t n_slots = (uint32_t)(plan.members.size() + plan.roots.size());
   const uint64_t tile_bytes = ((uint64_t)n_sweeps + n_slots + 1) * kTileWords * 8;
   uint64_t group = 1;
-  if (!o.drop && o.sweep_variant != 2 && gates_fit(1, share1)) {
+  if (!o.drop && o.sweep_variant != 2 && gates_fit(1, share1) && one_tile_gen != plan_gen) {
     const uint64_t by_items = (1ull << 31) / ((uint64_t)std::max(n_sweeps, 1u) * kTileWords);
     group = std::max<uint64_t>(1, std::min(tiles, std::min(kTileScratch / tile_bytes, by_items)));
   }
-  d_sens.ensure(group * std::max<uint32_t>(n_slots, 1) * kTileWords * 8);
-  d_out.ensure(group * std::max<uint32_t>(n_sweeps, 1) * kTileWords * 8);
+  auto scratch = [&](uint64_t n) {
+    d_sens.ensure(n * std::max<uint32_t>(n_slots, 1) * kTileWords * 8);
+    d_out.ensure(n * std::max<uint32_t>(n_sweeps, 1) * kTileWords * 8);
+  };
   d_count.ensure(std::max<uint64_t>(F, 1) * 8);
   d_first.ensure(std::max<uint64_t>(F, 1) * 8);
   d_lastflag.ensure(std::max<uint64_t>(F, 1));
@@ -406,6 +409,7 @@ void fsimb_handle::run(const fsimb_opts* opts) {
     } else if (o.tune && tiles) {
       if (!tuned_holds()) {
         const auto t0 = std::chrono::steady_clock::now();
+        scratch(1);
         tune_shape(s);
         tune_ms_now =
             std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
@@ -446,6 +450,16 @@ void fsimb_handle::run(const fsimb_opts* opts) {
   } else if (n_sweeps) {
     sched = &use_schedule(M, threads, s);
     smem = std::max<size_t>(16, sweep_vals_bytes(sched->max_live, M));
+  }
+  try {
+    scratch(group);
+  } catch (const CudaError&) {
+    if (group == 1) throw;
+    one_tile_gen = plan_gen;
+    group = 1;
+    d_sens.release();
+    d_out.release();
+    scratch(1);
   }
   // control words: the error word, then a work counter per tile
   int* err_word = d_queue.as<int>();
@@ -907,11 +921,14 @@ int fsimb_good_values(const fsimb_handle* hc, uint64_t round, uint64_t* out, uin
   CK(cudaSetDevice(h->device));
   const uint64_t tile = round / kTileWords, lane = round % kTileWords;
   const uint32_t bits = h->pats.bits(round);
-  h->d_round.ensure(n * 8);
+  // into the run's scratch where it is large enough (a full device may have
+  // no room for more)
+  DevBuf& b = h->d_sens.n >= n * 8 ? h->d_sens : h->d_out.n >= n * 8 ? h->d_out : h->d_round;
+  b.ensure(n * 8);
   launch_round(h->d_good.as<uint64_t>() + (tile * h->nl.N) * kTileWords + lane, h->nl.N,
-               bits >= 64 ? ~0ull : ((1ull << bits) - 1), h->d_round.as<uint64_t>(), h->stream);
+               bits >= 64 ? ~0ull : ((1ull << bits) - 1), b.as<uint64_t>(), h->stream);
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(out, h->d_round.p, n * 8, cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaMemcpyAsync(out, b.p, n * 8, cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   API_END(h)
 }

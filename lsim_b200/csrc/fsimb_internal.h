@@ -238,6 +238,7 @@ struct fsimb_handle {
   fsimb::DevBuf d_roots, d_members, d_traced, d_traced_slot, d_inj, d_exact;
   fsimb::DevBuf d_pwords, d_good, d_out, d_sens, d_count, d_first, d_lastflag, d_queue;
   fsimb::DevBuf d_root_list[2], d_sweep_list, d_exact_list[2], d_nout, d_tune_list;
+  uint64_t one_tile_gen = 0;  // plan_gen whose group of tiles found no room on the device
   uint64_t good_tiles = 0;  // tiles held in d_good
   uint64_t good_P = 0;
   bool pats_uploaded = false;  // d_pwords holds the current patterns

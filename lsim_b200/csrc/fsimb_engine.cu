@@ -677,17 +677,27 @@ void fsimb_handle::run(const fsimb_opts* opts) {
   ++launches;
   CK(cudaGetLastError());
   const size_t record_bytes = F * sizeof(fsimb_fault_result);
+  const double last_ms = stats.ms_compute;  // of the run before
   cudaEvent_t e4 = ev(4);
-  // The records come back to pageable memory the first time and to
-  // page-locked memory from a handle's second run of the size on: locking
-  // takes 1.3 ms and 0.5 ms per MB, a pageable copy 20 us more at 300 KB and
-  // 1 ms more at 24 MB.
-  const bool again = host_records.size() > F;
-  const bool pinned = h_records.n >= record_bytes + 16 || (again && h_records.try_ensure(record_bytes + 16));
-  if (pinned)
+  // The records come back to pageable memory first, and to page-locked memory
+  // once locking is cheap against the run (in count mode it runs beside the
+  // kernels) or the pageable copies have cost as much.  Locking takes 1.1 to 4 ms
+  // and 0.3 to 3 ms per MB, a pageable copy 10 us more at 45 KB, 17 us at 130 KB, 0.1 ms
+  // at 1.3 MB, 0.3 to 0.6 ms at 4 MB and 0.8 ms at 24 MB.  Locked on its second run, a
+  // handle of 400 gates and 64 patterns took 2.5 ms for it, against 0.15 ms.
+  const double record_mb = (double)record_bytes * 1e-6, lock_us = 1500 + 500 * record_mb;
+  bool pinned = h_records.n >= record_bytes + 16;
+  if (!pinned && host_records.size() > F &&
+      (last_ms * 1e3 > lock_us * (o.drop ? 10 : 2) || paged_us > lock_us)) {
+    pinned = h_records.try_ensure(record_bytes + 16);
+    paged_us = 0;
+  }
+  if (pinned) {
     std::vector<fsimb_fault_result>().swap(host_records);
-  else
+  } else {
     host_records.resize(F + 1);
+    paged_us += 12 + 80 * record_mb;
+  }
   char* dst = pinned ? h_records.as<char>() : reinterpret_cast<char*>(host_records.data());
   CK(cudaMemcpyAsync(dst, d_records.p, record_bytes + 16, cudaMemcpyDeviceToHost, s));
   CK(cudaEventRecord(e4, s));

@@ -248,6 +248,7 @@ struct fsimb_handle {
   // host_records after a batch's run.
   fsimb::DevBuf d_records, d_round;
   fsimb::PinnedBuf h_records;
+  double paged_us = 0;  // what pageable record copies have cost so far
   std::vector<fsimb_fault_result> host_records;
   const fsimb_fault_result* records = nullptr;
   uint64_t n_records = 0;

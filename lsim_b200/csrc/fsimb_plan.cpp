@@ -236,6 +236,9 @@ void build_circuit_plan(const Netlist& nl, CircuitPlan& C, bool sweeps) {
   for (uint32_t l = 0; l < nl.n_levels; ++l)
     P.max_level_width = std::max<uint32_t>(P.max_level_width, nl.level_off[l + 1] - nl.level_off[l]);
 
+  build_gate_recs(nl, P.net.gates);
+  if (!sweeps) return;
+
   // Per-element fanout facts.
   C.mux_below.assign(N, 0);
   P.po_drv.assign(N, 0);
@@ -265,8 +268,7 @@ void build_circuit_plan(const Netlist& nl, CircuitPlan& C, bool sweeps) {
   // What sweeps evaluate, and the peak number of live values (interval graph
   // of [level, highest reading level]), over all gates and over the stored
   // ones; a schedule may need a few more slots to honour residues.
-  build_gate_recs(nl, P.net.gates);
-  if (sweeps) {
+  {
     auto peak = [&](const std::vector<uint32_t>& last) {
       std::vector<int64_t> delta(nl.n_levels + 2, 0);
       for (uint32_t e = 0; e < N; ++e)

@@ -281,8 +281,9 @@ constexpr uint64_t kSplitRecords = 256;  // records a level from which ANDs and 
 // 0: AND family (AND, NAND, OR, NOR, INV, CLKBUF, PO), 1: XOR family, 2: MUX.
 uint32_t gate_family(uint8_t type);
 void build_plan(const Netlist& nl, const std::vector<Fault>& faults, Plan& plan);
-// Without `sweeps` (no fault will be simulated) base.net holds the gate
-// records only.
+// Without `sweeps` (no fault will be simulated) it holds the sizes, the
+// levels and the gate records only: what the good machine reads (200,000 gates:
+// 13 ms with the fanout facts and FFRs, 2 without).
 void build_circuit_plan(const Netlist& nl, CircuitPlan& cplan, bool sweeps = true);
 // Roots, members, traced faults and sweeps of a fault list; the circuit's
 // per-element vectors (net, gate_fo, po_drv, nfp_prefix) stay in

@@ -415,7 +415,7 @@ def run_ours(args):
         "data": "synthetic", "config": _config(world, faults_sharded),
         "e2e": {"value": e2e, "unit": UNIT,
                 "h2d_bytes_per_step": int(words.nbytes),
-                "d2h_bytes_per_step": int(F * 17)},
+                "d2h_bytes_per_step": int(F * 32 + 16)},  # the records and the error word
         "gpu_launches": int(launches),
         "gate_word_evals_per_s": {
             "sweep_dense": gwe / (ms / 1e3) * (world if not faults_sharded else 1),

@@ -769,10 +769,10 @@ struct fsimb_batch {
       for (size_t i = 0; i < members.size(); ++i)
         if (a.M[i] == m) {
           a.cls[i] = (int)a.shapes.size();
-          t = std::max(t, pick_sweep_threads(schedule_at(i, m), m));
+          t = std::max(t, pick_sweep_threads(schedule_at(i, m)));
         }
       if (!t) continue;
-      a.shapes.push_back(ClassShape{m, (int)std::min<uint32_t>(threads ? threads : t, sweep_max_threads(m))});
+      a.shapes.push_back(ClassShape{m, threads ? threads : (int)t});
     }
     return a;
   }
@@ -987,7 +987,7 @@ struct fsimb_batch {
       const ClassShape def = a.shapes[c];
       std::vector<ClassShape> cands{def};
       for (int T : {32, 64, 128, 256, 384, 512, 768, 1024})
-        if (T <= (int)sweep_max_threads(def.M) && T != def.threads) cands.push_back(ClassShape{def.M, T});
+        if (T != def.threads) cands.push_back(ClassShape{def.M, T});
       float best_ms = 1e30f;
       ClassShape best = def;
       bool best_is_default = false;
@@ -1165,7 +1165,7 @@ void fsimb_batch::run(const fsimb_batch_opts* opts) {
   }
   stats.device_bytes = exec.device_bytes();
   stats.h2d_bytes = h2d;
-  stats.d2h_bytes = exec.F_total * 17 + sizeof(int);
+  stats.d2h_bytes = exec.F_total * 17;
 }
 
 // -------------------------------------------------------------------- C ABI

@@ -160,7 +160,6 @@ bool default_sweep_shape(const Plan& plan, const std::function<const Schedule&(i
     exact[bi] = true;
     vals[bi] = sched_fits(sc, M, share1) ? sweep_vals_bytes(sc.max_live, M) : share1 + 1;
   }
-  threads = std::min<int>(threads, (int)sweep_max_threads(M));
   return true;
 }
 
@@ -405,7 +404,7 @@ void fsimb_handle::run(const fsimb_opts* opts) {
         if (o.words_per_item || M == 1)
           throw no_room(std::max(plan.max_live, cached_schedule(M).max_live), M, budget, ctas);
       }
-      threads = o.block_threads ? (int)o.block_threads : (int)pick_sweep_threads(cached_schedule(M), M);
+      threads = o.block_threads ? (int)o.block_threads : (int)pick_sweep_threads(cached_schedule(M));
     } else if (o.tune && tiles) {
       if (!tuned_holds()) {
         const auto t0 = std::chrono::steady_clock::now();
@@ -419,7 +418,6 @@ void fsimb_handle::run(const fsimb_opts* opts) {
     } else if (!default_shape(M, threads)) {
       M = 0;
     }
-    threads = std::min<int>(threads, (int)sweep_max_threads(M));
     if (!M) {  // no schedule fits: the global-memory sweep
       if (o.sweep_variant == 1) throw no_room(cached_schedule(1).max_live, 1, share1, 1);
       wide = true;
@@ -704,7 +702,7 @@ void fsimb_handle::run(const fsimb_opts* opts) {
   CK(cudaStreamSynchronize(s));
   uint64_t kerr = 0;
   std::memcpy(&kerr, dst + record_bytes, sizeof kerr);
-  if (kerr) throw CudaError{"a sweep kernel reached its time limit waiting for a record copy; results discarded"};
+  if (kerr) throw CudaError{"a sweep kernel's wait test reached its time limit; results discarded"};
   if (!o.drop) {
     for (uint64_t g = 0; g < n_groups; ++g) {
       float x = 0;

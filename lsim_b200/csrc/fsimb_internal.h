@@ -79,14 +79,13 @@ inline void upload(DevBuf& b, const std::vector<T>& v, cudaStream_t s) {
   if (!v.empty()) CK(cudaMemcpyAsync(b.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s));
 }
 
-// Largest sweep CTA for M words per item (the kernels' register caps).
-inline uint32_t sweep_max_threads(int) { return 1024; }
+// Largest sweep CTA (the kernels' register caps).
+constexpr uint32_t kMaxSweepThreads = 1024;
 
 // Sweep CTA size for one thread per record of a level: the multiple of 32
 // that splits the typical (90th percentile) level into equal rounds, so no
 // thread idles long before the per-level barrier.
-inline uint32_t pick_sweep_threads(const Schedule& sc, int M) {
-  const uint32_t tmax = sweep_max_threads(M);
+inline uint32_t pick_sweep_threads(const Schedule& sc) {
   std::vector<uint32_t> widths;
   for (size_t l = 0; l + 1 < sc.rec_off.size(); ++l)
     if (sc.rec_off[l + 1] > sc.rec_off[l]) widths.push_back(sc.rec_off[l + 1] - sc.rec_off[l]);
@@ -100,7 +99,7 @@ inline uint32_t pick_sweep_threads(const Schedule& sc, int M) {
   for (uint32_t k = 1; k <= 64; ++k) {
     uint32_t t = (w + k - 1) / k;
     t = std::max<uint32_t>(64, (t + 31) / 32 * 32);
-    if (t > tmax) continue;
+    if (t > kMaxSweepThreads) continue;
     const double cost = (double)k * t + 8.0 * k;  // issued slots + per-round overhead
     if (cost < best_cost) {
       best_cost = cost;

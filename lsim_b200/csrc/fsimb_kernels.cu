@@ -220,6 +220,7 @@ __global__ void k_good_level(GoodView a, uint32_t lo, uint32_t hi) {
 }
 
 // ---------------------------------------------------------------- bounded wait
+// (the wait test's only: the sweeps' barriers are the CTA's own)
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
@@ -729,14 +730,13 @@ __device__ __forceinline__ void sweep_item(uint64_t* vals, unsigned long long* a
   if (tid < M) out_row[w0 + tid] = acc[tid];
 }
 
-// Test hook: a wait on a barrier that nothing completes runs out and the
-// launch reports an error.
-__device__ __forceinline__ bool sweep_wait_test(uint64_t* bar, uint64_t wait_ns, int* err) {
+// Test hook of the error word: a wait on a barrier that nothing completes runs
+// out and the launch reports it.  Nothing else in a sweep waits on an mbarrier.
+__device__ __forceinline__ void sweep_wait_test(uint64_t* bar, uint64_t wait_ns, int* err) {
   if (threadIdx.x == 0) {
     mbar_init(bar, 1);
     if (!mbar_wait(bar, 0, wait_ns)) atomicExch(err, 1);
   }
-  return false;
 }
 
 // Register caps: 1,024 threads an SM at up to 4 words per item.  D: the stream
@@ -1218,7 +1218,7 @@ uint32_t launch_good(const GoodView& a, const uint32_t* level_off, int n_sms, cu
     for (uint32_t l = 0; l < a.n_levels; ++l) {
       const uint64_t n = (uint64_t)(level_off[l + 1] - level_off[l]) * a.W;
       if (!n) continue;
-      const uint64_t blocks = std::min<uint64_t>((n + 255) / 256, 148ull * 64);
+      const uint64_t blocks = std::min<uint64_t>((n + 255) / 256, 64ull * n_sms);
       k_good_level<<<(unsigned)blocks, 256, 0, s>>>(a, level_off[l], level_off[l + 1]);
       ++launches;
     }

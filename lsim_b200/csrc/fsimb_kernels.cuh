@@ -225,7 +225,7 @@ cudaError_t launch_sweep(int M, bool direct, int threads, int blocks, size_t sme
                          cudaStream_t s);
 cudaError_t sweep_set_smem(int M, bool direct, size_t smem);
 cudaError_t sweep_occupancy(int M, bool direct, int threads, size_t smem, int* blocks_per_sm);
-// M in {1, 2}; 256 threads per CTA.
+// M in {1, 2}; threads a multiple of 32, at most 1,024.
 cudaError_t launch_sweep_wide(int M, int threads, int blocks, const SweepWideArgs& a, cudaStream_t s);
 cudaError_t sweep_wide_occupancy(int M, int threads, int* blocks_per_sm);
 // Time limit of the wait test's wait.

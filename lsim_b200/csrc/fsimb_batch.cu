@@ -303,7 +303,6 @@ void BatchExec::layout(const std::vector<BatchJob>& jobs, const std::vector<Clas
   // Sweep classes: shapes[c] runs the jobs with cls == c.
   classes.clear();
   uint32_t n_counters = 0;
-  for (size_t& a : smem_attr) a = 0;
   for (size_t ci = 0; ci < shapes.size(); ++ci) {
     const ClassShape& sh = shapes[ci];
     SweepClass k;
@@ -392,19 +391,11 @@ void BatchExec::size_class(SweepClass& k, const ClassShape& sh) {
                      std::to_string(sh.M) + " word(s) per item; shared memory holds " +
                      std::to_string(share / (8 * sh.M))};
   k.smem = std::max<size_t>(16, vals);
-  size_t& attr = smem_attr[m_slot(sh.M) + 4 * k.direct];
-  attr = std::max(attr, k.smem);
-  CK(sweep_batch_set_smem(sh.M, k.direct, attr));
+  CK(sweep_batch_set_smem(sh.M, k.direct, share));
   k.occ = 0;
   CK(sweep_batch_occupancy(sh.M, k.direct, sh.threads, k.smem, &k.occ));
   if (k.occ < 1) throw LimitError{"batch sweep kernel does not fit on an SM with this shape"};
   k.blocks = (int)std::min<unsigned long long>((unsigned long long)n_sms * k.occ, k.n_items);
-}
-
-void BatchExec::apply_attributes() {
-  for (int M : {1, 2, 4, 8})
-    for (bool direct : {false, true})
-      if (const size_t a = smem_attr[m_slot(M) + 4 * direct]) CK(sweep_batch_set_smem(M, direct, a));
 }
 
 uint64_t BatchExec::enqueue(cudaStream_t s, bool good_only, bool with_events, cudaEvent_t* ev) {
@@ -1088,7 +1079,6 @@ void fsimb_batch::run(const fsimb_batch_opts* opts) {
     exec.concurrent = !o.serial_classes;
     exec.invalidate_graph();
   }
-  exec.apply_attributes();  // the autotuner may have changed them
   if (graph) {
     launches = exec.run_graph(stream, s);
   } else {

@@ -87,8 +87,6 @@ class BatchExec {
   uint64_t static_bytes = 0, desc_bytes = 0;
   uint64_t ctl_bytes = 256;  // one work counter per swept circuit
   BatchSweepParams params{};  // launch parameters being built (32 KB)
-  // dynamic smem limit set per words-per-item kernel, without and with direct records
-  size_t smem_attr[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   cudaEvent_t* class_events = nullptr;  // direct launches: recorded after each class
   // Classes run as concurrent branches (one stream each), so CTAs of small
   // circuits can share SMs with the CTAs of large ones.
@@ -123,9 +121,6 @@ class BatchExec {
   uint64_t upload_static(const std::vector<BatchJob>& jobs, cudaStream_t s);
   // Shared memory and grid of a class for a shape.
   void size_class(SweepClass& k, const ClassShape& sh);
-  // Sets each class's dynamic shared-memory limit on its kernel (a
-  // per-kernel attribute other launch sequences may have changed).
-  void apply_attributes();
   // Enqueues the launch sequence; returns the number of kernels.  With
   // with_events, ev[0] is recorded after the good machine, ev[1] after the sweeps.
   uint64_t enqueue(cudaStream_t s, bool good_only, bool with_events, cudaEvent_t* ev);

@@ -212,7 +212,7 @@ void fsimb_handle::tune_shape(cudaStream_t s) {
     if (!sched_fits(cached_schedule(M), M, share1)) continue;
     const Schedule& sc = use_schedule(M, T, s);
     const size_t smem = std::max<size_t>(16, sweep_vals_bytes(sc.max_live, M));
-    CK(sweep_set_smem(M, sc.direct, smem));
+    CK(sweep_set_smem(M, sc.direct, share1));
     int got = 0;
     CK(sweep_occupancy(M, sc.direct, T, smem, &got));
     if (got < 1) continue;
@@ -474,7 +474,7 @@ void fsimb_handle::run(const fsimb_opts* opts) {
   CK(cudaEventRecord(e2, s));
 
   if (!wide && n_sweeps) {
-    CK(sweep_set_smem(M, sched->direct, smem));
+    CK(sweep_set_smem(M, sched->direct, share1));
     CK(sweep_occupancy(M, sched->direct, threads, smem, &occ_got));
     if (occ_got < 1) throw LimitError{"sweep kernel does not fit on an SM with this shape"};
     blocks = n_sms * occ_got;

@@ -209,6 +209,9 @@ struct BatchUnits {
 void launch_good_batch(const BatchUnits& u, unsigned long long n_units, cudaStream_t s);
 cudaError_t launch_sweep_batch(int M, bool direct, int threads, int blocks, size_t smem, const BatchSweepParams& p,
                                cudaStream_t s);
+// Lets launches take up to `smem` bytes of dynamic shared memory.  The limit
+// is the kernel's, shared by all threads and handles: every caller sets the
+// largest CTA's, so that none lowers it between another's setting and launch.
 cudaError_t sweep_batch_set_smem(int M, bool direct, size_t smem);
 cudaError_t sweep_batch_occupancy(int M, bool direct, int threads, size_t smem, int* blocks_per_sm);
 void launch_ffr_batch(const BatchUnits& u, unsigned long long n_units, cudaStream_t s);
@@ -223,7 +226,7 @@ uint32_t launch_good(const GoodView& a, const uint32_t* level_off, int n_sms, cu
 // cudaErrorInvalidValue when M is unsupported.
 cudaError_t launch_sweep(int M, bool direct, int threads, int blocks, size_t smem, const SweepArgs& a,
                          cudaStream_t s);
-cudaError_t sweep_set_smem(int M, bool direct, size_t smem);
+cudaError_t sweep_set_smem(int M, bool direct, size_t smem);  // as sweep_batch_set_smem
 cudaError_t sweep_occupancy(int M, bool direct, int threads, size_t smem, int* blocks_per_sm);
 // M in {1, 2}; threads a multiple of 32, at most 1,024.
 cudaError_t launch_sweep_wide(int M, int threads, int blocks, const SweepWideArgs& a, cudaStream_t s);

@@ -117,9 +117,6 @@ struct fsimb_server {
   fsimb_server_opts opts{};
 
   std::mutex circuits_mu;  // guards `circuits` growth
-  // Held while kernel attributes are set and the launches that rely on them
-  // are issued (circuit registration queries occupancy with its own sizes).
-  std::mutex attr_mu;
   std::vector<std::unique_ptr<ResidentCircuit>> circuits;
 
   std::mutex mu;  // guards everything below
@@ -461,9 +458,7 @@ struct fsimb_server {
       r->job.cls = cls;
       s.jobs.push_back(r->job);
     }
-    std::lock_guard<std::mutex> g(attr_mu);
     s.exec.layout(s.jobs, shapes, false, s.stream);
-    s.exec.apply_attributes();
     CK(cudaEventRecord(s.e0, s.stream));
     s.exec.enqueue(s.stream, false, false, nullptr);
     s.exec.fetch_async(s.stream);
